@@ -47,28 +47,28 @@ def _case(name, do, model, weights, kv, streams=1, shortest=0, context=0, tokens
 def listed():
     return [
         # the smallest model and hardly any context: launches and latency
-        _case("decode 1, 1.7B, start of a chat", "decode", "1.7b", "tq2", "f16", context=24),
+        _case("decode 1 1.7B start of a chat", "decode", "1.7b", "tq2", "f16", context=24),
         # the headline of bench.py: one stream at 4096 tokens
-        _case("decode 1, 8B, 4096", "decode", "8b", "tq2", "f16", context=4096),
+        _case("decode 1 8B 4096", "decode", "8b", "tq2", "f16", context=4096),
         # one reader of a long document on a 1-bit model, INT8 cache
-        _case("decode 1, 4B 1-bit, q8 20000", "decode", "4b", "q1", "q8", context=20001),
+        _case("decode 1 4B 1-bit q8 20000", "decode", "4b", "q1", "q8", context=20001),
         # a handful of chats, ragged
-        _case("decode 5, 8B 1-bit, 90-700", "decode", "8b", "q1", "f16", streams=5, shortest=90, context=700, preset="balanced"),
+        _case("decode 5 8B 1-bit 90-700", "decode", "8b", "q1", "f16", streams=5, shortest=90, context=700, preset="balanced"),
         # a half-full server with the densest cache format
-        _case("decode 24, 4B, q4 100-1500", "decode", "4b", "tq2", "q4", streams=24, shortest=100, context=1500, preset="balanced"),
+        _case("decode 24 4B q4 100-1500", "decode", "4b", "tq2", "q4", streams=24, shortest=100, context=1500, preset="balanced"),
         # the serving benchmark: 64 streams, prompts of 128 to 2048 tokens, INT8 cache, Balanced preset
-        _case("decode 64, 4B, q8 128-2048", "decode", "4b", "tq2", "q8", streams=64, shortest=128, context=2048, preset="balanced"),
+        _case("decode 64 4B q8 128-2048", "decode", "4b", "tq2", "q8", streams=64, shortest=128, context=2048, preset="balanced"),
         # bench.py's aggregate: 64 streams at 1024 tokens
-        _case("decode 64, 8B, 1024", "decode", "8b", "tq2", "f16", streams=64, context=1024),
+        _case("decode 64 8B 1024", "decode", "8b", "tq2", "f16", streams=64, context=1024),
         # a draft of eight tokens checked at a long context
-        _case("verify 9, 8B, 4096", "verify", "8b", "tq2", "f16", context=4096, tokens=9),
+        _case("verify 9 8B 4096", "verify", "8b", "tq2", "f16", context=4096, tokens=9),
         # an ordinary prompt of odd length into the INT8 cache
-        _case("prompt 777, 4B, q8", "prompt", "4b", "tq2", "q8", tokens=777),
+        _case("prompt 777 4B q8", "prompt", "4b", "tq2", "q8", tokens=777),
         # the longest prompt that is one chunk: time to first token of bench.py
-        _case("prompt 4096, 8B", "prompt", "8b", "tq2", "f16", tokens=4096),
+        _case("prompt 4096 8B", "prompt", "8b", "tq2", "f16", tokens=4096),
         # checkpoints in the common block formats, which are used as stored
-        _case("decode 1, 8B q4_k, 300", "decode", "8b", "q4_k", "f16", context=300),
-        _case("prompt 500, 4B q8_0", "prompt", "4b", "q8_0", "f16", tokens=500),
+        _case("decode 1 8B q4_k 300", "decode", "8b", "q4_k", "f16", context=300),
+        _case("prompt 500 4B q8_0", "prompt", "4b", "q8_0", "f16", tokens=500),
     ]
 
 
