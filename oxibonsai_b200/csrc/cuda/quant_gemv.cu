@@ -3,16 +3,17 @@
 //
 // Replaces the reference's per-format single-GEMV wrappers cuda_gemv_q4_0 / q8_0, cuda_gemv_q{2..8}k
 // and cuda_gemv_fp8_* (crates/oxibonsai-kernels/src/gpu_backend/cuda_q_std_kernels.rs:200-,
-// cuda_k_quant_kernels.rs:640-, cuda_fp8_kernels.rs:300-) with one kernel templated on the block
-// decoder.  One warp owns a row: for 32-element blocks every lane decodes a whole block per step
-// (32 blocks = 1024 inputs per warp step), for 256-element super-blocks the 32 lanes share a block,
-// eight elements each.  Accumulation is f32, lanes are folded with shuffles, optional fused RMSNorm
-// of the input (every warp recomputes the mean square from L1/L2-resident x) and residual add.
+// cuda_k_quant_kernels.rs:640-, cuda_fp8_kernels.rs:300-) with kernels templated on the block decoder.
+// Products and sums are f32, with optional fused RMSNorm of the input and residual add.
+// quant_stream_kernel (below) serves matrices whose rows can be copied in 16-byte units; quant_gemv_kernel and its
+// batched form take the rest: one warp owns a row, for 32-element blocks every lane decodes a whole block per step
+// (32 blocks = 1024 inputs per warp step), for 256-element super-blocks the 32 lanes share a block, eight elements each.
 // Block layouts are the ones documented in csrc/core/blocks.hpp and csrc/core/kquants.hpp.
 #include <cuda_bf16.h>
 #include <cuda_fp8.h>
 
 #include "common.cuh"
+#include "tcgen05.cuh"
 
 namespace bonsai {
 
@@ -67,6 +68,408 @@ struct DecBF16 { static constexpr int kElems = 32, kBytes = 64;
 struct DecF32 { static constexpr int kElems = 32, kBytes = 128;
   static __device__ float at(const uint8_t* p, int i) { float v; memcpy(&v, p + 4 * i, 4); return v; } };
 
+// ---- streamed rows ------------------------------------------------------------------------------------------------------
+// One or two tokens over a matrix of blocks.  The rows of a matrix are one contiguous byte string, so a CTA owns a range of
+// rows and a producer lane streams it through a shared-memory ring with bulk copies (the first stages before it waits for the
+// kernel ahead: weights depend on nothing).  Blocks of 18, 34, 110 or 210 bytes are no friends of wide global loads; out of
+// shared memory the aligned words around a block cost at most two wavefronts each.
+// A lane decodes 32 consecutive weights of a row per step, a warp 1024: it keeps its 32 inputs (times the norm weights) of
+// every token in registers for the whole range of rows, so an input is loaded once per CTA.  A group's codes are multiplied as
+// exact integers and the scale is applied once per group; a minimum is multiplied into the group's sum of inputs, made once.
+// K is spread over KW warps; their partial sums stay in shared memory until the end, where they are added in K order.
+// What bounds it: instructions.  24576 x 4096 in Q4_0 takes 19.6 M warp instructions (some six per weight with addresses, shuffles and
+// the hand-over of stages), half of the issue slots; more rows side by side do not help.  24576 x 4096, one token: Q4_0 27.8 us, Q8_0
+// 25.9 (4.1 TB/s), Q4_K 27.9, Q6_K 40.8, F16 40.7 (4.9 TB/s).  Before (a warp per row, one byte load per weight) the matrices of a
+// quarter-depth 8B model in Q4_K took 113 us on average, now 20; a token of it 4370 us, now 850.
+constexpr int kQsMaxWarps = 16;
+constexpr int kQsMaxStages = 8;
+constexpr int kQsRing = 112 * 1024;
+constexpr int kQsRows = 256;        // rows of a CTA whose partial sums are kept
+
+__device__ __forceinline__ uint64_t qs_pack(float a, float b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t qs_fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ uint64_t qs_add2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ float qs_sum2(uint64_t a) {
+  float x, y;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a));
+  return x + y;
+}
+
+// Integers become floats without a conversion: a field of a word that lies at bit `at` of a float with exponent 2^(23 - at) counts in
+// ones above the base 2^(23 - at), which is then taken off exactly, two values at a time.
+__device__ __forceinline__ float qs_int(uint32_t v) { return __uint_as_float(0x4B000000u | v) - 8388608.0f; }   // v < 2^23
+template <int AT>
+__device__ __forceinline__ float qs_raw(uint32_t w, uint32_t mask) { return __uint_as_float((w & (mask << AT)) | ((150u - AT) << 23)); }
+template <int A0, int A1>
+__device__ __forceinline__ uint64_t qs_take(float a, float b, float less) {
+  return qs_add2(qs_pack(a, b), qs_pack(-(float)(1 << (23 - A0)) - less, -(float)(1 << (23 - A1)) - less));
+}
+// nibbles n, n + 1 (n even) of w, minus `less`: five nibbles of a word lie inside a mantissa, the other three after one shift
+__device__ __forceinline__ uint64_t qs_nibbles(uint32_t w, int n, float less) {
+  const uint32_t u = w >> 20;
+  if (n == 0) return qs_take<0, 4>(qs_raw<0>(w, 15u), qs_raw<4>(w, 15u), less);
+  if (n == 2) return qs_take<8, 12>(qs_raw<8>(w, 15u), qs_raw<12>(w, 15u), less);
+  if (n == 4) return qs_take<16, 0>(qs_raw<16>(w, 15u), qs_raw<0>(u, 15u), less);
+  return qs_take<4, 8>(qs_raw<4>(u, 15u), qs_raw<8>(u, 15u), less);
+}
+// signed bytes b, b + 1 of w, w with its sign bits flipped
+__device__ __forceinline__ uint64_t qs_bytes(uint32_t w, int b) {
+  const float x = __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7650u + (uint32_t)b)), y = __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7651u + (uint32_t)b));
+  return qs_add2(qs_pack(x, y), qs_pack(-8388736.0f, -8388736.0f));
+}
+// two integers below 2^23, minus `less`
+__device__ __forceinline__ uint64_t qs_ints(uint32_t a, uint32_t b, float less) {
+  return qs_take<0, 0>(__uint_as_float(0x4B000000u | a), __uint_as_float(0x4B000000u | b), less);
+}
+
+// NW words at p: aligned to A bytes (2, 4 or 16)
+template <int NW, int A>
+__device__ __forceinline__ void qs_words(const uint8_t* p, uint32_t* out) {
+  if (A == 16 && NW % 4 == 0) {
+#pragma unroll
+    for (int i = 0; i < NW / 4; ++i) {
+      const uint4 v = reinterpret_cast<const uint4*>(p)[i];
+      out[4 * i] = v.x; out[4 * i + 1] = v.y; out[4 * i + 2] = v.z; out[4 * i + 3] = v.w;
+    }
+  } else if (A >= 4) {
+#pragma unroll
+    for (int i = 0; i < NW; ++i) out[i] = reinterpret_cast<const uint32_t*>(p)[i];
+  } else {
+    const uint32_t odd = (uint32_t)(reinterpret_cast<uintptr_t>(p) & 2u);
+    const uint32_t* a = reinterpret_cast<const uint32_t*>(p - odd);
+    uint32_t w[NW + 1];
+#pragma unroll
+    for (int i = 0; i <= NW; ++i) w[i] = a[i];       // the word behind the last block lies in the ring's slack
+#pragma unroll
+    for (int i = 0; i < NW; ++i) out[i] = __funnelshift_r(w[i], w[i + 1], odd * 8);
+  }
+}
+__device__ __forceinline__ uint32_t qs_u16(const uint8_t* p) { return *reinterpret_cast<const uint16_t*>(p); }
+__device__ __forceinline__ float qs_f16(const uint8_t* p) { return __half2float(__ushort_as_half((unsigned short)qs_u16(p))); }
+
+// 32 weights: block number b (of 32) of the row at `row`.  Weights j, j + 1 (j even) are s[j / (32 / kScales)] * q2(j) - m[...].
+#define QS_HEAD(scales, mins) static constexpr int kScales = scales; static constexpr bool kMin = mins; float s[scales], m[mins ? scales : 1];
+struct QsQ4_0 { QS_HEAD(1, false) uint32_t w[4];
+  __device__ void load(const uint8_t* row, int b) { const uint8_t* p = row + b * 18; s[0] = qs_f16(p); qs_words<4, 2>(p + 2, w); }
+  __device__ uint64_t q2(int j) const { return qs_nibbles(w[j >> 3], j & 7, 8.0f); } };
+struct QsQ8_0 { QS_HEAD(1, false) uint32_t w[8];
+  __device__ void load(const uint8_t* row, int b) { const uint8_t* p = row + b * 34; s[0] = qs_f16(p); qs_words<8, 2>(p + 2, w);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) w[i] ^= 0x80808080u; }
+  __device__ uint64_t q2(int j) const { return qs_bytes(w[j >> 2], j & 3); } };
+template <bool E5M2> struct QsFp8 { QS_HEAD(1, false) uint32_t w[8];
+  __device__ void load(const uint8_t* row, int b) { const uint8_t* p = row + b * 34; s[0] = qs_f16(p + 32); qs_words<8, 2>(p, w); }
+  __device__ uint64_t q2(int j) const {
+    const __half2_raw h = __nv_cvt_fp8x2_to_halfraw2((__nv_fp8x2_storage_t)(w[j >> 2] >> (8 * (j & 3))), E5M2 ? __NV_E5M2 : __NV_E4M3);
+    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&h));
+    return qs_pack(f.x, f.y); } };
+struct QsTq2_256 { QS_HEAD(1, false) uint32_t w[2];
+  __device__ void load(const uint8_t* row, int b) { const uint8_t* p = row + (b >> 3) * 66; s[0] = qs_f16(p + 64); qs_words<2, 2>(p + 8 * (b & 7), w); }
+  __device__ float q(int j) const { const uint32_t c = (w[j >> 4] >> (2 * (j & 15))) & 3u; return c == 0 ? -1.0f : (c == 2 ? 1.0f : 0.0f); }
+  __device__ uint64_t q2(int j) const { return qs_pack(q(j), q(j + 1)); } };
+struct QsQ2K { QS_HEAD(2, true) uint32_t w[2];
+  __device__ void load(const uint8_t* row, int b) {
+    const uint8_t* p = row + (b >> 3) * 84;
+    const int j = b & 7;
+    const float d = qs_f16(p + 80), dm = qs_f16(p + 82);
+    const uint32_t sc = qs_u16(p + 2 * j);
+    s[0] = d * qs_int(sc & 15u); m[0] = dm * qs_int((sc >> 4) & 15u); s[1] = d * qs_int((sc >> 8) & 15u); m[1] = dm * qs_int(sc >> 12);
+    qs_words<2, 4>(p + 16 + 8 * j, w); }
+  __device__ uint64_t q2(int j) const { const uint32_t v = w[j >> 4] >> (2 * (j & 15)); return qs_take<0, 2>(qs_raw<0>(v, 3u), qs_raw<2>(v, 3u), 0.0f); } };
+struct QsQ3K { QS_HEAD(2, false) uint32_t w[2], h[1];
+  __device__ void load(const uint8_t* row, int b) {
+    const uint8_t* p = row + (b >> 3) * 110;
+    const int j = b & 7;
+    const float d = qs_f16(p + 108);
+    const uint32_t sc = p[96 + j];
+    s[0] = d * (qs_int(sc & 15u) - 8.0f); s[1] = d * (qs_int(sc >> 4) - 8.0f);
+    qs_words<2, 2>(p + 32 + 8 * j, w); qs_words<1, 2>(p + 4 * j, h); }
+  __device__ uint32_t q(int j) const { return ((w[j >> 4] >> (2 * (j & 15))) & 3u) | (((h[0] >> j) & 1u) << 2); }
+  __device__ uint64_t q2(int j) const { return qs_ints(q(j), q(j + 1), 4.0f); } };
+__device__ __forceinline__ void qs_k6(const uint32_t* t, int j, float d, float dm, float& s, float& m) {   // t: the 12 scale bytes
+  s = d * qs_int(((t[0] >> (4 * j)) & 15u) | (((t[2] >> (2 * j)) & 3u) << 4));
+  m = dm * qs_int(((t[1] >> (4 * j)) & 15u) | (((t[2] >> (16 + 2 * j)) & 3u) << 4));
+}
+struct QsQ4K { QS_HEAD(1, true) uint32_t w[4];
+  __device__ void load(const uint8_t* row, int b) {
+    const uint8_t* p = row + (b >> 3) * 144;
+    uint32_t t[4];
+    qs_words<4, 16>(p, t);
+    const __half2 dd = *reinterpret_cast<const __half2*>(t);
+    qs_k6(t + 1, b & 7, __low2float(dd), __high2float(dd), s[0], m[0]);
+    qs_words<4, 16>(p + 16 + 16 * (b & 7), w); }
+  __device__ uint64_t q2(int j) const { return qs_nibbles(w[j >> 3], j & 7, 0.0f); } };
+struct QsQ5K { QS_HEAD(1, true) uint32_t w[4], h[1];
+  __device__ void load(const uint8_t* row, int b) {
+    const uint8_t* p = row + (b >> 3) * 176;
+    uint32_t t[4];
+    qs_words<4, 16>(p, t);
+    const __half2 dd = *reinterpret_cast<const __half2*>(t);
+    qs_k6(t + 1, b & 7, __low2float(dd), __high2float(dd), s[0], m[0]);
+    qs_words<4, 16>(p + 48 + 16 * (b & 7), w); qs_words<1, 4>(p + 16 + 4 * (b & 7), h); }
+  __device__ uint32_t q(int j) const { return ((w[j >> 3] >> (4 * (j & 7))) & 15u) | (((h[0] >> j) & 1u) << 4); }
+  __device__ uint64_t q2(int j) const { return qs_ints(q(j), q(j + 1), 0.0f); } };
+struct QsQ6K { QS_HEAD(2, false) uint32_t w[4], h[2];
+  __device__ void load(const uint8_t* row, int b) {
+    const uint8_t* p = row + (b >> 3) * 210;
+    const int j = b & 7;
+    const float d = qs_f16(p + 208);
+    const uint32_t sc = qs_u16(p + 192 + 2 * j);
+    s[0] = d * (float)(int8_t)(sc & 255u); s[1] = d * (float)(int8_t)(sc >> 8);
+    qs_words<4, 2>(p + 16 * j, w); qs_words<2, 2>(p + 128 + 8 * j, h); }
+  __device__ uint32_t q(int j) const { return ((w[j >> 3] >> (4 * (j & 7))) & 15u) | (((h[j >> 4] >> (2 * (j & 15))) & 3u) << 4); }
+  __device__ uint64_t q2(int j) const { return qs_ints(q(j), q(j + 1), 32.0f); } };
+struct QsQ8K { QS_HEAD(1, false) uint32_t w[8];
+  __device__ void load(const uint8_t* row, int b) {
+    const uint8_t* p = row + (b >> 3) * 292;
+    s[0] = *reinterpret_cast<const float*>(p);
+    qs_words<8, 4>(p + 4 + 32 * (b & 7), w);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) w[i] ^= 0x80808080u; }
+  __device__ uint64_t q2(int j) const { return qs_bytes(w[j >> 2], j & 3); } };
+struct QsF16 { QS_HEAD(1, false) uint32_t w[16];
+  __device__ void load(const uint8_t* row, int b) { s[0] = 1.0f; qs_words<16, 16>(row + b * 64, w); }
+  __device__ uint64_t q2(int j) const { const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[j >> 1])); return qs_pack(f.x, f.y); } };
+struct QsBF16 { QS_HEAD(1, false) uint32_t w[16];
+  __device__ void load(const uint8_t* row, int b) { s[0] = 1.0f; qs_words<16, 16>(row + b * 64, w); }
+  __device__ uint64_t q2(int j) const { return qs_pack(__uint_as_float(w[j >> 1] << 16), __uint_as_float(w[j >> 1] & 0xFFFF0000u)); } };
+struct QsF32 { QS_HEAD(1, false) uint32_t w[32];
+  __device__ void load(const uint8_t* row, int b) { s[0] = 1.0f; qs_words<32, 16>(row + b * 128, w); }
+  __device__ uint64_t q2(int j) const { return qs_pack(__uint_as_float(w[j]), __uint_as_float(w[j + 1])); } };
+#undef QS_HEAD
+
+struct QsParams {
+  const uint8_t* w;
+  const float* x;          // [NB][x_ld]
+  const float* norm_w;
+  float* out;              // [NB][out_ld]
+  const float* residual;   // [NB][out_ld]
+  float eps;
+  int x_ld, out_ld, N, K, R, KW, RW, stages;
+  long long row_bytes;
+};
+
+template <typename D, int NB>
+__global__ void __launch_bounds__(kQsMaxWarps * 32 + 32, 1) quant_stream_kernel(QsParams p) {
+  constexpr int U = NB == 1 && sizeof(D) < 64 ? 2 : 1;      // what the registers hold (F16: two rows 87 us, one 67)
+  extern __shared__ __align__(128) uint8_t qs_smem[];     // ring, 16 bytes of slack, one token's inputs, partial sums [rows][NB][KW]
+  __shared__ uint64_t full[kQsMaxStages], empty[kQsMaxStages];
+  __shared__ float s_sq[NB][kQsMaxWarps];
+  __shared__ int s_failed;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5, nwarps = p.KW * p.RW;
+  const int nchunks = (p.N + p.R - 1) / p.R;
+  const int c0 = (int)(((long long)blockIdx.x * nchunks) / gridDim.x), c1 = (int)(((long long)(blockIdx.x + 1) * nchunks) / gridDim.x);
+  const int stage_bytes = (int)(p.R * p.row_bytes);
+  float* xbuf = reinterpret_cast<float*>(qs_smem + (((size_t)p.stages * stage_bytes + 16 + 127) & ~(size_t)127));   // [K / 32][36]
+  float* part = xbuf + (p.K >> 5) * 36;
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (t == 0) {
+    for (int i = 0; i < p.stages; ++i) {
+      tc::mbar_init(&full[i], 1);
+      tc::mbar_init(&empty[i], nwarps);
+    }
+    tc::mbar_fence_init();
+    s_failed = 0;
+  }
+  __syncthreads();
+  bool failed = false;
+  if (warp == nwarps) {
+    if (lane == 0) {
+      for (int c = c0; c < c1 && !failed; ++c) {
+        const int i = c - c0, st = i % p.stages;
+        if (!tc::mbar_wait_sleep<40>(&empty[st], ((i / p.stages) & 1) ^ 1)) { failed = true; break; }
+        const uint32_t bytes = (uint32_t)(min(p.R, p.N - c * p.R) * p.row_bytes);      // a multiple of 16: the caller checked
+        tc::mbar_arrive_expect_tx(&full[st], bytes);
+        tc::bulk_g2s(qs_smem + (size_t)st * stage_bytes, p.w + (size_t)c * p.R * p.row_bytes, bytes, &full[st]);
+      }
+    }
+  } else {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const int kw = warp % p.KW, rw = warp / p.KW;
+    const int b = kw * 32 + lane;                 // this lane's block of 32 inputs
+    const bool live = b * 32 < p.K;
+    uint64_t x2[NB][16];
+    float xs[NB][D::kScales];
+#pragma unroll
+    for (int n = 0; n < NB; ++n) {
+      // coalesced loads into padded shared memory, from there 32 neighbours per lane (strided global loads took 4 us)
+      const float4* xp = reinterpret_cast<const float4*>(p.x + (size_t)n * p.x_ld);
+      const float4* np = reinterpret_cast<const float4*>(p.norm_w);
+      float sq = 0.0f;
+      for (int i = t; i < (p.K >> 2); i += nwarps * 32) {
+        float4 v = xp[i];
+        if (p.norm_w != nullptr) {
+          const float4 g = __ldg(np + i);
+          sq += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
+          v.x *= g.x; v.y *= g.y; v.z *= g.z; v.w *= g.w;
+        }
+        *reinterpret_cast<float4*>(xbuf + (i >> 3) * 36 + (i & 7) * 4) = v;
+      }
+      sq = warp_sum(sq);
+      if (lane == 0) s_sq[n][warp] = sq;
+      asm volatile("bar.sync 1, %0;" ::"r"(nwarps * 32) : "memory");
+      float xv[32];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const float4 v = live ? *reinterpret_cast<const float4*>(xbuf + b * 36 + i * 4) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        xv[4 * i] = v.x; xv[4 * i + 1] = v.y; xv[4 * i + 2] = v.z; xv[4 * i + 3] = v.w;
+      }
+#pragma unroll
+      for (int i = 0; i < 16; ++i) x2[n][i] = qs_pack(xv[2 * i], xv[2 * i + 1]);
+      constexpr int G = 32 / D::kScales;
+#pragma unroll
+      for (int g = 0; g < D::kScales; ++g) {
+        xs[n][g] = 0.0f;
+#pragma unroll
+        for (int i = 0; i < G; ++i) xs[n][g] += xv[g * G + i];
+      }
+      if (n + 1 < NB) asm volatile("bar.sync 1, %0;" ::"r"(nwarps * 32) : "memory");
+    }
+    for (int c = c0; c < c1 && !failed; ++c) {
+      const int i = c - c0, st = i % p.stages, rows = min(p.R, p.N - c * p.R);
+      if (!tc::mbar_wait(&full[st], (i / p.stages) & 1)) { failed = true; break; }
+      const uint8_t* chunk = qs_smem + (size_t)st * stage_bytes;
+      // U rows side by side: their loads, sums and shuffles overlap
+      for (int r = rw; r < rows; r += U * p.RW) {
+        float acc[U][NB];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+          for (int n = 0; n < NB; ++n) acc[u][n] = 0.0f;
+        if (live) {
+          D d[U];
+#pragma unroll
+          for (int u = 0; u < U; ++u) d[u].load(chunk + (size_t)min(r + u * p.RW, rows - 1) * p.row_bytes, b);
+          constexpr int G2 = 16 / D::kScales;
+#pragma unroll
+          for (int g = 0; g < D::kScales; ++g) {
+            uint64_t a[U][NB];
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+#pragma unroll
+              for (int n = 0; n < NB; ++n) a[u][n] = 0ull;
+#pragma unroll
+            for (int k = 0; k < G2; ++k)
+#pragma unroll
+              for (int u = 0; u < U; ++u) {
+                const uint64_t q = d[u].q2((g * G2 + k) * 2);
+#pragma unroll
+                for (int n = 0; n < NB; ++n) a[u][n] = qs_fma2(q, x2[n][g * G2 + k], a[u][n]);
+              }
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+#pragma unroll
+              for (int n = 0; n < NB; ++n) {
+                acc[u][n] = fmaf(d[u].s[g], qs_sum2(a[u][n]), acc[u][n]);
+                if (D::kMin) acc[u][n] = fmaf(-d[u].m[g], xs[n][g], acc[u][n]);
+              }
+          }
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+          for (int u = 0; u < U; ++u)
+#pragma unroll
+            for (int n = 0; n < NB; ++n) acc[u][n] += __shfl_xor_sync(0xffffffffu, acc[u][n], o);
+        if (lane == 0) {
+#pragma unroll
+          for (int u = 0; u < U; ++u)
+#pragma unroll
+            for (int n = 0; n < NB; ++n)
+              if (r + u * p.RW < rows) part[((size_t)(i * p.R + r + u * p.RW) * NB + n) * p.KW + kw] = acc[u][n];
+        }
+      }
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(&empty[st]);
+    }
+  }
+  if (failed) s_failed = 1;      // a copy that never arrived: its rows come out as NaN instead of numbers made of old data
+  __syncthreads();
+  if (warp >= nwarps) return;
+  float inv[NB];
+#pragma unroll
+  for (int n = 0; n < NB; ++n) {
+    float ss = 0.0f;
+    for (int k = 0; k < nwarps; ++k) ss += s_sq[n][k];
+    inv[n] = p.norm_w != nullptr ? 1.0f / sqrtf(ss / (float)p.K + p.eps) : 1.0f;
+  }
+  const int row0 = c0 * p.R, rows = min(c1 * p.R, p.N) - row0;
+  for (int i = t; i < rows; i += nwarps * 32) {
+#pragma unroll
+    for (int n = 0; n < NB; ++n) {
+      float v = 0.0f;
+      for (int k = 0; k < p.KW; ++k) v += part[((size_t)i * NB + n) * p.KW + k];
+      const size_t o = (size_t)n * p.out_ld + row0 + i;
+      p.out[o] = s_failed ? __int_as_float(0x7FFFFFFF) : (p.residual ? p.residual[o] : 0.0f) + v * inv[n];
+    }
+  }
+}
+
+// Whether a matrix can be streamed, and how: chunks of R rows that start and end on 16-byte boundaries (a last chunk of fewer rows
+// must end on one too), two stages at least, inputs in 16-byte loads, at most sixteen warps over K.
+template <typename D>
+static bool qs_plan(QsParams& p, int& grid, size_t& smem, int nb) {
+  constexpr int unroll = sizeof(D) < 64 ? 2 : 1;
+  if (p.K % 32 != 0 || p.K > kQsMaxWarps * 1024 || p.x_ld % 4 != 0) return false;
+  if (((reinterpret_cast<uintptr_t>(p.w) | reinterpret_cast<uintptr_t>(p.x) | reinterpret_cast<uintptr_t>(p.norm_w)) & 15) != 0) return false;
+  if (((long long)p.N * p.row_bytes) % 16 != 0) return false;
+  int R = 1;
+  while ((R * p.row_bytes) % 16 != 0) R *= 2;                    // 1 to 8: a row has an even number of bytes
+  p.KW = (p.K + 1023) / 1024;
+  p.RW = 1;
+  while (p.RW * 2 * p.KW <= kQsMaxWarps && p.RW < 8) p.RW *= 2;
+  while (R < p.RW) R *= 2;
+  if (unroll == 2 && R == p.RW && 2 * R * p.row_bytes <= kQsRing / 3) R *= 2;      // two rows for every warp over rows, three copies ahead
+  if (R * p.row_bytes > kQsRing / 2) return false;
+  p.R = R;
+  const long long stage = R * p.row_bytes;
+  p.stages = (int)(kQsRing / stage < kQsMaxStages ? kQsRing / stage : kQsMaxStages);
+  if (p.stages < 2) return false;
+  const int nchunks = (p.N + R - 1) / R;
+  grid = nchunks < 148 ? nchunks : 148;
+  const int most = kQsRows / R;                                   // chunks of a CTA
+  if ((nchunks + grid - 1) / grid > most) grid = (nchunks + most - 1) / most;
+  const int per = (nchunks + grid - 1) / grid;
+  if (p.stages > per) p.stages = per < 2 ? 2 : per;
+  smem = (((size_t)p.stages * stage + 16 + 127) & ~(size_t)127) + (size_t)(p.K / 32) * 36 * sizeof(float) + (size_t)per * R * nb * p.KW * sizeof(float);
+  return smem <= 220 * 1024;
+}
+
+template <typename D>
+static QsParams qs_params(const void* w, const float* x, int x_ld, const float* norm_w, float eps, float* out, const float* residual, int out_ld,
+                          int N, int K) {
+  QsParams p{};
+  p.w = (const uint8_t*)w; p.x = x; p.norm_w = norm_w; p.out = out; p.residual = residual; p.eps = eps;
+  p.x_ld = x_ld; p.out_ld = out_ld; p.N = N; p.K = K;
+  p.row_bytes = (long long)(K / D::kElems) * D::kBytes;
+  return p;
+}
+
+template <typename D, int NB>
+static int qs_launch(const QsParams& p, int grid, size_t smem, cudaStream_t st) {
+  static bool configured[64] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return BONSAI_CUDA_LAUNCH_FAILED;
+  if (!configured[dev]) {
+    if (cudaFuncSetAttribute(quant_stream_kernel<D, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024) != cudaSuccess) return BONSAI_CUDA_LAUNCH_FAILED;
+    configured[dev] = true;
+  }
+  const cudaError_t e = launch_pdl(quant_stream_kernel<D, NB>, dim3(grid), dim3((p.KW * p.RW + 1) * 32), smem, st, p);
+  return e == cudaSuccess ? BONSAI_CUDA_OK : BONSAI_CUDA_LAUNCH_FAILED;
+}
+
 template <typename D>
 __global__ void __launch_bounds__(256) quant_gemv_kernel(const uint8_t* __restrict__ w, const float* __restrict__ x,
                                                         const float* __restrict__ norm_w, float eps, float* __restrict__ out,
@@ -106,10 +509,14 @@ __global__ void __launch_bounds__(256) quant_gemv_kernel(const uint8_t* __restri
   }
 }
 
-template <typename D>
+template <typename D, typename Q>
 static int launch_quant_gemv(const void* w, const float* x, const float* norm_w, float eps, float* out, const float* residual, int N, int K,
                              cudaStream_t st) {
   if (K % D::kElems != 0) return BONSAI_CUDA_BAD_ARG;
+  QsParams p = qs_params<D>(w, x, K, norm_w, eps, out, residual, N, N, K);
+  int sgrid;
+  size_t smem;
+  if (qs_plan<Q>(p, sgrid, smem, 1)) return qs_launch<Q, 1>(p, sgrid, smem, st);
   int grid = (N + 7) / 8;
   if (grid > 148 * 8) grid = 148 * 8;
   quant_gemv_kernel<D><<<grid, 256, 0, st>>>((const uint8_t*)w, x, norm_w, eps, out, residual, N, K);
@@ -174,13 +581,27 @@ __global__ void __launch_bounds__(256) quant_gemv_batched_kernel(const uint8_t* 
   }
 }
 
-template <typename D>
+template <typename D, typename Q>
 static int launch_quant_gemv_batched(const void* w, const float* x, int x_ld, const float* norm_w, float eps, float* out, const float* residual,
                                      int out_ld, int N, int K, int B, cudaStream_t st) {
   if (K % D::kElems != 0) return BONSAI_CUDA_BAD_ARG;
   int grid = (N + 7) / 8;
   if (grid > 148 * 8) grid = 148 * 8;
   const uint8_t* wp = (const uint8_t*)w;
+  {
+    QsParams p = qs_params<D>(w, x, x_ld, norm_w, eps, out, residual, out_ld, N, K);
+    int sgrid, rc = BONSAI_CUDA_OK;
+    size_t smem;
+    if (qs_plan<Q>(p, sgrid, smem, 2)) {
+      for (int b = 0; b < B && rc == BONSAI_CUDA_OK; b += 2) {       // the second pair's weights come from L2 when the matrix fits there
+        p.x = x + (size_t)b * x_ld;
+        p.out = out + (size_t)b * out_ld;
+        p.residual = residual ? residual + (size_t)b * out_ld : nullptr;
+        rc = b + 1 < B ? qs_launch<Q, 2>(p, sgrid, smem, st) : qs_launch<Q, 1>(p, sgrid, smem, st);
+      }
+      return rc;
+    }
+  }
   // groups of up to eight rows: the weights of a later group come from L2 when the matrix fits there
   for (int b0 = 0; b0 < B; b0 += 8) {
     const int nb = B - b0 < 8 ? B - b0 : 8;
@@ -255,20 +676,20 @@ int bonsai_quant_gemv(int type, const void* w, const float* x, const float* norm
   using namespace bonsai;
   if (N <= 0 || K <= 0) return BONSAI_CUDA_BAD_ARG;
   switch (type) {
-    case 0: return launch_quant_gemv<DecF32>(w, x, norm_w, eps, out, residual, N, K, stream);
-    case 1: return launch_quant_gemv<DecF16>(w, x, norm_w, eps, out, residual, N, K, stream);
-    case 30: return launch_quant_gemv<DecBF16>(w, x, norm_w, eps, out, residual, N, K, stream);
-    case 2: return launch_quant_gemv<DecQ4_0>(w, x, norm_w, eps, out, residual, N, K, stream);
-    case 8: return launch_quant_gemv<DecQ8_0>(w, x, norm_w, eps, out, residual, N, K, stream);
-    case 10: return launch_quant_gemv<DecQ2K>(w, x, norm_w, eps, out, residual, N, K, stream);
-    case 11: return launch_quant_gemv<DecQ3K>(w, x, norm_w, eps, out, residual, N, K, stream);
-    case 12: return launch_quant_gemv<DecQ4K>(w, x, norm_w, eps, out, residual, N, K, stream);
-    case 13: return launch_quant_gemv<DecQ5K>(w, x, norm_w, eps, out, residual, N, K, stream);
-    case 14: return launch_quant_gemv<DecQ6K>(w, x, norm_w, eps, out, residual, N, K, stream);
-    case 15: return launch_quant_gemv<DecQ8K>(w, x, norm_w, eps, out, residual, N, K, stream);
-    case 35: return launch_quant_gemv<DecTq2_256>(w, x, norm_w, eps, out, residual, N, K, stream);
-    case 43: return launch_quant_gemv<DecFp8<false>>(w, x, norm_w, eps, out, residual, N, K, stream);
-    case 44: return launch_quant_gemv<DecFp8<true>>(w, x, norm_w, eps, out, residual, N, K, stream);
+    case 0: return launch_quant_gemv<DecF32, QsF32>(w, x, norm_w, eps, out, residual, N, K, stream);
+    case 1: return launch_quant_gemv<DecF16, QsF16>(w, x, norm_w, eps, out, residual, N, K, stream);
+    case 30: return launch_quant_gemv<DecBF16, QsBF16>(w, x, norm_w, eps, out, residual, N, K, stream);
+    case 2: return launch_quant_gemv<DecQ4_0, QsQ4_0>(w, x, norm_w, eps, out, residual, N, K, stream);
+    case 8: return launch_quant_gemv<DecQ8_0, QsQ8_0>(w, x, norm_w, eps, out, residual, N, K, stream);
+    case 10: return launch_quant_gemv<DecQ2K, QsQ2K>(w, x, norm_w, eps, out, residual, N, K, stream);
+    case 11: return launch_quant_gemv<DecQ3K, QsQ3K>(w, x, norm_w, eps, out, residual, N, K, stream);
+    case 12: return launch_quant_gemv<DecQ4K, QsQ4K>(w, x, norm_w, eps, out, residual, N, K, stream);
+    case 13: return launch_quant_gemv<DecQ5K, QsQ5K>(w, x, norm_w, eps, out, residual, N, K, stream);
+    case 14: return launch_quant_gemv<DecQ6K, QsQ6K>(w, x, norm_w, eps, out, residual, N, K, stream);
+    case 15: return launch_quant_gemv<DecQ8K, QsQ8K>(w, x, norm_w, eps, out, residual, N, K, stream);
+    case 35: return launch_quant_gemv<DecTq2_256, QsTq2_256>(w, x, norm_w, eps, out, residual, N, K, stream);
+    case 43: return launch_quant_gemv<DecFp8<false>, QsFp8<false>>(w, x, norm_w, eps, out, residual, N, K, stream);
+    case 44: return launch_quant_gemv<DecFp8<true>, QsFp8<true>>(w, x, norm_w, eps, out, residual, N, K, stream);
     default: return BONSAI_CUDA_BAD_ARG;
   }
 }
@@ -278,22 +699,22 @@ int bonsai_quant_gemv_batched(int type, const void* w, const float* x, int x_ld,
                               const float* residual, int out_ld, int N, int K, int B, cudaStream_t stream) {
   using namespace bonsai;
   if (N <= 0 || K <= 0 || B <= 0 || x_ld < K || out_ld < N) return BONSAI_CUDA_BAD_ARG;
-#define BONSAI_QGB(D) return launch_quant_gemv_batched<D>(w, x, x_ld, norm_w, eps, out, residual, out_ld, N, K, B, stream)
+#define BONSAI_QGB(...) return launch_quant_gemv_batched<__VA_ARGS__>(w, x, x_ld, norm_w, eps, out, residual, out_ld, N, K, B, stream)
   switch (type) {
-    case 0: BONSAI_QGB(DecF32);
-    case 1: BONSAI_QGB(DecF16);
-    case 30: BONSAI_QGB(DecBF16);
-    case 2: BONSAI_QGB(DecQ4_0);
-    case 8: BONSAI_QGB(DecQ8_0);
-    case 10: BONSAI_QGB(DecQ2K);
-    case 11: BONSAI_QGB(DecQ3K);
-    case 12: BONSAI_QGB(DecQ4K);
-    case 13: BONSAI_QGB(DecQ5K);
-    case 14: BONSAI_QGB(DecQ6K);
-    case 15: BONSAI_QGB(DecQ8K);
-    case 35: BONSAI_QGB(DecTq2_256);
-    case 43: BONSAI_QGB(DecFp8<false>);
-    case 44: BONSAI_QGB(DecFp8<true>);
+    case 0: BONSAI_QGB(DecF32, QsF32);
+    case 1: BONSAI_QGB(DecF16, QsF16);
+    case 30: BONSAI_QGB(DecBF16, QsBF16);
+    case 2: BONSAI_QGB(DecQ4_0, QsQ4_0);
+    case 8: BONSAI_QGB(DecQ8_0, QsQ8_0);
+    case 10: BONSAI_QGB(DecQ2K, QsQ2K);
+    case 11: BONSAI_QGB(DecQ3K, QsQ3K);
+    case 12: BONSAI_QGB(DecQ4K, QsQ4K);
+    case 13: BONSAI_QGB(DecQ5K, QsQ5K);
+    case 14: BONSAI_QGB(DecQ6K, QsQ6K);
+    case 15: BONSAI_QGB(DecQ8K, QsQ8K);
+    case 35: BONSAI_QGB(DecTq2_256, QsTq2_256);
+    case 43: BONSAI_QGB(DecFp8<false>, QsFp8<false>);
+    case 44: BONSAI_QGB(DecFp8<true>, QsFp8<true>);
     default: return BONSAI_CUDA_BAD_ARG;
   }
 #undef BONSAI_QGB

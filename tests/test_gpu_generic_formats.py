@@ -197,3 +197,26 @@ def test_standalone_rmsnorm_and_residual_add():
     a, b = torch.randn(100003, generator=g).to(dev), torch.randn(100003, generator=g).to(dev)
     want = a + b
     assert torch.equal(K.residual_add(a, b), want)
+
+
+@pytest.mark.parametrize("name,tid,tol", TYPES)
+@pytest.mark.parametrize("n,k", [(8, 256), (44, 2560), (1201, 2560), (600, 4096), (24, 12288), (16, 16384), (16, 16640)])
+def test_streamed_rows_of_every_format(name, tid, tol, n, k):
+    """Few rows, odd row counts (whose bytes cannot be copied in 16-byte units for some formats), widths that leave lanes of the last warp
+    idle, the widest matrix that is streamed and one beyond it; one to three tokens."""
+    from oxibonsai_b200.core.blocks import dequantize, quantize
+    from oxibonsai_b200.ops import cuda_ops as K
+    dev = torch.device("cuda:0")
+    rng = np.random.default_rng(n + k)
+    q = quantize(tid, rng.normal(size=(n, k)).astype(np.float32) * 0.05)
+    wd = torch.from_numpy(dequantize(tid, q).reshape(n, k)).double()
+    qd = torch.from_numpy(q).to(dev)
+    nw = torch.from_numpy(rng.uniform(0.5, 1.5, k).astype(np.float32))
+    for batch in (1, 2, 3):
+        x = torch.from_numpy(rng.normal(size=(batch, k)).astype(np.float32))
+        res = torch.from_numpy(rng.normal(size=(batch, n)).astype(np.float32))
+        y = K.quant_gemv_batched(tid, qd, n, k, x.to(dev), norm_w=nw.to(dev), eps=1e-6, residual=res.to(dev)).cpu().double()
+        xn = nw.double() * x.double() * torch.rsqrt((x.double() ** 2).mean(dim=1, keepdim=True) + 1e-6)
+        # every sum runs over at most K / 32 + 64 rounded steps of terms whose magnitudes add up to |x| |W|, with minima taken off separately
+        terms = xn.abs() @ wd.abs().T * (3.0 if name in ("Q2_K", "Q4_K", "Q5_K") else 1.0) + res.abs()
+        assert ((y - (xn @ wd.T + res.double())).abs() <= 2.0 ** -23 * (k / 32 + 64) * terms).all(), (name, batch)
