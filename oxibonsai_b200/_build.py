@@ -35,7 +35,7 @@ NVCC_FLAGS = ["-std=c++17", "-O3", "-lineinfo", "-shared", "-Xcompiler", "-fPIC"
 
 def _sources(kind: str) -> list[Path]:
     pats = {"host": ["capi_*.cpp", "core/*.cpp", "cpu/*.cpp", "runtime/*.cpp"], "cuda": ["cuda/*.cu", "comm/*.cu"],
-            "layered": ["layered/*.cu", "cuda/sampler.cu", "cuda/bitgemm_prefill.cu"]}[kind]
+            "layered": ["layered/*.cu", "cuda/sampler.cu", "cuda/bitgemm_prefill.cu", "cuda/gemm_pair.cu"]}[kind]
     out: list[Path] = []
     for p in pats:
         out += sorted(CSRC.glob(p))

@@ -46,6 +46,8 @@ int bonsai_attn_decode_qkv_f16(const float*, int, const float*, const float*, fl
 int bonsai_norm_to_f16_hmma(const float*, int, const float*, float, int, int, void*, int, cudaStream_t);
 int bonsai_bitgemm_hmma(const void*, const void*, const void*, int, float*, const float*, void*, int, int, int, int, int, cudaStream_t);
 int bonsai_bitgemm_hmma_tp(const void*, const void*, const void*, const void*, int, float*, const float*, int, int, int, int, cudaStream_t);
+int bonsai_gemm_pair(const void*, const void*, int, float*, const float*, void*, int*, int, int, int, int, int, int, int, cudaStream_t);
+int bonsai_expand_rows(const void*, const void*, int, int, int, void*, cudaStream_t);
 int bonsai_attn_prefill_order(const float*, int, int, const int*, int, int, int, int, int, const void*, const void*, const float*,
                               const float*, void*, int, int, cudaStream_t);
 int bonsai_embed_rows_f16(const void*, const int*, float*, int, int, int, cudaStream_t);
@@ -235,6 +237,7 @@ static int decode_step(Runner& r, const uint64_t* sp, int batch, int flags, int 
 enum PrefillPtr {
   PP_TOKENS = 0, PP_POSITIONS, PP_H, PP_XN, PP_QKV, PP_Q, PP_ATTN, PP_ACT, PP_STATUS,
   PP_SM_ATTN, PP_SM_ACC, PP_SM_ML, PP_SM_CTR,   // small chunks: f32 attention output and split-KV workspace for kSmallChunk rows
+  PP_WEXP, PP_WEXP_ELEMS,         // scratch matrix of expanded weights (pointer, f16 elements as a plain integer)
   PP_GEMM_WS, PP_GEMM_WS_BYTES,   // workspace of the GEMM's balanced work distribution (pointer, size as a plain integer)
   PP_COUNT
 };
@@ -242,12 +245,33 @@ enum PrefillPtr {
 // Chunks of at most this many tokens run like a decode batch (mma.sync GEMMs, split-KV attention); the small-chunk
 // workspace holds kSmallChunk rows of kSmallSplits splits.
 constexpr int kSmallChunk = 32, kSmallSplits = 16;
+// Chunks of more than 64 tokens expand the weights once and multiply densely (pair_gemm) where the scratch matrix holds all of them,
+// larger matrices from kPairTokens tokens on.  In place / expanded, us: 6144 x 4096, 65 tokens 34 / 24, 192 tokens 44 / 25;
+// 24576 x 4096, 65 tokens 61 / 85, 192 tokens 78 / 90, 256 tokens 91 / 94, 384 tokens 134 / 102.
+constexpr int kPairTokens = 256;
 
 static inline int pf_gemm(Runner& r, const void* codes, const void* scales, const void* x, int x_ld, float* out_f32, const float* residual,
                           void* out_f16, int* status, int n_rows, int K, int T, int epi, int out_ld, int sms, const void* dense_w,
                           cudaStream_t st) {
   return bonsai_bitgemm_prefill_ws(codes, scales, x, x_ld, out_f32, residual, out_f16, status, n_rows, K, T, epi, out_ld, sms, dense_w,
                                    r.gemm_ws, r.gemm_ws_bytes, 1, st);
+}
+
+// A packed GEMM over many tokens: the weights are expanded to f16 slab by slab (256 rows at least) into a scratch matrix that stays in
+// L2, and multiplied by the dense kernel on pairs of SMs.
+static int pair_gemm(const void* codes, const void* scales, const void* x, int x_ld, float* out_f32, const float* residual, void* out_f16,
+                     int* status, int n_rows, int K, int T, int epi, int out_ld, int sms, void* scratch, size_t scratch_elems, cudaStream_t st) {
+  const int most = (int)(scratch_elems / (size_t)K < (size_t)n_rows ? scratch_elems / (size_t)K : (size_t)n_rows);
+  const int slabs = (n_rows + most - 1) / most, per = ((n_rows + slabs - 1) / slabs + 255) / 256 * 256;
+  const int step = slabs == 1 ? n_rows : (per <= most ? per : most / 256 * 256);      // most >= 256: the caller checked
+  for (int r0 = 0; r0 < n_rows; r0 += step) {
+    const int rows = n_rows - r0 < step ? n_rows - r0 : step;
+    RC(bonsai_expand_rows(codes, scales, r0, rows, K, scratch, st));
+    RC(bonsai_gemm_pair(scratch, x, x_ld, out_f32 ? out_f32 + r0 : nullptr, residual ? residual + r0 : nullptr,
+                        out_f16 ? static_cast<char*>(out_f16) + (size_t)(epi == 2 ? r0 / 2 : r0) * 2 : nullptr, status, rows, K, T, epi, out_ld,
+                        sms, 0, st));
+  }
+  return 0;
 }
 
 // One chunk of T prompt tokens of the sequence in `slot`, starting at position pos0: batched
@@ -295,8 +319,12 @@ static int prefill_chunk(Runner& r, const uint64_t* sp, const uint64_t* pp, int 
     return hm ? bonsai_norm_to_f16_hmma(h, hidden, w, r.eps, T, hidden, xn, xn_ld, st)
               : bonsai_norm_to_f16_paired(h, hidden, w, r.eps, T, hidden, xn, xn_ld, 0, st);
   };
+  void* wexp = P<void>(pp[PP_WEXP]);
+  const size_t wexp_elems = (size_t)pp[PP_WEXP_ELEMS];
   auto gemm = [&](const void* codes, const void* scales, const void* x, int x_ld, float* out_f32, const float* residual, void* out_f16,
                   int n_rows, int K, int epi, int out_ld) {
+    if (T > 64 && wexp_elems >= (size_t)256 * K && (T >= kPairTokens || (size_t)n_rows * K <= wexp_elems))
+      return pair_gemm(codes, scales, x, x_ld, out_f32, residual, out_f16, status, n_rows, K, T, epi, out_ld, sms, wexp, wexp_elems, st);
     return hm ? bonsai_bitgemm_hmma(codes, scales, x, x_ld, out_f32, residual, out_f16, n_rows, K, T, epi, out_ld, st)
               : pf_gemm(r, codes, scales, x, x_ld, out_f32, residual, out_f16, status, n_rows, K, T, epi, out_ld, sms, nullptr, st);
   };

@@ -20,6 +20,15 @@ constexpr uint32_t kSpinLimit = 1u << 24;  // ~ a second of polling; far beyond 
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
+// One lane of a converged warp, for the instructions that a single thread issues.  Behind this predicate the compiler knows that one
+// thread is active and keeps descriptors and addresses in uniform registers; behind `lane == 0` it wraps every tcgen05 and TMA
+// instruction into a loop over the lanes that might be active.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\tselp.u32 %0, 1, 0, e;\n\t}" : "=r"(p));
+  return p != 0;
+}
+
 // ---- mbarrier ---------------------------------------------------------------------------------
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");

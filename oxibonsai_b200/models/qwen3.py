@@ -410,9 +410,13 @@ class Qwen3Runner(SlotState):
                   "sm_ml": torch.zeros((sm, nq, ss, 2), **f32), "sm_ctr": torch.zeros(sm * max(1, nkv), **i32)})
         if b["gemm_ws"] is None:
             b["gemm_ws"] = self._gemm_ws = K.new_gemm_workspace(dev)
-        order = ["tokens", "positions", "h", "xn", "qkv", "q", "attn", "act", "status", "sm_attn", "sm_acc", "sm_ml", "sm_ctr", "gemm_ws"]
-        assert len(order) + 1 == K._pf().bonsai_runner_prefill_ptr_count()
-        b["ptrs"] = (C.c_uint64 * (len(order) + 1))(*[b[k].data_ptr() for k in order], b["gemm_ws"].numel())
+        # scratch for expanded weights: the largest matrix, at most 104 MB (slabs of it then pass through L2), at least 256 rows
+        mats = [m for lw in w.layers[:1] for m in (lw.qkv, lw.o, lw.gate_up, lw.down)]
+        b["wexp"] = torch.empty(max(256 * max(m.k for m in mats), min(52 << 20, max(m.n * m.k for m in mats))), **f16)
+        order = ["tokens", "positions", "h", "xn", "qkv", "q", "attn", "act", "status", "sm_attn", "sm_acc", "sm_ml", "sm_ctr"]
+        ptrs = [b[k].data_ptr() for k in order] + [b["wexp"].data_ptr(), b["wexp"].numel(), b["gemm_ws"].data_ptr(), b["gemm_ws"].numel()]
+        assert len(ptrs) == K._pf().bonsai_runner_prefill_ptr_count()
+        b["ptrs"] = (C.c_uint64 * len(ptrs))(*ptrs)
         self._pf = b
         return b
 

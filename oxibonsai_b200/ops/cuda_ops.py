@@ -742,6 +742,43 @@ def dense_gemm_f16(w: torch.Tensor, x: torch.Tensor, out: torch.Tensor | None = 
     return out
 
 
+_gp_declared = False
+
+
+def _gp():
+    global _gp_declared
+    l = _pf()
+    if not _gp_declared:
+        declare({"bonsai_gemm_pair": [_vp, _vp, _i, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _vp],
+                 "bonsai_expand_rows": [_vp, _vp, _i, _i, _i, _vp, _vp]})
+        _gp_declared = True
+    return l
+
+
+def expand_rows(w: PlanarWeight, row0: int = 0, rows: int | None = None) -> torch.Tensor:
+    """Rows of a packed matrix as f16 [rows, K] in paired-K order (the operand of :func:`gemm_pair` for prompt chunks)."""
+    rows = w.n - row0 if rows is None else rows
+    out = torch.empty((rows, w.k), dtype=torch.float16, device=w.codes.device)
+    check(_gp().bonsai_expand_rows(w.codes.data_ptr(), w.scales.data_ptr(), row0, rows, w.k, out.data_ptr(), stream()), "expand_rows")
+    return out
+
+
+def gemm_pair(w: torch.Tensor, x: torch.Tensor, epi: int = 0, residual: torch.Tensor | None = None, out: torch.Tensor | None = None,
+              status: torch.Tensor | None = None, sms: int = 148, tile_tokens: int = 0) -> torch.Tensor:
+    """out[T, N] = epilogue(x[T, K] @ w[N, K]^T) for f16 operands on pairs of SMs.  ``epi``: 0 f32 store, 1 f32 residual add, 2 f16 SwiGLU
+    over interleaved gate / up rows (paired-K order), 3 f16 store.  ``tile_tokens``: tokens per tile, 0 = chosen by size."""
+    T, n = x.shape[0], w.shape[0]
+    assert w.dtype == torch.float16 and x.dtype == torch.float16 and w.is_contiguous() and x.shape[1] == w.shape[1]
+    if out is None:
+        out = torch.empty((T, n // 2 if epi == 2 else n), dtype=torch.float32 if epi <= 1 else torch.float16, device=x.device)
+    if status is None:
+        status = torch.zeros(1, dtype=torch.int32, device=x.device)
+    check(_gp().bonsai_gemm_pair(w.data_ptr(), x.data_ptr(), x.stride(0), out.data_ptr() if epi <= 1 else None, ptr(residual),
+                                 out.data_ptr() if epi >= 2 else None, status.data_ptr(), n, w.shape[1], T, epi, out.stride(0), sms, tile_tokens,
+                                 stream()), "gemm_pair")
+    return out
+
+
 def bitgemm_prefill(w: PlanarWeight, x_paired: torch.Tensor, epi: int = 0, residual: torch.Tensor | None = None,
                     out: torch.Tensor | None = None, status: torch.Tensor | None = None, sms: int = 148,
                     balanced: bool | str = "auto") -> torch.Tensor:

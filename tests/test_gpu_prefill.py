@@ -153,3 +153,47 @@ def test_bitgemm_hmma_matches_fp32(ty, rows, cols, T):
         want = torch.nn.functional.silu(ref[:, 0::2]) * ref[:, 1::2]
         got = ys.cpu()[:, K.hmma_k_index(rows // 2)].double()
         assert (got - want).abs().max().item() <= 3e-3 * want.abs().max().item() + 1e-4
+
+
+@pytest.mark.parametrize("ty", [TQ2_0_G128, Q1_0_G128])
+def test_expanded_rows_are_the_decoded_weights(ty):
+    from oxibonsai_b200.ops import cuda_ops as K
+    n, k = 77, 384
+    raw, want = _random_quant(ty, n, k, 5)
+    w = K.PlanarWeight(n, k, torch.device(DEV))
+    w.fill_from_gguf(torch.from_numpy(np.array(raw, copy=True)).to(DEV), ty, k, 0, n)
+    want = want.half()
+    perm = K.paired_k_index(k)
+    for row0, rows in ((0, n), (5, 1), (40, 37)):
+        assert torch.equal(K.expand_rows(w, row0, rows).cpu()[:, perm], want[row0:row0 + rows])
+
+
+@pytest.mark.parametrize("rows,cols,T,tile", [(1, 64, 1, 0), (130, 64, 33, 32), (256, 192, 256, 256), (300, 320, 257, 0), (514, 4096, 77, 48), (1024, 448, 700, 240)])
+@pytest.mark.parametrize("sms", [2, 6, 148])
+def test_pair_gemm_matches_fp64(rows, cols, T, tile, sms):
+    """Remainders of rows (256 per tile), tokens (any multiple of 16 per tile) and stages (six 64-input blocks), one cluster for all
+    tiles and one for each."""
+    from oxibonsai_b200.ops import cuda_ops as K
+    g = torch.Generator(device=DEV).manual_seed(rows + T)
+    w = (torch.randn((rows, cols), device=DEV, generator=g) * cols ** -0.5).half()
+    x = torch.randn((T, cols), device=DEV, generator=g).half()
+    res = torch.randn((T, rows), device=DEV, generator=g)
+    want, terms = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    # products are exact in f32; every addition of the accumulator may drop one unit in the last place
+    bound = 2.0 ** -23 * (cols + 4) * (terms + res.abs().double())
+    a, b = (K.gemm_pair(w, x, e, residual=r, status=status, sms=sms, tile_tokens=tile) for e, r in ((0, None), (1, res)))
+    assert ((a.double() - want).abs() <= bound).all() and ((b.double() - want - res.double()).abs() <= bound).all()
+    half = 2.0 ** -11
+    assert ((K.gemm_pair(w, x, 3, status=status, sms=sms, tile_tokens=tile).double() - want).abs() <= bound + half * want.abs() + 2.0 ** -25).all()
+    if rows % 2 == 0:
+        gate, up = want[:, 0::2], want[:, 1::2]
+        act = torch.nn.functional.silu(gate) * up
+        n = rows // 2
+        wide = torch.zeros((T, (n + 15) // 16 * 16), dtype=torch.float16, device=DEV)      # paired-K order moves inputs within eight
+        K.gemm_pair(w, x, 2, out=wide, status=status, sms=sms, tile_tokens=tile)
+        got = wide[:, K.paired_k_index(wide.shape[1], DEV)][:, :n].double()
+        # |d silu| <= 1.1 |d gate|; the fast exponential and division add 2^-20
+        slack = 1.1 * bound[:, 0::2] * up.abs() + gate.abs() * bound[:, 1::2] + (half + 2.0 ** -20) * act.abs() + 2.0 ** -24
+        assert ((got - act).abs() <= slack).all()
+    assert status.item() == 0
