@@ -7,8 +7,8 @@
 // sequence (everything before the chunk plus the causal part of the chunk) in blocks of 64 from the
 // page pool, and keeps the online-softmax state in registers (flash-attention style).  The score
 // and value products run on the tensor cores through warp-level mma (m16n8k16, f16 in / f32
-// accumulate); the matrix sizes per CTA (64 x 64 x head_dim) are too small to amortise a
-// TMEM-resident tcgen05 pipeline, and the prefill time is dominated by the GEMMs.
+// accumulate).  Chunks of head size 128 over f16, INT8 and INT4 pages go to the tcgen05 kernel (attention_prefill_tc.cu); this one
+// has the other head size, f32 pages, pages that are no multiple of 64 tokens and the hmma-K output order.
 //
 // q: f32 [T][nq][hd] (already normalised and rotated); output: f16 [T][nq*hd] in the paired-K order
 // that the attention-output GEMM consumes.  KV formats: F32 / F16 / Q8 / Q4 pages (dequantised to
@@ -295,19 +295,27 @@ __global__ void __launch_bounds__(128, 3) attn_prefill_kernel(const float* __res
   }
 }
 
+int attn_prefill_tc(const float*, int, int, const int*, int, int, int, int, int, const void*, const void*, const float*, const float*, void*, int,
+                    void*, size_t, cudaStream_t);
+
 }  // namespace bonsai
 
 extern "C" {
 
 // q f32 [T][nq][hd]; block_table: the sequence's page list; the chunk's first token sits at pos0.
 // out f16 [T][out_ld]; k_order 0 = paired-K (operand order of the tcgen05 GEMM), 1 = hmma-K (the mma.sync GEMM; needs
-// nq * hd to be a multiple of 128).
-int bonsai_attn_prefill_order(const float* q, int T, int pos0, const int* block_table, int nq, int nkv, int hd, int kvt, int page_size,
-                              const void* kpool, const void* vpool, const float* kscale, const float* vscale, void* out, int out_ld,
-                              int k_order, cudaStream_t stream) {
+// nq * hd to be a multiple of 128).  scratch (f16 elements, may be null): where INT8 / INT4 rows are decoded to for the tcgen05 kernel,
+// 2 * nkv * hd per key, keys rounded up to 128; without it, or when it is too small, the mma.sync kernel decodes them itself.
+int bonsai_attn_prefill_ws(const float* q, int T, int pos0, const int* block_table, int nq, int nkv, int hd, int kvt, int page_size,
+                           const void* kpool, const void* vpool, const float* kscale, const float* vscale, void* out, int out_ld,
+                           int k_order, void* scratch, size_t scratch_elems, cudaStream_t stream) {
   using namespace bonsai;
   if (k_order < 0 || k_order > 1 || (k_order == 1 && (nq * hd) % 128 != 0)) return BONSAI_CUDA_BAD_ARG;
   if (T < 1 || (hd != 64 && hd != 128) || nq % nkv != 0 || kvt < 0 || kvt > 3) return BONSAI_CUDA_BAD_ARG;
+  if (k_order == 0) {
+    const int rc = attn_prefill_tc(q, T, pos0, block_table, nq, nkv, hd, kvt, page_size, kpool, vpool, kscale, vscale, out, out_ld, scratch, scratch_elems, stream);
+    if (rc != BONSAI_CUDA_BAD_ARG) return rc;   // bad argument = not a form of that kernel
+  }
   PfKvPool kv{(const uint8_t*)kpool, (const uint8_t*)vpool, kscale, vscale, page_size, nkv, hd, kvt};
   dim3 grid(nq, (T + 63) / 64);
   const float sc = 1.0f / sqrtf((float)hd);
@@ -326,6 +334,12 @@ int bonsai_attn_prefill_order(const float* q, int T, int pos0, const int* block_
     attn_prefill_kernel<64><<<grid, 128, smem, stream>>>(q, T, pos0, block_table, kv, nq, sc, (__half*)out, out_ld, k_order);
   }
   return launch_status();
+}
+
+int bonsai_attn_prefill_order(const float* q, int T, int pos0, const int* block_table, int nq, int nkv, int hd, int kvt, int page_size,
+                              const void* kpool, const void* vpool, const float* kscale, const float* vscale, void* out, int out_ld,
+                              int k_order, cudaStream_t stream) {
+  return bonsai_attn_prefill_ws(q, T, pos0, block_table, nq, nkv, hd, kvt, page_size, kpool, vpool, kscale, vscale, out, out_ld, k_order, nullptr, 0, stream);
 }
 
 // out f16 [T][out_ld] in paired-K order.

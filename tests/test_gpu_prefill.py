@@ -197,3 +197,48 @@ def test_pair_gemm_matches_fp64(rows, cols, T, tile, sms):
         slack = 1.1 * bound[:, 0::2] * up.abs() + gate.abs() * bound[:, 1::2] + (half + 2.0 ** -20) * act.abs() + 2.0 ** -24
         assert ((got - act).abs() <= slack).all()
     assert status.item() == 0
+
+
+@pytest.mark.parametrize("nq,nkv,T,pos0,kvt,page", [(3, 3, 1, 0, 1, 64), (8, 8, 129, 0, 1, 64), (4, 2, 128, 127, 1, 128), (8, 2, 65, 63, 1, 64), (8, 1, 300, 50, 1, 64),
+                                                    (8, 2, 200, 77, 2, 16), (8, 2, 31, 400, 3, 64), (4, 1, 513, 1000, 2, 64)])
+def test_tensor_memory_prompt_attention(nq, nkv, T, pos0, kvt, page):
+    """Group sizes 1 to 8, one to several blocks of query rows and key tiles, contexts that end inside and on tiles, every page format;
+    whatever lies behind the last key (here NaN) does not enter."""
+    import math
+    from oxibonsai_b200.ops import cuda_ops as K
+    g = torch.Generator(device=DEV).manual_seed(T + pos0)
+    rand = lambda *shape: torch.randn(shape, device=DEV, generator=g)  # noqa: E731
+    n = pos0 + T
+    pages = (n + page - 1) // page
+    table = torch.randperm(pages + 3, device=DEV, generator=g)[:pages].to(torch.int32)
+    pools, scales, rows = [], [], []
+    for _ in range(2):
+        x = rand(pages + 3, nkv, page, 128)
+        s = None
+        if kvt == 1:
+            q = x.half()
+            d = q.double()
+        else:
+            top = 127 if kvt == 2 else 7
+            s = (x.abs().amax(-1) / top).contiguous()
+            c = (x / s[..., None]).round().clamp(-top, top)
+            d = c.double() * s.double()[..., None]
+            q = c.to(torch.int8) if kvt == 2 else ((c + 8).to(torch.uint8)[..., 0::2] | ((c + 8).to(torch.uint8)[..., 1::2] << 4))
+        rows.append(d[table.long()].transpose(1, 2).reshape(-1, nkv, 128)[:n])
+        if n % page:
+            (q if s is None else s)[int(table[-1]), :, n % page:] = float("nan")
+        pools.append(q.contiguous())
+        scales.append(s)
+    query = rand(T, nq, 128)
+    got = torch.full((T, nq * 128), float("nan"), dtype=torch.float16, device=DEV)
+    scratch = torch.empty(2 * nkv * 128 * ((n + 127) // 128 * 128), dtype=torch.float16, device=DEV)
+    K.attn_prefill(query, pos0, table, nq, nkv, 128, kvt, page, *pools, *scales, out=got, scratch=scratch)
+    hidden = torch.arange(n, device=DEV)[None] > pos0 + torch.arange(T, device=DEV)[:, None]
+    for h in range(nq):
+        score = query[:, h].double() @ rows[0][:, h * nkv // nq].T / math.sqrt(128)
+        p = score.masked_fill(hidden, -math.inf).softmax(-1)
+        v = rows[1][:, h * nkv // nq]
+        # f16 queries and rows move a score by at most 3 * 2^-11 of the sum of its products' magnitudes, f16 probabilities a weight by 2^-11
+        moved = (query[:, h].double().abs() @ rows[0][:, h * nkv // nq].abs().T / math.sqrt(128) * 3 * 2.0 ** -11).amax(-1, keepdim=True)
+        bound = (2 * moved + 2.0 ** -10) * (p @ v.abs()) + 2.0 ** -10 * (p @ v).abs() + 1e-6
+        assert ((got[:, K.paired_k_index(nq * 128, DEV)].double()[:, h * 128:(h + 1) * 128] - p @ v).abs() <= bound).all(), h
