@@ -271,7 +271,7 @@ __global__ void norm_to_f16_hmma_kernel(const float* __restrict__ x, int x_ld, c
   const float* xr = x + (size_t)blockIdx.x * x_ld;
   __half* orow = out + (size_t)blockIdx.x * out_ld;
   if (vec) {
-    norm_row_to_f16(xr, w, eps, K, orow, s32, [](int k) { return hmma_k_pos(k); });
+    norm_row_to_f16<K_HMMA>(xr, w, eps, K, orow, s32);
     return;
   }
   float inv = 1.0f;
@@ -360,8 +360,9 @@ int bonsai_bitgemm_hmma_tp(const void* comm, const void* codes, const void* scal
 int bonsai_norm_to_f16_hmma(const float* x, int x_ld, const float* w, float eps, int T, int K, void* out, int out_ld, cudaStream_t stream) {
   if (T < 1 || K % 128 != 0) return BONSAI_CUDA_BAD_ARG;
   // one block per token: a block as wide as the row allows keeps the two passes short (few tokens = few blocks)
-  const int threads = K >= 4096 ? 1024 : (K >= 2048 ? 512 : 256);
-  const int vec = (x_ld % 4 == 0) && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) % 16 == 0);   // 16-byte loads
+  const int threads = K >= 4096 ? 512 : 256;
+  const int vec = (x_ld % 4 == 0) && (out_ld % 2 == 0) && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) % 16 == 0) &&
+                  (reinterpret_cast<uintptr_t>(out) % 4 == 0);   // 16-byte loads, 4-byte stores
   const cudaError_t e = bonsai::launch_pdl(bonsai::norm_to_f16_hmma_kernel, dim3(T), dim3(threads), 0, stream, x, x_ld, w, eps, K, (__half*)out,
                                            out_ld, vec);
   return e == cudaSuccess ? BONSAI_CUDA_OK : BONSAI_CUDA_LAUNCH_FAILED;

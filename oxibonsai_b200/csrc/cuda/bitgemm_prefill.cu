@@ -719,8 +719,8 @@ __global__ void norm_to_f16_paired_kernel(const float* __restrict__ x, int x_ld,
   const float* xr = x + (size_t)tok * x_ld;
   __half* orow = out + (size_t)tok * out_ld;
   if (vec) {
-    if (natural) norm_row_to_f16(xr, w, eps, K, orow, s32, [](int k) { return k; });
-    else norm_row_to_f16(xr, w, eps, K, orow, s32, [](int k) { return paired_k(k); });
+    if (natural) norm_row_to_f16<K_NATURAL>(xr, w, eps, K, orow, s32);
+    else norm_row_to_f16<K_PAIRED>(xr, w, eps, K, orow, s32);
     return;
   }
   float inv = 1.0f;
@@ -886,8 +886,9 @@ int bonsai_norm_to_f16_paired(const float* x, int x_ld, const float* w, float ep
                               cudaStream_t stream) {
   if (T < 1 || K % 16 != 0) return BONSAI_CUDA_BAD_ARG;
   // one block per token; with few tokens (decode batches) a wide block keeps the two passes short
-  const int threads = T <= 128 ? (K >= 4096 ? 1024 : (K >= 2048 ? 512 : 256)) : 256;
-  const int vec = (x_ld % 4 == 0) && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) % 16 == 0);   // 16-byte loads
+  const int threads = T <= 128 ? (K >= 4096 ? 512 : 256) : 256;
+  const int vec = (x_ld % 4 == 0) && (out_ld % 8 == 0) &&
+                  ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(out)) % 16 == 0);   // 16-byte loads and stores
   const cudaError_t e = bonsai::launch_pdl(bonsai::norm_to_f16_paired_kernel, dim3(T), dim3(threads), 0, stream, x, x_ld, w, eps, K, (__half*)out,
                                            out_ld, natural, vec);
   return e == cudaSuccess ? BONSAI_CUDA_OK : BONSAI_CUDA_LAUNCH_FAILED;

@@ -46,48 +46,72 @@ __device__ __forceinline__ float block_sum(float v, float* smem32) {
   return t;
 }
 
-// One row: y = rmsnorm(x) * w (a plain copy when w is null), written as f16 at position pos(k) of the output row.
-// The row is read once with 16-byte loads and kept in registers between the sum of squares and the scaling (up to
-// 16 * blockDim.x elements; longer rows are read twice).  Needs 16-byte aligned rows and K % 4 == 0.
-template <class PosFn>
+// position of logical input k inside its 128-input group in the hmma-K order
+__host__ __device__ inline int hmma_k_pos(int k) {
+  const int r = k & 127, wq = r >> 4, e = r & 15;
+  const int c = wq >> 1, j = wq & 1, plane = e >> 3, p = e & 3, h = (e >> 2) & 1;
+  return (k & ~127) | ((j * 4 + p) * 16 + plane * 8 + 2 * c + h);
+}
+
+// One row: y = rmsnorm(x) * w (a plain copy when w is null) as f16 in the K order that the consumer reads.
+// A thread takes eight neighbouring inputs, so that every order stores whole words: in natural and paired-K order (inputs k and k + 4
+// of every eight side by side) they are one 16-byte word, in hmma-K order four pairs (k, k + 4).  The row is read once and kept in
+// registers between the sum of squares and the scaling (up to 16 * blockDim.x elements; longer rows are read twice).  Needs 16-byte
+// aligned rows and K % 8 == 0.
+enum KOrder { K_NATURAL = 0, K_PAIRED = 1, K_HMMA = 2 };
+template <int ORDER>
 __device__ __forceinline__ void norm_row_to_f16(const float* __restrict__ xr, const float* __restrict__ w, float eps, int K,
-                                                __half* __restrict__ orow, float* s32, PosFn pos) {
-  constexpr int kKeep = 4;
-  const int nch = K >> 2;
+                                                __half* __restrict__ orow, float* s32) {
+  constexpr int kKeep = 2;
+  const int nch = K >> 3;
   const float4* x4 = reinterpret_cast<const float4*>(xr);
-  float4 v[kKeep];
+  float4 v[kKeep][2];
   float ss = 0.0f;
 #pragma unroll
   for (int i = 0; i < kKeep; ++i) {
     const int c = threadIdx.x + i * blockDim.x;
-    v[i] = c < nch ? x4[c] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    ss += v[i].x * v[i].x + v[i].y * v[i].y + v[i].z * v[i].z + v[i].w * v[i].w;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      v[i][h] = c < nch ? x4[2 * c + h] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      ss += v[i][h].x * v[i][h].x + v[i][h].y * v[i][h].y + v[i][h].z * v[i][h].z + v[i][h].w * v[i][h].w;
+    }
   }
-  for (int c = threadIdx.x + kKeep * blockDim.x; c < nch; c += blockDim.x) {
-    const float4 t = x4[c];
-    ss += t.x * t.x + t.y * t.y + t.z * t.z + t.w * t.w;
-  }
+  for (int c = threadIdx.x + kKeep * blockDim.x; c < nch; c += blockDim.x)
+    for (int h = 0; h < 2; ++h) {
+      const float4 t = x4[2 * c + h];
+      ss += t.x * t.x + t.y * t.y + t.z * t.z + t.w * t.w;
+    }
   float inv = 1.0f;
   if (w != nullptr) {
     ss = block_sum(ss, s32);
     inv = 1.0f / sqrtf(ss / (float)K + eps);
   }
-  auto emit = [&](int c, float4 t) {
+  auto emit = [&](int c, float4 a, float4 b) {
     if (w != nullptr) {
-      const float4 ww = reinterpret_cast<const float4*>(w)[c];
-      t.x *= ww.x * inv; t.y *= ww.y * inv; t.z *= ww.z * inv; t.w *= ww.w * inv;
+      const float4 wa = reinterpret_cast<const float4*>(w)[2 * c], wb = reinterpret_cast<const float4*>(w)[2 * c + 1];
+      a.x *= wa.x * inv; a.y *= wa.y * inv; a.z *= wa.z * inv; a.w *= wa.w * inv;
+      b.x *= wb.x * inv; b.y *= wb.y * inv; b.z *= wb.z * inv; b.w *= wb.w * inv;
     }
-    orow[pos(4 * c)] = __float2half_rn(t.x);
-    orow[pos(4 * c + 1)] = __float2half_rn(t.y);
-    orow[pos(4 * c + 2)] = __float2half_rn(t.z);
-    orow[pos(4 * c + 3)] = __float2half_rn(t.w);
+    __align__(16) __half2 h[4];
+    if (ORDER == K_NATURAL) {
+      h[0] = __floats2half2_rn(a.x, a.y); h[1] = __floats2half2_rn(a.z, a.w); h[2] = __floats2half2_rn(b.x, b.y); h[3] = __floats2half2_rn(b.z, b.w);
+    } else {
+      h[0] = __floats2half2_rn(a.x, b.x); h[1] = __floats2half2_rn(a.y, b.y); h[2] = __floats2half2_rn(a.z, b.z); h[3] = __floats2half2_rn(a.w, b.w);
+    }
+    if (ORDER == K_HMMA) {
+      const int pos = hmma_k_pos(8 * c);
+#pragma unroll
+      for (int p = 0; p < 4; ++p) *reinterpret_cast<__half2*>(orow + pos + p * 16) = h[p];
+    } else {
+      *reinterpret_cast<uint4*>(orow + 8 * c) = *reinterpret_cast<const uint4*>(h);
+    }
   };
 #pragma unroll
   for (int i = 0; i < kKeep; ++i) {
     const int c = threadIdx.x + i * blockDim.x;
-    if (c < nch) emit(c, v[i]);
+    if (c < nch) emit(c, v[i][0], v[i][1]);
   }
-  for (int c = threadIdx.x + kKeep * blockDim.x; c < nch; c += blockDim.x) emit(c, x4[c]);
+  for (int c = threadIdx.x + kKeep * blockDim.x; c < nch; c += blockDim.x) emit(c, x4[2 * c], x4[2 * c + 1]);
 }
 
 // Dot of one packed word (16 ternary weights, scaled by 2^-63) with 16 floats.
@@ -101,13 +125,6 @@ __device__ __forceinline__ float dot_word16(uint32_t w, const float* x) {
     acc = fmaf(wb, x[8 + i], acc);
   }
   return acc;
-}
-
-// position of logical input k inside its 128-input group in the hmma-K order
-__host__ __device__ inline int hmma_k_pos(int k) {
-  const int r = k & 127, wq = r >> 4, e = r & 15;
-  const int c = wq >> 1, j = wq & 1, plane = e >> 3, p = e & 3, h = (e >> 2) & 1;
-  return (k & ~127) | ((j * 4 + p) * 16 + plane * 8 + 2 * c + h);
 }
 
 // Launch with programmatic dependent launch enabled: the kernel may start while its predecessor in
