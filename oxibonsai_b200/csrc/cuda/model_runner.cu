@@ -46,6 +46,7 @@ int bonsai_attn_decode_qkv_f16(const float*, int, const float*, const float*, fl
 int bonsai_norm_to_f16_hmma(const float*, int, const float*, float, int, int, void*, int, cudaStream_t);
 int bonsai_bitgemm_hmma(const void*, const void*, const void*, int, float*, const float*, void*, int, int, int, int, int, cudaStream_t);
 int bonsai_bitgemm_hmma_tp(const void*, const void*, const void*, const void*, int, float*, const float*, int, int, int, int, cudaStream_t);
+int bonsai_bitgemm_batch(const void*, const void*, const void*, int, float*, const float*, void*, int*, int, int, int, int, int, int, cudaStream_t);
 int bonsai_gemm_pair(const void*, const void*, int, float*, const float*, void*, int*, int, int, int, int, int, int, int, cudaStream_t);
 int bonsai_expand_rows(const void*, const void*, int, int, int, void*, cudaStream_t);
 int bonsai_attn_prefill_ws(const float*, int, int, const int*, int, int, int, int, int, const void*, const void*, const float*,
@@ -301,12 +302,15 @@ static int prefill_chunk(Runner& r, const uint64_t* sp, const uint64_t* pp, int 
   const int xn_ld = hidden > qd ? hidden : qd;
   const int* bt = P<int>(sp[SP_BLOCK_TABLE]) + (size_t)slot * r.ic[IC_MAX_PAGES];
 
-  // Chunks of up to 32 tokens (speculative verification, short prompts) run like a decode batch: the packed GEMMs on
-  // mma.sync with register-expanded weights (activations in hmma-K order) and, once the chunk's K/V rows are appended,
+  // Chunks of up to 32 tokens (speculative verification, short prompts) run like a decode batch: the packed GEMMs of one
+  // (on tensor-parallel ranks mma.sync with register-expanded weights, activations in hmma-K order) and, once the chunk's K/V rows are appended,
   // the split-KV decode attention with one "sequence" per token (all share the page list; token i sees positions
   // <= pos0 + i), which spreads a long context over the GPU where the prompt kernel would run one CTA per head.
   // Larger chunks use the tcgen05 GEMM (paired-K order) and the prompt attention kernel.
-  const bool hm = r.ic[IC_FAST] != 5 && T <= kSmallChunk && hidden % 128 == 0 && qd % 128 == 0 && inter % 128 == 0;
+  const bool small = r.ic[IC_FAST] != 5 && T <= kSmallChunk && hidden % 128 == 0 && qd % 128 == 0 && inter % 128 == 0;
+  // One GPU: the packed GEMMs of up to 64 tokens go through tensor memory (bitgemm_batch.cu, paired-K order).
+  const bool batch = !tp && T <= 64 && r.ic[IC_FAST] != 5;
+  const bool hm = small && !batch;
   // Tensor parallel, up to 16 tokens (a speculative verification pass): the row-parallel GEMMs exchange their partial sums
   // in the epilogue, as in the batched decode step, instead of GEMM + two-shot all-reduce (three more launches and two flag
   // barriers per exchange).
@@ -325,6 +329,7 @@ static int prefill_chunk(Runner& r, const uint64_t* sp, const uint64_t* pp, int 
                   int n_rows, int K, int epi, int out_ld) {
     if (T > 64 && wexp_elems >= (size_t)256 * K && (T >= kPairTokens || (size_t)n_rows * K <= wexp_elems))
       return pair_gemm(codes, scales, x, x_ld, out_f32, residual, out_f16, status, n_rows, K, T, epi, out_ld, sms, wexp, wexp_elems, st);
+    if (batch) return bonsai_bitgemm_batch(codes, scales, x, x_ld, out_f32, residual, out_f16, status, n_rows, K, T, epi, out_ld, 0, st);
     return hm ? bonsai_bitgemm_hmma(codes, scales, x, x_ld, out_f32, residual, out_f16, n_rows, K, T, epi, out_ld, st)
               : pf_gemm(r, codes, scales, x, x_ld, out_f32, residual, out_f16, status, n_rows, K, T, epi, out_ld, sms, nullptr, st);
   };
@@ -341,12 +346,13 @@ static int prefill_chunk(Runner& r, const uint64_t* sp, const uint64_t* pp, int 
                                   P<float>(r.gp[GP_ROPE_SIN]), positions, bt, 0, q, T, nq, nkv, hd, kvt,
                                   r.ic[IC_PAGE_SIZE], P<void>(pool.k), P<void>(pool.v), P<float>(pool.ks),
                                   P<float>(pool.vs), st));
-    if (hm) {
+    if (small) {
       float* attn32 = P<float>(pp[PP_SM_ATTN]);
       RC(bonsai_attn_decode(q, positions, bt, 0, T, nq, nkv, hd, kvt, r.ic[IC_PAGE_SIZE], P<void>(pool.k),
                             P<void>(pool.v), P<float>(pool.ks), P<float>(pool.vs), sm_splits, P<float>(pp[PP_SM_ACC]),
                             P<float>(pp[PP_SM_ML]), P<int>(pp[PP_SM_CTR]), attn32, 0, st));
-      RC(bonsai_norm_to_f16_hmma(attn32, qd, nullptr, r.eps, T, qd, attn, qd, st));
+      RC(hm ? bonsai_norm_to_f16_hmma(attn32, qd, nullptr, r.eps, T, qd, attn, qd, st)
+            : bonsai_norm_to_f16_paired(attn32, qd, nullptr, r.eps, T, qd, attn, qd, 0, st));
     } else {
       RC(bonsai_attn_prefill_ws(q, T, pos0, bt, nq, nkv, hd, kvt, r.ic[IC_PAGE_SIZE], P<void>(pool.k), P<void>(pool.v), P<float>(pool.ks),
                                 P<float>(pool.vs), attn, qd, 0, wexp, wexp_elems, st));
@@ -423,24 +429,25 @@ static int decode_step_batched(Runner& r, const uint64_t* sp, const uint64_t* pp
   r.gemm_ws = P<void>(pp[PP_GEMM_WS]);
   r.gemm_ws_bytes = (size_t)pp[PP_GEMM_WS_BYTES];
   const int xn_ld = hidden > qd ? hidden : qd;
-  // Small batches run the packed GEMMs on mma.sync with register-expanded weights (bitgemm_hmma.cu, activations in
-  // hmma-K order); the tcgen05 kernel (paired-K order) takes over where it measured faster.  QKV / O / gate-up / down
-  // of the 8B model in us: 8 tokens 15.7 / 8.3 / 24.6 / 20.9 against 17.8 / 17.6 / 32.8 / 24.7, 32 tokens 23.9 / 12.7 /
-  // 40.2 / 33.3 against 21.8 / 25.0 / 38.4 / 30.7, 64 tokens 39.6 / 20.6 / 66.0 / 51.7 against 26.3 / 26.1 / 43.4 / 39.0:
-  // everything up to 32 sequences, and the O projection (few rows, short K) up to 64.
+  // Tensor-parallel ranks run the packed GEMMs of small batches on mma.sync with register-expanded weights (bitgemm_hmma.cu,
+  // activations in hmma-K order; everything up to 32 sequences, the O projection up to 64), the tcgen05 kernel of bitgemm_prefill.cu
+  // (paired-K order) takes the larger ones.
   const bool hm_ok = r.ic[IC_FAST] != 5 && hidden % 128 == 0 && qd % 128 == 0 && inter % 128 == 0;
   // Tensor parallel, up to 16 sequences: the two row-parallel GEMMs carry the all-reduce + residual add in their epilogue
   // ({value, tag} messages).  That doubles the bytes on the wire, which is right while the exchange is latency-bound;
   // measured at 64 sequences (2 MB per peer per exchange) it lost to partial sums + the one-shot all-reduce kernel
   // (TP = 2: 7.3 against 6.2 ms per step), so larger batches keep that path.
   const bool tp_fused = tp && hm_ok && batch <= 16;
-  const bool hm_all = hm_ok && batch <= 32, hm_o = hm_ok && batch <= 64;
+  // One GPU: the packed GEMMs of up to 64 sequences go through tensor memory (bitgemm_batch.cu, paired-K order).
+  const bool tm = !tp && batch <= 64 && r.ic[IC_FAST] != 5;
+  const bool hm_all = !tm && hm_ok && batch <= 32, hm_o = !tm && hm_ok && batch <= 64;
   auto to_f16 = [&](bool hm, const float* src, int src_ld, const float* w, int K, void* dst, int dst_ld) {
     return hm ? bonsai_norm_to_f16_hmma(src, src_ld, w, r.eps, batch, K, dst, dst_ld, st)
               : bonsai_norm_to_f16_paired(src, src_ld, w, r.eps, batch, K, dst, dst_ld, 0, st);
   };
   auto gemm = [&](bool hm, const void* codes, const void* scales, const void* x, int x_ld, float* out_f32, const float* residual,
                   void* out_f16, int n_rows, int K, int epi, int out_ld) {
+    if (tm) return bonsai_bitgemm_batch(codes, scales, x, x_ld, out_f32, residual, out_f16, status, n_rows, K, batch, epi, out_ld, 0, st);
     return hm ? bonsai_bitgemm_hmma(codes, scales, x, x_ld, out_f32, residual, out_f16, n_rows, K, batch, epi, out_ld, st)
               : pf_gemm(r, codes, scales, x, x_ld, out_f32, residual, out_f16, status, n_rows, K, batch, epi, out_ld, sms, nullptr, st);
   };

@@ -751,7 +751,8 @@ def _gp():
     l = _pf()
     if not _gp_declared:
         declare({"bonsai_gemm_pair": [_vp, _vp, _i, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _vp],
-                 "bonsai_expand_rows": [_vp, _vp, _i, _i, _i, _vp, _vp]})
+                 "bonsai_expand_rows": [_vp, _vp, _i, _i, _i, _vp, _vp],
+                 "bonsai_bitgemm_batch": [_vp, _vp, _vp, _i, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _vp]})
         _gp_declared = True
     return l
 
@@ -761,6 +762,22 @@ def expand_rows(w: PlanarWeight, row0: int = 0, rows: int | None = None) -> torc
     rows = w.n - row0 if rows is None else rows
     out = torch.empty((rows, w.k), dtype=torch.float16, device=w.codes.device)
     check(_gp().bonsai_expand_rows(w.codes.data_ptr(), w.scales.data_ptr(), row0, rows, w.k, out.data_ptr(), stream()), "expand_rows")
+    return out
+
+
+def bitgemm_batch(w: PlanarWeight, x_paired: torch.Tensor, epi: int = 0, residual: torch.Tensor | None = None, out: torch.Tensor | None = None,
+                  status: torch.Tensor | None = None, split: int = 0) -> torch.Tensor:
+    """out[T, N] = epilogue(W x) for T <= 64 tokens, the expanded weights in tensor memory.  ``epi``: 0 f32 store, 1 f32 residual add, 2 f16
+    SwiGLU over interleaved gate / up rows (paired-K order).  ``split``: CTAs that share a tile's K range, 0 = chosen by size."""
+    T = x_paired.shape[0]
+    assert x_paired.dtype == torch.float16 and x_paired.shape[1] == w.k
+    if out is None:
+        out = torch.empty((T, (w.n // 2 + 7) // 8 * 8 if epi == 2 else w.n), dtype=torch.float32 if epi <= 1 else torch.float16, device=x_paired.device)
+    if status is None:
+        status = torch.zeros(1, dtype=torch.int32, device=x_paired.device)
+    check(_gp().bonsai_bitgemm_batch(w.codes.data_ptr(), w.scales.data_ptr(), x_paired.data_ptr(), x_paired.stride(0),
+                                     out.data_ptr() if epi <= 1 else None, ptr(residual), out.data_ptr() if epi == 2 else None,
+                                     status.data_ptr(), w.n, w.k, T, epi, out.stride(0), split, stream()), "bitgemm_batch")
     return out
 
 

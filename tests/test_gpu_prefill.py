@@ -242,3 +242,36 @@ def test_tensor_memory_prompt_attention(nq, nkv, T, pos0, kvt, page):
         moved = (query[:, h].double().abs() @ rows[0][:, h * nkv // nq].abs().T / math.sqrt(128) * 3 * 2.0 ** -11).amax(-1, keepdim=True)
         bound = (2 * moved + 2.0 ** -10) * (p @ v.abs()) + 2.0 ** -10 * (p @ v).abs() + 1e-6
         assert ((got[:, K.paired_k_index(nq * 128, DEV)].double()[:, h * 128:(h + 1) * 128] - p @ v).abs() <= bound).all(), h
+
+
+@pytest.mark.parametrize("ty", [TQ2_0_G128, Q1_0_G128])
+@pytest.mark.parametrize("rows,cols,T,split", [(1, 128, 1, 0), (128, 128, 16, 1), (130, 384, 17, 2), (144, 640, 33, 3), (272, 1152, 64, 8), (2560, 512, 9, 1), (20000, 256, 40, 2)])
+def test_batch_gemm_through_tensor_memory(ty, rows, cols, T, split):
+    """One block of inputs and fewer blocks than CTAs in a cluster, remainders of rows (128 per tile), of blocks (four per copy, six slots)
+    and of tokens (16, 32, 64), shares of the tokens that do not come out even, several tiles per cluster."""
+    from oxibonsai_b200.ops import cuda_ops as K
+    raw, dense = _random_quant(ty, rows, cols, rows + T)
+    w = K.PlanarWeight(rows, cols, torch.device(DEV))
+    w.fill_from_gguf(torch.from_numpy(np.array(raw, copy=True)).to(DEV), ty, cols, 0, rows)
+    g = torch.Generator(device=DEV).manual_seed(T)
+    x = torch.randn((T, cols), device=DEV, generator=g).half()
+    res = torch.randn((T, rows), device=DEV, generator=g)
+    paired = torch.empty_like(x)
+    paired[:, K.paired_k_index(cols, DEV)] = x
+    dense = dense.to(DEV).double()
+    want, terms = x.double() @ dense.T, x.double().abs() @ dense.abs().T
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    bound = 2.0 ** -23 * (cols + 16) * (terms + res.abs().double())      # products are exact in f32, sums may drop a last place each
+    a = K.bitgemm_batch(w, paired, 0, status=status, split=split)
+    b = K.bitgemm_batch(w, paired, 1, residual=res, status=status, split=split)
+    assert ((a.double() - want).abs() <= bound).all() and ((b.double() - want - res.double()).abs() <= bound).all()
+    assert torch.equal(a, K.bitgemm_batch(w, paired, 0, split=split))
+    if rows % 2 == 0:
+        gate, up = want[:, 0::2], want[:, 1::2]
+        act = torch.nn.functional.silu(gate) * up
+        wide = torch.zeros((T, (rows // 2 + 15) // 16 * 16), dtype=torch.float16, device=DEV)
+        K.bitgemm_batch(w, paired, 2, out=wide, status=status, split=split)
+        got = wide[:, K.paired_k_index(wide.shape[1], DEV)][:, :rows // 2].double()
+        slack = 1.1 * bound[:, 0::2] * up.abs() + gate.abs() * bound[:, 1::2] + (2.0 ** -11 + 2.0 ** -20) * act.abs() + 2.0 ** -24
+        assert ((got - act).abs() <= slack).all()
+    assert status.item() == 0
