@@ -687,6 +687,8 @@ int launch_decode_d(int dpl, int G, dim3 grid, size_t smem, cudaStream_t st, con
   }
 }
 
+int attn_decode_quant(const float*, const int*, const int*, int, int, int, int, int, int, const void*, const void*, const float*, const float*, int, float*,
+                      float*, int*, float*, int, float, cudaStream_t);
 int attn_decode_mma_f16(const float* q, const int* positions, const int* block_table, int max_pages, int batch, int nq, int nkv,
                         int page_size, const void* kpool, const void* vpool, int nsplit, float* ws_acc, float* ws_ml, int* counters,
                         float* out, int extra_len, float sm_scale, cudaStream_t stream);
@@ -742,6 +744,11 @@ int bonsai_attn_decode(const float* q, const int* positions, const int* block_ta
     // tensor-core path; it declines (BAD_ARG) shapes it does not cover and the CUDA-core kernels below take over
     const int rc = attn_decode_mma_f16(q, positions, block_table, max_pages, batch, nq, nkv, page_size, kpool, vpool, nsplit, ws_acc,
                                        ws_ml, counters, out, extra_len, sc, stream);
+    if (rc != BONSAI_CUDA_BAD_ARG) return rc;
+  }
+  if (hd == 128 && (kvt == KV_Q8 || kvt == KV_Q4) && !g_attn_force_cuda_cores) {
+    const int rc = attn_decode_quant(q, positions, block_table, max_pages, batch, nq, nkv, kvt, page_size, kpool, vpool, kscale, vscale, nsplit, ws_acc,
+                                     ws_ml, counters, out, extra_len, sc, stream);
     if (rc != BONSAI_CUDA_BAD_ARG) return rc;
   }
   if (hd == 128 && kvt != KV_F32 && (G == 1 || G == 2 || G == 4) && (page_size & (page_size - 1)) == 0) {

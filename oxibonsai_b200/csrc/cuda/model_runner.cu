@@ -12,6 +12,7 @@
 // Tensor parallelism: q/k/v and gate/up are column-parallel (local heads / local intermediate
 // rows), attn-output and down are row-parallel (local K slice).  With tp_size > 1 the row-parallel
 // GEMVs write partial sums and the fused all-reduce+residual kernel of csrc/comm combines them.
+#include <algorithm>
 #include <vector>
 
 #include "common.cuh"
@@ -132,6 +133,8 @@ static int qkv_attention_run(Runner& r, const uint64_t* lp, const uint64_t* sp, 
                                               P<void>(pool.k), P<void>(pool.v), nsplit, ws_acc, ws_ml, counters, attn, st);
     if (rc != BONSAI_CUDA_BAD_ARG) return rc;   // bad argument = not a shape of the fused kernel
   }
+  // INT8 / INT4 pages: the tensor-core kernel has two CTAs on an SM; more splits than fill those only add partial sums
+  if (n > 1 && (kvt == 2 || kvt == 3) && hd == 128) nsplit = std::max(1, std::min(nsplit, 2 * 148 / (nkv * n)));
   RC(bonsai_qknorm_rope_kvstore(qkv, qkv_n, P<float>(lp[LP_Q_NORM]), P<float>(lp[LP_K_NORM]), r.eps, P<float>(r.gp[GP_ROPE_COS]),
                                 P<float>(r.gp[GP_ROPE_SIN]), positions, bt, mp, q, n, nq, nkv, hd, kvt, r.ic[IC_PAGE_SIZE], P<void>(pool.k),
                                 P<void>(pool.v), P<float>(pool.ks), P<float>(pool.vs), st));

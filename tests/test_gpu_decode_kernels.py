@@ -373,3 +373,50 @@ def test_cluster_merge_of_decode_attention_matches_the_global_merge(nq, nkv, nsp
             sc = torch.einsum("hd,htd->ht", q[b], Kc.repeat_interleave(G, 0)) / hd ** 0.5
             ref = torch.einsum("ht,htd->hd", torch.softmax(sc, -1), Vc.repeat_interleave(G, 0))
             assert (got[b] - ref).abs().max().item() <= 4e-3 * max(1.0, ref.abs().max().item()), (lens, nsplit, b)
+
+
+@pytest.mark.parametrize("nq,nkv,nsplit", [(3, 3, 1), (4, 2, 3), (8, 2, 16), (8, 1, 2)])
+@pytest.mark.parametrize("kvt", [2, 3])
+def test_quantised_decode_attention_keeps_32_bit_queries_and_probabilities(nq, nkv, nsplit, kvt):
+    """Group sizes 1 to 8; contexts of one token, of a tile and one more, of many; row scales over six orders of magnitude, some zero,
+    growing along the context (the reference scale moves up); whatever lies behind the last key does not enter."""
+    import math
+    from oxibonsai_b200.ops import cuda_ops as K
+    g = torch.Generator(device=DEV).manual_seed(nq + nsplit)
+    rand = lambda *shape: torch.randn(shape, device=DEV, generator=g)  # noqa: E731
+    lens, page = [1, 16, 17, 333, 1500], 32
+    pages = [(n + page - 1) // page for n in lens]
+    table = torch.zeros((len(lens), max(pages)), dtype=torch.int32, device=DEV)
+    order, at = torch.randperm(sum(pages), device=DEV, generator=g).to(torch.int32), 0
+    for b, n in enumerate(pages):
+        table[b, :n] = order[at:at + n]
+        at += n
+    top = 127 if kvt == 2 else 7
+    pools, scales, values = [], [], []
+    for which in range(2):
+        x = rand(sum(pages), nkv, page, 128)
+        c = (x / x.abs().amax(-1, keepdim=True) * top).round()
+        s = x.abs().amax(-1) / top
+        if which == 1:
+            s = s * torch.exp(4 * rand(*s.shape))
+            for b, n in enumerate(lens):                     # larger and larger values
+                s[table[b, :pages[b]].long()] *= torch.logspace(-3, 0, pages[b] * page, device=DEV).view(pages[b], 1, page)
+            s[rand(*s.shape) > 2] = 0.0
+        pools.append((c.to(torch.int8) if kvt == 2 else ((c + 8).to(torch.uint8)[..., 0::2] | ((c + 8).to(torch.uint8)[..., 1::2] << 4))).contiguous())
+        values.append(c.double() * s.double()[..., None])
+        for b, n in enumerate(lens):
+            if n % page:
+                s[int(table[b, pages[b] - 1]), :, n % page:] = float("nan")
+        scales.append(s.contiguous())
+    q = rand(len(lens), nq, 128) * torch.exp(3 * rand(len(lens), nq, 1))
+    q[0, 0] = 0.0
+    pos = torch.tensor([n - 1 for n in lens], dtype=torch.int32, device=DEV)
+    got = K.attn_decode(q, pos, table, nq, nkv, 128, kvt, page, *pools, *scales, nsplit=nsplit)
+    for b, n in enumerate(lens):
+        k, v = (x[table[b, :pages[b]].long()].transpose(1, 2).reshape(-1, nkv, 128)[:n] for x in values)
+        for h in range(nq):
+            kh, vh, qh = k[:, h * nkv // nq], v[:, h * nkv // nq], q[b, h].double()
+            p = (kh @ qh / math.sqrt(128)).softmax(0)
+            # two f16 terms leave 2^-22 of an operand, a tile's sums some 2^-21: 2^-20 of a score's products, and of a weighted value
+            moved = 2.0 ** -20 * (kh.abs() @ qh.abs() / math.sqrt(128)).max()
+            assert ((got[b, h].double() - p @ vh).abs() <= (2 * moved + 2.0 ** -19) * (p @ vh.abs()) + 1e-30).all(), (b, h)
