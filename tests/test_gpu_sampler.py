@@ -113,3 +113,25 @@ def test_allow_mask_constrains_every_path():
         temps, topks, topps = torch.tensor([1.5], device=DEV), torch.tensor([k], dtype=torch.int32, device=DEV), torch.tensor([1.0], device=DEV)
         for _ in range(50):
             assert K.sample(lg, temps, topks, topps, rng, allow_mask=mask).item() in allowed
+
+
+@pytest.mark.parametrize("vocab,k,ties,masked", [(300, 299, False, False), (1025, 1, False, False), (4097, 1024, False, False), (5000, 40, True, False),
+                                                 (40001, 40, False, True), (40004, 200, True, True), (3000, 7, None, False), (70, 40, False, True)])
+def test_gathered_candidates_are_the_top_k(vocab, k, ties, masked):
+    """Rows shorter and longer than the block, odd rows, k from one to the block, ties at the threshold (by index), every entry equal (more
+    candidates than the block holds), masks that leave threads without an entry or fewer entries than k."""
+    from oxibonsai_b200.ops import cuda_ops as K
+    g = torch.Generator().manual_seed(vocab + k)
+    lg = torch.zeros((1, vocab)) if ties is None else torch.randn((1, vocab), generator=g) * 2
+    if ties:
+        lg = lg.round()
+    mask = torch.randint(-2 ** 31, 2 ** 31 - 1, (1, (vocab + 31) // 32), generator=g, dtype=torch.int32) if masked else None
+    rows = np.arange(vocab)
+    seen = rows if mask is None else rows[(mask[0].numpy()[rows >> 5].view(np.uint32) >> (rows & 31).astype(np.uint32)) & 1 == 1]
+    args = [torch.tensor([v], dtype=d, device=DEV) for v, d in ((0.9, torch.float32), (k, torch.int32), (0.95, torch.float32))]
+    rng, state = torch.tensor([99], dtype=torch.int64, device=DEV), 99
+    for _ in range(20):
+        tok = K.sample(lg.to(DEV), *args, rng, allow_mask=None if mask is None else mask.to(DEV)).item()
+        ref, state, allowed = _reference_sample(lg[0].numpy()[seen], 0.9, k, 0.95, state)
+        assert tok == seen[ref] and tok in seen[sorted(allowed)]
+        assert (rng.item() & ((1 << 64) - 1)) == state
