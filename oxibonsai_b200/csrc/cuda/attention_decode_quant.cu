@@ -6,8 +6,8 @@
 //   * codes are exact in f16; a pair of them comes out of a packed word with a byte or nibble shuffle under an exponent and one exact HADD2;
 //   * a query and a probability are two f16 terms, x = hi + lo (22 bits): the group's heads are rows 0..G-1 of the first operand as hi
 //     and rows 8..8+G-1 as lo, rows that the instruction computes anyway, and the two sums meet in one lane;
-//   * a head's queries are scaled by a power of two to [2^7, 2^8), a probability times its row's scale by the power of two that brings the
-//     largest scale so far to [1, 2), and by 2^14: neither leaves the range in which the two terms hold 22 bits;
+//   * a head's queries are scaled by a power of two to [2^7, 2^8), its probabilities times their rows' scales, tile by tile, to [2^14, 2^15):
+//     neither leaves the range in which the two terms hold 22 bits;
 //   * the dimensions and tokens of a tile may come in any order as long as both operands agree, so that every lane loads whole 16-byte
 //     words of the rows straight into registers, a tile ahead.
 // Scores, maxima, sums and accumulators are f32; the error against 64 bits is that of the CUDA-core kernel (2.7e-7 over 64 sequences of
@@ -68,7 +68,10 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? 1 : 2) attn_decode_quant_ke
   asm volatile("griddepcontrol.wait;" ::: "memory");
   const int len = p.positions[b] + 1 + p.extra_len;
   int chunk = (len + nsplit - 1) / nsplit;
-  chunk = (chunk + 15) & ~15;               // tiles of 16 never straddle a split or (page_size is a multiple of 16) a page
+  // Tiles of 16 never straddle a split or (page_size is a multiple of 16) a page, and a split has a tile for each of its warps at least;
+  // splits that are left without tokens leave, and a single part needs no merge.
+  chunk = max((chunk + 15) & ~15, NW * 16);
+  if (split * chunk >= len) return;
   const int t0 = split * chunk, t1 = min(len, t0 + chunk), ntiles = t1 > t0 ? (t1 - t0 + 15) >> 4 : 0;
   const int* bt = p.block_table + (size_t)b * p.max_pages;
   const int pshift = 31 - __clz(p.page_size), pmask = p.page_size - 1;
@@ -136,7 +139,7 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? 1 : 2) attn_decode_quant_ke
   float o[16][2];          // dimensions 32 c + i and 32 c + 16 + i of head `row`
 #pragma unroll
   for (int i = 0; i < 16; ++i) o[i][0] = o[i][1] = 0.0f;
-  float m = -INFINITY, l = 0.0f, ref = 0.0f;      // ref: power of two at or below the largest value scale so far, the same in all lanes
+  float m = -INFINITY, l = 0.0f;
 
   for (int j = warp; j < ntiles; j += NW) {
     Tile nxt;
@@ -169,17 +172,6 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? 1 : 2) attn_decode_quant_ke
     }
     // ---- softmax; the scales of tokens 8 n + 2c + e ----------------------------------------------------------------------------------------
     const int tb = t0 + j * 16;
-    float top = lane < 16 ? 0.0f : cur.s;
-#pragma unroll
-    for (int x = 8; x > 0; x >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, x));
-    top = __shfl_sync(0xffffffffu, top, 16);
-    float fit = 1.0f;                                    // what a grown reference takes off the sums so far
-    if (top > 2.0f * ref || ref == 0.0f) {
-      const float to = top < 1e30f ? qa_pow2(fmaxf(top, 1e-30f)) : 1.0f;
-      fit = ref / to;
-      ref = to;
-    }
-    const float inv_ref = 16384.0f / ref;
     float pr[2][2], mx = m;
 #pragma unroll
     for (int n = 0; n < 2; ++n)
@@ -193,29 +185,32 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? 1 : 2) attn_decode_quant_ke
     mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
     mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
     const float down = mx == -INFINITY ? 1.0f : expf(m - mx);
-    float ps = 0.0f;
-    uint32_t pa[4];
+    float ps = 0.0f, x[2][2], top = 0.0f;
 #pragma unroll
-    for (int n = 0; n < 2; ++n) {
-      float x[2];
+    for (int n = 0; n < 2; ++n)
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
         const float vs = __shfl_sync(0xffffffffu, cur.s, 16 + 8 * n + 2 * c + e);
         const float pe = mx == -INFINITY ? 0.0f : expf(pr[n][e] - mx);
         ps += pe;
-        x[e] = pe * (vs * inv_ref);
+        x[n][e] = pe * vs;
+        top = fmaxf(top, x[n][e]);
       }
-      qa_split(x[0], x[1], pa[2 * n], pa[2 * n + 1]);
-    }
+    top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 1));
+    top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 2));
+    // the head's largest weight of the tile comes to [2^14, 2^15); weights below 2^-110 lose digits
+    const float unit = top < 1e30f ? qa_pow2(fmaxf(top, 7.8e-34f)) * (1.0f / 16384.0f) : 1.0f, up = 1.0f / unit;
+    uint32_t pa[4];
+#pragma unroll
+    for (int n = 0; n < 2; ++n) qa_split(x[n][0] * up, x[n][1] * up, pa[2 * n], pa[2 * n + 1]);
     l = l * down + ps;
     m = mx;
     // a tile's product starts from zero (the tensor core would truncate a long running sum); its hi and lo rows are in one lane
-    const float keep = down * fit;
     auto add = [&](int i, uint32_t b0, uint32_t b1) {
       float t[4] = {0.0f, 0.0f, 0.0f, 0.0f};
       qa_mma(t, pa, b0, b1);
-      o[i][0] = fmaf(o[i][0], keep, t[0] + t[2]);
-      o[i][1] = fmaf(o[i][1], keep, t[1] + t[3]);
+      o[i][0] = fmaf(t[0] + t[2], unit, o[i][0] * down);
+      o[i][1] = fmaf(t[1] + t[3], unit, o[i][1] * down);
     };
     // ---- O += P V: MMA i has, in column `row`, dimension 16 row + i -------------------------------------------------------------------------------
     {
@@ -250,16 +245,16 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? 1 : 2) attn_decode_quant_ke
   }
   l += __shfl_xor_sync(0xffffffffu, l, 1);
   l += __shfl_xor_sync(0xffffffffu, l, 2);
+  const int parts = (len + chunk - 1) / chunk;
 
   // ---- the CTA's warps, then the splits: as in attention_decode.cu ------------------------------------------------------------------------------
   constexpr int stride = hd + 2;
   if (row < G) {
     float* dst = qa_sh + ((size_t)warp * G + row) * stride;
-    const float unit = ref * (1.0f / 16384.0f);
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
-      dst[32 * c + i] = o[i][0] * unit;
-      dst[32 * c + 16 + i] = o[i][1] * unit;
+      dst[32 * c + i] = o[i][0];
+      dst[32 * c + 16 + i] = o[i][1];
     }
     if (c == 0) {
       dst[hd] = m;
@@ -281,19 +276,19 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? 1 : 2) attn_decode_quant_ke
       L += f * src[hd + 1];
     }
     const size_t head = (size_t)b * p.nq + kvh * G + g;
-    if (nsplit == 1) {
+    if (parts == 1) {
       p.out[head * hd + d] = L > 0.0f ? a / L : 0.0f;
     } else {
       p.ws_acc[(head * nsplit + split) * hd + d] = a;
       if (d == 0) *reinterpret_cast<float2*>(p.ws_ml + (head * nsplit + split) * 2) = make_float2(M, L);
     }
   }
-  if (nsplit == 1) return;
+  if (parts == 1) return;
   __threadfence();
   __syncthreads();
   if (threadIdx.x == 0) {
     int* ctr = p.counters + (size_t)b * p.nkv + kvh;
-    s_last = atomicAdd(ctr, 1) == nsplit - 1;
+    s_last = atomicAdd(ctr, 1) == parts - 1;
     if (s_last) *ctr = 0;
   }
   __syncthreads();
@@ -306,20 +301,20 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? 1 : 2) attn_decode_quant_ke
     const float* ac = p.ws_acc + head * nsplit * hd + d;
     // eight splits per step, all of a step's loads before the first use
     float M = -INFINITY;
-    for (int s0 = 0; s0 < nsplit; s0 += 8) {
+    for (int s0 = 0; s0 < parts; s0 += 8) {
       float x[8];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) x[i] = s0 + i < nsplit ? __ldcg(ml + s0 + i).x : -INFINITY;
+      for (int i = 0; i < 8; ++i) x[i] = s0 + i < parts ? __ldcg(ml + s0 + i).x : -INFINITY;
 #pragma unroll
       for (int i = 0; i < 8; ++i) M = fmaxf(M, x[i]);
     }
     float a = 0.0f, L = 0.0f;
-    for (int s0 = 0; s0 < nsplit; s0 += 8) {
+    for (int s0 = 0; s0 < parts; s0 += 8) {
       float2 x[8];
       float y[8];
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
-        const bool ok = s0 + i < nsplit;
+        const bool ok = s0 + i < parts;
         x[i] = ok ? __ldcg(ml + s0 + i) : make_float2(-INFINITY, 0.0f);
         y[i] = ok ? __ldcg(ac + (size_t)(s0 + i) * hd) : 0.0f;
       }

@@ -379,8 +379,9 @@ def test_cluster_merge_of_decode_attention_matches_the_global_merge(nq, nkv, nsp
 @pytest.mark.parametrize("kvt", [2, 3])
 def test_quantised_decode_attention_keeps_32_bit_queries_and_probabilities(nq, nkv, nsplit, kvt):
     """Group sizes 1 to 8; contexts of one token, of a tile and one more, of many; row scales over six orders of magnitude, some zero,
-    growing along the context (the reference scale moves up); whatever lies behind the last key does not enter."""
+    growing along the context; whatever lies behind the last key does not enter."""
     import math
+    DEV = _dev()
     from oxibonsai_b200.ops import cuda_ops as K
     g = torch.Generator(device=DEV).manual_seed(nq + nsplit)
     rand = lambda *shape: torch.randn(shape, device=DEV, generator=g)  # noqa: E731
@@ -419,4 +420,7 @@ def test_quantised_decode_attention_keeps_32_bit_queries_and_probabilities(nq, n
             p = (kh @ qh / math.sqrt(128)).softmax(0)
             # two f16 terms leave 2^-22 of an operand, a tile's sums some 2^-21: 2^-20 of a score's products, and of a weighted value
             moved = 2.0 ** -20 * (kh.abs() @ qh.abs() / math.sqrt(128)).max()
-            assert ((got[b, h].double() - p @ vh).abs() <= (2 * moved + 2.0 ** -19) * (p @ vh.abs()) + 1e-30).all(), (b, h)
+            # a weight below 2^-17 of its tile's largest is held to 2^-39 of that one instead, times codes up to 127 and sixteen tokens
+            small = 2.0 ** -28 * (p @ vh.abs()).max()
+            worst = ((got[b, h].double() - p @ vh).abs() / ((2 * moved + 2.0 ** -19) * (p @ vh.abs()) + small + 1e-30)).max().item()
+            assert worst <= 1.0, (b, h, worst, moved.item(), (p @ vh.abs()).min().item())
