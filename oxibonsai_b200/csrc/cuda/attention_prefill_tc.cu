@@ -156,10 +156,10 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_prefill_tc_kernel(const __
   } else if (warp == 9) {
     const uint32_t ids = tc::idesc_f32acc(tc::FMT_F16, tc::FMT_F16, 128, 128), idv = ids | (1u << 16);
     for (int j = 0; j <= n1 && !failed; ++j) {
-      if (j < n1 && !tc::mbar_wait_warp<0>(&k_full[j & 1], (j >> 1) & 1, lane)) { failed = true; break; }
+      if (j < n1 && !__all_sync(0xffffffffu, tc::mbar_wait(&k_full[j & 1], (j >> 1) & 1))) { failed = true; break; }
       if (j > 0) {
         const int i = j - 1;
-        if (!tc::mbar_wait_warp<0>(&v_full[i & 1], (i >> 1) & 1, lane)) { failed = true; break; }
+        if (!__all_sync(0xffffffffu, tc::mbar_wait(&v_full[i & 1], (i >> 1) & 1))) { failed = true; break; }
         if (i * 128 + 128 > total) {      // rows behind the last key may hold anything; 0 x anything has to be 0
           uint8_t* v = sV + (i & 1) * kAtTile;
           for (int r = (total & 127) * 16 + lane; r < 128 * 16; r += 32)
@@ -171,7 +171,7 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_prefill_tc_kernel(const __
       for (int u = 0; u < 2; ++u) {
         const int n = u ? n1 : n0;
         if (j > 0 && j <= n) {
-          if (!tc::mbar_wait_warp<0>(&p_ready[u], (j - 1) & 1, lane)) { failed = true; break; }
+          if (!__all_sync(0xffffffffu, tc::mbar_wait(&p_ready[u], (j - 1) & 1))) { failed = true; break; }
           tc::tc_fence_after();
           if (tc::elect_one()) {
             const uint64_t dv = at_desc_v(tc::smem_u32(sV + ((j - 1) & 1) * kAtTile));
@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_prefill_tc_kernel(const __
     const int first_masked = (p.pos0 + tok_first + u * TOK + 1) >> 7;       // tiles from here on hold keys that some row does not see
     float m = 0.0f, l = 0.0f;
     for (int j = 0; j < n; ++j) {
-      if (!tc::mbar_wait_warp<0>(&s_full[u], j & 1, lane)) { failed = true; break; }
+      if (!__all_sync(0xffffffffu, tc::mbar_wait(&s_full[u], j & 1))) { failed = true; break; }
       tc::tc_fence_after();
       float s[128];
 #pragma unroll

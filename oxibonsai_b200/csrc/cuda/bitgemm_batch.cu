@@ -16,10 +16,10 @@
 // The K range of a 128-row tile is cut over the S CTAs of a cluster, so that projections with few rows fill the GPU too; each CTA
 // then adds up, in CTA order, the partial sums of its share of the tokens, which the others wrote into its shared memory.  A cluster
 // takes tile after tile; the accumulators and the exchange are double-buffered.
-// What bounds it: the expanders' chain of wait, expansion and store, some 0.26 us per 16 K weights and SM (1.5 instructions per weight for
-// shift, mask and scale would allow 0.12), and about 5 us per launch.  us at 4 / 16 / 32 / 64 tokens (before: the better of bitgemm_hmma and
-// bitgemm_prefill): 6144 x 4096 10.5 / 11.2 / 12.9 / 16.5 (16.0 / 16.7 / 20.7 / 24.0), 4096 x 4096 9.5 / 10.1 / 11.8 / 14.6 (8.4 / 9.0 / 13.3 /
-// 22.1), 24576 x 4096 21.6 / 22.6 / 26.5 / 40.1 (24.5 / 25.4 / 38.3 / 44.7), 4096 x 12288 15.1 / 15.5 / 16.6 / 19.0 (21.4 / 23.0 / 31.5 / 43.3).
+// What bounds it: the expanders' chain of wait, expansion and store, some 0.23 us per 16 K weights and SM (1.5 instructions per weight for
+// shift, mask and scale would allow 0.12), and about 5 us per launch.  us at 8 / 32 / 64 tokens (before: the better of bitgemm_hmma and
+// bitgemm_prefill): 6144 x 4096 10.2 / 12.1 / 15.7 (16.0 / 20.7 / 24.0), 4096 x 4096 9.3 / 11.2 / 14.1 (8.4 / 13.3 / 22.1), 24576 x 4096
+// 19.6 / 25.1 / 36.2 (24.5 / 38.3 / 44.7), 4096 x 12288 13.8 / 15.2 / 17.5 (21.4 / 31.5 / 41.1).
 #include <cuda.h>
 #include <cuda_fp16.h>
 
@@ -209,7 +209,7 @@ __global__ void __launch_bounds__(kGbThreads, 1) bitgemm_batch_kernel(const __gr
     }
     __syncwarp();
   } else if (warp < kGbEpiWarp) {
-    // thread = weight row of the tile
+    // thread = weight row of the tile; all lanes poll (one that passes the outcome on is a shuffle later: 24576 x 4096, 8 tokens 22.3 against 19.6 us)
     const int group = warp >> 2, r = t & 127;
     const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
     auto scale_of = [&](int tile, int kb) {
@@ -221,7 +221,7 @@ __global__ void __launch_bounds__(kGbThreads, 1) bitgemm_batch_kernel(const __gr
     __half next = scale_of(cid, group);         // scale of this group's next block, requested a block ahead
     for (int tile = cid; tile < row_tiles && !failed; tile += nclusters, it0 += nb) {
       for (int kb0 = 0; kb0 < nb && !failed; kb0 += 4) {
-        if (!tc::mbar_wait_warp<0>(&c_full[cs], cphase, lane)) { failed = true; break; }
+        if (!__all_sync(0xffffffffu, tc::mbar_wait(&c_full[cs], cphase))) { failed = true; break; }
         const int end = min(kb0 + 4, nb);
         for (int kb = kb0 + (group + 3 - (it0 + kb0) % 3) % 3; kb < end; kb += 3) {
           const int it = it0 + kb, s = it % kGbSlots;
@@ -242,7 +242,7 @@ __global__ void __launch_bounds__(kGbThreads, 1) bitgemm_batch_kernel(const __gr
                 o[wd * 8 + 4 + i] = *reinterpret_cast<const uint32_t*>(&hb);
               }
             if (h == 0) {
-              if (!tc::mbar_wait_warp<0>(&empty[s], ((it / kGbSlots) & 1) ^ 1, lane)) { failed = true; break; }
+              if (!__all_sync(0xffffffffu, tc::mbar_wait(&empty[s], ((it / kGbSlots) & 1) ^ 1))) { failed = true; break; }
               tc::tc_fence_after();
             }
             gb_st32(taddr + lanes + s * 64 + h * 32, o);
