@@ -108,8 +108,12 @@ __global__ void __launch_bounds__(NW * 32, 8 / NW) attn_decode_mma_kernel(MmaAtt
   if (p.qkv == nullptr) asm volatile("griddepcontrol.wait;" ::: "memory");
   const int len = p.positions[b] + 1 + p.extra_len;
   int chunk = (len + nsplit - 1) / nsplit;
-  chunk = (chunk + kMmaTile - 1) & ~(kMmaTile - 1);   // tiles never straddle a split boundary or (page_size >= 16) a page
+  // Tiles never straddle a split boundary or (page_size >= 16) a page, and a split has at least a tile for each of its warps: more splits
+  // would only lengthen the merge.  Those that are left without tokens (parts .. nsplit - 1) leave, a single part needs no merge
+  // (16 splits: 24 tokens of 16 / 8 heads 6.3 -> 4.1 us; 14 splits: five sequences of 90 to 700 12.7 -> 9.7 us).
+  chunk = max((chunk + kMmaTile - 1) & ~(kMmaTile - 1), kMmaTile * NW);
   const int t0 = split * chunk, t1 = min(len, t0 + chunk);
+  if (!CL && t0 >= len) return;
   const int ntiles = t1 > t0 ? (t1 - t0 + kMmaTile - 1) / kMmaTile : 0;
   const int* bt = p.block_table + (size_t)b * p.max_pages;
   const int pshift = 31 - __clz(p.page_size), pmask = p.page_size - 1;
@@ -255,6 +259,7 @@ __global__ void __launch_bounds__(NW * 32, 8 / NW) attn_decode_mma_kernel(MmaAtt
     __syncwarp();   // every lane is done with this buffer before the next iteration's copies overwrite it
   }
   cp_async_wait<0>();
+  const int parts = (len + chunk - 1) / chunk;      // a division: not on the way to the first tile
   l += __shfl_xor_sync(0xffffffffu, l, 1);
   l += __shfl_xor_sync(0xffffffffu, l, 2);
 
@@ -285,7 +290,7 @@ __global__ void __launch_bounds__(NW * 32, 8 / NW) attn_decode_mma_kernel(MmaAtt
     float* merge = sh + (size_t)kMmaWarps * G * stride;         // [nsplit][G][hd + 2], used in CTA 0 only
     float* lead = cluster.map_shared_rank(merge, 0);
     asm volatile("barrier.cluster.wait.aligned;" ::: "memory");   // the arrival at the top of the kernel: every CTA runs
-    for (int idx = threadIdx.x; idx < G * hd; idx += blockDim.x) {
+    for (int idx = (int)rank < parts ? threadIdx.x : G * hd; idx < G * hd; idx += blockDim.x) {
       const int g = idx / hd, d = idx - g * hd;
       float M = -INFINITY;
 #pragma unroll
@@ -311,11 +316,11 @@ __global__ void __launch_bounds__(NW * 32, 8 / NW) attn_decode_mma_kernel(MmaAtt
     float* s_f = sh;                                            // [G][nsplit] normalised weights of the splits
     for (int g = warp; g < G; g += kMmaWarps) {
       float M = -INFINITY;
-      for (int sp = lane; sp < nsplit; sp += 32) M = fmaxf(M, merge[((size_t)sp * G + g) * stride + hd]);
+      for (int sp = lane; sp < parts; sp += 32) M = fmaxf(M, merge[((size_t)sp * G + g) * stride + hd]);
 #pragma unroll
       for (int o2 = 16; o2 > 0; o2 >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o2));
       float L = 0.0f;
-      for (int sp = lane; sp < nsplit; sp += 32) {
+      for (int sp = lane; sp < parts; sp += 32) {
         const float ms = merge[((size_t)sp * G + g) * stride + hd];
         const float f = (ms == -INFINITY) ? 0.0f : __expf(ms - M);
         L += f * merge[((size_t)sp * G + g) * stride + hd + 1];
@@ -325,14 +330,14 @@ __global__ void __launch_bounds__(NW * 32, 8 / NW) attn_decode_mma_kernel(MmaAtt
       for (int o2 = 16; o2 > 0; o2 >>= 1) L += __shfl_xor_sync(0xffffffffu, L, o2);
       const float inv = L > 0.0f ? 1.0f / L : 0.0f;
       __syncwarp();
-      for (int sp = lane; sp < nsplit; sp += 32) s_f[g * nsplit + sp] *= inv;
+      for (int sp = lane; sp < parts; sp += 32) s_f[g * nsplit + sp] *= inv;
     }
     __syncthreads();
     const size_t hb = (size_t)b * p.nq + kvh * G;
     for (int idx = threadIdx.x; idx < G * hd; idx += blockDim.x) {
       const int g = idx / hd, d = idx - g * hd;
       float a = 0.0f;
-      for (int sp = 0; sp < nsplit; ++sp) a += s_f[g * nsplit + sp] * merge[((size_t)sp * G + g) * stride + d];
+      for (int sp = 0; sp < parts; ++sp) a += s_f[g * nsplit + sp] * merge[((size_t)sp * G + g) * stride + d];
       p.out[hb * hd + idx] = a;
     }
     return;
@@ -351,18 +356,23 @@ __global__ void __launch_bounds__(NW * 32, 8 / NW) attn_decode_mma_kernel(MmaAtt
       L += f * src[hd + 1];
     }
     const size_t oi = (((size_t)b * p.nq + kvh * G + g) * nsplit + split);
+    if (parts == 1) {
+      p.out[((size_t)b * p.nq + kvh * G + g) * hd + d] = L > 0.0f ? a / L : 0.0f;
+      continue;
+    }
     p.ws_acc[oi * hd + d] = a;
     if (d == 0) {
       p.ws_ml[oi * 2] = M;
       p.ws_ml[oi * 2 + 1] = L;
     }
   }
+  if (parts == 1) return;
   __threadfence();
   __syncthreads();
   if (threadIdx.x == 0) {
     int* ctr = p.counters + (size_t)b * p.nkv + kvh;
     const int prev = atomicAdd(ctr, 1);
-    s_last = (prev == nsplit - 1);
+    s_last = (prev == parts - 1);
     if (s_last) *ctr = 0;
   }
   __syncthreads();
@@ -382,11 +392,11 @@ __global__ void __launch_bounds__(NW * 32, 8 / NW) attn_decode_mma_kernel(MmaAtt
       const int idx = min((int)threadIdx.x + k * kMmaWarps * 32, G * hd - 1);
 #pragma unroll
       for (int i = 0; i < SB; ++i)
-        av[k][i] = sp0 + i < nsplit ? __ldcg(p.ws_acc + ((hb0 + idx / hd) * nsplit + sp0 + i) * hd + (idx % hd)) : 0.0f;
+        av[k][i] = sp0 + i < parts ? __ldcg(p.ws_acc + ((hb0 + idx / hd) * nsplit + sp0 + i) * hd + (idx % hd)) : 0.0f;
     }
   };
   load_acc(0);
-  for (int i = threadIdx.x; i < G * nsplit; i += blockDim.x) {
+  for (int i = threadIdx.x; i < G * nsplit; i += blockDim.x) {      // behind `parts`: old values, not used
     const float2 v = __ldcg(reinterpret_cast<const float2*>(p.ws_ml) + hb0 * nsplit + i);
     s_f[i] = v.x;
     s_l[i] = v.y;
@@ -394,11 +404,11 @@ __global__ void __launch_bounds__(NW * 32, 8 / NW) attn_decode_mma_kernel(MmaAtt
   __syncthreads();
   for (int g = warp; g < G; g += kMmaWarps) {   // one warp per query head of the group
     float M = -INFINITY;
-    for (int sp = lane; sp < nsplit; sp += 32) M = fmaxf(M, s_f[g * nsplit + sp]);
+    for (int sp = lane; sp < parts; sp += 32) M = fmaxf(M, s_f[g * nsplit + sp]);
 #pragma unroll
     for (int o2 = 16; o2 > 0; o2 >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o2));
     float L = 0.0f;
-    for (int sp = lane; sp < nsplit; sp += 32) {
+    for (int sp = lane; sp < parts; sp += 32) {
       const float ms = s_f[g * nsplit + sp];
       const float f = (ms == -INFINITY) ? 0.0f : __expf(ms - M);
       L += f * s_l[g * nsplit + sp];
@@ -408,19 +418,19 @@ __global__ void __launch_bounds__(NW * 32, 8 / NW) attn_decode_mma_kernel(MmaAtt
     for (int o2 = 16; o2 > 0; o2 >>= 1) L += __shfl_xor_sync(0xffffffffu, L, o2);
     const float inv = L > 0.0f ? 1.0f / L : 0.0f;
     __syncwarp();
-    for (int sp = lane; sp < nsplit; sp += 32) s_f[g * nsplit + sp] *= inv;
+    for (int sp = lane; sp < parts; sp += 32) s_f[g * nsplit + sp] *= inv;
   }
   __syncthreads();
   float a[NI];
 #pragma unroll
   for (int k = 0; k < NI; ++k) a[k] = 0.0f;
-  for (int sp0 = 0; sp0 < nsplit; sp0 += SB) {
+  for (int sp0 = 0; sp0 < parts; sp0 += SB) {
     if (sp0 > 0) load_acc(sp0);
 #pragma unroll
     for (int k = 0; k < NI; ++k) {
       const int idx = min((int)threadIdx.x + k * kMmaWarps * 32, G * hd - 1);
 #pragma unroll
-      for (int i = 0; i < SB; ++i) a[k] += (sp0 + i < nsplit ? s_f[(idx / hd) * nsplit + sp0 + i] : 0.0f) * av[k][i];
+      for (int i = 0; i < SB; ++i) a[k] += (sp0 + i < parts ? s_f[(idx / hd) * nsplit + sp0 + i] : 0.0f) * av[k][i];
     }
   }
 #pragma unroll
