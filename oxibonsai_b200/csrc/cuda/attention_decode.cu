@@ -698,7 +698,7 @@ static int g_attn_force_cuda_cores = 0;
 
 extern "C" {
 
-// 1: f16 caches with head_dim 128 use the CUDA-core kernel instead of the tensor-core one (comparisons, tests)
+// 1: f16, INT8 and INT4 caches with head_dim 128 use the CUDA-core kernel instead of the tensor-core ones (comparisons, tests)
 void bonsai_attn_decode_force_cuda_cores(int on) { bonsai::g_attn_force_cuda_cores = on; }
 
 // qkv: f32 [batch][qkv_stride] holding q | k | v heads.  Writes normalised+rotated q to q_out
@@ -741,7 +741,7 @@ int bonsai_attn_decode(const float* q, const int* positions, const int* block_ta
   if (smem > 48 * 1024) return BONSAI_CUDA_BAD_ARG;
   float sc = 1.0f / sqrtf((float)hd);
   if (hd == 128 && kvt == KV_F16 && !g_attn_force_cuda_cores) {
-    // tensor-core path; it declines (BAD_ARG) shapes it does not cover and the CUDA-core kernels below take over
+    // tensor-core paths; they decline (BAD_ARG) shapes that they do not cover and the CUDA-core kernels below take over
     const int rc = attn_decode_mma_f16(q, positions, block_table, max_pages, batch, nq, nkv, page_size, kpool, vpool, nsplit, ws_acc,
                                        ws_ml, counters, out, extra_len, sc, stream);
     if (rc != BONSAI_CUDA_BAD_ARG) return rc;

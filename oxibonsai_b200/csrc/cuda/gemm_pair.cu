@@ -15,7 +15,9 @@
 //
 // Packed weights (planar layout, common.cuh) are expanded to f16 once per prompt chunk, slab by slab into one scratch matrix that
 // stays in L2, in the paired-K order that the activations have.  Expanding inside the GEMM instead repeats the work for every 256
-// tokens and holds the tensor core to half its rate; measured figures at bonsai_bitgemm_pair.
+// tokens and holds the tensor core to half its rate.  4096 x 4096, dense, 4096 tokens: 124 us with the single-SM tile, 104 here
+// (1.32 PFLOP/s); 6144 x 4096 packed, 192 tokens: 44 us in place, 25 expanded first.  Issued by elected threads: 53 us instead of 17 for 64
+// blocks behind `lane == 0`.
 #include <cuda.h>
 #include <cuda_fp16.h>
 

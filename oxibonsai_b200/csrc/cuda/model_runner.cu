@@ -246,7 +246,7 @@ enum PrefillPtr {
   PP_COUNT
 };
 
-// Chunks of at most this many tokens run like a decode batch (mma.sync GEMMs, split-KV attention); the small-chunk
+// Chunks of at most this many tokens run like a decode batch (its GEMMs, split-KV attention); the small-chunk
 // workspace holds kSmallChunk rows of kSmallSplits splits.
 constexpr int kSmallChunk = 32, kSmallSplits = 16;
 // Chunks of more than 64 tokens expand the weights once and multiply densely (pair_gemm) where the scratch matrix holds all of them,

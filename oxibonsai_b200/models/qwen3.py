@@ -410,9 +410,7 @@ class Qwen3Runner(SlotState):
                   "sm_ml": torch.zeros((sm, nq, ss, 2), **f32), "sm_ctr": torch.zeros(sm * max(1, nkv), **i32)})
         if b["gemm_ws"] is None:
             b["gemm_ws"] = self._gemm_ws = K.new_gemm_workspace(dev)
-        # scratch for expanded weights: the largest matrix, at most 104 MB (slabs of it then pass through L2), at least 256 rows
-        mats = [m for lw in w.layers[:1] for m in (lw.qkv, lw.o, lw.gate_up, lw.down)]
-        b["wexp"] = torch.empty(max(256 * max(m.k for m in mats), min(52 << 20, max(m.n * m.k for m in mats))), **f16)
+        b["wexp"] = torch.empty(self._wexp_elems(), **f16)
         order = ["tokens", "positions", "h", "xn", "qkv", "q", "attn", "act", "status", "sm_attn", "sm_acc", "sm_ml", "sm_ctr"]
         ptrs = [b[k].data_ptr() for k in order] + [b["wexp"].data_ptr(), b["wexp"].numel(), b["gemm_ws"].data_ptr(), b["gemm_ws"].numel()]
         assert len(ptrs) == K._pf().bonsai_runner_prefill_ptr_count()
@@ -470,10 +468,28 @@ class Qwen3Runner(SlotState):
                                                       self.cfg.vocab, K.stream()), "tp_allgather_logits")
         return self.logits[:T]
 
+    def _wexp_elems(self) -> int:
+        """f16 scratch for expanded weights: the largest matrix, at most 104 MB (slabs of it then pass through L2), at least 256 rows."""
+        mats = [m for lw in self.w.layers[:1] for m in (lw.qkv, lw.o, lw.gate_up, lw.down)]
+        return max(256 * max(m.k for m in mats), min(52 << 20, max(m.n * m.k for m in mats)))
+
     def prefill_launches(self, n_tokens: int, chunk: int = 1024) -> int:
+        """Number of kernel launches of a prompt on one GPU over f16 pages."""
         full, tail = divmod(n_tokens, chunk)
-        small = K._pf().bonsai_runner_small_chunk()
-        per_chunk = lambda t: 1 + (9 if t <= small else 8) * self.cfg.layers     # small chunks convert the f32 attention rows separately
+        small, cfg = K._pf().bonsai_runner_small_chunk(), self.cfg
+        lw, elems = self.w.layers[0], self._wexp_elems()
+
+        def matrix(t: int, m) -> int:      # an expansion and a product per slab of the scratch, or one product (kPairTokens in the runner)
+            if t <= 64 or (t < 256 and m.n * m.k > elems):
+                return 1
+            most = min(elems // m.k, m.n)
+            slabs = -(-m.n // most)
+            per = -(-(-(-m.n // slabs)) // 256) * 256
+            step = m.n if slabs == 1 else per if per <= most else most // 256 * 256
+            return 2 * -(-m.n // step)
+
+        # beside the four matrices two norms, rotation + append and attention; small chunks convert the f32 attention rows separately
+        per_chunk = lambda t: 1 + (4 + (t <= small) + sum(matrix(t, m) for m in (lw.qkv, lw.o, lw.gate_up, lw.down))) * cfg.layers
         return full * per_chunk(chunk) + (per_chunk(tail) if tail else 0) + 2
 
     def set_comm(self, comm_handle: int) -> None:
