@@ -223,10 +223,11 @@ class GenericQwen3Engine:
         if self._wscratch is None:
             self._wscratch = torch.empty(max(c.hidden * c.inter, qd * c.hidden), dtype=torch.float16, device=dev)
         f32 = dict(dtype=torch.float32, device=dev)
+        status = torch.zeros(1, dtype=torch.int32, device=dev)       # of all products: a fill before each would also hold back its launch
 
         def mm(lin: _Linear, x16: torch.Tensor, out: torch.Tensor, residual: torch.Tensor | None = None) -> None:
             w16 = K.quant_to_f16(lin.type, lin.data, lin.n, lin.k, out=self._wscratch[: lin.n * lin.k].view(lin.n, lin.k), paired=True)
-            K.dense_gemm_f16(w16, x16, out=out, residual=residual)
+            K.dense_gemm_f16(w16, x16, out=out, status=status, residual=residual)
 
         done = 0
         while done < tokens.numel():
