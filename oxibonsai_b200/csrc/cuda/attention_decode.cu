@@ -100,8 +100,16 @@ __global__ void qknorm_rope_kvstore_kernel(const float* __restrict__ qkv, int qk
   }
 }
 
+// Sum over the half-warp, largest distance first.
+__device__ __forceinline__ float half_warp_sum(float v) {
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, o));
+  return v;
+}
+
 // The same for head size 128, a warp per (token, head): a lane has dimensions 2l, 2l + 1 and their rotation partners 64 further on, so
-// loads and stores are whole words and nothing passes through shared memory.  A block per head took 148 us for the 4096 x 48 heads of a
+// loads and stores are whole words and nothing passes through shared memory.  The squares are added in the block's order (a half-warp's
+// two sums are one of its warps, 32 dimensions), so that both kernels leave the same bits.  A block per head took 148 us for the 4096 x 48 heads of a
 // prompt, bound by its barriers and the number of blocks; 184 MB move, 28 us at the measured copy rate.
 __global__ void __launch_bounds__(256) qknorm_rope_kvstore_h128_kernel(const float* __restrict__ qkv, int qkv_stride, const float* __restrict__ q_norm,
                                                                        const float* __restrict__ k_norm, float eps, const float* __restrict__ rope_cos,
@@ -122,7 +130,10 @@ __global__ void __launch_bounds__(256) qknorm_rope_kvstore_h128_kernel(const flo
     const float2* wv = reinterpret_cast<const float2*>(is_q ? q_norm : k_norm);
     const float2 wl = wv[lane], wh = wv[32 + lane];
     const float2 c = reinterpret_cast<const float2*>(rope_cos + (size_t)pos * 64)[lane], s = reinterpret_cast<const float2*>(rope_sin + (size_t)pos * 64)[lane];
-    const float inv = 1.0f / sqrtf(warp_sum(lo.x * lo.x + lo.y * lo.y + hi.x * hi.x + hi.y * hi.y) / 128.0f + eps);
+    const float quarter_lo = __fadd_rn(half_warp_sum(__fmul_rn(lo.x, lo.x)), half_warp_sum(__fmul_rn(lo.y, lo.y)));      // dimensions 0-31, 32-63
+    const float quarter_hi = __fadd_rn(half_warp_sum(__fmul_rn(hi.x, hi.x)), half_warp_sum(__fmul_rn(hi.y, hi.y)));      // 64-95, 96-127
+    const float pair = __fadd_rn(quarter_lo, quarter_hi);                                                                 // warps 0 + 2, 1 + 3
+    const float inv = 1.0f / sqrtf(__fadd_rn(pair, __shfl_xor_sync(0xffffffffu, pair, 16)) / 128.0f + eps);
     const float2 a = make_float2(wl.x * lo.x * inv, wl.y * lo.y * inv), d = make_float2(wh.x * hi.x * inv, wh.y * hi.y * inv);
     lo = make_float2(a.x * c.x - d.x * s.x, a.y * c.y - d.y * s.y);
     hi = make_float2(a.x * s.x + d.x * c.x, a.y * s.y + d.y * c.y);

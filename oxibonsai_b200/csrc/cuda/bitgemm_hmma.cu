@@ -264,7 +264,7 @@ __global__ void __launch_bounds__(kGhWarps * 32) bitgemm_hmma_kernel(GhParams p,
 }
 
 // One block per token: y = rmsnorm(x) * w (or a plain copy when w is null) as f16 in hmma-K order.
-__global__ void norm_to_f16_hmma_kernel(const float* __restrict__ x, int x_ld, const float* __restrict__ w, float eps, int K,
+__global__ void __launch_bounds__(1024) norm_to_f16_hmma_kernel(const float* __restrict__ x, int x_ld, const float* __restrict__ w, float eps, int K,
                                         __half* __restrict__ out, int out_ld, int vec) {
   __shared__ float s32[32];
   asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -359,10 +359,10 @@ int bonsai_bitgemm_hmma_tp(const void* comm, const void* codes, const void* scal
 
 int bonsai_norm_to_f16_hmma(const float* x, int x_ld, const float* w, float eps, int T, int K, void* out, int out_ld, cudaStream_t stream) {
   if (T < 1 || K % 128 != 0) return BONSAI_CUDA_BAD_ARG;
-  // one block per token: a block as wide as the row allows keeps the two passes short (few tokens = few blocks)
-  const int threads = K >= 4096 ? 512 : 256;
   const int vec = (x_ld % 4 == 0) && (out_ld % 2 == 0) && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) % 16 == 0) &&
                   (reinterpret_cast<uintptr_t>(out) % 4 == 0);   // 16-byte loads, 4-byte stores
+  // one block per token: a block as wide as the row allows keeps the two passes short (few tokens = few blocks)
+  const int threads = bonsai::norm_threads(K, true) * (vec ? 1 : 2);
   const cudaError_t e = bonsai::launch_pdl(bonsai::norm_to_f16_hmma_kernel, dim3(T), dim3(threads), 0, stream, x, x_ld, w, eps, K, (__half*)out,
                                            out_ld, vec);
   return e == cudaSuccess ? BONSAI_CUDA_OK : BONSAI_CUDA_LAUNCH_FAILED;

@@ -711,7 +711,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) bitgemm_prefill_kernel(const __
 
 // One block per token: y = rmsnorm(x) * w (or a plain copy when w is null), written as f16 in the
 // paired-K order consumed by bitgemm_prefill.
-__global__ void norm_to_f16_paired_kernel(const float* __restrict__ x, int x_ld, const float* __restrict__ w, float eps, int K,
+__global__ void __launch_bounds__(1024) norm_to_f16_paired_kernel(const float* __restrict__ x, int x_ld, const float* __restrict__ w, float eps, int K,
                                           __half* __restrict__ out, int out_ld, int natural, int vec) {
   __shared__ float s32[32];
   // The GEMM behind may start at once: it sets up its barriers and tensor memory and requests packed weights, which nothing in the stream
@@ -889,10 +889,10 @@ int bonsai_bitgemm_prefill(const void* codes, const void* scales, const void* x_
 int bonsai_norm_to_f16_paired(const float* x, int x_ld, const float* w, float eps, int T, int K, void* out, int out_ld, int natural,
                               cudaStream_t stream) {
   if (T < 1 || K % 16 != 0) return BONSAI_CUDA_BAD_ARG;
-  // one block per token; with few tokens (decode batches) a wide block keeps the two passes short
-  const int threads = T <= 128 ? (K >= 4096 ? 512 : 256) : 256;
   const int vec = (x_ld % 4 == 0) && (out_ld % 8 == 0) &&
                   ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(out)) % 16 == 0);   // 16-byte loads and stores
+  // one block per token; with few tokens (decode batches) a wide block keeps the two passes short
+  const int threads = bonsai::norm_threads(K, T <= 128) * (vec ? 1 : 2);
   const cudaError_t e = bonsai::launch_pdl(bonsai::norm_to_f16_paired_kernel, dim3(T), dim3(threads), 0, stream, x, x_ld, w, eps, K, (__half*)out,
                                            out_ld, natural, vec);
   return e == cudaSuccess ? BONSAI_CUDA_OK : BONSAI_CUDA_LAUNCH_FAILED;

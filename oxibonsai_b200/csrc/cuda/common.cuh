@@ -56,35 +56,45 @@ __host__ __device__ inline int hmma_k_pos(int k) {
 // One row: y = rmsnorm(x) * w (a plain copy when w is null) as f16 in the K order that the consumer reads.
 // A thread takes eight neighbouring inputs, so that every order stores whole words: in natural and paired-K order (inputs k and k + 4
 // of every eight side by side) they are one 16-byte word, in hmma-K order four pairs (k, k + 4).  The row is read once and kept in
-// registers between the sum of squares and the scaling (up to 16 * blockDim.x elements; longer rows are read twice).  Needs 16-byte
+// registers between the sum of squares and the scaling (up to 32 * blockDim.x elements; longer rows are read twice).  Needs 16-byte
 // aligned rows and K % 8 == 0.
+//
+// The squares are added up as by 2 * blockDim.x threads with four neighbouring inputs each: a thread keeps the two sums apart, its half-warp
+// is a warp of that order, and warps are added last.  The order is part of the result: f16 rounds the rows, every product carries a
+// flipped bit on, and a short prompt over INT4 pages would move by 3 % with another one.  norm_threads gives the block size.
 enum KOrder { K_NATURAL = 0, K_PAIRED = 1, K_HMMA = 2 };
+__host__ __device__ inline int norm_threads(int K, bool wide) { return wide && K >= 4096 ? 512 : (wide && K >= 2048 ? 256 : 128); }
+__device__ __forceinline__ float norm_square4(float4 v) { return fmaf(v.w, v.w, fmaf(v.z, v.z, fmaf(v.x, v.x, __fmul_rn(v.y, v.y)))); }
 template <int ORDER>
 __device__ __forceinline__ void norm_row_to_f16(const float* __restrict__ xr, const float* __restrict__ w, float eps, int K,
                                                 __half* __restrict__ orow, float* s32) {
-  constexpr int kKeep = 2;
+  constexpr int kKeep = 4;
   const int nch = K >> 3;
   const float4* x4 = reinterpret_cast<const float4*>(xr);
   float4 v[kKeep][2];
-  float ss = 0.0f;
+  float ss[2] = {0.0f, 0.0f};
 #pragma unroll
   for (int i = 0; i < kKeep; ++i) {
     const int c = threadIdx.x + i * blockDim.x;
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       v[i][h] = c < nch ? x4[2 * c + h] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-      ss += v[i][h].x * v[i][h].x + v[i][h].y * v[i][h].y + v[i][h].z * v[i][h].z + v[i][h].w * v[i][h].w;
+      ss[h] = __fadd_rn(ss[h], norm_square4(v[i][h]));
     }
   }
   for (int c = threadIdx.x + kKeep * blockDim.x; c < nch; c += blockDim.x)
-    for (int h = 0; h < 2; ++h) {
-      const float4 t = x4[2 * c + h];
-      ss += t.x * t.x + t.y * t.y + t.z * t.z + t.w * t.w;
-    }
+    for (int h = 0; h < 2; ++h) ss[h] = __fadd_rn(ss[h], norm_square4(x4[2 * c + h]));
   float inv = 1.0f;
   if (w != nullptr) {
-    ss = block_sum(ss, s32);
-    inv = 1.0f / sqrtf(ss / (float)K + eps);
+    const int lane = threadIdx.x & 31, parts = blockDim.x >> 4;
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) ss[h] = __fadd_rn(ss[h], __shfl_xor_sync(0xffffffffu, ss[h], o));
+    if ((lane & 15) == 0) s32[threadIdx.x >> 4] = __fadd_rn(ss[0], ss[1]);
+    __syncthreads();
+    const float sum = warp_sum(lane < parts ? s32[lane] : 0.0f);
+    inv = 1.0f / sqrtf(sum / (float)K + eps);
   }
   auto emit = [&](int c, float4 a, float4 b) {
     if (w != nullptr) {

@@ -424,3 +424,28 @@ def test_quantised_decode_attention_keeps_32_bit_queries_and_probabilities(nq, n
             small = 2.0 ** -28 * (p @ vh.abs()).max()
             worst = ((got[b, h].double() - p @ vh).abs() / ((2 * moved + 2.0 ** -19) * (p @ vh.abs()) + small + 1e-30)).max().item()
             assert worst <= 1.0, (b, h, worst, moved.item(), (p @ vh.abs()).min().item())
+
+
+@pytest.mark.parametrize("nq,nkv,B", [(4, 2, 1), (3, 3, 37)])
+@pytest.mark.parametrize("kvt", [0, 1, 2, 3])
+def test_row_kernels_of_head_size_128_leave_the_same_bits(nq, nkv, B, kvt):
+    """Norm, rotation and append: a warp per head, and (rows at odd strides) a block per head."""
+    from oxibonsai_b200.ops import cuda_ops as K
+    dev = _dev()
+    g = torch.Generator(device=dev).manual_seed(B + kvt)
+    rand = lambda *shape: torch.randn(shape, device=dev, generator=g)  # noqa: E731
+    width, page = (nq + 2 * nkv) * 128, 16
+    odd = torch.zeros((B, width + 1), device=dev)
+    odd[:, :width] = rand(B, width) * rand(B, 1).exp()
+    table = torch.arange(4, dtype=torch.int32, device=dev).repeat(B, 1)
+    pos = torch.arange(B, dtype=torch.int32, device=dev)
+    norms, turn = (rand(128), rand(128)), (rand(64, 64), rand(64, 64))
+    outs = []
+    for rows in (odd[:, :width].contiguous(), odd[:, :width]):
+        pools = [torch.zeros((4, nkv, page, 64 if kvt == 3 else 128), dtype=K.KV_DTYPES[kvt], device=dev) for _ in range(2)]
+        scales = [torch.zeros((4, nkv, page), device=dev) if kvt >= 2 else None for _ in range(2)]
+        q = torch.zeros((B, nq, 128), device=dev)
+        K.qknorm_rope_kvstore(rows, *norms, 1e-6, *turn, pos, table, q, nq, nkv, 128, kvt, page, *pools, *scales)
+        outs.append([q, *pools, *(s for s in scales if s is not None)])
+    for a, b in zip(*outs):
+        assert torch.equal(a, b)

@@ -275,3 +275,53 @@ def test_batch_gemm_through_tensor_memory(ty, rows, cols, T, split):
         slack = 1.1 * bound[:, 0::2] * up.abs() + gate.abs() * bound[:, 1::2] + (2.0 ** -11 + 2.0 ** -20) * act.abs() + 2.0 ** -24
         assert ((got - act).abs() <= slack).all()
     assert status.item() == 0
+
+
+def _row_scale(x, threads):
+    """1 / rms of every row of x with the squares added in the order that the results depend on: thread t of `threads` adds groups t, t + threads, ..
+    of four neighbouring inputs, then warps by halves, then the warps' sums by halves.  One rounding to 32 bits per step."""
+    f = np.float32
+    T, k = x.shape
+    step = -(-k // (4 * threads)) * 4 * threads
+    v = np.zeros((T, step), dtype=np.float64)
+    v[:, :k] = x
+    v = v.reshape(T, -1, threads, 4)
+    acc = np.zeros((T, threads), dtype=f)
+    for i in range(v.shape[1]):
+        y = f(v[:, i, :, 1] ** 2)
+        for e in (0, 2, 3):
+            y = f(v[:, i, :, e] ** 2 + y.astype(np.float64))
+        acc = acc + y
+    def halves(a):
+        while a.shape[-1] > 1:
+            n = a.shape[-1] // 2
+            a = a[..., :n] + a[..., n:]
+        return a[..., 0]
+    warps = np.zeros((T, 32), dtype=f)
+    warps[:, :threads // 32] = halves(acc.reshape(T, threads // 32, 32))
+    return f(1) / np.sqrt(halves(warps) / f(k) + f(1e-6))
+
+
+@pytest.mark.parametrize("cols", [128, 1920, 2048, 2560, 4096, 12288, 33024])
+@pytest.mark.parametrize("T", [1, 128, 129])
+def test_row_norms_add_their_squares_in_a_fixed_order(cols, T):
+    """f16 rows that feed the products: their bits hang on the order of the sum, whatever the block and the width of its loads."""
+    from oxibonsai_b200.ops import cuda_ops as K
+    g = torch.Generator().manual_seed(cols + T)
+    x = torch.randn((T, cols), generator=g) * torch.randn((T, 1), generator=g).exp()
+    w = torch.randn(cols, generator=g)
+    def want(threads):
+        return x * (w * torch.from_numpy(_row_scale(x.numpy(), threads))[:, None])
+    few = 1024 if cols >= 4096 else (512 if cols >= 2048 else 256)
+    rows = want(few if T <= 128 else 256).half()
+    perm, hmma = K.paired_k_index(cols, DEV), K.hmma_k_index(cols)
+    assert torch.equal(K.norm_to_f16_paired(x.to(DEV), w.to(DEV), 1e-6)[:, perm].cpu(), rows)
+    assert torch.equal(K.norm_to_f16_paired(x.to(DEV), w.to(DEV), 1e-6, natural=True).cpu(), rows)
+    assert torch.equal(K.norm_to_f16_hmma(x.to(DEV), w.to(DEV), 1e-6).cpu()[:, hmma], want(few).half())
+    # rows off 16-byte boundaries: scalar loads, blocks of the full width
+    wide = torch.zeros((T, cols + 1), device=DEV)
+    wide[:, 1:] = x.to(DEV)
+    ref = x.double() * w.double() / (x.double().square().mean(-1, keepdim=True) + 1e-6).sqrt()
+    bound = 2.0 ** -11 * ref.abs() + cols * 2.0 ** -24 * ref.abs() + 2.0 ** -24
+    for got in (K.norm_to_f16_paired(wide[:, 1:], w.to(DEV), 1e-6)[:, perm].cpu(), K.norm_to_f16_hmma(wide[:, 1:], w.to(DEV), 1e-6).cpu()[:, hmma]):
+        assert ((got.double() - ref).abs() <= bound).all()
