@@ -738,11 +738,12 @@ int bonsai_qknorm_rope_kvstore(const float* qkv, int qkv_stride, const float* q_
 
 // q: f32 [batch][nq][hd] -> out f32 [batch][nq][hd].  Context length of sequence b is
 // positions[b] + 1 + extra_len.  ws_acc needs batch*nq*nsplit*hd floats, ws_ml batch*nq*nsplit*2,
-// counters batch*nkv ints that are zero between launches (the kernel resets them).
-int bonsai_attn_decode(const float* q, const int* positions, const int* block_table, int max_pages, int batch, int nq, int nkv,
-                       int hd, int kvt, int page_size, const void* kpool, const void* vpool, const float* kscale,
-                       const float* vscale, int nsplit, float* ws_acc, float* ws_ml, int* counters, float* out, int extra_len,
-                       cudaStream_t stream) {
+// counters batch*nkv ints that are zero between launches (the kernel resets them).  f32_rows: INT8 / INT4 rows are multiplied in f32 on the
+// CUDA cores whatever their shape.
+int bonsai_attn_decode_route(const float* q, const int* positions, const int* block_table, int max_pages, int batch, int nq, int nkv,
+                             int hd, int kvt, int page_size, const void* kpool, const void* vpool, const float* kscale,
+                             const float* vscale, int nsplit, float* ws_acc, float* ws_ml, int* counters, float* out, int extra_len,
+                             int f32_rows, cudaStream_t stream) {
   using namespace bonsai;
   if (hd % 32 != 0 || hd < 64 || hd > 256 || nq % nkv != 0 || nsplit < 1 || batch <= 0 || counters == nullptr) return BONSAI_CUDA_BAD_ARG;
   int G = nq / nkv, dpl = hd / 32;
@@ -757,7 +758,7 @@ int bonsai_attn_decode(const float* q, const int* positions, const int* block_ta
                                        ws_ml, counters, out, extra_len, sc, stream);
     if (rc != BONSAI_CUDA_BAD_ARG) return rc;
   }
-  if (hd == 128 && (kvt == KV_Q8 || kvt == KV_Q4) && !g_attn_force_cuda_cores) {
+  if (hd == 128 && (kvt == KV_Q8 || kvt == KV_Q4) && !g_attn_force_cuda_cores && !f32_rows) {
     const int rc = attn_decode_quant(q, positions, block_table, max_pages, batch, nq, nkv, kvt, page_size, kpool, vpool, kscale, vscale, nsplit, ws_acc,
                                      ws_ml, counters, out, extra_len, sc, stream);
     if (rc != BONSAI_CUDA_BAD_ARG) return rc;
@@ -776,6 +777,14 @@ int bonsai_attn_decode(const float* q, const int* positions, const int* block_ta
     case KV_Q4: return launch_decode_d<KV_Q4>(dpl, G, grid, smem, stream, q, positions, block_table, max_pages, pool, nq, sc, ws_acc, ws_ml, counters, out, extra_len);
     default: return BONSAI_CUDA_BAD_ARG;
   }
+}
+
+int bonsai_attn_decode(const float* q, const int* positions, const int* block_table, int max_pages, int batch, int nq, int nkv,
+                       int hd, int kvt, int page_size, const void* kpool, const void* vpool, const float* kscale,
+                       const float* vscale, int nsplit, float* ws_acc, float* ws_ml, int* counters, float* out, int extra_len,
+                       cudaStream_t stream) {
+  return bonsai_attn_decode_route(q, positions, block_table, max_pages, batch, nq, nkv, hd, kvt, page_size, kpool, vpool, kscale, vscale, nsplit,
+                                  ws_acc, ws_ml, counters, out, extra_len, 0, stream);
 }
 
 }  // extern "C"

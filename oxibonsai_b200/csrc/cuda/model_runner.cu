@@ -25,6 +25,8 @@ int bonsai_qknorm_rope_kvstore(const float*, int, const float*, const float*, fl
                                const int*, int, float*, int, int, int, int, int, int, void*, void*, float*, float*, cudaStream_t);
 int bonsai_attn_decode(const float*, const int*, const int*, int, int, int, int, int, int, int, const void*, const void*,
                        const float*, const float*, int, float*, float*, int*, float*, int, cudaStream_t);
+int bonsai_attn_decode_route(const float*, const int*, const int*, int, int, int, int, int, int, int, const void*, const void*,
+                             const float*, const float*, int, float*, float*, int*, float*, int, int, cudaStream_t);
 int bonsai_bitgemv_h2(const void*, const void*, const float*, const float*, float, float*, const float*, int, int, int, cudaStream_t);
 int bonsai_bitgemv_warp(const void*, const void*, const float*, const float*, float, float*, const float*, int, int, int, cudaStream_t);
 int bonsai_bitgemv_hmma(const void*, const void*, const float*, const float*, float, float*, const float*, int, int, int, cudaStream_t);
@@ -253,6 +255,16 @@ constexpr int kSmallChunk = 32, kSmallSplits = 16;
 // larger matrices from kPairTokens tokens on.  In place / expanded, us: 6144 x 4096, 65 tokens 34 / 24, 192 tokens 44 / 25;
 // 24576 x 4096, 65 tokens 61 / 85, 192 tokens 78 / 90, 256 tokens 91 / 94, 384 tokens 134 / 102.
 constexpr int kPairTokens = 256;
+// Prompts over INT4 pages.  A sum in another order flips a few f16 roundings of the rows behind it, and some four layers later those
+// have nothing in common (8e-4 of the logits over f16 pages); the keys and values of such rows then also take other INT4 codes, 0.4
+// standard deviations apart, which only many tokens average out.  Between the kernels that short chunks and prompts have always had and
+// the tensor-memory ones (quarter-depth models of 1.7B / 4B / 8B): 17 tokens 0.048 / 0.053, 64 tokens 0.024 / 0.031, 100 tokens 0.018 / 0.016 / 0.018,
+// 300 tokens 0.008 / 0.010 / 0.010; a draft of nine behind 64 tokens 0.002; the error against 64 bits is the same.  Sequences of up to
+// kInt4Tokens tokens keep the former ones (up to 32 tokens mma.sync GEMM and f32 decode attention, up to 64 the 64-token tile, then only mma.sync
+// attention: gemm_pair adds in the order of the 256-token tile, bit for bit), so that their answers stay what they were.  A draft behind a
+// context three times its length is not a prompt.
+constexpr int kInt4Tokens = 256;
+static inline bool int4_prompt(int kvt, int pos0, int T) { return kvt == 3 && pos0 + T <= kInt4Tokens && pos0 < 3 * T; }
 
 static inline int pf_gemm(Runner& r, const void* codes, const void* scales, const void* x, int x_ld, float* out_f32, const float* residual,
                           void* out_f16, int* status, int n_rows, int K, int T, int epi, int out_ld, int sms, const void* dense_w,
@@ -312,7 +324,9 @@ static int prefill_chunk(Runner& r, const uint64_t* sp, const uint64_t* pp, int 
   // Larger chunks use the tcgen05 GEMM (paired-K order) and the prompt attention kernel.
   const bool small = r.ic[IC_FAST] != 5 && T <= kSmallChunk && hidden % 128 == 0 && qd % 128 == 0 && inter % 128 == 0;
   // One GPU: the packed GEMMs of up to 64 tokens go through tensor memory (bitgemm_batch.cu, paired-K order).
-  const bool batch = !tp && T <= 64 && r.ic[IC_FAST] != 5;
+  const int kvt = slot_format(r, slot);                   // page format of this sequence
+  const bool settled = int4_prompt(kvt, pos0, T);         // kernels and sums as they have always been
+  const bool batch = !tp && T <= 64 && r.ic[IC_FAST] != 5 && !settled;
   const bool hm = small && !batch;
   // Tensor parallel, up to 16 tokens (a speculative verification pass): the row-parallel GEMMs exchange their partial sums
   // in the epilogue, as in the batched decode step, instead of GEMM + two-shot all-reduce (three more launches and two flag
@@ -337,7 +351,6 @@ static int prefill_chunk(Runner& r, const uint64_t* sp, const uint64_t* pp, int 
               : pf_gemm(r, codes, scales, x, x_ld, out_f32, residual, out_f16, status, n_rows, K, T, epi, out_ld, sms, nullptr, st);
   };
 
-  const int kvt = slot_format(r, slot);                   // page format of this sequence
   RC(bonsai_embed_rows_f16(P<void>(r.gp[GP_EMBD]), tokens, h, T, hidden, vocab, st));
   for (int l = 0; l < r.ic[IC_LAYERS]; ++l) {
     const uint64_t* lp = &r.lp[(size_t)l * LP_COUNT];
@@ -351,14 +364,14 @@ static int prefill_chunk(Runner& r, const uint64_t* sp, const uint64_t* pp, int 
                                   P<float>(pool.vs), st));
     if (small) {
       float* attn32 = P<float>(pp[PP_SM_ATTN]);
-      RC(bonsai_attn_decode(q, positions, bt, 0, T, nq, nkv, hd, kvt, r.ic[IC_PAGE_SIZE], P<void>(pool.k),
-                            P<void>(pool.v), P<float>(pool.ks), P<float>(pool.vs), sm_splits, P<float>(pp[PP_SM_ACC]),
-                            P<float>(pp[PP_SM_ML]), P<int>(pp[PP_SM_CTR]), attn32, 0, st));
+      RC(bonsai_attn_decode_route(q, positions, bt, 0, T, nq, nkv, hd, kvt, r.ic[IC_PAGE_SIZE], P<void>(pool.k),
+                                  P<void>(pool.v), P<float>(pool.ks), P<float>(pool.vs), sm_splits, P<float>(pp[PP_SM_ACC]),
+                                  P<float>(pp[PP_SM_ML]), P<int>(pp[PP_SM_CTR]), attn32, 0, settled, st));
       RC(hm ? bonsai_norm_to_f16_hmma(attn32, qd, nullptr, r.eps, T, qd, attn, qd, st)
             : bonsai_norm_to_f16_paired(attn32, qd, nullptr, r.eps, T, qd, attn, qd, 0, st));
     } else {
       RC(bonsai_attn_prefill_ws(q, T, pos0, bt, nq, nkv, hd, kvt, r.ic[IC_PAGE_SIZE], P<void>(pool.k), P<void>(pool.v), P<float>(pool.ks),
-                                P<float>(pool.vs), attn, qd, 0, wexp, wexp_elems, st));
+                                P<float>(pool.vs), attn, qd, 0, settled ? nullptr : wexp, settled ? 0 : wexp_elems, st));
     }
     if (!tp) {
       RC(gemm(P<void>(lp[LP_O_CODES]), P<void>(lp[LP_O_SCALES]), attn, qd, h, h, nullptr, hidden, qd, 1, hidden));

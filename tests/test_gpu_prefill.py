@@ -325,3 +325,54 @@ def test_row_norms_add_their_squares_in_a_fixed_order(cols, T):
     bound = 2.0 ** -11 * ref.abs() + cols * 2.0 ** -24 * ref.abs() + 2.0 ** -24
     for got in (K.norm_to_f16_paired(wide[:, 1:], w.to(DEV), 1e-6)[:, perm].cpu(), K.norm_to_f16_hmma(wide[:, 1:], w.to(DEV), 1e-6).cpu()[:, hmma]):
         assert ((got.double() - ref).abs() <= bound).all()
+
+
+@pytest.fixture(scope="module")
+def wide_head_gguf(tmp_path_factory):
+    from oxibonsai_b200.core import Qwen3Config, write_synthetic_gguf
+    p = tmp_path_factory.mktemp("gguf") / "wide_head.gguf"
+    write_synthetic_gguf(str(p), Qwen3Config(hidden=512, inter=1024, layers=2, heads=4, kv_heads=2, head_dim=128, vocab=1000, context=1024, name="wide"), seed=3)
+    return str(p)
+
+
+@pytest.mark.parametrize("T", [16, 32, 33, 64, 65, 256])
+def test_short_prompts_over_int4_pages_keep_their_kernels(T, wide_head_gguf):
+    """The cache rows that a prompt leaves behind are, bit for bit, those of the former kernels one by one: another order of their sums would flip
+    codes.  Above 64 tokens that includes products over expanded weights."""
+    from oxibonsai_b200.ops import cuda_ops as K
+    from oxibonsai_b200.runtime import EngineBuilder
+    eng = EngineBuilder().model_path(wide_head_gguf).max_seq_len(320).max_batch(2).kv_cache("q4").build()
+    r, cfg = eng.runner, eng.runner.cfg
+    prompt = torch.randint(0, cfg.vocab, (T,), generator=torch.Generator().manual_seed(T)).tolist()
+    eng.begin_sequence(prompt, T + 1, 0)
+    eng.prefill(prompt, 0, 0)
+    torch.cuda.synchronize()
+    got = [t.clone() for t in (eng.kv.k, eng.kv.v, eng.kv.k_scale, eng.kv.v_scale)]
+    for t in (eng.kv.k, eng.kv.v, eng.kv.k_scale, eng.kv.v_scale):
+        t.zero_()
+    nq, nkv, eps = cfg.heads, cfg.kv_heads, cfg.eps
+    table = r.block_table[:1].contiguous()
+    pos = torch.arange(T, dtype=torch.int32, device=DEV)
+    h = torch.index_select(r.w.embd, 0, torch.tensor(prompt, device=DEV)).float()
+    splits = max(1, min(16, 4 * 148 // (nkv * T)))
+    splits = 1 << (splits.bit_length() - 1)
+    to_f16, gemm = (K.norm_to_f16_hmma, K.bitgemm_hmma) if T <= 32 else (K.norm_to_f16_paired, K.bitgemm_prefill)
+    for l, lw in enumerate(r.w.layers):
+        pools = (eng.kv.k[l], eng.kv.v[l], eng.kv.k_scale[l], eng.kv.v_scale[l])
+        qkv = gemm(lw.qkv, to_f16(h, lw.attn_norm, eps))
+        q = torch.empty((T, nq, 128), device=DEV)
+        K.qknorm_rope_kvstore(qkv, lw.q_norm, lw.k_norm, eps, r.rope_cos, r.rope_sin, pos, table.expand(T, -1).contiguous(), q, nq, nkv, 128, 3, eng.kv.page_size, *pools)
+        if T <= 32:
+            K.lib().bonsai_attn_decode_force_cuda_cores(1)
+            try:
+                a = K.attn_decode(q, pos, table.expand(T, -1).contiguous(), nq, nkv, 128, 3, eng.kv.page_size, *pools, nsplit=splits)
+            finally:
+                K.lib().bonsai_attn_decode_force_cuda_cores(0)
+            a = to_f16(a.view(T, -1))
+        else:
+            a = K.attn_prefill(q, 0, table[0], nq, nkv, 128, 3, eng.kv.page_size, *pools)
+        h = gemm(lw.o, a, epi=1, residual=h)
+        h = gemm(lw.down, gemm(lw.gate_up, to_f16(h, lw.ffn_norm, eps), epi=2), epi=1, residual=h)
+    for a, b in zip(got, (eng.kv.k, eng.kv.v, eng.kv.k_scale, eng.kv.v_scale)):
+        assert torch.equal(a, b)
+    assert torch.equal(r._pf["h"][:T], h)
