@@ -403,7 +403,8 @@ class Qwen3Runner(SlotState):
              "h": torch.zeros((chunk, cfg.hidden), **f32), "xn": torch.zeros((chunk, max(cfg.hidden, qd)), **f16),
              "qkv": torch.zeros((chunk, (nq + 2 * nkv) * hd), **f32), "q": torch.zeros((chunk, nq, hd), **f32),
              "attn": torch.zeros((chunk, qd), **f16), "act": torch.zeros((chunk, w.inter_local), **f16),
-             "status": torch.zeros(1, **i32), "gemm_ws": getattr(self, "_gemm_ws", None)}
+             "status": self.status,       # the word that is read with the sampled tokens
+             "gemm_ws": getattr(self, "_gemm_ws", None)}
         # chunks of up to `sm` tokens run like a decode batch: f32 attention rows and the split-KV workspace for them
         sm, ss = K._pf().bonsai_runner_small_chunk(), K._pf().bonsai_runner_small_splits()
         b.update({"sm_attn": torch.zeros((sm, qd), **f32), "sm_acc": torch.zeros((sm, nq, ss, hd), **f32),

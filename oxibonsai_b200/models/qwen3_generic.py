@@ -29,6 +29,7 @@ from ..core.oracle import EOS_TOKEN, rope_table
 from ..ops import cuda_ops as K
 from ..runtime.presets import SamplingParams, SamplingPreset
 from .qwen3 import _f16_matrix, _norm_vector
+from .slot_state import SlotState
 
 SUPPORTED = (G.F32, G.F16, G.BF16, G.Q4_0, G.Q8_0, G.TQ2_0, G.F8_E4M3, G.F8_E5M2, G.Q2_K, G.Q3_K, G.Q4_K, G.Q5_K, G.Q6_K, G.Q8_K)
 
@@ -125,7 +126,10 @@ class GenericQwen3Engine:
         self._free_ranges = list(range(B - 1, -1, -1))
         self._slot_range: dict[int, int] = {}
         self.bt = torch.zeros((B, self.n_pages), **i32)
-        self.token = torch.zeros(B, **i32)          # last token of every slot: input of a step, and where the sampler writes
+        # [status word, last token of every slot]: the products of prompts record an expired wait in the first, the second is a step's input and
+        # where the sampler writes; one copy brings both to the host
+        self._ctl = torch.zeros(B + 1, **i32)
+        self.status, self.token = self._ctl[:1], self._ctl[1:]
         self.pos = torch.zeros(B, **i32)
         self.h = torch.zeros((B, c.hidden), **f32)
         self.qkv = torch.zeros((B, (c.heads + 2 * nkv) * hd), **f32)
@@ -142,7 +146,7 @@ class GenericQwen3Engine:
         self.allow_mask = torch.full((B, self.mask_words), -1, **i32)
         self._masked: set[int] = set()
         self._graphs: dict[tuple[int, bool], torch.cuda.CUDAGraph] = {}
-        self._host = torch.zeros(B, dtype=torch.int32).pin_memory()
+        self._host = torch.zeros(B + 1, dtype=torch.int32).pin_memory()
         self._pos_host = torch.zeros(B, dtype=torch.int32).pin_memory()
         self.nsplit = max(1, min(32, 296 // nkv))
 
@@ -223,11 +227,10 @@ class GenericQwen3Engine:
         if self._wscratch is None:
             self._wscratch = torch.empty(max(c.hidden * c.inter, qd * c.hidden), dtype=torch.float16, device=dev)
         f32 = dict(dtype=torch.float32, device=dev)
-        status = torch.zeros(1, dtype=torch.int32, device=dev)       # of all products: a fill before each would also hold back its launch
 
         def mm(lin: _Linear, x16: torch.Tensor, out: torch.Tensor, residual: torch.Tensor | None = None) -> None:
             w16 = K.quant_to_f16(lin.type, lin.data, lin.n, lin.k, out=self._wscratch[: lin.n * lin.k].view(lin.n, lin.k), paired=True)
-            K.dense_gemm_f16(w16, x16, out=out, status=status, residual=residual)
+            K.dense_gemm_f16(w16, x16, out=out, status=self.status, residual=residual)
 
         done = 0
         while done < tokens.numel():
@@ -331,7 +334,18 @@ class GenericQwen3Engine:
         K.sample(self.logits[s], self.temps[s], self.topks[s], self.topps[s], self.rng[s], out=self.token[s],
                  allow_mask=self.allow_mask[s] if mask is not None else None)
         self.pos[slot] = len(prompt)
-        return int(self.token[slot].item())
+        return self._read_tokens(slot + 1)[slot]
+
+    def _read_tokens(self, n: int) -> list[int]:
+        """The tokens of slots 0 .. n-1; raises instead when a kernel recorded an expired wait, since tokens computed from missing data are
+        never handed out."""
+        self._host[: n + 1].copy_(self._ctl[: n + 1], non_blocking=True)
+        torch.cuda.synchronize(self.device)
+        status, *tokens = self._host[: n + 1].tolist()
+        if status:
+            self.status.zero_()
+            raise K.CudaKernelError(f"a prompt reported status {status}: {SlotState.STATUS_TEXT.get(status, 'a bounded wait expired')}")
+        return tokens
 
     def step_batch(self, positions: Sequence[int], masks: dict | None = None) -> list[int]:
         """One decode step for slots 0 .. len(positions)-1; returns their sampled tokens."""
@@ -344,9 +358,7 @@ class GenericQwen3Engine:
             for s, m in masks.items():
                 self.set_mask(s, m)
         self.step(b, masked)
-        self._host[:b].copy_(self.token[:b], non_blocking=True)
-        torch.cuda.synchronize(self.device)
-        return self._host[:b].tolist()
+        return self._read_tokens(b)
 
     def move_slot(self, src: int, dst: int) -> None:
         for t in (self.bt, self.token, self.pos, self.temps, self.topks, self.topps, self.rng, self.allow_mask):

@@ -481,7 +481,10 @@ class InferenceEngine:
     def verify_greedy(self, tokens: Sequence[int], pos0: int, slot: int = 0) -> list[int]:
         """Greedy next-token choices of the model after each of ``tokens`` placed at positions pos0.. (one batched pass)."""
         t = torch.tensor([int(x) for x in tokens], dtype=torch.int32).pin_memory().to(self.device, non_blocking=True)
-        return self.runner.verify_greedy(t, slot, pos0).tolist()
+        r = self.runner
+        *choice, status = torch.cat([r.verify_greedy(t, slot, pos0), r.status]).tolist()      # one copy to the host
+        r.check_status(status)
+        return choice
 
     def verify_sampled(self, tokens: Sequence[int], pos0: int, draft_logits: torch.Tensor, temperature: float,
                        uniforms: Sequence[float], slot: int = 0) -> tuple[int, int]:

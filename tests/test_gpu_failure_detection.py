@@ -69,3 +69,51 @@ def test_engine_raises_when_the_status_word_is_set(tiny_gguf):
             pass
     assert int(eng.runner.status.item()) == 0    # cleared once reported
     assert eng.generate([1, 2, 3], 2)            # and the engine is usable again
+
+
+@pytest.mark.parametrize("call", ["prompt", "batch", "verification"])
+def test_expired_waits_of_prompts_batches_and_verification_are_reported(call, tiny_gguf):
+    """The word that the tensor-core GEMMs of these passes record an expired wait in is the one that is read with the tokens."""
+    from oxibonsai_b200.ops import cuda_ops as K
+    from oxibonsai_b200.runtime import EngineBuilder
+    eng = EngineBuilder().model_path(tiny_gguf).preset("greedy").max_seq_len(128).max_batch(2).build()
+    prompt = list(range(1, 41))
+    eng.open_sequence(prompt, 64, 0)
+    eng.open_sequence(prompt, 64, 1)
+    pass_of = {"prompt": lambda: eng.open_sequence(prompt, 64, 0), "batch": lambda: eng.step_batch([40, 40]), "verification": lambda: eng.verify_greedy([3, 4, 5], 40)}[call]
+    assert pass_of()
+    eng.runner._pf["status"].fill_(1)            # what a GEMM does whose pipeline stalls
+    with pytest.raises(K.CudaKernelError, match="stalled"):
+        pass_of()
+    assert int(eng.runner.status.item()) == 0 and pass_of()
+
+
+def test_expired_waits_of_block_format_prompts_are_reported(tiny_gguf, tmp_path, monkeypatch):
+    import torch
+    from oxibonsai_b200 import cli
+    from oxibonsai_b200.models.qwen3_generic import GenericQwen3Engine
+    from oxibonsai_b200.ops import cuda_ops as K
+    path = str(tmp_path / "tiny_q8_0.gguf")
+    cli.requantize_gguf(tiny_gguf, path, "q8_0")
+    eng = GenericQwen3Engine(path, max_seq_len=128, max_batch=2)
+    prompt = list(range(1, 41))
+
+    def first_token(slot):
+        eng.begin_sequence(prompt, 64, slot)
+        eng.prefill_slot(prompt, slot)
+        return eng.finish_sequence(prompt, slot)
+
+    good = [first_token(0), first_token(1)]
+    product = K.dense_gemm_f16
+
+    def stalled(*args, status=None, **kw):
+        out = product(*args, status=status, **kw)
+        status.fill_(1)
+        return out
+
+    monkeypatch.setattr(K, "dense_gemm_f16", stalled)
+    with pytest.raises(K.CudaKernelError, match="stalled"):
+        first_token(1)
+    monkeypatch.setattr(K, "dense_gemm_f16", product)
+    assert [first_token(0), first_token(1)] == good and len(eng.step_batch([40, 40])) == 2
+    torch.cuda.synchronize()
