@@ -296,7 +296,7 @@ __global__ void __launch_bounds__(128, 3) attn_prefill_kernel(const float* __res
 }
 
 int attn_prefill_tc(const float*, int, int, const int*, int, int, int, int, int, const void*, const void*, const float*, const float*, void*, int,
-                    void*, size_t, cudaStream_t);
+                    void*, size_t, int*, cudaStream_t);
 
 }  // namespace bonsai
 
@@ -305,15 +305,17 @@ extern "C" {
 // q f32 [T][nq][hd]; block_table: the sequence's page list; the chunk's first token sits at pos0.
 // out f16 [T][out_ld]; k_order 0 = paired-K (operand order of the tcgen05 GEMM), 1 = hmma-K (the mma.sync GEMM; needs
 // nq * hd to be a multiple of 128).  scratch (f16 elements, may be null): where INT8 / INT4 rows are decoded to for the tcgen05 kernel,
-// 2 * nkv * hd per key, keys rounded up to 128; without it, or when it is too small, the mma.sync kernel decodes them itself.
+// 2 * nkv * hd per key, keys rounded up to 128; without it, or when it is too small, the mma.sync kernel decodes them itself.  status (may be
+// null): 6 after a wait of the tcgen05 kernel expired, whose rows are then NaN.
 int bonsai_attn_prefill_ws(const float* q, int T, int pos0, const int* block_table, int nq, int nkv, int hd, int kvt, int page_size,
                            const void* kpool, const void* vpool, const float* kscale, const float* vscale, void* out, int out_ld,
-                           int k_order, void* scratch, size_t scratch_elems, cudaStream_t stream) {
+                           int k_order, void* scratch, size_t scratch_elems, int* status, cudaStream_t stream) {
   using namespace bonsai;
   if (k_order < 0 || k_order > 1 || (k_order == 1 && (nq * hd) % 128 != 0)) return BONSAI_CUDA_BAD_ARG;
   if (T < 1 || (hd != 64 && hd != 128) || nq % nkv != 0 || kvt < 0 || kvt > 3) return BONSAI_CUDA_BAD_ARG;
   if (k_order == 0) {
-    const int rc = attn_prefill_tc(q, T, pos0, block_table, nq, nkv, hd, kvt, page_size, kpool, vpool, kscale, vscale, out, out_ld, scratch, scratch_elems, stream);
+    const int rc = attn_prefill_tc(q, T, pos0, block_table, nq, nkv, hd, kvt, page_size, kpool, vpool, kscale, vscale, out, out_ld, scratch, scratch_elems, status,
+                                   stream);
     if (rc != BONSAI_CUDA_BAD_ARG) return rc;   // bad argument = not a form of that kernel
   }
   PfKvPool kv{(const uint8_t*)kpool, (const uint8_t*)vpool, kscale, vscale, page_size, nkv, hd, kvt};
@@ -339,7 +341,8 @@ int bonsai_attn_prefill_ws(const float* q, int T, int pos0, const int* block_tab
 int bonsai_attn_prefill_order(const float* q, int T, int pos0, const int* block_table, int nq, int nkv, int hd, int kvt, int page_size,
                               const void* kpool, const void* vpool, const float* kscale, const float* vscale, void* out, int out_ld,
                               int k_order, cudaStream_t stream) {
-  return bonsai_attn_prefill_ws(q, T, pos0, block_table, nq, nkv, hd, kvt, page_size, kpool, vpool, kscale, vscale, out, out_ld, k_order, nullptr, 0, stream);
+  return bonsai_attn_prefill_ws(q, T, pos0, block_table, nq, nkv, hd, kvt, page_size, kpool, vpool, kscale, vscale, out, out_ld, k_order, nullptr, 0, nullptr,
+                                stream);
 }
 
 // out f16 [T][out_ld] in paired-K order.

@@ -22,6 +22,7 @@
 namespace bonsai {
 
 constexpr int kAtThreads = 320;
+constexpr int kAtStalled = 6;                          // status of an expired wait
 constexpr int kAtTile = 128 * 128 * 2;                 // bytes of a [128][128] f16 tile: two halves of 64 columns, 128-byte swizzle
 constexpr int kAtSmem = 1024 + 6 * kAtTile;            // Q of two tiles, two stages of K and V
 
@@ -29,6 +30,7 @@ struct AtParams {
   const float* q;
   const int* bt;
   __half* out;
+  int* status;             // may be null
   int T, pos0, nq, nkv, page, paged, n_pad, out_ld;
   float scale;
 };
@@ -83,7 +85,6 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_prefill_tc_kernel(const __
   uint8_t* sV = base + 4 * kAtTile;
   __shared__ uint64_t k_full[2], k_empty[2], v_full[2], v_empty[2], s_full[2], p_ready[2], o_full[2];
   __shared__ uint32_t tmem_slot;
-  __shared__ int s_failed;
   const int t = threadIdx.x, warp = __shfl_sync(0xffffffffu, t >> 5, 0), lane = t & 31;
   const int kvh = blockIdx.x, tok_first = (gridDim.y - 1 - blockIdx.y) * 2 * TOK;      // the longest blocks go first
   const int total = p.pos0 + p.T;                      // keys of the sequence
@@ -104,7 +105,6 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_prefill_tc_kernel(const __
       tc::mbar_init(&p_ready[i], 4);
       tc::mbar_init(&o_full[i], 1);
     }
-    s_failed = 0;
     tc::mbar_fence_init();
   }
   asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -152,6 +152,7 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_prefill_tc_kernel(const __
             for (int x = 0; x < 2; ++x) at_load(dst + x * 16384 + h * 8192, m ? &vmap : &kmap, x * 64, row[h], full);
         }
       }
+      if (failed && p.status != nullptr) atomicExch(p.status, kAtStalled);
     }
   } else if (warp == 9) {
     const uint32_t ids = tc::idesc_f32acc(tc::FMT_F16, tc::FMT_F16, 128, 128), idv = ids | (1u << 16);
@@ -198,6 +199,7 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_prefill_tc_kernel(const __
       if (j < n1 && tc::elect_one()) tc::mma_commit(&k_empty[j & 1]);
       __syncwarp();
     }
+    if (failed && lane == 0 && p.status != nullptr) atomicExch(p.status, kAtStalled);
   } else {
     const int u = warp >> 2, n = u ? n1 : n0, r = t & 127;
     const int tok = tok_first + u * TOK + r / G, head = kvh * G + r % G, last = p.pos0 + tok;      // last key that this row sees
@@ -260,6 +262,7 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_prefill_tc_kernel(const __
       if (lane == 0) tc::mbar_arrive(&p_ready[u]);
     }
     if (!failed && n > 0 && !tc::mbar_wait_warp<0>(&o_full[u], 0, lane)) failed = true;
+    if (failed && lane == 0 && p.status != nullptr) atomicExch(p.status, kAtStalled);
     tc::tc_fence_after();
     if (tok_first + u * TOK < p.T) {
       const float inv = failed ? __int_as_float(0x7FFFFFFF) : (l > 0.0f ? 1.0f / l : 0.0f);      // an expired wait: NaN, not numbers
@@ -355,12 +358,12 @@ static int at_launch(const CUtensorMap& kmap, const CUtensorMap& vmap, const AtP
 // Arguments as bonsai_attn_prefill_order (k_order 0).  f16 pages of a multiple of 64 tokens are read in place; INT8 / INT4 pages are
 // decoded into scratch (f16 elements, 16-byte aligned), 2 * nkv * 128 per key.  Anything else: BAD_ARG, the caller has another kernel.
 int attn_prefill_tc(const float* q, int T, int pos0, const int* bt, int nq, int nkv, int hd, int kvt, int page, const void* kpool, const void* vpool,
-                    const float* kscale, const float* vscale, void* out, int out_ld, void* scratch, size_t scratch_elems, cudaStream_t st) {
+                    const float* kscale, const float* vscale, void* out, int out_ld, void* scratch, size_t scratch_elems, int* status, cudaStream_t st) {
   const int G = nkv > 0 && nq % nkv == 0 ? nq / nkv : 0, n = pos0 + T, n_pad = (n + 127) / 128 * 128;
   if (hd != 128 || (G != 1 && G != 2 && G != 4 && G != 8) || out_ld % 8 != 0) return BONSAI_CUDA_BAD_ARG;
   if (((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(kpool) | reinterpret_cast<uintptr_t>(vpool)) & 15) != 0)
     return BONSAI_CUDA_BAD_ARG;
-  AtParams p{q, bt, (__half*)out, T, pos0, nq, nkv, page, kvt == 1 ? 1 : 0, n_pad, out_ld, 1.4426950408889634f / sqrtf((float)hd)};
+  AtParams p{q, bt, (__half*)out, status, T, pos0, nq, nkv, page, kvt == 1 ? 1 : 0, n_pad, out_ld, 1.4426950408889634f / sqrtf((float)hd)};
   CUtensorMap kmap, vmap;
   if (kvt == 1) {
     if (page % 64 != 0 || !at_map(&kmap, kpool, 0x7FFFFFFFu) || !at_map(&vmap, vpool, 0x7FFFFFFFu)) return BONSAI_CUDA_BAD_ARG;

@@ -53,7 +53,7 @@ int bonsai_bitgemm_batch(const void*, const void*, const void*, int, float*, con
 int bonsai_gemm_pair(const void*, const void*, int, float*, const float*, void*, int*, int, int, int, int, int, int, int, cudaStream_t);
 int bonsai_expand_rows(const void*, const void*, int, int, int, void*, cudaStream_t);
 int bonsai_attn_prefill_ws(const float*, int, int, const int*, int, int, int, int, int, const void*, const void*, const float*,
-                           const float*, void*, int, int, void*, size_t, cudaStream_t);
+                           const float*, void*, int, int, void*, size_t, int*, cudaStream_t);
 int bonsai_embed_rows_f16(const void*, const int*, float*, int, int, int, cudaStream_t);
 int bonsai_bitgemv_s16_pf(const void*, const float*, const float*, float, float*, const float*, int, int, int, const void*, int*, const void*,
                           size_t, cudaStream_t);
@@ -371,7 +371,7 @@ static int prefill_chunk(Runner& r, const uint64_t* sp, const uint64_t* pp, int 
             : bonsai_norm_to_f16_paired(attn32, qd, nullptr, r.eps, T, qd, attn, qd, 0, st));
     } else {
       RC(bonsai_attn_prefill_ws(q, T, pos0, bt, nq, nkv, hd, kvt, r.ic[IC_PAGE_SIZE], P<void>(pool.k), P<void>(pool.v), P<float>(pool.ks),
-                                P<float>(pool.vs), attn, qd, 0, settled ? nullptr : wexp, settled ? 0 : wexp_elems, st));
+                                P<float>(pool.vs), attn, qd, 0, settled ? nullptr : wexp, settled ? 0 : wexp_elems, status, st));
     }
     if (!tp) {
       RC(gemm(P<void>(lp[LP_O_CODES]), P<void>(lp[LP_O_SCALES]), attn, qd, h, h, nullptr, hidden, qd, 1, hidden));

@@ -251,7 +251,8 @@ class GenericQwen3Engine:
                 vs = self.vscale[l] if self.vscale is not None else None
                 K.qknorm_rope_kvstore(qkv, w["q_norm"], w["k_norm"], eps, self.cos, self.sin, positions, bt, q, c.heads, c.kv_heads, c.head_dim,
                                       self.kvt, self.page, self.kpool[l], self.vpool[l], ks, vs)
-                a16 = K.attn_prefill(q, p0, self.bt[slot], c.heads, c.kv_heads, c.head_dim, self.kvt, self.page, self.kpool[l], self.vpool[l], ks, vs)
+                a16 = K.attn_prefill(q, p0, self.bt[slot], c.heads, c.kv_heads, c.head_dim, self.kvt, self.page, self.kpool[l], self.vpool[l], ks, vs,
+                                     status=self.status)
                 mm(w["o"], a16, h, residual=h)
                 xn = K.norm_to_f16_paired(h, w["ffn_norm"], eps)
                 mm(w["gate"], xn, gate)

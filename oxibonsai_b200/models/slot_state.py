@@ -31,7 +31,7 @@ class SlotState:
 
     STATUS_TEXT = {1: "a tile pipeline of the tensor-core GEMM stalled", 2: "a tensor-parallel peer did not deliver its partial sums",
                    3: "a tensor-parallel peer did not reach a barrier", 4: "a tensor-parallel peer did not enter an all-reduce",
-                   5: "the weight copy pipeline of a GEMV stalled"}
+                   5: "the weight copy pipeline of a GEMV stalled", 6: "a tile pipeline of the prompt attention stalled"}
 
     def check_status(self, value: int | None = None) -> None:
         """Raises when a kernel of an earlier step recorded an expired wait (``value``: the status word as already read by

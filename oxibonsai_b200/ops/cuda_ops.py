@@ -626,7 +626,7 @@ _PF_SIG = {
     "bonsai_norm_to_f16_paired": [_vp, _i, _vp, _f, _i, _i, _vp, _i, _i, _vp],
     "bonsai_attn_prefill": [_vp, _i, _i, _vp, _i, _i, _i, _i, _i, _vp, _vp, _vp, _vp, _vp, _i, _vp],
     "bonsai_attn_prefill_order": [_vp, _i, _i, _vp, _i, _i, _i, _i, _i, _vp, _vp, _vp, _vp, _vp, _i, _i, _vp],
-    "bonsai_attn_prefill_ws": [_vp, _i, _i, _vp, _i, _i, _i, _i, _i, _vp, _vp, _vp, _vp, _vp, _i, _i, _vp, C.c_size_t, _vp],
+    "bonsai_attn_prefill_ws": [_vp, _i, _i, _vp, _i, _i, _i, _i, _i, _vp, _vp, _vp, _vp, _vp, _i, _i, _vp, C.c_size_t, _vp, _vp],
     "bonsai_embed_rows_f16": [_vp, _vp, _vp, _i, _i, _i, _vp],
     "bonsai_runner_prefill_ptr_count": [],
     "bonsai_runner_small_chunk": [],
@@ -820,15 +820,17 @@ def bitgemm_prefill(w: PlanarWeight, x_paired: torch.Tensor, epi: int = 0, resid
 
 
 def attn_prefill(q: torch.Tensor, pos0: int, block_table_row: torch.Tensor, nq, nkv, hd, kvt, page_size, kpool, vpool, kscale=None,
-                 vscale=None, out: torch.Tensor | None = None, k_order: int = 0, scratch: torch.Tensor | None = None) -> torch.Tensor:
+                 vscale=None, out: torch.Tensor | None = None, k_order: int = 0, scratch: torch.Tensor | None = None,
+                 status: torch.Tensor | None = None) -> torch.Tensor:
     """Causal attention of a T-token chunk (q f32 [T, nq, hd]) over the sequence's pages; returns f16 [T, nq*hd] in paired-K
     order (``k_order`` 0, the tcgen05 GEMM's operand order) or hmma-K order (1, the mma.sync GEMM's).  ``scratch``: f16 elements into
-    which INT8 / INT4 rows are decoded (2 * nkv * hd per key, keys rounded up to 128); without it a slower kernel decodes them itself."""
+    which INT8 / INT4 rows are decoded (2 * nkv * hd per key, keys rounded up to 128); without it a slower kernel decodes them itself.
+    ``status``: int32 word that takes a code when a wait inside the kernel expires."""
     assert scratch is None or (scratch.dtype == torch.float16 and scratch.is_contiguous())
     T = q.shape[0]
     if out is None:
         out = torch.empty((T, nq * hd), dtype=torch.float16, device=q.device)
     check(_pf().bonsai_attn_prefill_ws(q.data_ptr(), T, pos0, block_table_row.data_ptr(), nq, nkv, hd, kvt, page_size, kpool.data_ptr(),
                                        vpool.data_ptr(), ptr(kscale), ptr(vscale), out.data_ptr(), out.stride(0), k_order, ptr(scratch),
-                                       0 if scratch is None else scratch.numel(), stream()), "attn_prefill")
+                                       0 if scratch is None else scratch.numel(), ptr(status), stream()), "attn_prefill")
     return out

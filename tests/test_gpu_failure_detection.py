@@ -117,3 +117,17 @@ def test_expired_waits_of_block_format_prompts_are_reported(tiny_gguf, tmp_path,
     monkeypatch.setattr(K, "dense_gemm_f16", product)
     assert [first_token(0), first_token(1)] == good and len(eng.step_batch([40, 40])) == 2
     torch.cuda.synchronize()
+
+
+def test_prompt_attention_takes_a_status_word(tiny_gguf):
+    """The tensor-memory kernel has waits that can expire: it is given the word in which the products of the same prompt record theirs, and
+    leaves it alone when all is well.  Its code has a text of its own."""
+    from oxibonsai_b200.models.slot_state import SlotState
+    from oxibonsai_b200.ops import cuda_ops as K
+    dev, T, nkv = _dev(), 200, 2
+    q = torch.randn((T, 4, 128), device=dev)
+    pools = [torch.randn((4, nkv, 64, 128), device=dev).half() for _ in range(2)]
+    table, status = torch.arange(4, dtype=torch.int32, device=dev), torch.zeros(1, dtype=torch.int32, device=dev)
+    a = K.attn_prefill(q, 0, table, 4, nkv, 128, K.KV_F16, 64, *pools, status=status)
+    assert int(status.item()) == 0 and torch.equal(a, K.attn_prefill(q, 0, table, 4, nkv, 128, K.KV_F16, 64, *pools))
+    assert "attention" in SlotState.STATUS_TEXT[6]
