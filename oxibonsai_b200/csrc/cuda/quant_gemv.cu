@@ -256,6 +256,7 @@ struct QsParams {
   const float* norm_w;
   float* out;              // [NB][out_ld]
   const float* residual;   // [NB][out_ld]
+  int* status;             // may be null; 5 after a copy that never arrived
   float eps;
   int x_ld, out_ld, N, K, R, KW, RW, stages;
   long long row_bytes;
@@ -395,7 +396,10 @@ __global__ void __launch_bounds__(kQsMaxWarps * 32 + 32, 1) quant_stream_kernel(
       if (lane == 0) tc::mbar_arrive(&empty[st]);
     }
   }
-  if (failed) s_failed = 1;      // a copy that never arrived: its rows come out as NaN instead of numbers made of old data
+  if (failed) {                  // a copy that never arrived: its rows come out as NaN instead of numbers made of old data
+    s_failed = 1;
+    if (lane == 0 && p.status != nullptr) atomicExch(p.status, 5);
+  }
   __syncthreads();
   if (warp >= nwarps) return;
   float inv[NB];
@@ -449,8 +453,9 @@ static bool qs_plan(QsParams& p, int& grid, size_t& smem, int nb) {
 
 template <typename D>
 static QsParams qs_params(const void* w, const float* x, int x_ld, const float* norm_w, float eps, float* out, const float* residual, int out_ld,
-                          int N, int K) {
+                          int N, int K, int* status) {
   QsParams p{};
+  p.status = status;
   p.w = (const uint8_t*)w; p.x = x; p.norm_w = norm_w; p.out = out; p.residual = residual; p.eps = eps;
   p.x_ld = x_ld; p.out_ld = out_ld; p.N = N; p.K = K;
   p.row_bytes = (long long)(K / D::kElems) * D::kBytes;
@@ -511,9 +516,9 @@ __global__ void __launch_bounds__(256) quant_gemv_kernel(const uint8_t* __restri
 
 template <typename D, typename Q>
 static int launch_quant_gemv(const void* w, const float* x, const float* norm_w, float eps, float* out, const float* residual, int N, int K,
-                             cudaStream_t st) {
+                             int* status, cudaStream_t st) {
   if (K % D::kElems != 0) return BONSAI_CUDA_BAD_ARG;
-  QsParams p = qs_params<D>(w, x, K, norm_w, eps, out, residual, N, N, K);
+  QsParams p = qs_params<D>(w, x, K, norm_w, eps, out, residual, N, N, K, status);
   int sgrid;
   size_t smem;
   if (qs_plan<Q>(p, sgrid, smem, 1)) return qs_launch<Q, 1>(p, sgrid, smem, st);
@@ -583,13 +588,13 @@ __global__ void __launch_bounds__(256) quant_gemv_batched_kernel(const uint8_t* 
 
 template <typename D, typename Q>
 static int launch_quant_gemv_batched(const void* w, const float* x, int x_ld, const float* norm_w, float eps, float* out, const float* residual,
-                                     int out_ld, int N, int K, int B, cudaStream_t st) {
+                                     int out_ld, int N, int K, int B, int* status, cudaStream_t st) {
   if (K % D::kElems != 0) return BONSAI_CUDA_BAD_ARG;
   int grid = (N + 7) / 8;
   if (grid > 148 * 8) grid = 148 * 8;
   const uint8_t* wp = (const uint8_t*)w;
   {
-    QsParams p = qs_params<D>(w, x, x_ld, norm_w, eps, out, residual, out_ld, N, K);
+    QsParams p = qs_params<D>(w, x, x_ld, norm_w, eps, out, residual, out_ld, N, K, status);
     int sgrid, rc = BONSAI_CUDA_OK;
     size_t smem;
     if (qs_plan<Q>(p, sgrid, smem, 2)) {
@@ -671,35 +676,36 @@ extern "C" {
 
 // out[N] = (residual or 0) + W (rmsnorm(x) or x) for a row-major matrix of GGUF blocks of `type`
 // (GGUF type ids: 0 F32, 1 F16, 30 BF16, 2 Q4_0, 8 Q8_0, 10-15 Q2_K..Q8_K, 35 TQ2_0, 43 / 44 FP8 E4M3 / E5M2).
-int bonsai_quant_gemv(int type, const void* w, const float* x, const float* norm_w, float eps, float* out, const float* residual,
-                      int N, int K, cudaStream_t stream) {
+// status (may be null): a word that takes code 5 when a wait for a copy of the matrix expired; its rows are then NaN.
+int bonsai_quant_gemv_status(int type, const void* w, const float* x, const float* norm_w, float eps, float* out, const float* residual,
+                             int N, int K, int* status, cudaStream_t stream) {
   using namespace bonsai;
   if (N <= 0 || K <= 0) return BONSAI_CUDA_BAD_ARG;
   switch (type) {
-    case 0: return launch_quant_gemv<DecF32, QsF32>(w, x, norm_w, eps, out, residual, N, K, stream);
-    case 1: return launch_quant_gemv<DecF16, QsF16>(w, x, norm_w, eps, out, residual, N, K, stream);
-    case 30: return launch_quant_gemv<DecBF16, QsBF16>(w, x, norm_w, eps, out, residual, N, K, stream);
-    case 2: return launch_quant_gemv<DecQ4_0, QsQ4_0>(w, x, norm_w, eps, out, residual, N, K, stream);
-    case 8: return launch_quant_gemv<DecQ8_0, QsQ8_0>(w, x, norm_w, eps, out, residual, N, K, stream);
-    case 10: return launch_quant_gemv<DecQ2K, QsQ2K>(w, x, norm_w, eps, out, residual, N, K, stream);
-    case 11: return launch_quant_gemv<DecQ3K, QsQ3K>(w, x, norm_w, eps, out, residual, N, K, stream);
-    case 12: return launch_quant_gemv<DecQ4K, QsQ4K>(w, x, norm_w, eps, out, residual, N, K, stream);
-    case 13: return launch_quant_gemv<DecQ5K, QsQ5K>(w, x, norm_w, eps, out, residual, N, K, stream);
-    case 14: return launch_quant_gemv<DecQ6K, QsQ6K>(w, x, norm_w, eps, out, residual, N, K, stream);
-    case 15: return launch_quant_gemv<DecQ8K, QsQ8K>(w, x, norm_w, eps, out, residual, N, K, stream);
-    case 35: return launch_quant_gemv<DecTq2_256, QsTq2_256>(w, x, norm_w, eps, out, residual, N, K, stream);
-    case 43: return launch_quant_gemv<DecFp8<false>, QsFp8<false>>(w, x, norm_w, eps, out, residual, N, K, stream);
-    case 44: return launch_quant_gemv<DecFp8<true>, QsFp8<true>>(w, x, norm_w, eps, out, residual, N, K, stream);
+    case 0: return launch_quant_gemv<DecF32, QsF32>(w, x, norm_w, eps, out, residual, N, K, status, stream);
+    case 1: return launch_quant_gemv<DecF16, QsF16>(w, x, norm_w, eps, out, residual, N, K, status, stream);
+    case 30: return launch_quant_gemv<DecBF16, QsBF16>(w, x, norm_w, eps, out, residual, N, K, status, stream);
+    case 2: return launch_quant_gemv<DecQ4_0, QsQ4_0>(w, x, norm_w, eps, out, residual, N, K, status, stream);
+    case 8: return launch_quant_gemv<DecQ8_0, QsQ8_0>(w, x, norm_w, eps, out, residual, N, K, status, stream);
+    case 10: return launch_quant_gemv<DecQ2K, QsQ2K>(w, x, norm_w, eps, out, residual, N, K, status, stream);
+    case 11: return launch_quant_gemv<DecQ3K, QsQ3K>(w, x, norm_w, eps, out, residual, N, K, status, stream);
+    case 12: return launch_quant_gemv<DecQ4K, QsQ4K>(w, x, norm_w, eps, out, residual, N, K, status, stream);
+    case 13: return launch_quant_gemv<DecQ5K, QsQ5K>(w, x, norm_w, eps, out, residual, N, K, status, stream);
+    case 14: return launch_quant_gemv<DecQ6K, QsQ6K>(w, x, norm_w, eps, out, residual, N, K, status, stream);
+    case 15: return launch_quant_gemv<DecQ8K, QsQ8K>(w, x, norm_w, eps, out, residual, N, K, status, stream);
+    case 35: return launch_quant_gemv<DecTq2_256, QsTq2_256>(w, x, norm_w, eps, out, residual, N, K, status, stream);
+    case 43: return launch_quant_gemv<DecFp8<false>, QsFp8<false>>(w, x, norm_w, eps, out, residual, N, K, status, stream);
+    case 44: return launch_quant_gemv<DecFp8<true>, QsFp8<true>>(w, x, norm_w, eps, out, residual, N, K, status, stream);
     default: return BONSAI_CUDA_BAD_ARG;
   }
 }
 
 // The same for B activation rows (a decode batch): x [B][x_ld], out and residual [B][out_ld].
-int bonsai_quant_gemv_batched(int type, const void* w, const float* x, int x_ld, const float* norm_w, float eps, float* out,
-                              const float* residual, int out_ld, int N, int K, int B, cudaStream_t stream) {
+int bonsai_quant_gemv_batched_status(int type, const void* w, const float* x, int x_ld, const float* norm_w, float eps, float* out,
+                                     const float* residual, int out_ld, int N, int K, int B, int* status, cudaStream_t stream) {
   using namespace bonsai;
   if (N <= 0 || K <= 0 || B <= 0 || x_ld < K || out_ld < N) return BONSAI_CUDA_BAD_ARG;
-#define BONSAI_QGB(...) return launch_quant_gemv_batched<__VA_ARGS__>(w, x, x_ld, norm_w, eps, out, residual, out_ld, N, K, B, stream)
+#define BONSAI_QGB(...) return launch_quant_gemv_batched<__VA_ARGS__>(w, x, x_ld, norm_w, eps, out, residual, out_ld, N, K, B, status, stream)
   switch (type) {
     case 0: BONSAI_QGB(DecF32, QsF32);
     case 1: BONSAI_QGB(DecF16, QsF16);
@@ -718,6 +724,16 @@ int bonsai_quant_gemv_batched(int type, const void* w, const float* x, int x_ld,
     default: return BONSAI_CUDA_BAD_ARG;
   }
 #undef BONSAI_QGB
+}
+
+int bonsai_quant_gemv(int type, const void* w, const float* x, const float* norm_w, float eps, float* out, const float* residual,
+                      int N, int K, cudaStream_t stream) {
+  return bonsai_quant_gemv_status(type, w, x, norm_w, eps, out, residual, N, K, nullptr, stream);
+}
+
+int bonsai_quant_gemv_batched(int type, const void* w, const float* x, int x_ld, const float* norm_w, float eps, float* out,
+                              const float* residual, int out_ld, int N, int K, int B, cudaStream_t stream) {
+  return bonsai_quant_gemv_batched_status(type, w, x, x_ld, norm_w, eps, out, residual, out_ld, N, K, B, nullptr, stream);
 }
 
 int bonsai_swiglu_rows(const float* gu, int gu_ld, float* out, int out_ld, int inter, int T, cudaStream_t stream) {

@@ -61,17 +61,16 @@ class _Linear:
                 out.append(p)
         return out
 
-    def __call__(self, x, norm_w=None, eps=1e-6, residual=None, out=None):
-        if x.dim() == 1:
-            return K.quant_gemv(self.type, self.data, self.n, self.k, x, norm_w, eps, residual, out)
-        return K.quant_gemv_batched(self.type, self.data, self.n, self.k, x, norm_w, eps, residual, out)
+    def __call__(self, x, norm_w=None, eps=1e-6, residual=None, out=None, status=None):
+        product = K.quant_gemv if x.dim() == 1 else K.quant_gemv_batched
+        return product(self.type, self.data, self.n, self.k, x, norm_w, eps, residual, out, status)
 
 
-def _project(mats: Sequence[_Linear], x: torch.Tensor, norm_w, eps: float, out: torch.Tensor) -> None:
+def _project(mats: Sequence[_Linear], x: torch.Tensor, norm_w, eps: float, out: torch.Tensor, status: torch.Tensor) -> None:
     """out[:, columns of mats[i]] = mats[i] (rmsnorm(x)) for a list of matrices that share the input."""
     c0 = 0
     for m in mats:
-        m(x, norm_w, eps, out=out[:, c0:c0 + m.n])
+        m(x, norm_w, eps, out=out[:, c0:c0 + m.n], status=status)
         c0 += m.n
 
 
@@ -126,8 +125,8 @@ class GenericQwen3Engine:
         self._free_ranges = list(range(B - 1, -1, -1))
         self._slot_range: dict[int, int] = {}
         self.bt = torch.zeros((B, self.n_pages), **i32)
-        # [status word, last token of every slot]: the products of prompts record an expired wait in the first, the second is a step's input and
-        # where the sampler writes; one copy brings both to the host
+        # [status word, last token of every slot]: the products record an expired wait in the first, the second is a step's input and where the
+        # sampler writes; one copy brings both to the host
         self._ctl = torch.zeros(B + 1, **i32)
         self.status, self.token = self._ctl[:1], self._ctl[1:]
         self.pos = torch.zeros(B, **i32)
@@ -192,17 +191,17 @@ class GenericQwen3Engine:
         h, qkv, pos, bt = self.h[s], self.qkv[s], self.pos[s], self.bt[s]
         h.copy_(torch.index_select(self.embd, 0, self.token[s].long()).float())      # no host sync: capturable
         for l, w in enumerate(self.layers):
-            _project(w["qkv"], h, w["attn_norm"], eps, qkv)
+            _project(w["qkv"], h, w["attn_norm"], eps, qkv, self.status)
             ks = self.kscale[l] if self.kscale is not None else None
             vs = self.vscale[l] if self.vscale is not None else None
             K.qknorm_rope_kvstore(qkv, w["q_norm"], w["k_norm"], eps, self.cos, self.sin, pos, bt, self.q[s], c.heads, c.kv_heads,
                                   c.head_dim, self.kvt, self.page, self.kpool[l], self.vpool[l], ks, vs)
             K.attn_decode(self.q[s], pos, bt, c.heads, c.kv_heads, c.head_dim, self.kvt, self.page, self.kpool[l], self.vpool[l], ks, vs,
                           nsplit=self.nsplit, out=self.attn[s])
-            w["o"](self.attn[s].view(hi - lo, -1), residual=h, out=h)
-            _project(w["gate_up"], h, w["ffn_norm"], eps, self.gu[s])
+            w["o"](self.attn[s].view(hi - lo, -1), residual=h, out=h, status=self.status)
+            _project(w["gate_up"], h, w["ffn_norm"], eps, self.gu[s], self.status)
             K.swiglu_rows(self.gu[s], c.inter, out=self.act[s])
-            w["down"](self.act[s], residual=h, out=h)
+            w["down"](self.act[s], residual=h, out=h, status=self.status)
         for b in range(lo, hi):
             K.f16gemv(self.lm_head, self.h[b], self.out_norm, eps, out=self.logits[b])
         if sample:
@@ -345,7 +344,7 @@ class GenericQwen3Engine:
         status, *tokens = self._host[: n + 1].tolist()
         if status:
             self.status.zero_()
-            raise K.CudaKernelError(f"a prompt reported status {status}: {SlotState.STATUS_TEXT.get(status, 'a bounded wait expired')}")
+            raise K.CudaKernelError(f"a pass reported status {status}: {SlotState.STATUS_TEXT.get(status, 'a bounded wait expired')}")
         return tokens
 
     def step_batch(self, positions: Sequence[int], masks: dict | None = None) -> list[int]:

@@ -210,9 +210,9 @@ def _mma():
 
 
 _QG_SIG = {
-    "bonsai_quant_gemv": [_i, _vp, _vp, _vp, _f, _vp, _vp, _i, _i, _vp],
+    "bonsai_quant_gemv_status": [_i, _vp, _vp, _vp, _f, _vp, _vp, _i, _i, _vp, _vp],
     "bonsai_swiglu": [_vp, _vp, _vp, _i, _vp],
-    "bonsai_quant_gemv_batched": [_i, _vp, _vp, _i, _vp, _f, _vp, _vp, _i, _i, _i, _i, _vp],
+    "bonsai_quant_gemv_batched_status": [_i, _vp, _vp, _i, _vp, _f, _vp, _vp, _i, _i, _i, _i, _vp, _vp],
     "bonsai_swiglu_rows": [_vp, _i, _vp, _i, _i, _i, _vp],
     "bonsai_quant_to_f16": [_i, _vp, _vp, _i, _i, _i, _vp],
 }
@@ -229,13 +229,15 @@ def _qg():
 
 
 def quant_gemv(type_id: int, w: torch.Tensor, n: int, k: int, x: torch.Tensor, norm_w: torch.Tensor | None = None, eps: float = 1e-6,
-               residual: torch.Tensor | None = None, out: torch.Tensor | None = None) -> torch.Tensor:
-    """out[n] = (residual) + W (rmsnorm(x)) for ``w`` = the raw GGUF bytes (uint8 CUDA tensor) of an [n, k] matrix of ``type_id`` blocks."""
+               residual: torch.Tensor | None = None, out: torch.Tensor | None = None, status: torch.Tensor | None = None) -> torch.Tensor:
+    """out[n] = (residual) + W (rmsnorm(x)) for ``w`` = the raw GGUF bytes (uint8 CUDA tensor) of an [n, k] matrix of ``type_id`` blocks.
+    ``status``: int32 word that takes code 5 when a wait for the matrix expires (the rows are NaN then)."""
     assert w.is_cuda and w.dtype == torch.uint8
     _f32c(x)
     if out is None:
         out = torch.empty(n, dtype=torch.float32, device=x.device)
-    check(_qg().bonsai_quant_gemv(type_id, w.data_ptr(), x.data_ptr(), ptr(norm_w), eps, out.data_ptr(), ptr(residual), n, k, stream()), "quant_gemv")
+    check(_qg().bonsai_quant_gemv_status(type_id, w.data_ptr(), x.data_ptr(), ptr(norm_w), eps, out.data_ptr(), ptr(residual), n, k, ptr(status),
+                                         stream()), "quant_gemv")
     return out
 
 
@@ -269,15 +271,15 @@ def residual_add(a: torch.Tensor, b: torch.Tensor) -> torch.Tensor:
 
 
 def quant_gemv_batched(type_id: int, w: torch.Tensor, n: int, k: int, x: torch.Tensor, norm_w: torch.Tensor | None = None, eps: float = 1e-6,
-                       residual: torch.Tensor | None = None, out: torch.Tensor | None = None) -> torch.Tensor:
+                       residual: torch.Tensor | None = None, out: torch.Tensor | None = None, status: torch.Tensor | None = None) -> torch.Tensor:
     """:func:`quant_gemv` for a batch: ``x`` [B, k] f32 (row stride >= k), ``out`` and ``residual`` [B, n] with one common row stride."""
     assert w.is_cuda and w.dtype == torch.uint8 and x.dim() == 2 and x.dtype == torch.float32 and x.stride(1) == 1
     B = x.shape[0]
     if out is None:
         out = torch.empty((B, n), dtype=torch.float32, device=x.device)
     assert out.stride(1) == 1 and (residual is None or (residual.stride(1) == 1 and residual.stride(0) == out.stride(0)))
-    check(_qg().bonsai_quant_gemv_batched(type_id, w.data_ptr(), x.data_ptr(), x.stride(0), ptr(norm_w), eps, out.data_ptr(), ptr(residual),
-                                          out.stride(0), n, k, B, stream()), "quant_gemv_batched")
+    check(_qg().bonsai_quant_gemv_batched_status(type_id, w.data_ptr(), x.data_ptr(), x.stride(0), ptr(norm_w), eps, out.data_ptr(), ptr(residual),
+                                                 out.stride(0), n, k, B, ptr(status), stream()), "quant_gemv_batched")
     return out
 
 

@@ -131,3 +131,22 @@ def test_prompt_attention_takes_a_status_word(tiny_gguf):
     a = K.attn_prefill(q, 0, table, 4, nkv, 128, K.KV_F16, 64, *pools, status=status)
     assert int(status.item()) == 0 and torch.equal(a, K.attn_prefill(q, 0, table, 4, nkv, 128, K.KV_F16, 64, *pools))
     assert "attention" in SlotState.STATUS_TEXT[6]
+
+
+def test_streamed_rows_take_the_status_word_of_the_engine(tiny_gguf, tmp_path, monkeypatch):
+    """Every product of a block-format decode step records an expired wait where the engine reads it with the tokens."""
+    from oxibonsai_b200 import cli
+    from oxibonsai_b200.models.qwen3_generic import GenericQwen3Engine
+    from oxibonsai_b200.ops import cuda_ops as K
+    path = str(tmp_path / "tiny_q8_0.gguf")
+    cli.requantize_gguf(tiny_gguf, path, "q8_0")
+    eng = GenericQwen3Engine(path, max_seq_len=64, max_batch=2)
+    words, product = [], K.quant_gemv_batched
+    monkeypatch.setattr(K, "quant_gemv_batched", lambda *a: (words.append(a[-1]), product(*a))[1])
+    eng._bind(0)
+    eng._forward(0, 1, True)
+    assert len(words) == 4 * eng.config.layers and all(w is eng.status for w in words) and eng._read_tokens(1)
+    eng.status.fill_(5)
+    with pytest.raises(K.CudaKernelError, match="copy pipeline"):
+        eng.step_batch([1])
+    assert eng.step_batch([1])
