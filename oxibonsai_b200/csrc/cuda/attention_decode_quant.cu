@@ -1,5 +1,5 @@
-// Split-KV decode attention for head_dim 128 over INT8 and INT4 pages on the warp-level tensor cores, with 32-bit queries and
-// probabilities.
+// Split-KV decode attention for head_dim 128 over INT8 and INT4 pages on the warp-level tensor cores, queries and probabilities as two f16
+// terms each (22 bits).
 //
 // The CUDA-core kernel (attention_decode.cu) spends some 190 warp instructions per token and kv head on products, shuffles and the
 // softmax bookkeeping; at 64 sequences of about 1100 tokens it took 145 us where the rows are 147 MB.  Here a warp handles 16 tokens:
@@ -10,10 +10,12 @@
 //     neither leaves the range in which the two terms hold 22 bits;
 //   * the dimensions and tokens of a tile may come in any order as long as both operands agree, so that every lane loads whole 16-byte
 //     words of the rows straight into registers, a tile ahead.
-// Scores, maxima, sums and accumulators are f32; the error against 64 bits is that of the CUDA-core kernel (2.7e-7 over 64 sequences of
-// 128 to 2048 tokens, 3.1e-7 over one of 20001).  32 / 8 heads, before and now: those 64 sequences 111 -> 45 us (3.3 TB/s), that one 40 -> 22 us,
-// 24 of 100 to 1500 in INT4 38 -> 24 us, one of 300 8.1 -> 9.2 us (its step: launch and merge).  Bound by instructions, some 20 per token and kv
-// head, and for few sequences by the chain of one tile.  Work decomposition, workspace and the last CTA's merge are those of the other kernels.
+// Scores, maxima, sums and accumulators are f32.  The error against 64 bits is no larger than that of the CUDA-core kernel's f32 products for
+// unit-normal queries and rows (one to 64 sequences of 16 to 20001 tokens: INT8 1.66e-7 and 1.78e-7, INT4 1.52e-7 and 1.71e-7); over INT8
+// rows and queries twice as large 2.9e-7 and 2.7e-7.  32 / 8 heads, before and now: 64 sequences of 128 to 2048 tokens 111 -> 46 us (3.2 TB/s),
+// one of 20001 40 -> 22 us, 24 of 100 to 1500 in INT4 38 -> 24 us, one of 300 8.1 -> 9.2 us (its step: launch and merge).  Bound by instructions,
+// some 20 per token and kv head, and for few sequences by the chain of one tile.  Work decomposition, workspace and the last CTA's merge
+// are those of the other kernels.
 #include <cuda_fp16.h>
 
 #include "common.cuh"
@@ -148,7 +150,10 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? 1 : 2) attn_decode_quant_ke
     float s[2][2];
 #pragma unroll
     for (int n = 0; n < 2; ++n) {
-      float acc[2][4] = {};          // two chains: half the latency and half the rounding
+      // INT4: two chains, whose sums of 11-bit times 4-bit products hardly round.  INT8: every product in a sum of its own, added up in f32: the
+      // tensor core cuts a running sum off where f32 rounds it (1.80 -> 1.66e-7 over unit queries, f32 1.78e-7; 64 sequences 62.6 -> 64.2 us).
+      constexpr int CH = KVT == 2 ? 8 : 2;
+      float acc[CH][4] = {};
 #pragma unroll
       for (int h = 0; h < KW; ++h) {
         const uint32_t w[4] = {cur.k[n][h].x, cur.k[n][h].y, cur.k[n][h].z, cur.k[n][h].w};
@@ -156,7 +161,7 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? 1 : 2) attn_decode_quant_ke
         for (int i = 0; i < 4; ++i) {
           if (KVT == 2) {
             const uint32_t x = w[i] ^ 0x80808080u;      // 1024 + code + 128 in a half
-            qa_mma(acc[i & 1], qa[h * 4 + i], qa_sub(__byte_perm(x, 0x64646464u, 0x4140), 0x64806480u), qa_sub(__byte_perm(x, 0x64646464u, 0x4342), 0x64806480u));
+            qa_mma(acc[h * 4 + i], qa[h * 4 + i], qa_sub(__byte_perm(x, 0x64646464u, 0x4140), 0x64806480u), qa_sub(__byte_perm(x, 0x64646464u, 0x4342), 0x64806480u));
           } else {
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
@@ -167,8 +172,14 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? 1 : 2) attn_decode_quant_ke
           }
         }
       }
-      s[n][0] = (acc[0][0] + acc[1][0]) + (acc[0][2] + acc[1][2]);
-      s[n][1] = (acc[0][1] + acc[1][1]) + (acc[0][3] + acc[1][3]);
+#pragma unroll
+      for (int step = 1; step < CH; step *= 2)
+#pragma unroll
+        for (int i = 0; i < CH; i += 2 * step)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) acc[i][e] += acc[i + step][e];
+      s[n][0] = acc[0][0] + acc[0][2];
+      s[n][1] = acc[0][1] + acc[0][3];
     }
     // ---- softmax; the scales of tokens 8 n + 2c + e ----------------------------------------------------------------------------------------
     const int tb = t0 + j * 16;

@@ -377,7 +377,7 @@ def test_cluster_merge_of_decode_attention_matches_the_global_merge(nq, nkv, nsp
 
 @pytest.mark.parametrize("nq,nkv,nsplit", [(3, 3, 1), (4, 2, 3), (8, 2, 16), (8, 1, 2)])
 @pytest.mark.parametrize("kvt", [2, 3])
-def test_quantised_decode_attention_keeps_32_bit_queries_and_probabilities(nq, nkv, nsplit, kvt):
+def test_quantised_decode_attention_with_queries_and_probabilities_in_two_f16_terms(nq, nkv, nsplit, kvt):
     """Group sizes 1 to 8; contexts of one token, of a tile and one more, of many; row scales over six orders of magnitude, some zero,
     growing along the context; whatever lies behind the last key does not enter."""
     import math
@@ -449,3 +449,42 @@ def test_row_kernels_of_head_size_128_leave_the_same_bits(nq, nkv, B, kvt):
         outs.append([q, *pools, *(s for s in scales if s is not None)])
     for a, b in zip(*outs):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("nq,nkv", [(16, 8), (32, 8)])
+@pytest.mark.parametrize("kvt", [2, 3])
+def test_quantised_decode_attention_is_no_further_off_than_f32_products(nq, nkv, kvt):
+    """Unit-normal queries and rows, contexts of a tile to thousands: the mean error against 64 bits, tensor cores and CUDA cores."""
+    import math
+    from oxibonsai_b200.ops import cuda_ops as K
+    dev, page = _dev(), 64
+    g = torch.Generator(device=dev).manual_seed(5)
+    rand = lambda *shape: torch.randn(shape, device=dev, generator=g)  # noqa: E731
+    off = [0.0, 0.0]
+    for lens in ([16, 24, 90], [300, 700, 411, 95, 512], [1500, 800, 100], [4096]) * 3:
+        pages = [-(-n // page) for n in lens]
+        table, at = torch.zeros((len(lens), max(pages)), dtype=torch.int32, device=dev), 0
+        for b, n in enumerate(pages):
+            table[b, :n] = torch.arange(at, at + n)
+            at += n
+        pools, scales, values = [], [], []
+        for _ in range(2):
+            x = rand(at, nkv, page, 128)
+            s = (x.abs().amax(-1) / (127 if kvt == 2 else 7)).contiguous()
+            c = (x / s[..., None]).round()
+            pools.append((c.to(torch.int8) if kvt == 2 else ((c + 8).to(torch.uint8)[..., 0::2] | ((c + 8).to(torch.uint8)[..., 1::2] << 4))).contiguous())
+            scales.append(s)
+            values.append(c.double() * s.double()[..., None])
+        q, pos = rand(len(lens), nq, 128), torch.tensor([n - 1 for n in lens], dtype=torch.int32, device=dev)
+        want = torch.empty((len(lens), nq, 128), dtype=torch.float64, device=dev)
+        for b, n in enumerate(lens):
+            k, v = (x[table[b, :pages[b]].long()].transpose(0, 1).reshape(nkv, -1, 128)[:, :n].repeat_interleave(nq // nkv, 0) for x in values)
+            want[b] = torch.einsum("hn,hnd->hd", (torch.einsum("hd,hnd->hn", q[b].double(), k) / math.sqrt(128)).softmax(-1), v)
+        for i in range(2):
+            K.lib().bonsai_attn_decode_force_cuda_cores(i)
+            try:
+                got = K.attn_decode(q, pos, table, nq, nkv, 128, kvt, page, *pools, *scales, nsplit=8)
+            finally:
+                K.lib().bonsai_attn_decode_force_cuda_cores(0)
+            off[i] += float((got.double() - want).norm() / want.norm())
+    assert off[0] <= 1.03 * off[1]          # means of twelve draws scatter by some 2 %
