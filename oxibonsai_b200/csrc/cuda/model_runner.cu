@@ -23,8 +23,6 @@ int bonsai_f16gemv(const void*, const float*, const float*, float, float*, int, 
 int bonsai_embed_f16(const void*, const int*, float*, int, int, cudaStream_t);
 int bonsai_qknorm_rope_kvstore(const float*, int, const float*, const float*, float, const float*, const float*, const int*,
                                const int*, int, float*, int, int, int, int, int, int, void*, void*, float*, float*, cudaStream_t);
-int bonsai_attn_decode(const float*, const int*, const int*, int, int, int, int, int, int, int, const void*, const void*,
-                       const float*, const float*, int, float*, float*, int*, float*, int, cudaStream_t);
 int bonsai_attn_decode_route(const float*, const int*, const int*, int, int, int, int, int, int, int, const void*, const void*,
                              const float*, const float*, int, float*, float*, int*, float*, int, int, cudaStream_t);
 int bonsai_bitgemv_h2(const void*, const void*, const float*, const float*, float, float*, const float*, int, int, int, cudaStream_t);
@@ -135,13 +133,14 @@ static int qkv_attention_run(Runner& r, const uint64_t* lp, const uint64_t* sp, 
                                               P<void>(pool.k), P<void>(pool.v), nsplit, ws_acc, ws_ml, counters, attn, st);
     if (rc != BONSAI_CUDA_BAD_ARG) return rc;   // bad argument = not a shape of the fused kernel
   }
+  const bool f32_rows = r.ic[IC_FAST] == 0;      // exact mode: quantised rows in f32
   // INT8 / INT4 pages: the tensor-core kernel has two CTAs on an SM; more splits than fill those only add partial sums
-  if (n > 1 && (kvt == 2 || kvt == 3) && hd == 128) nsplit = std::max(1, std::min(nsplit, 2 * 148 / (nkv * n)));
+  if (n > 1 && (kvt == 2 || kvt == 3) && hd == 128 && !f32_rows) nsplit = std::max(1, std::min(nsplit, 2 * 148 / (nkv * n)));
   RC(bonsai_qknorm_rope_kvstore(qkv, qkv_n, P<float>(lp[LP_Q_NORM]), P<float>(lp[LP_K_NORM]), r.eps, P<float>(r.gp[GP_ROPE_COS]),
                                 P<float>(r.gp[GP_ROPE_SIN]), positions, bt, mp, q, n, nq, nkv, hd, kvt, r.ic[IC_PAGE_SIZE], P<void>(pool.k),
                                 P<void>(pool.v), P<float>(pool.ks), P<float>(pool.vs), st));
-  return bonsai_attn_decode(q, positions, bt, mp, n, nq, nkv, hd, kvt, r.ic[IC_PAGE_SIZE], P<void>(pool.k), P<void>(pool.v),
-                            P<float>(pool.ks), P<float>(pool.vs), nsplit, ws_acc, ws_ml, counters, attn, 0, st);
+  return bonsai_attn_decode_route(q, positions, bt, mp, n, nq, nkv, hd, kvt, r.ic[IC_PAGE_SIZE], P<void>(pool.k), P<void>(pool.v),
+                                  P<float>(pool.ks), P<float>(pool.vs), nsplit, ws_acc, ws_ml, counters, attn, 0, f32_rows, st);
 }
 
 // The same for slots 0 .. batch-1: one launch (pair) per run of consecutive slots that share a page format.

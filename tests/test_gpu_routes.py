@@ -1,0 +1,44 @@
+"""Which kernels a call runs: a rule that stopped taking the fast kernel, or took it where it must not, would pass every comparison of numbers."""
+import pytest
+import torch
+
+from oxibonsai_b200.runtime.observability import kernel_histogram
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def kernels(run) -> dict[str, int]:
+    """Names of the kernels of one call of ``run`` and how often each was launched."""
+    table = kernel_histogram(run, iterations=1)
+    if not table:
+        pytest.skip("the profiler recorded no device activity")
+    return {name: row["count"] for name, row in table.items()}
+
+
+def launches(table: dict[str, int], part: str) -> int:
+    return sum(n for name, n in table.items() if part in name)
+
+
+@pytest.fixture(scope="module")
+def wide_head_gguf(tmp_path_factory):
+    from oxibonsai_b200.core import Qwen3Config, write_synthetic_gguf
+    p = tmp_path_factory.mktemp("gguf") / "wide_head.gguf"
+    write_synthetic_gguf(str(p), Qwen3Config(hidden=512, inter=1024, layers=2, heads=4, kv_heads=2, head_dim=128, vocab=1000, context=1024, name="wide"), seed=3)
+    return str(p)
+
+
+def engine(path, kv, max_batch=1, **kw):
+    from oxibonsai_b200.runtime.engine import InferenceEngine
+    return InferenceEngine(path, max_seq_len=1024, kv_dtype=kv, max_batch=max_batch, **kw)
+
+
+@pytest.mark.parametrize("kv", ["q8", "q4"])
+def test_exact_mode_multiplies_quantised_rows_in_f32(kv, wide_head_gguf):
+    ran = {}
+    for exact in (True, False):
+        eng = engine(wide_head_gguf, kv, exact=exact)
+        eng.open_sequence(list(range(1, 20)), 32, 0)
+        ran[exact] = kernels(lambda: eng.runner.step_eager(1))
+    assert launches(ran[True], "attn_decode") == 2 and not launches(ran[True], "attn_decode_quant")
+    assert launches(ran[False], "attn_decode") == 2 == launches(ran[False], "attn_decode_quant")
