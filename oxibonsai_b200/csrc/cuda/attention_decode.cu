@@ -700,6 +700,7 @@ int launch_decode_d(int dpl, int G, dim3 grid, size_t smem, cudaStream_t st, con
 
 int attn_decode_quant(const float*, const int*, const int*, int, int, int, int, int, int, const void*, const void*, const float*, const float*, int, float*,
                       float*, int*, float*, int, float, cudaStream_t);
+bool attn_decode_quant_takes(const float*, int, int, int, const void*, const void*);
 int attn_decode_mma_f16(const float* q, const int* positions, const int* block_table, int max_pages, int batch, int nq, int nkv,
                         int page_size, const void* kpool, const void* vpool, int nsplit, float* ws_acc, float* ws_ml, int* counters,
                         float* out, int extra_len, float sm_scale, cudaStream_t stream);
@@ -736,6 +737,12 @@ int bonsai_qknorm_rope_kvstore(const float* qkv, int qkv_stride, const float* q_
   return launch_status();
 }
 
+// Whether bonsai_attn_decode_route sends quantised rows of this shape to the tensor cores.
+int bonsai_attn_decode_on_tensor_cores(const float* q, int nq, int nkv, int hd, int kvt, int page_size, const void* kpool, const void* vpool, int f32_rows) {
+  using namespace bonsai;
+  return hd == 128 && (kvt == KV_Q8 || kvt == KV_Q4) && !g_attn_force_cuda_cores && !f32_rows && attn_decode_quant_takes(q, nq, nkv, page_size, kpool, vpool);
+}
+
 // q: f32 [batch][nq][hd] -> out f32 [batch][nq][hd].  Context length of sequence b is
 // positions[b] + 1 + extra_len.  ws_acc needs batch*nq*nsplit*hd floats, ws_ml batch*nq*nsplit*2,
 // counters batch*nkv ints that are zero between launches (the kernel resets them).  f32_rows: INT8 / INT4 rows are multiplied in f32 on the
@@ -758,11 +765,9 @@ int bonsai_attn_decode_route(const float* q, const int* positions, const int* bl
                                        ws_ml, counters, out, extra_len, sc, stream);
     if (rc != BONSAI_CUDA_BAD_ARG) return rc;
   }
-  if (hd == 128 && (kvt == KV_Q8 || kvt == KV_Q4) && !g_attn_force_cuda_cores && !f32_rows) {
-    const int rc = attn_decode_quant(q, positions, block_table, max_pages, batch, nq, nkv, kvt, page_size, kpool, vpool, kscale, vscale, nsplit, ws_acc,
-                                     ws_ml, counters, out, extra_len, sc, stream);
-    if (rc != BONSAI_CUDA_BAD_ARG) return rc;
-  }
+  if (bonsai_attn_decode_on_tensor_cores(q, nq, nkv, hd, kvt, page_size, kpool, vpool, f32_rows))
+    return attn_decode_quant(q, positions, block_table, max_pages, batch, nq, nkv, kvt, page_size, kpool, vpool, kscale, vscale, nsplit, ws_acc,
+                             ws_ml, counters, out, extra_len, sc, stream);
   if (hd == 128 && kvt != KV_F32 && (G == 1 || G == 2 || G == 4) && (page_size & (page_size - 1)) == 0) {
     switch (kvt) {
       case KV_F16: return launch_decode_h128<KV_F16>(G, grid, smem, stream, q, positions, block_table, max_pages, pool, nq, sc, ws_acc, ws_ml, counters, out, extra_len);

@@ -350,17 +350,22 @@ static int qa_launch(const QaParams& p, int batch, int nsplit, cudaStream_t st) 
   return e == cudaSuccess ? BONSAI_CUDA_OK : BONSAI_CUDA_LAUNCH_FAILED;
 }
 
-// Head size 128, INT8 (kvt 2) or INT4 (3) rows; BAD_ARG for group sizes, pages and alignments that the caller's other kernels take.
+// Head size 128, INT8 or INT4 rows: the group sizes, pages and alignments of this kernel.
+bool attn_decode_quant_takes(const float* q, int nq, int nkv, int page_size, const void* kpool, const void* vpool) {
+  const int G = nq / nkv;
+  return (G == 1 || G == 2 || G == 4 || G == 8) && page_size >= 16 && (page_size & (page_size - 1)) == 0 &&
+         ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(kpool) | reinterpret_cast<uintptr_t>(vpool)) & 15) == 0;
+}
+
+// kvt 2 (INT8) or 3 (INT4); BAD_ARG for what the caller's other kernels take.
 int attn_decode_quant(const float* q, const int* positions, const int* block_table, int max_pages, int batch, int nq, int nkv, int kvt, int page_size,
                       const void* kpool, const void* vpool, const float* kscale, const float* vscale, int nsplit, float* ws_acc, float* ws_ml, int* counters,
                       float* out, int extra_len, float sm_scale, cudaStream_t st) {
-  const int G = nq / nkv;
-  if ((reinterpret_cast<uintptr_t>(q) & 15) != 0 || page_size < 16 || (page_size & (page_size - 1)) != 0 || ((reinterpret_cast<uintptr_t>(kpool) | reinterpret_cast<uintptr_t>(vpool)) & 15) != 0)
-    return BONSAI_CUDA_BAD_ARG;
+  if (!attn_decode_quant_takes(q, nq, nkv, page_size, kpool, vpool)) return BONSAI_CUDA_BAD_ARG;
   QaParams p{q, positions, block_table, (const uint8_t*)kpool, (const uint8_t*)vpool, kscale, vscale, ws_acc, ws_ml, counters, out,
              max_pages, nq, nkv, page_size, extra_len, sm_scale};
 #define BONSAI_QA(g) (kvt == 2 ? qa_launch<2, g>(p, batch, nsplit, st) : qa_launch<3, g>(p, batch, nsplit, st))
-  switch (G) {
+  switch (nq / nkv) {
     case 1: return BONSAI_QA(1);
     case 2: return BONSAI_QA(2);
     case 4: return BONSAI_QA(4);

@@ -23,6 +23,7 @@ int bonsai_f16gemv(const void*, const float*, const float*, float, float*, int, 
 int bonsai_embed_f16(const void*, const int*, float*, int, int, cudaStream_t);
 int bonsai_qknorm_rope_kvstore(const float*, int, const float*, const float*, float, const float*, const float*, const int*,
                                const int*, int, float*, int, int, int, int, int, int, void*, void*, float*, float*, cudaStream_t);
+int bonsai_attn_decode_on_tensor_cores(const float*, int, int, int, int, int, const void*, const void*, int);
 int bonsai_attn_decode_route(const float*, const int*, const int*, int, int, int, int, int, int, int, const void*, const void*,
                              const float*, const float*, int, float*, float*, int*, float*, int, int, cudaStream_t);
 int bonsai_bitgemv_h2(const void*, const void*, const float*, const float*, float, float*, const float*, int, int, int, cudaStream_t);
@@ -134,8 +135,9 @@ static int qkv_attention_run(Runner& r, const uint64_t* lp, const uint64_t* sp, 
     if (rc != BONSAI_CUDA_BAD_ARG) return rc;   // bad argument = not a shape of the fused kernel
   }
   const bool f32_rows = r.ic[IC_FAST] == 0;      // exact mode: quantised rows in f32
-  // INT8 / INT4 pages: the tensor-core kernel has two CTAs on an SM; more splits than fill those only add partial sums
-  if (n > 1 && (kvt == 2 || kvt == 3) && hd == 128 && !f32_rows) nsplit = std::max(1, std::min(nsplit, 2 * 148 / (nkv * n)));
+  // INT8 / INT4 pages on the tensor cores: two CTAs on an SM; more splits than fill those only add partial sums
+  if (n > 1 && bonsai_attn_decode_on_tensor_cores(q, nq, nkv, hd, kvt, r.ic[IC_PAGE_SIZE], P<void>(pool.k), P<void>(pool.v), f32_rows))
+    nsplit = std::max(1, std::min(nsplit, 2 * 148 / (nkv * n)));
   RC(bonsai_qknorm_rope_kvstore(qkv, qkv_n, P<float>(lp[LP_Q_NORM]), P<float>(lp[LP_K_NORM]), r.eps, P<float>(r.gp[GP_ROPE_COS]),
                                 P<float>(r.gp[GP_ROPE_SIN]), positions, bt, mp, q, n, nq, nkv, hd, kvt, r.ic[IC_PAGE_SIZE], P<void>(pool.k),
                                 P<void>(pool.v), P<float>(pool.ks), P<float>(pool.vs), st));

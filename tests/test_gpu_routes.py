@@ -1,4 +1,6 @@
 """Which kernels a call runs: a rule that stopped taking the fast kernel, or took it where it must not, would pass every comparison of numbers."""
+import json
+
 import pytest
 import torch
 
@@ -14,6 +16,22 @@ def kernels(run) -> dict[str, int]:
     if not table:
         pytest.skip("the profiler recorded no device activity")
     return {name: row["count"] for name, row in table.items()}
+
+
+def grids(run, part: str, tmp_path) -> list[list[int]]:
+    """Grids of the launches of one call of ``run`` whose kernel's name holds ``part``."""
+    from torch.profiler import ProfilerActivity, profile
+    run()
+    torch.cuda.synchronize()
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        run()
+        torch.cuda.synchronize()
+    prof.export_chrome_trace(str(tmp_path / "trace.json"))
+    events = json.loads((tmp_path / "trace.json").read_text())["traceEvents"]
+    out = [e["args"]["grid"] for e in events if part in e.get("name", "") and "grid" in e.get("args", {})]
+    if not out and not any("grid" in e.get("args", {}) for e in events):
+        pytest.skip("the profiler recorded no launches")
+    return out
 
 
 def launches(table: dict[str, int], part: str) -> int:
@@ -42,3 +60,15 @@ def test_exact_mode_multiplies_quantised_rows_in_f32(kv, wide_head_gguf):
         ran[exact] = kernels(lambda: eng.runner.step_eager(1))
     assert launches(ran[True], "attn_decode") == 2 and not launches(ran[True], "attn_decode_quant")
     assert launches(ran[False], "attn_decode") == 2 == launches(ran[False], "attn_decode_quant")
+
+
+@pytest.mark.parametrize("page,splits", [(8, 9), (64, 4)])
+def test_splits_of_quantised_attention_follow_the_kernel(page, splits, tmp_path):
+    """Pages of eight tokens stay on the CUDA cores, four CTAs an SM; the tensor-core kernel has two."""
+    from oxibonsai_b200.core import Qwen3Config, write_synthetic_gguf
+    path = str(tmp_path / "groups.gguf")
+    write_synthetic_gguf(path, Qwen3Config(hidden=512, inter=1024, layers=1, heads=16, kv_heads=8, head_dim=128, vocab=1000, context=1024, name="groups"), seed=3)
+    eng = engine(path, "q8", max_batch=8, page_size=page)
+    for slot in range(8):
+        eng.open_sequence(list(range(1, 20)), 32, slot)
+    assert grids(lambda: eng.runner.step_eager(8), "attn_decode", tmp_path) == [[8, splits, 8]]
