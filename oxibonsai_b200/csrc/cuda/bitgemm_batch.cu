@@ -23,6 +23,9 @@
 #include <cuda.h>
 #include <cuda_fp16.h>
 
+#include <atomic>
+#include <mutex>
+
 #include "common.cuh"
 #include "tcgen05.cuh"
 
@@ -369,13 +372,17 @@ static cudaLaunchConfig_t gb_config(cudaLaunchAttribute* attr, int clusters, int
   return cfg;
 }
 
-// How many clusters of each size the device holds at once (the CTA's shared memory allows one per SM whatever the tokens are).
+// How many clusters of each size the device holds at once (the CTA's shared memory allows one per SM whatever the tokens are); null when the
+// device does not say.  The table is published behind its flag: threads that come first together ask one after another.
 static const int* gb_clusters() {
   static int held[64][kGbMaxSplit + 1];
-  static bool known[64] = {};
+  static std::atomic<bool> known[64];
+  static std::mutex asking;
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
-  if (!known[dev]) {
+  if (known[dev].load(std::memory_order_acquire)) return held[dev];
+  std::lock_guard<std::mutex> lock(asking);
+  if (!known[dev].load(std::memory_order_relaxed)) {
     if (cudaFuncSetAttribute(bitgemm_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024) != cudaSuccess) return nullptr;
     for (int s = 1; s <= kGbMaxSplit; ++s) {
       cudaLaunchAttribute attr[2];
@@ -385,7 +392,7 @@ static const int* gb_clusters() {
       held[dev][s] = n;
     }
     (void)cudaGetLastError();
-    known[dev] = true;
+    known[dev].store(true, std::memory_order_release);
   }
   return held[dev];
 }

@@ -72,3 +72,37 @@ def test_splits_of_quantised_attention_follow_the_kernel(page, splits, tmp_path)
     for slot in range(8):
         eng.open_sequence(list(range(1, 20)), 32, slot)
     assert grids(lambda: eng.runner.step_eager(8), "attn_decode", tmp_path) == [[8, splits, 8]]
+
+
+def test_threads_that_make_the_first_batch_product_together_get_the_same_rows():
+    """The table of what the device holds is filled by the first call: in a process of its own, eight threads start with it at once."""
+    import subprocess
+    import sys
+    code = """
+import threading, torch
+from oxibonsai_b200.ops import cuda_ops as K
+dev = torch.device("cuda:0")
+w = K.PlanarWeight(512, 1024, dev)
+w.codes.random_(-2**31, 2**31 - 1)
+w.scales.fill_(0.01)
+x = torch.randn((5, 1024), device=dev).half()
+K._gp()
+torch.cuda.synchronize()
+out, go = [None] * 8, threading.Barrier(8)
+def run(i):
+    torch.cuda.set_device(0)
+    with torch.cuda.stream(torch.cuda.Stream()):
+        y, st = torch.empty((5, 512), device=dev), torch.zeros(1, dtype=torch.int32, device=dev)
+        torch.cuda.current_stream().synchronize()
+        go.wait()
+        K.bitgemm_batch(w, x, out=y, status=st)
+        torch.cuda.current_stream().synchronize()
+        out[i] = y
+threads = [threading.Thread(target=run, args=(i,)) for i in range(8)]
+[t.start() for t in threads]
+[t.join() for t in threads]
+assert all(torch.equal(out[0], y) for y in out)
+print("alike")
+"""
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "alike" in r.stdout, r.stderr[-2000:]
