@@ -129,7 +129,7 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? 1 : 2) attn_decode_quant_ke
     }
     top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 1));
     top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 2));
-    const float unit = top > 1e-30f && top < 1e30f ? qa_pow2(top) * 0.0078125f : 1.0f;
+    const float unit = top > 1e-30f && top < INFINITY ? qa_pow2(top) * 0.0078125f : 1.0f;
     const float up = 1.0f / unit;            // a power of two: exact
     q_back = unit;
 #pragma unroll
@@ -210,7 +210,7 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? 1 : 2) attn_decode_quant_ke
     top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 1));
     top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 2));
     // the head's largest weight of the tile comes to [2^14, 2^15); weights below 2^-110 lose digits
-    const float unit = top < 1e30f ? qa_pow2(fmaxf(top, 7.8e-34f)) * (1.0f / 16384.0f) : 1.0f, up = 1.0f / unit;
+    const float unit = top < INFINITY ? qa_pow2(fmaxf(top, 7.8e-34f)) * (1.0f / 16384.0f) : 1.0f, up = 1.0f / unit;
     uint32_t pa[4];
 #pragma unroll
     for (int n = 0; n < 2; ++n) qa_split(x[n][0] * up, x[n][1] * up, pa[2 * n], pa[2 * n + 1]);

@@ -488,3 +488,22 @@ def test_quantised_decode_attention_is_no_further_off_than_f32_products(nq, nkv,
                 K.lib().bonsai_attn_decode_force_cuda_cores(0)
             off[i] += float((got.double() - want).norm() / want.norm())
     assert off[0] <= 1.03 * off[1]          # means of twelve draws scatter by some 2 %
+
+
+@pytest.mark.parametrize("kvt", [2, 3])
+@pytest.mark.parametrize("size", [1e30, 2e35])
+def test_quantised_decode_attention_holds_large_values(kvt, size):
+    """Rows whose scales come close to the end of f32's range (and, times codes, stay inside): weights keep their digits, nothing overflows."""
+    from oxibonsai_b200.ops import cuda_ops as K
+    dev, nq, nkv, n = _dev(), 4, 2, 40
+    g = torch.Generator(device=dev).manual_seed(1)
+    codes = [torch.randint(-7, 8, (1, nkv, 64, 128), device=dev, generator=g) for _ in range(2)]
+    pools = [(c.to(torch.int8) if kvt == 2 else ((c + 8).to(torch.uint8)[..., 0::2] | ((c + 8).to(torch.uint8)[..., 1::2] << 4))).contiguous() for c in codes]
+    scales = [torch.full((1, nkv, 64), 0.05, device=dev), torch.full((1, nkv, 64), size, device=dev)]
+    q = torch.randn((1, nq, 128), device=dev, generator=g)
+    table, pos = torch.zeros((1, 1), dtype=torch.int32, device=dev), torch.tensor([n - 1], dtype=torch.int32, device=dev)
+    got = K.attn_decode(q, pos, table, nq, nkv, 128, kvt, 64, *pools, *scales, nsplit=2)
+    k, v = (c[0, :, :n].double().repeat_interleave(nq // nkv, 0) * float(s.double()[0, 0, 0]) for c, s in zip(codes, scales))
+    p = (torch.einsum("hd,hnd->hn", q[0].double(), k) / 128 ** 0.5).softmax(-1)
+    want, terms = torch.einsum("hn,hnd->hd", p, v), torch.einsum("hn,hnd->hd", p, v.abs())
+    assert ((got[0].double() - want).abs() <= 2.0 ** -17 * terms).all()          # scores of some 4 x 2^-20 and weighted values of 2^-19
