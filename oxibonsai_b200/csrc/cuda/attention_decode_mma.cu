@@ -109,11 +109,11 @@ __global__ void __launch_bounds__(NW * 32, 8 / NW) attn_decode_mma_kernel(MmaAtt
   const int len = p.positions[b] + 1 + p.extra_len;
   int chunk = (len + nsplit - 1) / nsplit;
   // Tiles never straddle a split boundary or (page_size >= 16) a page, and a split has at least a tile for each of its warps: more splits
-  // would only lengthen the merge.  Those that are left without tokens (parts .. nsplit - 1) leave, a single part needs no merge
+  // would only lengthen the merge.  Those that are left without tokens (parts .. nsplit - 1, never the first) leave, a single part needs no merge
   // (16 splits: 24 tokens of 16 / 8 heads 6.3 -> 4.1 us; 14 splits: five sequences of 90 to 700 12.7 -> 9.7 us).
   chunk = max((chunk + kMmaTile - 1) & ~(kMmaTile - 1), kMmaTile * NW);
   const int t0 = split * chunk, t1 = min(len, t0 + chunk);
-  if (!CL && t0 >= len) return;
+  if (!CL && split > 0 && t0 >= len) return;
   const int ntiles = t1 > t0 ? (t1 - t0 + kMmaTile - 1) / kMmaTile : 0;
   const int* bt = p.block_table + (size_t)b * p.max_pages;
   const int pshift = 31 - __clz(p.page_size), pmask = p.page_size - 1;
@@ -147,7 +147,7 @@ __global__ void __launch_bounds__(NW * 32, 8 / NW) attn_decode_mma_kernel(MmaAtt
   if (p.qkv != nullptr) {
     // a warp per item: the G query heads, plus the new token's K and V rows in the CTA that owns position len - 1
     float* qs = sh;                                          // [G][128] normalised, rotated, scaled queries
-    const int pos = len - 1;
+    const int pos = max(len - 1, 0);
     const bool owner = pos >= t0 && pos < t1;
     const float* raw = p.qkv + (size_t)b * p.qkv_stride;
     for (int it = warp; it < G + (owner ? 2 : 0); it += kMmaWarps) {
@@ -259,7 +259,7 @@ __global__ void __launch_bounds__(NW * 32, 8 / NW) attn_decode_mma_kernel(MmaAtt
     __syncwarp();   // every lane is done with this buffer before the next iteration's copies overwrite it
   }
   cp_async_wait<0>();
-  const int parts = (len + chunk - 1) / chunk;      // a division: not on the way to the first tile
+  const int parts = max(1, (len + chunk - 1) / chunk);      // a division: not on the way to the first tile
   l += __shfl_xor_sync(0xffffffffu, l, 1);
   l += __shfl_xor_sync(0xffffffffu, l, 2);
 

@@ -71,9 +71,9 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? 1 : 2) attn_decode_quant_ke
   const int len = p.positions[b] + 1 + p.extra_len;
   int chunk = (len + nsplit - 1) / nsplit;
   // Tiles of 16 never straddle a split or (page_size is a multiple of 16) a page, and a split has a tile for each of its warps at least;
-  // splits that are left without tokens leave, and a single part needs no merge.
+  // splits that are left without tokens leave (the first one stays: rows over no tokens are zero), and a single part needs no merge.
   chunk = max((chunk + 15) & ~15, NW * 16);
-  if (split * chunk >= len) return;
+  if (split > 0 && split * chunk >= len) return;
   const int t0 = split * chunk, t1 = min(len, t0 + chunk), ntiles = t1 > t0 ? (t1 - t0 + 15) >> 4 : 0;
   const int* bt = p.block_table + (size_t)b * p.max_pages;
   const int pshift = 31 - __clz(p.page_size), pmask = p.page_size - 1;
@@ -256,7 +256,7 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? 1 : 2) attn_decode_quant_ke
   }
   l += __shfl_xor_sync(0xffffffffu, l, 1);
   l += __shfl_xor_sync(0xffffffffu, l, 2);
-  const int parts = (len + chunk - 1) / chunk;
+  const int parts = max(1, (len + chunk - 1) / chunk);
 
   // ---- the CTA's warps, then the splits: as in attention_decode.cu ------------------------------------------------------------------------------
   constexpr int stride = hd + 2;

@@ -507,3 +507,19 @@ def test_quantised_decode_attention_holds_large_values(kvt, size):
     p = (torch.einsum("hd,hnd->hn", q[0].double(), k) / 128 ** 0.5).softmax(-1)
     want, terms = torch.einsum("hn,hnd->hd", p, v), torch.einsum("hn,hnd->hd", p, v.abs())
     assert ((got[0].double() - want).abs() <= 2.0 ** -17 * terms).all()          # scores of some 4 x 2^-20 and weighted values of 2^-19
+
+
+@pytest.mark.parametrize("kvt", [0, 1, 2, 3])
+@pytest.mark.parametrize("nsplit", [1, 4])
+def test_decode_attention_over_no_tokens_is_zero(kvt, nsplit):
+    """A sequence without a single key beside one that has some: its rows are written, as zeros."""
+    from oxibonsai_b200.ops import cuda_ops as K
+    dev, nq, nkv = _dev(), 4, 2
+    g = torch.Generator(device=dev).manual_seed(1)
+    pools = [torch.randint(-7, 8, (2, nkv, 64, 64 if kvt == 3 else 128), device=dev, generator=g).to(K.KV_DTYPES[kvt]) for _ in range(2)]
+    scales = [torch.ones((2, nkv, 64), device=dev) if kvt >= 2 else None for _ in range(2)]
+    q = torch.randn((2, nq, 128), device=dev, generator=g)
+    table, pos = torch.tensor([[0], [1]], dtype=torch.int32, device=dev), torch.tensor([-1, 9], dtype=torch.int32, device=dev)
+    out = torch.full((2, nq, 128), float("nan"), device=dev)
+    K.attn_decode(q, pos, table, nq, nkv, 128, kvt, 64, *pools, *scales, nsplit=nsplit, out=out)
+    assert not out[0].any() and torch.isfinite(out[1]).all() and out[1].any()
