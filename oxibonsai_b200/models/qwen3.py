@@ -411,13 +411,24 @@ class Qwen3Runner(SlotState):
                   "sm_ml": torch.zeros((sm, nq, ss, 2), **f32), "sm_ctr": torch.zeros(sm * max(1, nkv), **i32)})
         if b["gemm_ws"] is None:
             b["gemm_ws"] = self._gemm_ws = K.new_gemm_workspace(dev)
-        b["wexp"] = torch.empty(self._wexp_elems(), **f16)
+        b["wexp"] = None                     # see _prompt_scratch
         order = ["tokens", "positions", "h", "xn", "qkv", "q", "attn", "act", "status", "sm_attn", "sm_acc", "sm_ml", "sm_ctr"]
-        ptrs = [b[k].data_ptr() for k in order] + [b["wexp"].data_ptr(), b["wexp"].numel(), b["gemm_ws"].data_ptr(), b["gemm_ws"].numel()]
+        ptrs = [b[k].data_ptr() for k in order] + [0, 0, b["gemm_ws"].data_ptr(), b["gemm_ws"].numel()]
         assert len(ptrs) == K._pf().bonsai_runner_prefill_ptr_count()
         b["ptrs"] = (C.c_uint64 * len(ptrs))(*ptrs)
         self._pf = b
         return b
+
+    def _prompt_scratch(self, b: dict, n_tokens: int, slot: int) -> None:
+        """The scratch matrix that prompt chunks of ``n_tokens`` use (expanded weights; f16 rows of a quantised cache): allocated by the first
+        prompt that does, so that a runner of decode steps and short prompts has none.  Without room for it, chunks keep to the kernels
+        that need none."""
+        if b["wexp"] is None and (n_tokens > 64 or (n_tokens > K._pf().bonsai_runner_small_chunk() and self.slot_formats[slot] in (K.KV_Q8, K.KV_Q4))):
+            try:
+                b["wexp"] = torch.empty(self._wexp_elems(), dtype=torch.float16, device=self.device)
+            except torch.OutOfMemoryError:
+                b["wexp"] = torch.empty(0, dtype=torch.float16, device=self.device)
+            b["ptrs"][len(b["ptrs"]) - 4], b["ptrs"][len(b["ptrs"]) - 3] = b["wexp"].data_ptr(), b["wexp"].numel()
 
     def prefill(self, tokens: torch.Tensor, slot: int, pos0: int = 0, chunk: int = 1024) -> None:
         """Runs prompt ``tokens`` (int32 device tensor) of the sequence in ``slot`` starting at position ``pos0``;
@@ -425,6 +436,7 @@ class Qwen3Runner(SlotState):
         n = tokens.numel()
         chunk = max(1, min(chunk, self.prefill_capacity))
         b = self._prefill_buffers(min(chunk, max(n, 1)))
+        self._prompt_scratch(b, min(chunk, n), slot)
         lib = K._pf()
         done = 0
         while done < n:
@@ -448,6 +460,7 @@ class Qwen3Runner(SlotState):
         call) for the rejection test of sampled speculative decoding."""
         T = tokens.numel()
         b = self._prefill_buffers(max(64, T))
+        self._prompt_scratch(b, T, slot)
         with nvtx.range(f"verify[slot={slot},pos={pos0},T={T}]"):
             return self._verify_logits(tokens, slot, pos0, T, b)
 
@@ -472,7 +485,7 @@ class Qwen3Runner(SlotState):
     def _wexp_elems(self) -> int:
         """f16 scratch for expanded weights: the largest matrix, at most 104 MB (slabs of it then pass through L2), at least 256 rows."""
         mats = [m for lw in self.w.layers[:1] for m in (lw.qkv, lw.o, lw.gate_up, lw.down)]
-        return max(256 * max(m.k for m in mats), min(52 << 20, max(m.n * m.k for m in mats)))
+        return max(256 * max((m.k for m in mats), default=0), min(52 << 20, max((m.n * m.k for m in mats), default=0)))
 
     def prefill_launches(self, n_tokens: int, chunk: int = 1024) -> int:
         """Number of kernel launches of a prompt on one GPU over f16 pages."""

@@ -106,3 +106,24 @@ print("alike")
 """
     r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and "alike" in r.stdout, r.stderr[-2000:]
+
+
+def test_prompt_scratch_is_allocated_by_the_first_long_prompt(wide_head_gguf):
+    """Decode steps, verification and short prompts run without it; where it does not fit, long prompts run without it too."""
+    prompt = [int(t) for t in torch.randint(0, 1000, (200,), generator=torch.Generator().manual_seed(1))]
+    tokens = []
+    for room in (True, False):
+        eng = engine(wide_head_gguf, "f16", max_batch=2)
+        eng.open_sequence(prompt[:40], 64, 0)
+        eng.open_sequence(prompt[:64], 80, 1)
+        eng.step_batch([40, 64])
+        eng.verify_greedy([1, 2, 3], 41)
+        assert eng.runner._pf["wexp"] is None
+        if not room:
+            eng.runner._wexp_elems = lambda: 1 << 45
+        tokens.append(eng.open_sequence(prompt, 300, 0))
+        assert eng.runner._pf["wexp"].numel() == (eng.runner._wexp_elems() if room else 0)
+        ran = kernels(lambda: eng.runner.prefill(torch.tensor(prompt, dtype=torch.int32, device=DEV), 0, 0))
+        assert launches(ran, "expand_rows") == launches(ran, "gemm_pair") == (8 if room else 0) and launches(ran, "bitgemm_prefill") == (0 if room else 8)
+        tokens.append(eng.runner.logits[0].clone())
+    assert tokens[0] == tokens[2] and torch.equal(tokens[1], tokens[3])
