@@ -813,8 +813,8 @@ int bonsai_bitgemm_prefill_ws(const void* codes, const void* scales, const void*
   if (K % 128 != 0 || n_rows < 1 || T < 1 || epi < 0 || epi > 3 || x_ld % 8 != 0) return BONSAI_CUDA_BAD_ARG;
   if ((epi <= 1 && out_f32 == nullptr) || (epi == 1 && residual == nullptr) || (epi >= 2 && out_f16 == nullptr)) return BONSAI_CUDA_BAD_ARG;
   // dense operands and more than one 64-token tile: pairs of SMs (gemm_pair.cu; 4096 x 4096 and 128 tokens: 31.5 -> 18.9 us, 4096
-  // tokens: 120 -> 104 us)
-  if (dense_w != nullptr && T > 64 && x_ld >= K && status != nullptr && ((reinterpret_cast<uintptr_t>(dense_w) | reinterpret_cast<uintptr_t>(x_f16)) & 15) == 0)
+  // tokens: 120 -> 104 us); the same sums, bit for bit
+  if (dense_w != nullptr && T > 64 && (epi != 2 || (n_rows % 2 == 0 && out_ld >= (n_rows / 2 + 7) / 8 * 8)) && x_ld >= K && status != nullptr && ((reinterpret_cast<uintptr_t>(dense_w) | reinterpret_cast<uintptr_t>(x_f16)) & 15) == 0)
     return bonsai_gemm_pair(dense_w, x_f16, x_ld, out_f32, residual, out_f16, status, n_rows, K, T, epi, out_ld, sms, 0, stream);
   const int tok = T <= 64 ? 64 : 256;
   CUtensorMap xmap, amap;

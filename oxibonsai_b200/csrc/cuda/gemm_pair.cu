@@ -299,15 +299,16 @@ static int launch_pair(const void* w, const void* x, int x_ld, GpParams p, int s
 extern "C" {
 
 // x_f16 [T][x_ld], w_f16 [n_rows][K] in one K order, 16-byte aligned, K a multiple of 64, x_ld of 8.  epi 0: out_f32 = W x; 1: out_f32 =
-// residual + W x; 2: out_f16 = SwiGLU over interleaved gate / up rows (paired-K order); 3: out_f16 = W x.  tile_tok: tokens per tile
-// (a multiple of 16 up to 256), 0 = chosen here.
+// residual + W x; 2: out_f16 = SwiGLU over interleaved gate / up rows (paired-K order, out_ld at least n_rows / 2 rounded up to 8); 3: out_f16 =
+// W x.  tile_tok: tokens per tile (a multiple of 16 up to 256), 0 = chosen here.
 int bonsai_gemm_pair(const void* w_f16, const void* x_f16, int x_ld, float* out_f32, const float* residual, void* out_f16, int* status, int n_rows,
                      int K, int T, int epi, int out_ld, int sms, int tile_tok, cudaStream_t stream) {
   using namespace bonsai;
   if (K < 64 || K % 64 != 0 || n_rows < 1 || T < 1 || epi < 0 || epi > 3 || x_ld < K || x_ld % 8 != 0 || status == nullptr) return BONSAI_CUDA_BAD_ARG;
   if (((reinterpret_cast<uintptr_t>(w_f16) | reinterpret_cast<uintptr_t>(x_f16)) & 15) != 0) return BONSAI_CUDA_BAD_ARG;
   if (tile_tok < 0 || tile_tok > 256 || tile_tok % 16 != 0) return BONSAI_CUDA_BAD_ARG;
-  if ((epi <= 1 && out_f32 == nullptr) || (epi == 1 && residual == nullptr) || (epi >= 2 && out_f16 == nullptr) || (epi == 2 && n_rows % 2 != 0))
+  if ((epi <= 1 && out_f32 == nullptr) || (epi == 1 && residual == nullptr) || (epi >= 2 && out_f16 == nullptr) ||
+      (epi == 2 && (n_rows % 2 != 0 || out_ld < (n_rows / 2 + 7) / 8 * 8)))
     return BONSAI_CUDA_BAD_ARG;
   return launch_pair(w_f16, x_f16, x_ld, GpParams{out_f32, residual, (__half*)out_f16, status, n_rows, K, T, epi, out_ld, tile_tok}, sms, stream);
 }

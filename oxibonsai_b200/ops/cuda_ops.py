@@ -786,11 +786,12 @@ def bitgemm_batch(w: PlanarWeight, x_paired: torch.Tensor, epi: int = 0, residua
 def gemm_pair(w: torch.Tensor, x: torch.Tensor, epi: int = 0, residual: torch.Tensor | None = None, out: torch.Tensor | None = None,
               status: torch.Tensor | None = None, sms: int = 148, tile_tokens: int = 0) -> torch.Tensor:
     """out[T, N] = epilogue(x[T, K] @ w[N, K]^T) for f16 operands on pairs of SMs.  ``epi``: 0 f32 store, 1 f32 residual add, 2 f16 SwiGLU
-    over interleaved gate / up rows (paired-K order), 3 f16 store.  ``tile_tokens``: tokens per tile, 0 = chosen by size."""
+    over interleaved gate / up rows (paired-K order, rows of a multiple of eight), 3 f16 store.  ``tile_tokens``: tokens per tile, 0 = chosen by
+    size."""
     T, n = x.shape[0], w.shape[0]
     assert w.dtype == torch.float16 and x.dtype == torch.float16 and w.is_contiguous() and x.shape[1] == w.shape[1]
     if out is None:
-        out = torch.empty((T, n // 2 if epi == 2 else n), dtype=torch.float32 if epi <= 1 else torch.float16, device=x.device)
+        out = torch.empty((T, (n // 2 + 7) // 8 * 8 if epi == 2 else n), dtype=torch.float32 if epi <= 1 else torch.float16, device=x.device)
     if status is None:
         status = torch.zeros(1, dtype=torch.int32, device=x.device)
     check(_gp().bonsai_gemm_pair(w.data_ptr(), x.data_ptr(), x.stride(0), out.data_ptr() if epi <= 1 else None, ptr(residual),

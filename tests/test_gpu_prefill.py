@@ -199,6 +199,26 @@ def test_pair_gemm_matches_fp64(rows, cols, T, tile, sms):
     assert status.item() == 0
 
 
+@pytest.mark.parametrize("rows", [300, 302, 306, 320])
+def test_pair_gemm_gated_units_stay_inside_their_rows(rows):
+    """SwiGLU rows in paired-K order take whole groups of eight: the output has room for them, and a row without it is refused."""
+    from oxibonsai_b200.ops import cuda_ops as K
+    g = torch.Generator(device=DEV).manual_seed(rows)
+    w, x = (torch.randn(s, device=DEV, generator=g).half() for s in ((rows, 256), (70, 256)))
+    out = K.gemm_pair(w, x, epi=2)
+    unit, width = rows // 2, (rows // 2 + 7) // 8 * 8
+    assert out.shape == (70, width)
+    gate, up = (x.double() @ w[i::2].double().T for i in range(2))
+    want = torch.nn.functional.silu(gate) * up
+    got = torch.zeros((70, (width + 15) // 16 * 16), dtype=torch.float16, device=DEV)
+    got[:, :width] = out
+    got = got[:, K.paired_k_index(got.shape[1], DEV)][:, :unit].double()
+    assert ((got - want).abs() <= 2.0 ** -10 * want.abs() + 1e-3).all()
+    if width != unit:
+        with pytest.raises(K.CudaKernelError):
+            K.gemm_pair(w, x, epi=2, out=torch.empty((70, unit), dtype=torch.float16, device=DEV))
+
+
 @pytest.mark.parametrize("nq,nkv,T,pos0,kvt,page", [(3, 3, 1, 0, 1, 64), (8, 8, 129, 0, 1, 64), (4, 2, 128, 127, 1, 128), (8, 2, 65, 63, 1, 64), (8, 1, 300, 50, 1, 64),
                                                     (8, 2, 200, 77, 2, 16), (8, 2, 31, 400, 3, 64), (4, 1, 513, 1000, 2, 64)])
 def test_tensor_memory_prompt_attention(nq, nkv, T, pos0, kvt, page):
