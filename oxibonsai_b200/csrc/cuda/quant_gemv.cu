@@ -462,6 +462,15 @@ static QsParams qs_params(const void* w, const float* x, int x_ld, const float* 
   return p;
 }
 
+// Rows of x that one launch takes: two where the matrix is streamed, else up to eight.
+template <typename D, typename Q>
+static int qs_rows(const void* w, int N, int K) {
+  QsParams p = qs_params<D>(w, nullptr, K, nullptr, 0.0f, nullptr, nullptr, N, N, K, nullptr);
+  int grid;
+  size_t smem;
+  return qs_plan<Q>(p, grid, smem, 2) ? 2 : 8;
+}
+
 template <typename D, int NB>
 static int qs_launch(const QsParams& p, int grid, size_t smem, cudaStream_t st) {
   static bool configured[64] = {};
@@ -734,6 +743,29 @@ int bonsai_quant_gemv(int type, const void* w, const float* x, const float* norm
 int bonsai_quant_gemv_batched(int type, const void* w, const float* x, int x_ld, const float* norm_w, float eps, float* out,
                               const float* residual, int out_ld, int N, int K, int B, cudaStream_t stream) {
   return bonsai_quant_gemv_batched_status(type, w, x, x_ld, norm_w, eps, out, residual, out_ld, N, K, B, nullptr, stream);
+}
+
+// Rows of x that a launch of bonsai_quant_gemv_batched takes for this matrix (inputs in rows of 16-byte multiples); 0 for a type it does not know.
+int bonsai_quant_gemv_rows(int type, const void* w, int N, int K) {
+  using namespace bonsai;
+  if (N <= 0 || K <= 0) return 0;
+  switch (type) {
+    case 0: return qs_rows<DecF32, QsF32>(w, N, K);
+    case 1: return qs_rows<DecF16, QsF16>(w, N, K);
+    case 30: return qs_rows<DecBF16, QsBF16>(w, N, K);
+    case 2: return qs_rows<DecQ4_0, QsQ4_0>(w, N, K);
+    case 8: return qs_rows<DecQ8_0, QsQ8_0>(w, N, K);
+    case 10: return qs_rows<DecQ2K, QsQ2K>(w, N, K);
+    case 11: return qs_rows<DecQ3K, QsQ3K>(w, N, K);
+    case 12: return qs_rows<DecQ4K, QsQ4K>(w, N, K);
+    case 13: return qs_rows<DecQ5K, QsQ5K>(w, N, K);
+    case 14: return qs_rows<DecQ6K, QsQ6K>(w, N, K);
+    case 15: return qs_rows<DecQ8K, QsQ8K>(w, N, K);
+    case 35: return qs_rows<DecTq2_256, QsTq2_256>(w, N, K);
+    case 43: return qs_rows<DecFp8<false>, QsFp8<false>>(w, N, K);
+    case 44: return qs_rows<DecFp8<true>, QsFp8<true>>(w, N, K);
+    default: return 0;
+  }
 }
 
 int bonsai_swiglu_rows(const float* gu, int gu_ld, float* out, int out_ld, int inter, int T, cudaStream_t stream) {

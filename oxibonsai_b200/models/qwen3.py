@@ -488,7 +488,7 @@ class Qwen3Runner(SlotState):
         return max(256 * max((m.k for m in mats), default=0), min(52 << 20, max((m.n * m.k for m in mats), default=0)))
 
     def prefill_launches(self, n_tokens: int, chunk: int = 1024) -> int:
-        """Number of kernel launches of a prompt on one GPU over f16 pages."""
+        """Number of kernel launches of a prompt on one GPU over f16 pages, the copy of its last row included."""
         full, tail = divmod(n_tokens, chunk)
         small, cfg = K._pf().bonsai_runner_small_chunk(), self.cfg
         lw, elems = self.w.layers[0], self._wexp_elems()

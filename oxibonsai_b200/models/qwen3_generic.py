@@ -7,7 +7,7 @@ forward_cuda_fp8.rs) and their prefill variants (crates/oxibonsai-kernels/src/gp
 cuda_k_quant_prefill/*, cuda_fp8_prefill.rs).  Q / K / V and gate / up are stored as one matrix each where their block
 types agree (rows of a block format concatenate byte for byte), so a decode step is 9 launches per layer, issued from
 Python and captured once per batch size into a CUDA graph.  Up to ``max_batch`` sequences decode together: the batched
-GEMV decodes every weight once and multiplies it into up to eight activation rows, and attention, KV append and the sampler
+GEMV streams every matrix once for two activation rows (a matrix that cannot be streamed, once for eight), and attention, KV append and the sampler
 are the batch kernels of the native engine.  The engine has the slot interface the continuous-batching scheduler drives
 (``begin_sequence`` / ``prefill`` / ``finish_sequence`` / ``step_batch`` / ``move_slot`` / ``close_sequence``).  Prompts of at least ``prefill_min`` tokens run in chunks through the tensor cores: each weight
 matrix is decoded once per chunk into an f16 scratch matrix (csrc/cuda/quant_gemv.cu, bonsai_quant_to_f16) and multiplied
@@ -177,10 +177,8 @@ class GenericQwen3Engine:
         return len(self._slot_range) / self.max_batch
 
     def kernel_launches_per_step(self, batch: int = 1) -> int:
-        lw = self.layers[0]
-        groups = -(-batch // 8)          # the batched GEMV takes eight rows per launch
-        per_layer = 5 + groups * (len(lw["qkv"]) + len(lw["gate_up"]) + 2)       # rope/KV store, attention (3), SwiGLU + projections
-        return per_layer * self.config.layers + 3 + batch + 1                    # embedding (3), LM head per row, sampler
+        products = sum(-(-batch // K.quant_gemv_rows(m.type, m.data, m.n, m.k)) for lw in self.layers for m in (*lw["qkv"], lw["o"], *lw["gate_up"], lw["down"]))
+        return products + 5 * self.config.layers + 3 + batch + 1      # rope/KV store, attention (3), SwiGLU; embedding (3), LM head per row, sampler
 
     # ---- forward ---------------------------------------------------------------------------------------------------------------
     def _forward(self, lo: int, hi: int, sample: bool, masked: bool = False) -> None:

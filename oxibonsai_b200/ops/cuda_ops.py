@@ -213,6 +213,7 @@ _QG_SIG = {
     "bonsai_quant_gemv_status": [_i, _vp, _vp, _vp, _f, _vp, _vp, _i, _i, _vp, _vp],
     "bonsai_swiglu": [_vp, _vp, _vp, _i, _vp],
     "bonsai_quant_gemv_batched_status": [_i, _vp, _vp, _i, _vp, _f, _vp, _vp, _i, _i, _i, _i, _vp, _vp],
+    "bonsai_quant_gemv_rows": [_i, _vp, _i, _i],
     "bonsai_swiglu_rows": [_vp, _i, _vp, _i, _i, _i, _vp],
     "bonsai_quant_to_f16": [_i, _vp, _vp, _i, _i, _i, _vp],
 }
@@ -281,6 +282,11 @@ def quant_gemv_batched(type_id: int, w: torch.Tensor, n: int, k: int, x: torch.T
     check(_qg().bonsai_quant_gemv_batched_status(type_id, w.data_ptr(), x.data_ptr(), x.stride(0), ptr(norm_w), eps, out.data_ptr(), ptr(residual),
                                                  out.stride(0), n, k, B, ptr(status), stream()), "quant_gemv_batched")
     return out
+
+
+def quant_gemv_rows(type_id: int, w: torch.Tensor, n: int, k: int) -> int:
+    """Rows of ``x`` that one launch of :func:`quant_gemv_batched` takes: two where the matrix is streamed, else eight."""
+    return _qg().bonsai_quant_gemv_rows(type_id, w.data_ptr(), n, k)
 
 
 def swiglu_rows(gu: torch.Tensor, inter: int, out: torch.Tensor | None = None) -> torch.Tensor:

@@ -127,3 +127,29 @@ def test_prompt_scratch_is_allocated_by_the_first_long_prompt(wide_head_gguf):
         assert launches(ran, "expand_rows") == launches(ran, "gemm_pair") == (8 if room else 0) and launches(ran, "bitgemm_prefill") == (0 if room else 8)
         tokens.append(eng.runner.logits[0].clone())
     assert tokens[0] == tokens[2] and torch.equal(tokens[1], tokens[3])
+
+
+@pytest.mark.parametrize("n", [20, 40, 65, 300, 1024, 1100])
+def test_prefill_launches_counts_what_a_prompt_launches(n, wide_head_gguf):
+    eng = engine(wide_head_gguf, "f16", max_batch=2)
+    eng._bind_slot(0, 1024)
+    tokens = torch.randint(0, 1000, (min(n, 1024),), dtype=torch.int32, device=DEV)
+    pieces = [tokens] if n <= 1024 else [tokens, tokens[:n - 1024]]
+    ran = sum(launches(kernels(lambda p=p: eng.runner.prefill(p, 0, 0)), "bonsai") for p in pieces)
+    assert eng.runner.prefill_launches(n) == ran - (len(pieces) - 1) + 1
+
+
+@pytest.mark.parametrize("batch", [1, 2, 3, 6])
+def test_launches_of_a_block_format_step(batch, wide_head_gguf, tmp_path):
+    """Products per pair of rows where the matrix is streamed."""
+    from oxibonsai_b200 import cli
+    from oxibonsai_b200.models.qwen3_generic import GenericQwen3Engine
+    path = str(tmp_path / "wide_q8_0.gguf")
+    cli.requantize_gguf(wide_head_gguf, path, "q8_0")
+    eng = GenericQwen3Engine(path, max_seq_len=128, max_batch=6)
+    for slot in range(batch):
+        eng._bind(slot)
+    ran = kernels(lambda: eng._forward(0, batch, True))
+    products = launches(ran, "quant_stream") + launches(ran, "quant_gemv")
+    assert products == 4 * eng.config.layers * -(-batch // 2)
+    assert eng.kernel_launches_per_step(batch) == products + 5 * eng.config.layers + 4 + batch
