@@ -153,3 +153,59 @@ def test_launches_of_a_block_format_step(batch, wide_head_gguf, tmp_path):
     products = launches(ran, "quant_stream") + launches(ran, "quant_gemv")
     assert products == 4 * eng.config.layers * -(-batch // 2)
     assert eng.kernel_launches_per_step(batch) == products + 5 * eng.config.layers + 4 + batch
+
+
+@pytest.mark.parametrize("n", [65, 255, 256, 300])
+def test_weights_expanded_slab_by_slab_give_the_same_prompt(n, tmp_path):
+    """A scratch of 256 rows of the widest matrix: gate / up passes in slabs (the last one smaller) that overwrite one another, below 256 tokens
+    the larger matrices stay packed.  Every sum runs in the same order, so logits and cache are those of one slab, bit for bit."""
+    from oxibonsai_b200.core import Qwen3Config, write_synthetic_gguf
+    path = str(tmp_path / "slabs.gguf")
+    cfg = Qwen3Config(hidden=512, inter=1152, layers=2, heads=4, kv_heads=2, head_dim=128, vocab=1000, context=1024, name="slabs")
+    write_synthetic_gguf(path, cfg, seed=5)
+    prompt = [int(t) for t in torch.randint(0, 1000, (n,), generator=torch.Generator().manual_seed(n))]
+    seen = []
+    for small in (True, False):
+        eng = engine(path, "f16")
+        if small:
+            eng.runner._wexp_elems = lambda: 256 * 1152
+        eng.open_sequence(prompt, n + 8, 0)
+        seen.append((eng.runner.logits[0].clone(), eng.kv.k.clone(), eng.kv.v.clone()))
+        tokens = torch.tensor(prompt, dtype=torch.int32, device=DEV)
+        ran = kernels(lambda: eng.runner.prefill(tokens, 0, 0))
+        # rows of 512, 512, 512 and 1152 inputs: qkv 1024, o 512, gate / up 2304, down 512 of them
+        slabs = (0 if n < 256 else 2) + 1 + (0 if n < 256 else 5) + (0 if n < 256 else 2) if small else 4
+        packed = 3 if small and n < 256 else 0
+        assert launches(ran, "expand_rows") == launches(ran, "gemm_pair") == 2 * slabs and launches(ran, "bitgemm_prefill") == 2 * packed
+    for a, b in zip(*seen):
+        assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("kvt,page,hd,scratch,order,tensor_memory", [(1, 64, 128, 0, 0, True), (1, 16, 128, 0, 0, False), (1, 128, 128, 0, 0, True), (1, 64, 64, 0, 0, False), (1, 64, 128, 0, 1, False),
+                                                                    (0, 64, 128, 0, 0, False), (2, 16, 128, 2 * 2 * 128 * 256, 0, True), (3, 64, 128, 2 * 2 * 128 * 256, 0, True),
+                                                                    (2, 64, 128, 2 * 2 * 128 * 256 - 1, 0, False), (3, 64, 128, 0, 0, False)])
+def test_prompt_attention_takes_the_kernel_of_its_form(kvt, page, hd, scratch, order, tensor_memory):
+    from oxibonsai_b200.ops import cuda_ops as K
+    T, nkv = 200, 2
+    q, pages = torch.randn((T, 4, hd), device=DEV), -(-T // page)
+    row = hd // 2 if kvt == 3 else hd
+    pools = [torch.zeros((pages, nkv, page, row), dtype=K.KV_DTYPES[kvt], device=DEV) for _ in range(2)]
+    scales = [torch.ones((pages, nkv, page), device=DEV) if kvt >= 2 else None for _ in range(2)]
+    table = torch.arange(pages, dtype=torch.int32, device=DEV)
+    room = torch.empty(scratch, dtype=torch.float16, device=DEV) if scratch else None
+    ran = kernels(lambda: K.attn_prefill(q, 0, table, 4, nkv, hd, kvt, page, *pools, *scales, k_order=order, scratch=room))
+    assert launches(ran, "attn_prefill_tc") == int(tensor_memory) and launches(ran, "attn_prefill") == 1
+    assert launches(ran, "kv_to_f16") == int(tensor_memory and kvt >= 2)
+
+
+@pytest.mark.parametrize("kvt,page,nq,part", [(1, 64, 4, "attn_decode_mma"), (2, 64, 4, "attn_decode_quant"), (3, 16, 16, "attn_decode_quant"), (2, 8, 4, "attn_decode_h128"), (3, 24, 4, "attn_decode_kernel"),
+                                              (2, 8, 16, "attn_decode_kernel"), (0, 64, 4, "attn_decode_kernel")])
+def test_decode_attention_takes_the_kernel_of_its_form(kvt, page, nq, part):
+    from oxibonsai_b200.ops import cuda_ops as K
+    nkv, pages = 2, 4
+    pools = [torch.zeros((pages, nkv, page, 64 if kvt == 3 else 128), dtype=K.KV_DTYPES[kvt], device=DEV) for _ in range(2)]
+    scales = [torch.ones((pages, nkv, page), device=DEV) if kvt >= 2 else None for _ in range(2)]
+    table, pos = torch.arange(pages, dtype=torch.int32, device=DEV)[None], torch.tensor([20], dtype=torch.int32, device=DEV)
+    q = torch.randn((1, nq, 128), device=DEV)
+    ran = kernels(lambda: K.attn_decode(q, pos, table, nq, nkv, 128, kvt, page, *pools, *scales, nsplit=4))
+    assert launches(ran, "attn_decode") == 1 == launches(ran, part)
