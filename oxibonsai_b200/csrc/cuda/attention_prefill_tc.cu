@@ -131,6 +131,7 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_prefill_tc_kernel(const __
 
   if (warp == 8) {
     if (tc::elect_one()) {
+      int issued[2] = {0, 0};
       for (int j = 0; j < n1 && !failed; ++j) {
         const int st = j & 1;
         const uint32_t ph = ((j >> 1) & 1) ^ 1;
@@ -150,8 +151,11 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_prefill_tc_kernel(const __
           for (int h = 0; h < 2; ++h)
 #pragma unroll
             for (int x = 0; x < 2; ++x) at_load(dst + x * 16384 + h * 8192, m ? &vmap : &kmap, x * 64, row[h], full);
+          ++issued[m];
         }
       }
+      tc::mbar_drain(k_full, issued[0], 2);
+      tc::mbar_drain(v_full, issued[1], 2);
       if (failed && p.status != nullptr) atomicExch(p.status, kAtStalled);
     }
   } else if (warp == 9) {

@@ -156,31 +156,33 @@ __global__ void __launch_bounds__(kGbThreads, 1) bitgemm_batch_kernel(const __gr
 
   if (warp == kGbCodeWarp) {
     if (tc::elect_one()) {
-      int s = 0;
+      int s = 0, issued = 0;
       uint32_t phase = 1;
       for (int tile = cid; tile < row_tiles && !failed; tile += nclusters)
-        for (int kb = 0; kb < nb; kb += 4) {
+        for (int kb = 0; kb < nb; kb += 4, ++issued) {
           if (!tc::mbar_wait_sleep<100>(&c_empty[s], phase)) { failed = true; break; }
           tc::mbar_arrive_expect_tx(&c_full[s], kGbCodeBytes);
           gb_load(sC + s * kGbCodeBytes, &cmap, (g0 + kb) * 8, tile * 128, &c_full[s]);
           if (++s == nC) { s = 0; phase ^= 1; }
         }
       if (failed) atomicExch(p.status, 1);
+      tc::mbar_drain(c_full, issued, nC);
     }
     __syncwarp();
   } else if (warp == kGbActWarp) {
     if (tc::elect_one()) {
       asm volatile("griddepcontrol.wait;" ::: "memory");
-      int s = 0;
+      int s = 0, issued = 0;
       uint32_t phase = 1;
       for (int tile = cid; tile < row_tiles && !failed; tile += nclusters)
-        for (int kb = 0; kb < nb; ++kb) {
+        for (int kb = 0; kb < nb; ++kb, ++issued) {
           if (!tc::mbar_wait_sleep<100>(&a_empty[s], phase)) { failed = true; break; }
           tc::mbar_arrive_expect_tx(&a_full[s], act_bytes);
           gb_load3(sB + s * act_bytes, &xmap, (g0 + kb) * 2, &a_full[s]);
           if (++s == nA) { s = 0; phase ^= 1; }
         }
       if (failed) atomicExch(p.status, 1);
+      tc::mbar_drain(a_full, issued, nA);
     }
     __syncwarp();
   } else if (warp >= kGbMmaWarp) {

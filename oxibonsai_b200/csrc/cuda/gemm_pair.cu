@@ -114,11 +114,11 @@ __global__ void __launch_bounds__(kGpThreads, 1) __cluster_dims__(2, 1, 1) gemm_
     if (tc::elect_one()) {
       asm volatile("griddepcontrol.wait;" ::: "memory");
       const uint32_t bytes = 2u * (kGpABytes + (uint32_t)tn * kGpBlock);      // both CTAs' weight rows and halves of the tokens
-      int s = 0;
+      int s = 0, issued = 0;
       uint32_t phase = 1;
       for (int tile = cid; tile < ntiles && !failed; tile += nclusters) {
         const int row0 = (tile / tok_tiles) * 256 + (int)rank * 128, tok0 = (tile % tok_tiles) * tn + (int)rank * (tn >> 1);
-        for (int kb = 0; kb < nblk; ++kb) {
+        for (int kb = 0; kb < nblk; ++kb, ++issued) {
           if (!tc::mbar_wait(&empty[s], phase)) { failed = true; break; }
           const uint32_t bar = gp_map(tc::smem_u32(&full[s]), 0);
           if (rank == 0) tc::mbar_arrive_expect_tx(&full[s], bytes);
@@ -128,6 +128,7 @@ __global__ void __launch_bounds__(kGpThreads, 1) __cluster_dims__(2, 1, 1) gemm_
         }
       }
       if (failed) atomicExch(p.status, 1);
+      if (rank == 0) tc::mbar_drain(full, issued, kGpStages);      // both CTAs' copies; the other one waits at the barrier below
     }
   } else if (warp == kGpEpiWarps + 1) {
     if (rank == 0 && tc::elect_one()) {

@@ -288,13 +288,15 @@ __global__ void __launch_bounds__(kQsMaxWarps * 32 + 32, 1) quant_stream_kernel(
   bool failed = false;
   if (warp == nwarps) {
     if (lane == 0) {
-      for (int c = c0; c < c1 && !failed; ++c) {
+      int issued = 0;
+      for (int c = c0; c < c1 && !failed; ++c, ++issued) {
         const int i = c - c0, st = i % p.stages;
         if (!tc::mbar_wait_sleep<40>(&empty[st], ((i / p.stages) & 1) ^ 1)) { failed = true; break; }
         const uint32_t bytes = (uint32_t)(min(p.R, p.N - c * p.R) * p.row_bytes);      // a multiple of 16: the caller checked
         tc::mbar_arrive_expect_tx(&full[st], bytes);
         tc::bulk_g2s(qs_smem + (size_t)st * stage_bytes, p.w + (size_t)c * p.R * p.row_bytes, bytes, &full[st]);
       }
+      tc::mbar_drain(full, issued, p.stages);
     }
   } else {
     asm volatile("griddepcontrol.wait;" ::: "memory");

@@ -8,7 +8,7 @@
 //  * one elected thread issues tcgen05.mma and tcgen05.commit; accumulators live in TMEM and are
 //    read back with tcgen05.ld (warp w may touch TMEM lanes 32*(w%4) .. 32*(w%4)+31);
 //  * every wait has an iteration limit; on expiry the kernel records an error code and leaves,
-//    after freeing any TMEM it holds, so a lost signal can never hang the device.
+//    after its copies have landed (mbar_drain) and any TMEM it holds is free, so a lost signal can never hang the device.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -94,6 +94,12 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, i
     }
   }
   return __shfl_sync(0xffffffffu, ok, 0) != 0;
+}
+
+// The thread that filled a ring of stages leaves when its copies have landed (stage i % stages, its barrier in phase i / stages): behind an expired
+// wait of another warp nothing else would keep the block, and copies in flight would land in the shared memory of the next one.
+__device__ __forceinline__ void mbar_drain(uint64_t* full, int issued, int stages) {
+  for (int i = issued > stages ? issued - stages : 0; i < issued; ++i) mbar_wait(&full[i % stages], (uint32_t)(i / stages) & 1);
 }
 
 // ---- async proxy ------------------------------------------------------------------------------
