@@ -25,6 +25,7 @@
 
 #include <atomic>
 #include <mutex>
+#include <type_traits>
 
 #include "common.cuh"
 #include "tcgen05.cuh"
@@ -230,28 +231,38 @@ __global__ void __launch_bounds__(kGbThreads, 1) bitgemm_batch_kernel(const __gr
         const int end = min(kb0 + 4, nb);
         for (int kb = kb0 + (group + 3 - (it0 + kb0) % 3) % 3; kb < end; kb += 3) {
           const int it = it0 + kb, s = it % kGbSlots;
-          const __half2 d2 = __half2half2(__hmul(next, __float2half(128.0f)));
+          // A masked code is +-2^-7 or 0 and the scale is taken times 128; a row of the warp with a scale of 512 or more (none in earnest) takes the
+          // other order, which leaves every f16 scale in range.
+          const __half d = next;
           next = scale_of(tile, kb + 3);
+          auto block = [&](auto large) {
+            const __half2 up = __half2half2(__float2half(128.0f)), d2 = large ? __half2half2(d) : __hmul2(__half2half2(d), up);
+            auto weights = [&](uint32_t m) {
+              const __half2 c = *reinterpret_cast<const __half2*>(&m), w = large ? __hmul2(__hmul2(c, up), d2) : __hmul2(c, d2);
+              return *reinterpret_cast<const uint32_t*>(&w);
+            };
 #pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const uint4 code = *reinterpret_cast<const uint4*>(sC + cs * kGbCodeBytes + tc::sw128_offset(r, 2 * (kb - kb0) + h));
-            const uint32_t w4[4] = {code.x, code.y, code.z, code.w};
-            uint32_t o[32];
+            for (int h = 0; h < 2; ++h) {
+              const uint4 code = *reinterpret_cast<const uint4*>(sC + cs * kGbCodeBytes + tc::sw128_offset(r, 2 * (kb - kb0) + h));
+              const uint32_t w4[4] = {code.x, code.y, code.z, code.w};
+              uint32_t o[32];
 #pragma unroll
-            for (int wd = 0; wd < 4; ++wd)
+              for (int wd = 0; wd < 4; ++wd)
 #pragma unroll
-              for (int i = 0; i < 4; ++i) {
-                const uint32_t ma = (w4[wd] << (12 - 4 * i)) & 0xA000A000u, mb = (w4[wd] << (13 - 4 * i)) & 0xA000A000u;
-                const __half2 ha = __hmul2(*reinterpret_cast<const __half2*>(&ma), d2), hb = __hmul2(*reinterpret_cast<const __half2*>(&mb), d2);
-                o[wd * 8 + i] = *reinterpret_cast<const uint32_t*>(&ha);
-                o[wd * 8 + 4 + i] = *reinterpret_cast<const uint32_t*>(&hb);
+                for (int i = 0; i < 4; ++i) {
+                  o[wd * 8 + i] = weights((w4[wd] << (12 - 4 * i)) & 0xA000A000u);
+                  o[wd * 8 + 4 + i] = weights((w4[wd] << (13 - 4 * i)) & 0xA000A000u);
+                }
+              if (h == 0) {
+                if (!__all_sync(0xffffffffu, tc::mbar_wait(&empty[s], ((it / kGbSlots) & 1) ^ 1))) return false;
+                tc::tc_fence_after();
               }
-            if (h == 0) {
-              if (!__all_sync(0xffffffffu, tc::mbar_wait(&empty[s], ((it / kGbSlots) & 1) ^ 1))) { failed = true; break; }
-              tc::tc_fence_after();
+              gb_st32(taddr + lanes + s * 64 + h * 32, o);
             }
-            gb_st32(taddr + lanes + s * 64 + h * 32, o);
-          }
+            return true;
+          };
+          if (__any_sync(0xffffffffu, __hge(__habs(d), __float2half(512.0f)))) failed = !block(std::true_type{});
+          else failed = !block(std::false_type{});
           if (failed) break;
           asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
           tc::tc_fence_before();

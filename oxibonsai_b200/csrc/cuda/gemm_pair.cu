@@ -235,13 +235,13 @@ __global__ void __launch_bounds__(256) expand_rows_kernel(const uint32_t* __rest
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const size_t j = i + u * stride;
-      const __half2 d2 = __half2half2(__hmul(sc[u], __float2half(128.0f)));
+      const __half2 d2 = __half2half2(sc[u]), up = __half2half2(__float2half(128.0f));
       const uint32_t v = (j & 1) ? w[u] << 1 : w[u];
       uint32_t o[4];
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
         const uint32_t m = (v << (12 - 4 * k)) & 0xA000A000u;       // +-2^-7 or 0, two weights four inputs apart
-        const __half2 h = __hmul2(*reinterpret_cast<const __half2*>(&m), d2);
+        const __half2 h = __hmul2(__hmul2(*reinterpret_cast<const __half2*>(&m), up), d2);      // in this order any f16 scale stays in range
         o[k] = *reinterpret_cast<const uint32_t*>(&h);
       }
       if (j < total) out[j] = make_uint4(o[0], o[1], o[2], o[3]);

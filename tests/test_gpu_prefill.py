@@ -396,3 +396,25 @@ def test_short_prompts_over_int4_pages_keep_their_kernels(T, wide_head_gguf):
     for a, b in zip(got, (eng.kv.k, eng.kv.v, eng.kv.k_scale, eng.kv.v_scale)):
         assert torch.equal(a, b)
     assert torch.equal(r._pf["h"][:T], h)
+
+
+@pytest.mark.parametrize("scale", [6e-8, 3e-5, 511.5, 512.0, 60000.0])
+def test_batch_gemm_takes_every_scale_of_the_format(scale):
+    """Group scales are f16: the smallest subnormal to the largest, one row with it among ordinary ones and all rows."""
+    from oxibonsai_b200.ops import cuda_ops as K
+    g = torch.Generator(device=DEV).manual_seed(1)
+    raw, _ = _random_quant(TQ2_0_G128, 200, 512, 3)
+    w = K.PlanarWeight(200, 512, torch.device(DEV)).fill_from_gguf(torch.from_numpy(np.array(raw, copy=True)).to(DEV), TQ2_0_G128, 512, 0, 200)
+    x = (torch.randn((20, 512), device=DEV, generator=g) * 1e-3).half()
+    paired = torch.empty_like(x)
+    paired[:, K.paired_k_index(512, DEV)] = x
+    w.scales.fill_(1.0)
+    signs = K.expand_rows(w)[:, K.paired_k_index(512, DEV)].double()      # -1, 0, +1
+    assert signs.abs().max() == 1.0
+    for rows in (slice(77, 78), slice(0, 200)):
+        w.scales.fill_(0.02)
+        w.scales[rows] = scale
+        dense = signs * w.scales.double().repeat_interleave(128, 1)
+        assert torch.equal(K.expand_rows(w)[:, K.paired_k_index(512, DEV)].double(), dense)
+        want, terms = x.double() @ dense.T, x.double().abs() @ dense.abs().T
+        assert ((K.bitgemm_batch(w, paired).double() - want).abs() <= 2.0 ** -23 * 528 * terms).all()
