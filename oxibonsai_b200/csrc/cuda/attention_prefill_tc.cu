@@ -9,7 +9,8 @@
 //   warps 0-3, 4-7   softmax of a tile: a thread owns a query row, reads its 128 scores from TMEM, and leaves P as f16 in their
 //               place, from where the second product takes it as its first operand; no shuffles, no shared memory
 // The sums are rescaled only when a row's maximum has grown by more than 2^8 since its scale was set (P stays below 2^8 then, well
-// inside f16, and keeps its relative precision); a tile that needs it rescales O in TMEM.
+// inside f16, and keeps its relative precision); a tile that needs it rescales O in TMEM.  That, and two query tiles taking turns on the
+// tensor core, are published ideas (FlashAttention-4).
 // Scores are base-2 (scale and log2 e are folded into the f16 queries), sums and maxima f32, P f16, as in the other kernel.
 // Both products of a 128 x 128 tile take 1024 cycles of the tensor core, its 16 K exponentials as many of the MUFU: what is left is
 // their overlap.  Figures at attn_prefill_tc below.
@@ -355,8 +356,8 @@ static int at_launch(const CUtensorMap& kmap, const CUtensorMap& vmap, const AtP
   return e == cudaSuccess ? BONSAI_CUDA_OK : BONSAI_CUDA_LAUNCH_FAILED;
 }
 
-// Measured, 32 / 8 heads (before, on mma.sync): a prompt of 4096 174 us, 788 TFLOP/s (1034); of 777 22.5 us (78.9), INT8 pages 25.1 with
-// their decoding (107.6); 512 tokens behind 8000 160 us (744); 333 behind 1000 33.5 us (121); 64 9.8 us (10.0).  Error against 64 bits
+// Measured, 32 / 8 heads (before, on mma.sync): a prompt of 4096 147 us, 937 TFLOP/s (1034); of 777 19.9 us (78.9), INT8 pages 22.9 with
+// their decoding (107.6); 512 tokens behind 8000 127 us (744); 333 behind 1000 28.3 us (121); 64 10.4 us (10.0).  Error against 64 bits
 // 3.2e-4 in both kernels.
 //
 // Arguments as bonsai_attn_prefill_order (k_order 0).  f16 pages of a multiple of 64 tokens are read in place; INT8 / INT4 pages are

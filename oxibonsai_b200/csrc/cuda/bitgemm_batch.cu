@@ -12,14 +12,14 @@
 //   warps 16-17  MMA issuers, every other block each, with an accumulator of its own;  warp 18: codes (TMA tiles of 128 rows x 512 inputs,
 //                before the kernel ahead has ended);  warp 19: activations
 // Waits, MMAs and commits hold their thread for some 100 cycles each whatever they move, so a block is as deep as the slots allow and
-// two threads issue: blocks of 64 inputs with one issuer took 0.33 us each, 24576 x 4096 and 16 tokens 33 us (now 22; three issuers 24).
+// two threads issue: blocks of 64 inputs with one issuer took 0.33 us each, 24576 x 4096 and 16 tokens 33 us (with two 22, with three 24).
 // The K range of a 128-row tile is cut over the S CTAs of a cluster, so that projections with few rows fill the GPU too; each CTA
 // then adds up, in CTA order, the partial sums of its share of the tokens, which the others wrote into its shared memory.  A cluster
 // takes tile after tile; the accumulators and the exchange are double-buffered.
-// What bounds it: the expanders' chain of wait, expansion and store, some 0.23 us per 16 K weights and SM (1.5 instructions per weight for
-// shift, mask and scale would allow 0.12), and about 5 us per launch.  us at 8 / 32 / 64 tokens (before: the better of bitgemm_hmma and
-// bitgemm_prefill): 6144 x 4096 10.2 / 12.1 / 15.7 (16.0 / 20.7 / 24.0), 4096 x 4096 9.3 / 11.2 / 14.1 (8.4 / 13.3 / 22.1), 24576 x 4096
-// 19.6 / 25.1 / 36.2 (24.5 / 38.3 / 44.7), 4096 x 12288 13.8 / 15.2 / 17.5 (21.4 / 31.5 / 41.1).
+// What bounds it: the expanders' chain of wait, expansion and store, 0.27 us per 16 K weights and SM (a slope over K; 0.28 at 64 tokens; 1.5
+// instructions per weight for shift, mask and scale would allow 0.12), and 5 to 7 us per launch.  us at 8 / 32 / 64 tokens (before: the better of
+// bitgemm_hmma and bitgemm_prefill): 6144 x 4096 10.2 / 12.1 / 15.7 (16.0 / 20.7 / 24.0), 4096 x 4096 9.5 / 11.0 / 13.8 (8.4 / 13.3 / 22.1),
+// 24576 x 4096 19.4 / 24.6 / 36.3 (24.5 / 38.3 / 44.7), 4096 x 12288 13.2 / 14.4 / 17.0 (21.4 / 31.5 / 41.1).
 #include <cuda.h>
 #include <cuda_fp16.h>
 

@@ -24,7 +24,8 @@
 //     in registers and meet in shared memory once at the end; partials are added in warp order, so results do not
 //     depend on timing.
 // Per (tile, group) block a thread issues 16 logic ops, 4 MMAs, 4 loads, 8 integer multiplies that build the
-// zero-padded B operands and a dozen f32 ops: ~0.8 instructions per weight.
+// zero-padded B operands and a dozen f32 ops: ~0.8 instructions per weight.  The whole kernel executes twice that (24576 x 4096: 4.93 M warp
+// instructions, 1.57 per weight): every CTA quantises the activations, and waits, reductions and stores come on top.
 //
 // Epilogues: store, residual add, SwiGLU over interleaved gate/up rows, and the tensor-parallel one: every finished
 // row goes to all peers as one 8-byte {value, tag} store and the same thread polls its own slots for the peers'
