@@ -367,7 +367,7 @@ static int prefill_chunk(Runner& r, const uint64_t* sp, const uint64_t* pp, int 
       float* attn32 = P<float>(pp[PP_SM_ATTN]);
       RC(bonsai_attn_decode_route(q, positions, bt, 0, T, nq, nkv, hd, kvt, r.ic[IC_PAGE_SIZE], P<void>(pool.k),
                                   P<void>(pool.v), P<float>(pool.ks), P<float>(pool.vs), sm_splits, P<float>(pp[PP_SM_ACC]),
-                                  P<float>(pp[PP_SM_ML]), P<int>(pp[PP_SM_CTR]), attn32, 0, settled, st));
+                                  P<float>(pp[PP_SM_ML]), P<int>(pp[PP_SM_CTR]), attn32, 0, settled || r.ic[IC_FAST] == 0, st));
       RC(hm ? bonsai_norm_to_f16_hmma(attn32, qd, nullptr, r.eps, T, qd, attn, qd, st)
             : bonsai_norm_to_f16_paired(attn32, qd, nullptr, r.eps, T, qd, attn, qd, 0, st));
     } else {

@@ -64,6 +64,19 @@ def test_exact_mode_multiplies_quantised_rows_in_f32(kv, wide_head_gguf):
     assert launches(ran[False], "attn_decode") == 2 == launches(ran[False], "attn_decode_quant")
 
 
+@pytest.mark.parametrize("kv", ["q8", "q4"])
+def test_exact_mode_verifies_quantised_rows_in_f32(kv, wide_head_gguf):
+    """Drafted tokens go through a small chunk, whose attention is the decode kernel's (behind 300 tokens: no short INT4 prompt)."""
+    ran = {}
+    for exact in (True, False):
+        eng = engine(wide_head_gguf, kv, exact=exact)
+        eng._bind_slot(0, 400)
+        drafted = torch.arange(1, 6, dtype=torch.int32, device=DEV)
+        ran[exact] = kernels(lambda: eng.runner.verify_logits(drafted, 0, 300))
+    assert launches(ran[True], "attn_decode") == 2 and not launches(ran[True], "attn_decode_quant")
+    assert launches(ran[False], "attn_decode") == 2 == launches(ran[False], "attn_decode_quant")
+
+
 @pytest.mark.parametrize("page,splits", [(8, 9), (64, 4)])
 def test_splits_of_quantised_attention_follow_the_kernel(page, splits, tmp_path):
     """Pages of eight tokens stay on the CUDA cores, four CTAs an SM; the tensor-core kernel has two."""
