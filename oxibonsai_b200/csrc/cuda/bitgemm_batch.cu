@@ -9,17 +9,20 @@
 // and the activations:
 //   warps 0-11   expanders in three groups of four; group e fills the operand slots e and e + 3 of six, 128 inputs each
 //   warps 12-15  epilogue
-//   warps 16-17  MMA issuers, every other block each, with an accumulator of its own;  warp 18: codes (TMA tiles of 128 rows x 512 inputs,
-//                before the kernel ahead has ended);  warp 19: activations
-// Waits, MMAs and commits hold their thread for some 100 cycles each whatever they move, so a block is as deep as the slots allow and
-// two threads issue: blocks of 64 inputs with one issuer took 0.33 us each, 24576 x 4096 and 16 tokens 33 us (with two 22, with three 24).
+//   warps 16-17  MMA issuers, every other block each, with an accumulator of its own;  warp 18: asks L2 for the weights of the CTA's share;
+//                warp 19: activations
 // The K range of a 128-row tile is cut over the S CTAs of a cluster, so that projections with few rows fill the GPU too; each CTA
 // then adds up, in CTA order, the partial sums of its share of the tokens, which the others wrote into its shared memory.  A cluster
 // takes tile after tile; the accumulators and the exchange are double-buffered.
-// What bounds it: the expanders' chain of wait, expansion and store, 0.27 us per 16 K weights and SM (a slope over K; 0.28 at 64 tokens; 1.5
-// instructions per weight for shift, mask and scale would allow 0.12), and 5 to 7 us per launch.  us at 8 / 32 / 64 tokens (before: the better of
-// bitgemm_hmma and bitgemm_prefill): 6144 x 4096 10.2 / 12.1 / 15.7 (16.0 / 20.7 / 24.0), 4096 x 4096 9.5 / 11.0 / 13.8 (8.4 / 13.3 / 22.1),
-// 24576 x 4096 19.4 / 24.6 / 36.3 (24.5 / 38.3 / 44.7), 4096 x 12288 13.2 / 14.4 / 17.0 (21.4 / 31.5 / 41.1).
+// What bounds it: chains.  A block of 16 K weights takes 390 cycles of an SM: the expanders' integer pipe (a mask per pair of weights), and behind it
+// their chain of load, expansion, store and barriers (300 with the expansion taken out, whatever the MMAs and the tokens are; 256 is the
+// tensor pipe at 64 tokens).  Around the blocks stand set-up 2600, the first activations 1900, drain and exchange 2000, sums and stores 600 to 1700 cycles.
+// Two issuers, since waits, MMAs and commits hold their thread for some 100 cycles each whatever they move (one 33 us, three 24 us where two took 22).
+// Codes come by plain loads, 32 bytes of its row per thread: through a ring of TMA copies the barriers cost 484 cycles a block, and copies small
+// enough for one group each kept their thread busy for 420.
+// us at 8 / 24 / 64 tokens behind its norm, weights from memory: 6144 x 4096 9.7 / 10.0 / 10.6 (with codes by TMA, four warps and a store per value in the
+// epilogue 11.0 / 13.3 / 17.4), 4096 x 4096 7.4 / 7.9 / 10.5 (10.0 / 12.3 / 15.8), 24576 x 4096 18.6 / 19.4 / 25.1 (20.5 / 28.3 / 42.2), 4096 x 12288 12.7 / 13.9 / 16.3
+// (13.5 / 16.2 / 21.1).
 #include <cuda.h>
 #include <cuda_fp16.h>
 
@@ -34,8 +37,7 @@ namespace bonsai {
 
 constexpr int kGbSlots = 6;                            // operand slots in TMEM, one 128-input block (64 columns) each
 constexpr int kGbGroups = 3, kGbIssuers = 2;
-constexpr int kGbMaxCodes = 5, kGbMaxActs = 12;        // stages of codes (512 inputs) and of activations (128 inputs)
-constexpr int kGbCodeBytes = 128 * 128;                // 128 rows x 512 inputs
+constexpr int kGbMaxActs = 12;                         // stages of activations (128 inputs)
 constexpr int kGbEpiWarp = 4 * kGbGroups, kGbMmaWarp = kGbEpiWarp + 4, kGbCodeWarp = kGbMmaWarp + kGbIssuers, kGbActWarp = kGbCodeWarp + 1;
 constexpr int kGbThreads = (kGbActWarp + 1) * 32;
 constexpr int kGbMaxSplit = 8;
@@ -43,23 +45,22 @@ constexpr int kGbMaxSplit = 8;
 // meet the same issuer (a wait must not be more than a phase behind its barrier): their numbers are multiples of the issuers.
 constexpr int kGbAccCol = kGbSlots * 64;
 // What shared memory holds beside the exchange.
-__host__ __device__ inline int gb_code_stages(int tok) { return tok == 64 ? 3 : 5; }
-__host__ __device__ inline int gb_act_stages(int tok) { return tok == 64 ? 6 : (tok == 32 ? 10 : 12); }
+__host__ __device__ inline int gb_act_stages(int tok) { return tok == 64 ? 8 : 12; }
+// Tokens that a CTA of a cluster finishes: whole groups of four, which travel as one 16-byte store.
+__host__ __device__ inline int gb_share(int T, int split) { return ((T + split - 1) / split + 3) & ~3; }
 
 struct GbParams {
+  const uint4* codes;      // planar rows of K / 4 bytes
   const __half* scales;
   float* out_f32;          // epi 0, 1
   const float* residual;   // epi 1
   __half* out_f16;         // epi 2: SwiGLU over interleaved gate / up rows, paired-K order
   int* status;
   int n_rows, K, T, epi, out_ld, split, tok;           // tok: T rounded up to 16, 32 or 64
+  int first[kGbMaxSplit + 1];                          // CTA i of a cluster takes the 128-input blocks first[i] .. first[i + 1] - 1
+  uint32_t up[8];                                      // powers of two: see the expansion
 };
 
-__device__ __forceinline__ void gb_load(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
-  asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(tc::smem_u32(dst)),
-               "l"(map), "r"(x), "r"(y), "r"(tc::smem_u32(bar))
-               : "memory");
-}
 __device__ __forceinline__ void gb_load3(void* dst, const CUtensorMap* map, int z, uint64_t* bar) {
   asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %2, %3}], [%4];" ::"r"(tc::smem_u32(dst)),
                "l"(map), "r"(0), "r"(z), "r"(tc::smem_u32(bar))
@@ -86,9 +87,25 @@ __device__ __forceinline__ uint32_t gb_map(uint32_t addr, uint32_t rank) {
   asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
   return r;
 }
-__device__ __forceinline__ void gb_st_remote(uint32_t addr, float v) { asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory"); }
+__device__ __forceinline__ void gb_st_remote4(uint32_t addr, const uint32_t* v) {
+  asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]) : "memory");
+}
 __device__ __forceinline__ void gb_arrive_remote(uint32_t bar) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ bool gb_test(uint64_t* bar, uint32_t parity) {      // asks and does not wait
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(tc::smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+__device__ __forceinline__ void gb_prefetch(const CUtensorMap* map, int x, int y) {
+  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global [%0, {%1, %2}];" ::"l"(map), "r"(x), "r"(y) : "memory");
 }
 // bounded wait that also acquires what other CTAs of the cluster wrote before they arrived; every lane polls
 __device__ __forceinline__ bool gb_wait_cluster(uint64_t* bar, uint32_t parity) {
@@ -107,79 +124,90 @@ __device__ __forceinline__ bool gb_wait_cluster(uint64_t* bar, uint32_t parity) 
 }
 
 __global__ void __launch_bounds__(kGbThreads, 1) bitgemm_batch_kernel(const __grid_constant__ CUtensorMap cmap, const __grid_constant__ CUtensorMap xmap,
-                                                                     GbParams p) {
+                                                                     const __grid_constant__ GbParams p) {
   extern __shared__ uint8_t gb_smem[];
-  uint8_t* base = (uint8_t*)(((uintptr_t)gb_smem + 1023) & ~(uintptr_t)1023);
-  uint8_t* sC = base;                                                       // codes
-  const int nC = gb_code_stages(p.tok), nA = gb_act_stages(p.tok), act_bytes = p.tok * 256;
-  uint8_t* sB = base + nC * kGbCodeBytes;                                    // activations
-  float* sR = reinterpret_cast<float*>(sB + nA * act_bytes);                 // partial sums [2][split][share of the tokens][128 rows]
-  __shared__ uint64_t c_full[kGbMaxCodes], c_empty[kGbMaxCodes], a_full[kGbMaxActs], a_empty[kGbMaxActs], full[kGbSlots], empty[kGbSlots], accf[2], acce[2], red[2];
+  uint8_t* sB = (uint8_t*)(((uintptr_t)gb_smem + 1023) & ~(uintptr_t)1023);  // activations
+  const int nA = gb_act_stages(p.tok), act_bytes = p.tok * 256;
+  float* sR = reinterpret_cast<float*>(sB + nA * act_bytes);                 // partial sums [2][split][share of the tokens / 4][128 rows][4]
+  __shared__ uint64_t a_full[kGbMaxActs], a_empty[kGbMaxActs], full[kGbSlots], empty[kGbSlots], accf[2], acce[2], red[2];
   __shared__ uint32_t tmem_slot;
+  __shared__ int s_failed;
   const int t = threadIdx.x, warp = __shfl_sync(0xffffffffu, t >> 5, 0), lane = t & 31;
-  const int S = p.split, rank = blockIdx.x % S, cid = blockIdx.x / S, nclusters = gridDim.x / S;
+  const int S = p.split, rank = blockIdx.x, cid = blockIdx.y, nclusters = gridDim.y;
   const int groups = p.K >> 7, row_tiles = (p.n_rows + 127) >> 7;
-  const int g0 = rank * groups / S, nb = (rank + 1) * groups / S - g0;      // this CTA's 128-input blocks of every tile
-  const int share = (p.tok + S - 1) / S;                                   // tokens that a CTA of the cluster finishes
+  const int g0 = p.first[rank], nb = p.first[rank + 1] - g0;                // this CTA's 128-input blocks of every tile
+  const int share = gb_share(p.T, S);                                      // tokens that a CTA of the cluster finishes
   const int sets = p.tok <= 32 ? 2 : 1;                                    // of accumulators
   // Blocks are numbered through over the CTA's tiles: block `it` goes through group it % 3, slot it % 6, issuer it % 2.
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+
+  // Expanders: thread = weight row of the tile.  Codes and scales come straight to the thread that expands them, the next block's while this one is
+  // expanded, and the first before anything is set up; warp 18 brings all of the CTA's share into L2.
+  int tile = cid, kb = warp >> 2;             // the group's next block
+  const uint4* code_at = p.codes;
+  const __half* scale_at = p.scales;
+  auto settle = [&] {                         // (tile, kb) and the addresses, kb counted from the tile's first block
+    while (kb >= nb) { kb -= nb; tile += nclusters; }
+    if (tile < row_tiles) {
+      const size_t row = min(tile * 128 + (t & 127), p.n_rows - 1);
+      code_at = p.codes + row * (size_t)(2 * groups) + 2 * (g0 + kb);
+      scale_at = p.scales + row * groups + g0 + kb;
+    }
+  };
+  uint4 code0 = make_uint4(0u, 0u, 0u, 0u), code1 = code0;
+  __half scale = __float2half(0.0f);
+  auto request = [&] {
+    code0 = __ldg(code_at);
+    code1 = __ldg(code_at + 1);
+    scale = __ldg(scale_at);
+  };
+  if (warp < kGbEpiWarp) {
+    settle();
+    if (tile < row_tiles) request();
+  }
   if (warp == kGbMmaWarp) {
     tc::tmem_alloc(&tmem_slot, 512);
     tc::tmem_relinquish();
   }
-  if (t == 0) {
-    for (int i = 0; i < nC; ++i) {
-      tc::mbar_init(&c_full[i], 1);
-      tc::mbar_init(&c_empty[i], 4 * kGbGroups);
+  if (t == 0) s_failed = 0;
+  if (t < kGbMaxActs) {
+    tc::mbar_init(&a_full[t], 1);
+    tc::mbar_init(&a_empty[t], 1);
+    if (t < kGbSlots) {
+      tc::mbar_init(&full[t], 4);              // the expander warps of the group
+      tc::mbar_init(&empty[t], 1);
     }
-    for (int i = 0; i < nA; ++i) {
-      tc::mbar_init(&a_full[i], 1);
-      tc::mbar_init(&a_empty[i], 1);
-    }
-    for (int i = 0; i < kGbSlots; ++i) {
-      tc::mbar_init(&full[i], 4);              // the expander warps of the group
-      tc::mbar_init(&empty[i], 1);
-    }
-    for (int i = 0; i < 2; ++i) {
-      tc::mbar_init(&accf[i], kGbIssuers);
-      tc::mbar_init(&acce[i], 4);
-      tc::mbar_init(&red[i], 4 * S);
+    if (t < 2) {
+      tc::mbar_init(&accf[t], kGbIssuers);
+      tc::mbar_init(&acce[t], 4);
+      tc::mbar_init(&red[t], 4 * S);
     }
     tc::mbar_fence_init();
   }
   tc::tc_fence_before();
   __syncthreads();
-  if (S > 1) asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  if (S > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");      // met before the first exchange
   tc::tc_fence_after();
   const uint32_t taddr = tmem_slot;
   bool failed = false;
 
   if (warp == kGbCodeWarp) {
     if (tc::elect_one()) {
-      int s = 0, issued = 0;
-      uint32_t phase = 1;
-      for (int tile = cid; tile < row_tiles && !failed; tile += nclusters)
-        for (int kb = 0; kb < nb; kb += 4, ++issued) {
-          if (!tc::mbar_wait_sleep<100>(&c_empty[s], phase)) { failed = true; break; }
-          tc::mbar_arrive_expect_tx(&c_full[s], kGbCodeBytes);
-          gb_load(sC + s * kGbCodeBytes, &cmap, (g0 + kb) * 8, tile * 128, &c_full[s]);
-          if (++s == nC) { s = 0; phase ^= 1; }
-        }
-      if (failed) atomicExch(p.status, 1);
-      tc::mbar_drain(c_full, issued, nC);
+      for (int tl = cid; tl < row_tiles; tl += nclusters)
+        for (int k = 0; k < nb; k += 4) gb_prefetch(&cmap, (g0 + k) * 8, tl * 128);
     }
     __syncwarp();
   } else if (warp == kGbActWarp) {
     if (tc::elect_one()) {
+      asm volatile("prefetch.tensormap [%0];" ::"l"(&xmap) : "memory");
       asm volatile("griddepcontrol.wait;" ::: "memory");
       int s = 0, issued = 0;
       uint32_t phase = 1;
-      for (int tile = cid; tile < row_tiles && !failed; tile += nclusters)
-        for (int kb = 0; kb < nb; ++kb, ++issued) {
+      for (int tl = cid; tl < row_tiles && !failed; tl += nclusters)
+        for (int k = 0; k < nb; ++k, ++issued) {
           if (!tc::mbar_wait_sleep<100>(&a_empty[s], phase)) { failed = true; break; }
           tc::mbar_arrive_expect_tx(&a_full[s], act_bytes);
-          gb_load3(sB + s * act_bytes, &xmap, (g0 + kb) * 2, &a_full[s]);
+          gb_load3(sB + s * act_bytes, &xmap, (g0 + k) * 2, &a_full[s]);
           if (++s == nA) { s = 0; phase ^= 1; }
         }
       if (failed) atomicExch(p.status, 1);
@@ -190,24 +218,28 @@ __global__ void __launch_bounds__(kGbThreads, 1) bitgemm_batch_kernel(const __gr
     if (tc::elect_one()) {
       const uint32_t idesc = tc::idesc_f32acc(tc::FMT_F16, tc::FMT_F16, 128, (uint32_t)p.tok);
       const int me = warp - kGbMmaWarp;
-      int it0 = 0, seg = 0;
-      for (int tile = cid; tile < row_tiles && !failed; tile += nclusters, ++seg, it0 += nb) {
+      int s = me, as = me, seg = 0, k = me;              // slot, stage and block, two further each time
+      uint32_t sphase = 0, aphase = 0;
+      for (int tl = cid; tl < row_tiles && !failed; tl += nclusters, ++seg, k -= nb) {
         const int ab = sets == 2 ? seg & 1 : 0, use = sets == 2 ? seg >> 1 : seg;
         if (!tc::mbar_wait(&acce[ab], (use & 1) ^ 1)) { failed = true; break; }
         tc::tc_fence_after();
         const uint32_t acc = taddr + kGbAccCol + (ab * kGbIssuers + me) * p.tok;
         bool fresh = true;
-        for (int kb = (it0 + me) & 1; kb < nb; kb += 2) {
-          const int it = it0 + kb, s = it % kGbSlots, as = it % nA;
-          if (!tc::mbar_wait(&a_full[as], (it / nA) & 1) || !tc::mbar_wait(&full[s], (it / kGbSlots) & 1)) { failed = true; break; }
+        for (; k < nb; k += kGbIssuers) {
+          // both barriers are asked before either answer is needed
+          const bool there = gb_test(&a_full[as], aphase), filled = gb_test(&full[s], sphase);
+          if ((!there && !tc::mbar_wait(&a_full[as], aphase)) || (!filled && !tc::mbar_wait(&full[s], sphase))) { failed = true; break; }
           tc::tc_fence_after();
           const uint64_t db = tc::smem_desc_sw128(tc::smem_u32(sB + as * act_bytes));
 #pragma unroll
-          for (uint32_t k = 0; k < 8; ++k)
-            gb_mma(acc, taddr + s * 64 + k * 8, db + (k >> 2) * (uint32_t)(p.tok * 128 >> 4) + (k & 3) * 2, idesc, !(fresh && k == 0));
+          for (uint32_t i = 0; i < 8; ++i)
+            gb_mma(acc, taddr + s * 64 + i * 8, db + (i >> 2) * (uint32_t)(p.tok * 128 >> 4) + (i & 3) * 2, idesc, !(fresh && i == 0));
           fresh = false;
           tc::mma_commit(&empty[s]);
           tc::mma_commit(&a_empty[as]);
+          if ((s += kGbIssuers) >= kGbSlots) { s -= kGbSlots; sphase ^= 1; }
+          if ((as += kGbIssuers) >= nA) { as -= nA; aphase ^= 1; }
         }
         tc::mma_commit(&accf[ab]);
       }
@@ -215,143 +247,166 @@ __global__ void __launch_bounds__(kGbThreads, 1) bitgemm_batch_kernel(const __gr
     }
     __syncwarp();
   } else if (warp < kGbEpiWarp) {
-    // thread = weight row of the tile; all lanes poll (one that passes the outcome on is a shuffle later: 24576 x 4096, 8 tokens 22.3 against 19.6 us)
-    const int group = warp >> 2, r = t & 127;
+    // What is not expansion costs as much as the expansion here - an instruction of a warp is some five cycles behind the one before it, a barrier
+    // asked a hundred - so counters run along instead of being computed from the block's number, and barriers are asked before the answer is needed.
     const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
-    auto scale_of = [&](int tile, int kb) {
-      while (kb >= nb) { kb -= nb; tile += nclusters; }
-      return tile < row_tiles ? __ldg(p.scales + (size_t)min(tile * 128 + r, p.n_rows - 1) * groups + g0 + kb) : __float2half(0.0f);
-    };
-    int it0 = 0, cs = 0;
-    uint32_t cphase = 0;
-    __half next = scale_of(cid, group);         // scale of this group's next block, requested a block ahead
-    for (int tile = cid; tile < row_tiles && !failed; tile += nclusters, it0 += nb) {
-      for (int kb0 = 0; kb0 < nb && !failed; kb0 += 4) {
-        if (!__all_sync(0xffffffffu, tc::mbar_wait(&c_full[cs], cphase))) { failed = true; break; }
-        const int end = min(kb0 + 4, nb);
-        for (int kb = kb0 + (group + 3 - (it0 + kb0) % 3) % 3; kb < end; kb += 3) {
-          const int it = it0 + kb, s = it % kGbSlots;
-          // A masked code is +-2^-7 or 0 and the scale is taken times 128; a row of the warp with a scale of 512 or more (none in earnest) takes the
-          // other order, which leaves every f16 scale in range.
-          const __half d = next;
-          next = scale_of(tile, kb + 3);
-          auto block = [&](auto large) {
-            const __half2 up = __half2half2(__float2half(128.0f)), d2 = large ? __half2half2(d) : __hmul2(__half2half2(d), up);
-            auto weights = [&](uint32_t m) {
-              const __half2 c = *reinterpret_cast<const __half2*>(&m), w = large ? __hmul2(__hmul2(c, up), d2) : __hmul2(c, d2);
-              return *reinterpret_cast<const uint32_t*>(&w);
-            };
+    int s = warp >> 2;                          // operand slot: group and group + 3 in turn
+    uint32_t sphase = 1;
+    while (tile < row_tiles) {
+      // A masked code is +-2^-7 or 0 and the scale is taken times 128; a row of the warp with a scale of 512 or more (none in earnest) takes the
+      // other order, which leaves every f16 scale in range.  The shifts (by 12 - 4 i and 13 - 4 i) are products: the masks and counters already fill the
+      // pipe that shifts run on (432 -> 390 cycles a block).
+      const __half d = scale;
+      const uint4 codes[2] = {code0, code1};
+      const bool vacant = gb_test(&empty[s], sphase);
+      kb += kGbGroups;
+      code_at += 2 * kGbGroups;
+      scale_at += kGbGroups;
+      if (kb >= nb) settle();
+      if (tile < row_tiles) request();
+      auto block = [&](auto large) {
+        const __half2 up = __half2half2(__float2half(128.0f)), d2 = large ? __half2half2(d) : __hmul2(__half2half2(d), up);
+        auto weights = [&](uint32_t m) {
+          const __half2 c = *reinterpret_cast<const __half2*>(&m), w = large ? __hmul2(__hmul2(c, up), d2) : __hmul2(c, d2);
+          return *reinterpret_cast<const uint32_t*>(&w);
+        };
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              const uint4 code = *reinterpret_cast<const uint4*>(sC + cs * kGbCodeBytes + tc::sw128_offset(r, 2 * (kb - kb0) + h));
-              const uint32_t w4[4] = {code.x, code.y, code.z, code.w};
-              uint32_t o[32];
+        for (int h = 0; h < 2; ++h) {
+          const uint32_t w4[4] = {codes[h].x, codes[h].y, codes[h].z, codes[h].w};
+          uint32_t o[32];
 #pragma unroll
-              for (int wd = 0; wd < 4; ++wd)
+          for (int wd = 0; wd < 4; ++wd)
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                  o[wd * 8 + i] = weights((w4[wd] << (12 - 4 * i)) & 0xA000A000u);
-                  o[wd * 8 + 4 + i] = weights((w4[wd] << (13 - 4 * i)) & 0xA000A000u);
-                }
-              if (h == 0) {
-                if (!__all_sync(0xffffffffu, tc::mbar_wait(&empty[s], ((it / kGbSlots) & 1) ^ 1))) return false;
-                tc::tc_fence_after();
-              }
-              gb_st32(taddr + lanes + s * 64 + h * 32, o);
+            for (int i = 0; i < 4; ++i) {
+              o[wd * 8 + i] = weights((w4[wd] * p.up[2 * i]) & 0xA000A000u);
+              o[wd * 8 + 4 + i] = weights((w4[wd] * p.up[2 * i + 1]) & 0xA000A000u);
             }
-            return true;
-          };
-          if (__any_sync(0xffffffffu, __hge(__habs(d), __float2half(512.0f)))) failed = !block(std::true_type{});
-          else failed = !block(std::false_type{});
-          if (failed) break;
-          asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-          tc::tc_fence_before();
-          __syncwarp();
-          if (lane == 0) tc::mbar_arrive(&full[s]);
+          if (h == 0) {
+            if (!__all_sync(0xffffffffu, vacant) && !__all_sync(0xffffffffu, tc::mbar_wait(&empty[s], sphase))) return false;
+            tc::tc_fence_after();
+          }
+          gb_st32(taddr + lanes + s * 64 + h * 32, o);
         }
-        __syncwarp();
-        if (lane == 0) tc::mbar_arrive(&c_empty[cs]);
-        if (++cs == nC) { cs = 0; cphase ^= 1; }
-      }
-    }
-    if (failed && lane == 0) atomicExch(p.status, 1);
-  } else {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    constexpr int CB = 16;
-    const int a = t - kGbEpiWarp * 32, quarter = warp & 3;
-    const uint32_t lanes = (uint32_t)(quarter * 32) << 16;
-    const int tok_lo = rank * share, tok_hi = min(p.T, tok_lo + share);
-    const uint32_t share_inv = (65536u + share - 1) / share;      // c / share for c < 64
-    int seg = 0, it0 = 0;
-    for (int tile = cid; tile < row_tiles; tile += nclusters, ++seg, it0 += nb) {
-      const int rb = seg & 1, ab = sets == 2 ? rb : 0, use = sets == 2 ? seg >> 1 : seg, row = tile * 128 + a;
-      const bool row_ok = row < p.n_rows;
-      if (!tc::mbar_wait_warp<64>(&accf[ab], use & 1, lane)) { failed = true; break; }
-      tc::tc_fence_after();
-      float* mine = sR + (size_t)rb * S * share * 128;
-      const uint32_t mine_at = tc::smem_u32(mine + a);
-      const uint32_t acc = taddr + lanes + kGbAccCol + ab * kGbIssuers * p.tok;
-      const int one = nb == 1 ? it0 & 1 : 0;        // a tile of one block was in one issuer's accumulator only
-      for (int c0 = 0; c0 < p.T; c0 += CB) {
-        uint32_t v[CB], w[CB];
-        tc::tmem_ld16(acc + one * p.tok + c0, v);
-        if (nb > 1) tc::tmem_ld16(acc + p.tok + c0, w);
-        tc::tmem_wait_ld();
-        if (nb > 1) {
-#pragma unroll
-          for (int j = 0; j < CB; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) + __uint_as_float(w[j]));
-        }
-#pragma unroll
-        for (int j = 0; j < CB; ++j) {
-          const int c = c0 + j, to = (int)((uint32_t)c * share_inv >> 16);
-          const uint32_t at = mine_at + (uint32_t)(rank * share + c - to * share) * 512;
-          if (c < p.T) gb_st_remote(S > 1 ? gb_map(at, (uint32_t)to) : at, __uint_as_float(v[j]));
-        }
-      }
+        return true;
+      };
+      if (__any_sync(0xffffffffu, __hge(__habs(d), __float2half(512.0f)))) failed = !block(std::true_type{});
+      else failed = !block(std::false_type{});
+      if (failed) break;
+      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       tc::tc_fence_before();
       __syncwarp();
-      if (lane == 0) tc::mbar_arrive(&acce[ab]);
-      if (lane < S) gb_arrive_remote(gb_map(tc::smem_u32(&red[rb]), (uint32_t)lane));
-      if (!gb_wait_cluster(&red[rb], (seg >> 1) & 1)) { failed = true; break; }
-      __syncwarp();
-      // this CTA's tokens, eight at a time: partial sums in CTA order, the residuals as a block before the stores (they usually alias)
-      for (int c0 = tok_lo; c0 < tok_hi; c0 += 8) {
-        float v[8], res[8];
+      if (lane == 0) tc::mbar_arrive(&full[s]);
+      if (s >= kGbGroups) { s -= kGbGroups; sphase ^= 1; }
+      else s += kGbGroups;
+    }
+  }
+  if (S > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  if (warp < kGbMmaWarp) {
+    // A tile's end is a chain (drain, exchange, sum, store): few, wide accesses and short loops.  Warps 12-15 take it beside the expansion of the next
+    // tile; the last tile has the expanders' warps too, every group a quarter of the tokens.  us of 64 / 24 / 5 tokens with four warps, a store per
+    // value and loops unrolled over tokens (the start's form): 6144 x 4096 16.2 / 12.3 / 10.0, 24576 x 4096 40.2 / 26.6 / 19.5.
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    constexpr int CB = 16;
+    const int a = t & 127, part = warp >= kGbEpiWarp ? 0 : 1 + (warp >> 2);
+    const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
+    const int tok_lo = rank * share, tok_hi = min(p.T, tok_lo + share), quads = share >> 2;
+    const uint32_t share_inv = (65536u + share - 1) / share;      // c / share for c < 64
+    const int last = (row_tiles - 1 - cid) / nclusters;            // the CTA's last tile, counted from 0
+    for (int seg = part == 0 ? 0 : last; seg <= last; ++seg) {
+      const int rb = seg & 1, ab = sets == 2 ? rb : 0, use = sets == 2 ? seg >> 1 : seg, row = (cid + seg * nclusters) * 128 + a;
+      const int parts = seg == last ? 1 + kGbGroups : 1;
+      const bool row_ok = row < p.n_rows;
+      // the residuals of a group of four tokens are requested a group ahead, the first group's before the sums are there (they usually alias the outputs)
+      float res[4];
+      auto residuals = [&](int c) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) res[j] = p.epi == 1 && row_ok && c0 + j < tok_hi ? p.residual[(size_t)(c0 + j) * p.out_ld + row] : 0.0f;
+        for (int j = 0; j < 4; ++j) res[j] = row_ok && c + j < tok_hi ? p.residual[(size_t)(c + j) * p.out_ld + row] : 0.0f;
+      };
+      if (p.epi == 1) residuals(tok_lo + 4 * part);
+      const float4* mine = reinterpret_cast<const float4*>(sR) + (size_t)rb * S * quads * 128 + a;
+      if (part == 0 && !failed) failed = !tc::mbar_wait_warp<20>(&accf[ab], use & 1, lane);
+      // The expanders have not followed the tiles before: their accumulator barrier may be phases ahead of what they could wait for.
+      if (parts > 1) {                                               // all sixteen warps come here, whatever failed
+        tc::tc_fence_before();
+        asm volatile("bar.sync 2, %0;" ::"n"(kGbMmaWarp * 32) : "memory");
+      }
+      if (!failed) {
+        tc::tc_fence_after();
+        const uint32_t mine_at = tc::smem_u32(mine) + (uint32_t)(rank * quads) * 2048;
+        const uint32_t acc = taddr + lanes + kGbAccCol + ab * kGbIssuers * p.tok;
+        const int one = nb == 1 ? seg & 1 : 0;        // a tile of one block was in one issuer's accumulator only
+#pragma unroll 1
+        for (int c0 = CB * part; c0 < p.T; c0 += CB * parts) {
+          uint32_t v[CB], w[CB];
+          tc::tmem_ld16(acc + one * p.tok + c0, v);
+          if (nb > 1) tc::tmem_ld16(acc + p.tok + c0, w);
+          tc::tmem_wait_ld();
+          if (nb > 1) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          v[j] = 0.0f;
-          if (c0 + j < tok_hi)
-            for (int i = 0; i < S; ++i) v[j] += mine[((size_t)i * share + (c0 + j - tok_lo)) * 128 + a];
+            for (int j = 0; j < CB; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) + __uint_as_float(w[j]));
+          }
+#pragma unroll
+          for (int j = 0; j < CB; j += 4) {
+            const int c = c0 + j, to = (int)((uint32_t)c * share_inv >> 16);
+            const uint32_t at = mine_at + (uint32_t)((c - to * share) >> 2) * 2048;
+            if (c < p.T) gb_st_remote4(gb_map(at, (uint32_t)to), v + j);
+          }
+        }
+        tc::tc_fence_before();
+        __syncwarp();
+      }
+      if (parts > 1) asm volatile("bar.sync 1, %0;" ::"n"(kGbMmaWarp * 32) : "memory");
+      if (failed) continue;
+      if (part == 0) {
+        if (lane == 0) tc::mbar_arrive(&acce[ab]);
+        if (lane < S) gb_arrive_remote(gb_map(tc::smem_u32(&red[rb]), (uint32_t)lane));
+      }
+      if (!__all_sync(0xffffffffu, gb_wait_cluster(&red[rb], (seg >> 1) & 1))) { failed = true; continue; }
+      // this CTA's tokens, four at a time: partial sums in CTA order
+#pragma unroll 1
+      for (int c = tok_lo + 4 * part; c < tok_hi; c += 4 * parts) {
+        float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        const float4* src = mine + (size_t)((c - tok_lo) >> 2) * 128;
+#pragma unroll 2
+        for (int i = 0; i < S; ++i, src += quads * 128) {
+          const float4 x = *src;
+          v[0] += x.x; v[1] += x.y; v[2] += x.z; v[3] += x.w;
         }
         if (p.epi == 2) {
           const bool odd = lane & 1;      // gate (even) and up (odd) rows are neighbouring lanes; each finishes every other token
           const int o = row >> 1;
-          __half* dst = p.out_f16 + ((o & ~7) | ((o & 3) << 1) | ((o >> 2) & 1));
+          __half* dst = p.out_f16 + ((o & ~7) | ((o & 3) << 1) | ((o >> 2) & 1)) + (size_t)(c + odd) * p.out_ld;
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
+          for (int j = 0; j < 2; ++j) {
             const float keep = odd ? v[2 * j + 1] : v[2 * j], other = __shfl_xor_sync(0xffffffffu, odd ? v[2 * j] : v[2 * j + 1], 1);
             const float g = odd ? other : keep, u = odd ? keep : other;
-            const int c = c0 + 2 * j + (odd ? 1 : 0);
-            if (row_ok && c < tok_hi) dst[(size_t)c * p.out_ld] = __float2half_rn(g / (1.0f + __expf(-g)) * u);
+            if (row_ok && c + 2 * j + odd < tok_hi) dst[(size_t)(2 * j) * p.out_ld] = __float2half_rn(g / (1.0f + __expf(-g)) * u);
           }
         } else {
+          if (p.epi == 1) {
 #pragma unroll
-          for (int j = 0; j < 8; ++j)
-            if (row_ok && c0 + j < tok_hi) p.out_f32[(size_t)(c0 + j) * p.out_ld + row] = p.epi == 1 ? res[j] + v[j] : v[j];
+            for (int j = 0; j < 4; ++j) v[j] += res[j];
+            residuals(c + 4 * parts);
+          }
+          float* dst = p.out_f32 + (size_t)c * p.out_ld + row;
+          if (row_ok) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j, dst += p.out_ld)
+              if (c + j < tok_hi) *dst = v[j];
+          }
         }
       }
       __syncwarp();
     }
     if (failed && lane == 0) atomicExch(p.status, 1);
   }
+  if (failed) s_failed = 1;
   tc::tc_fence_before();
   __syncthreads();
   tc::tc_fence_after();
   if (warp == kGbMmaWarp) tc::tmem_dealloc(taddr, 512);
-  // nobody leaves while another CTA of the cluster may still write to it (after an expired wait it would)
-  if (S > 1) asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  // Whoever has its last sums is written to no more and leaves; after an expired wait it stays until the others have left or wait here too.
+  if (S > 1 && s_failed) asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 static bool gb_maps(CUtensorMap* cmap, CUtensorMap* xmap, const void* codes, int n_rows, int K, const void* x, int x_ld, int T, int tok) {
@@ -359,19 +414,19 @@ static bool gb_maps(CUtensorMap* cmap, CUtensorMap* xmap, const void* codes, int
   cuuint64_t xd[3] = {64, (cuuint64_t)T, (cuuint64_t)K / 64}, xst[2] = {(cuuint64_t)x_ld * 2, 128};      // [K / 64][T][64]
   cuuint32_t cbox[2] = {32, 128}, xbox[3] = {64, (cuuint32_t)tok, 2}, estr[3] = {1, 1, 1};
   return cuTensorMapEncodeTiled(cmap, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, const_cast<void*>(codes), cd, cst, cbox, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                                CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS &&
+                                CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS &&
          cuTensorMapEncodeTiled(xmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void*>(x), xd, xst, xbox, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                                 CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 static size_t gb_smem_bytes(int tok, int split) {
-  const int share = (tok + split - 1) / split;
-  return 1024 + (size_t)gb_code_stages(tok) * kGbCodeBytes + (size_t)gb_act_stages(tok) * tok * 256 + (size_t)2 * split * share * 128 * sizeof(float);
+  const int share = gb_share(tok, split);
+  return 1024 + (size_t)gb_act_stages(tok) * tok * 256 + (size_t)2 * split * share * 128 * sizeof(float);
 }
 
 static cudaLaunchConfig_t gb_config(cudaLaunchAttribute* attr, int clusters, int split, size_t smem, cudaStream_t st) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(clusters * split);
+  cfg.gridDim = dim3(split, clusters);
   cfg.blockDim = dim3(kGbThreads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
@@ -429,13 +484,15 @@ int bonsai_bitgemm_batch(const void* codes, const void* scales, const void* x_f1
   const int most = groups < kGbMaxSplit ? groups : kGbMaxSplit;
   if (split > most) split = most;
   if (split == 0 || held[split] < 1) {
-    // rounds of tiles times the 128-input blocks that a CTA goes through, plus what a tile costs whatever its depth (accumulator drain and
-    // exchange, six blocks' time) and a cluster for its size.  16 tokens, us by split 1 / 2 / 3 / 4 / 6: 6144 x 4096 15.8 / 11.3 / 11.8 / 11.4 / 12.9;
-    // 24576 x 4096 27.0 / 22.7 / 25.3 / 27.1 / 35.4; 4096 x 12288 38.4 / 20.3 / 17.0 / 15.4 / 15.7; 2560 x 4096 15.6 / 9.2 / 7.8 / 7.9 / 8.7.
+    // Rounds of tiles times the 128-input blocks that a CTA goes through, plus what a tile costs whatever its depth (accumulator drain and
+    // exchange, six blocks' time), and for the cluster's size what waiting for one more CTA costs: 1.5 blocks' time, 2.8 with the 33 to 64 tokens' sums to
+    // exchange, where more than four CTAs never paid.  us by split 1 / 2 / 3 / 4 / 6 behind the norm at 8 tokens: 6144 x 4096 13.0 / 9.7 / 13.1 / 9.4 / 10.2;
+    // 24576 x 4096 22.0 / 18.6 / 20.3 / 20.6 / 26.4; 4096 x 12288 28.6 / 17.9 / 16.2 / 12.7 / 16.0; 2560 x 4096 13.0 / 9.2 / 8.0 / 6.9 / 7.0; 2560 x 9728 23.7 / 15.1 / 12.5 /
+    // 10.9 / 10.1; at 64 tokens 2560 x 4096 14.3 / 10.3 / 9.4 / 8.5 / 10.3, 2560 x 9728 25.6 / 16.4 / 14.9 / 11.8 / 14.2.
     long long best = -1;
-    for (int s = 1; s <= most; ++s) {
+    for (int s = 1; s <= (T > 32 && most > 4 ? 4 : most); ++s) {
       if (held[s] < 1) continue;
-      const long long rounds = (tiles + held[s] - 1) / held[s], cost = rounds * ((groups + s - 1) / s + 6) + 3 * s;
+      const long long rounds = (tiles + held[s] - 1) / held[s], cost = 10 * rounds * ((groups + s - 1) / s + 6) + (T > 32 ? 28 : 15) * s;
       if (best < 0 || cost < best) {
         best = cost;
         split = s;
@@ -446,7 +503,8 @@ int bonsai_bitgemm_batch(const void* codes, const void* scales, const void* x_f1
   const int tok = T <= 16 ? 16 : (T <= 32 ? 32 : 64);
   CUtensorMap cmap, xmap;
   if (!gb_maps(&cmap, &xmap, codes, n_rows, K, x_f16, x_ld, T, tok)) return BONSAI_CUDA_BAD_ARG;
-  GbParams p{(const __half*)scales, out_f32, residual, (__half*)out_f16, status, n_rows, K, T, epi, out_ld, split, tok};
+  GbParams p{(const uint4*)codes, (const __half*)scales, out_f32, residual, (__half*)out_f16, status, n_rows, K, T, epi, out_ld, split, tok, {}, {1u << 12, 1u << 13, 1u << 8, 1u << 9, 1u << 4, 1u << 5, 1u, 2u}};
+  for (int i = 0; i <= split; ++i) p.first[i] = i * groups / split;
   cudaLaunchAttribute attr[2];
   const int clusters = tiles < held[split] ? tiles : held[split];
   // the request is that of 64 tokens, so that one CTA has an SM whatever the batch is

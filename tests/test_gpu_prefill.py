@@ -297,6 +297,29 @@ def test_batch_gemm_through_tensor_memory(ty, rows, cols, T, split):
     assert status.item() == 0
 
 
+@pytest.mark.parametrize("T", [1, 5, 12, 33, 64])
+@pytest.mark.parametrize("split", [3, 5, 7, 8])
+def test_batch_gemm_shares_of_tokens(T, split):
+    """Groups of four tokens handed out over the CTAs of a cluster: CTAs without tokens, with fewer than four, unequal shares of blocks, a last
+    tile of fewer rows, one tile and several per cluster (148 / 3 clusters at most)."""
+    from oxibonsai_b200.ops import cuda_ops as K
+    for rows, cols in ((200, 1152), (64 * 128 + 6, 1152)):
+        raw, dense = _random_quant(TQ2_0_G128, rows, cols, rows + T)
+        w = K.PlanarWeight(rows, cols, torch.device(DEV))
+        w.fill_from_gguf(torch.from_numpy(np.array(raw, copy=True)).to(DEV), TQ2_0_G128, cols, 0, rows)
+        g = torch.Generator(device=DEV).manual_seed(T + split)
+        x = torch.randn((T, cols), device=DEV, generator=g).half()
+        res = torch.randn((T, rows), device=DEV, generator=g)
+        paired = torch.empty_like(x)
+        paired[:, K.paired_k_index(cols, DEV)] = x
+        dense = dense.to(DEV).double()
+        want, terms = x.double() @ dense.T + res.double(), x.double().abs() @ dense.abs().T + res.abs().double()
+        status = torch.zeros(1, dtype=torch.int32, device=DEV)
+        got = K.bitgemm_batch(w, paired, 1, residual=res, status=status, split=split)
+        assert ((got.double() - want).abs() <= 2.0 ** -23 * (cols + 16) * terms).all()      # products are exact in f32, sums may drop a last place each
+        assert status.item() == 0
+
+
 def _row_scale(x, threads):
     """1 / rms of every row of x with the squares added in the order that the results depend on: thread t of `threads` adds groups t, t + threads, ..
     of four neighbouring inputs, then warps by halves, then the warps' sums by halves.  One rounding to 32 bits per step."""
