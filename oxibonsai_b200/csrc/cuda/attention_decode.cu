@@ -115,8 +115,10 @@ __global__ void __launch_bounds__(256) qknorm_rope_kvstore_h128_kernel(const flo
                                                                        const float* __restrict__ k_norm, float eps, const float* __restrict__ rope_cos,
                                                                        const float* __restrict__ rope_sin, const int* __restrict__ positions,
                                                                        const int* __restrict__ block_table, int max_pages, float* __restrict__ q_out,
-                                                                       int nq, int batch, KvPool pool) {
-  // no early signal to the next kernel: decode attention requests cached rows before it waits, and this kernel writes the newest
+                                                                       int nq, int batch, KvPool pool, int early) {
+  // early: the next kernel reads no rows and no queries before it waits for this one (the CUDA-core decode attention requests cached rows, and this
+  // kernel writes the newest)
+  if (early) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
   const int nkv = pool.kv_heads, heads = nq + 2 * nkv, lane = threadIdx.x & 31;
   const long long unit = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
@@ -699,12 +701,36 @@ int launch_decode_d(int dpl, int G, dim3 grid, size_t smem, cudaStream_t st, con
 }
 
 int attn_decode_quant(const float*, const int*, const int*, int, int, int, int, int, int, const void*, const void*, const float*, const float*, int, float*,
-                      float*, int*, float*, int, float, cudaStream_t);
+                      float*, long long, int*, float*, int, float, cudaStream_t);
 bool attn_decode_quant_takes(const float*, int, int, int, const void*, const void*);
 int attn_decode_mma_f16(const float* q, const int* positions, const int* block_table, int max_pages, int batch, int nq, int nkv,
                         int page_size, const void* kpool, const void* vpool, int nsplit, float* ws_acc, float* ws_ml, int* counters,
                         float* out, int extra_len, float sm_scale, cudaStream_t stream);
 static int g_attn_force_cuda_cores = 0;
+
+}  // namespace bonsai
+
+namespace bonsai {
+
+int qknorm_rope_kvstore(const float* qkv, int qkv_stride, const float* q_norm, const float* k_norm, float eps, const float* rope_cos,
+                        const float* rope_sin, const int* positions, const int* block_table, int max_pages, float* q_out, int batch, int nq,
+                        int nkv, int hd, int kvt, int page_size, void* kpool, void* vpool, float* kscale, float* vscale, int early, cudaStream_t stream) {
+  if (hd % 32 != 0 || hd < 64 || hd > 256 || kvt < 0 || kvt > 3 || batch <= 0) return BONSAI_CUDA_BAD_ARG;
+  KvPool pool{(uint8_t*)kpool, (uint8_t*)vpool, kscale, vscale, page_size, nkv, hd, kvt};
+  dim3 grid(nq + 2 * nkv, batch);
+  const uintptr_t ends = reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(q_norm) | reinterpret_cast<uintptr_t>(k_norm) |
+                         reinterpret_cast<uintptr_t>(rope_cos) | reinterpret_cast<uintptr_t>(rope_sin) | reinterpret_cast<uintptr_t>(q_out) |
+                         reinterpret_cast<uintptr_t>(kpool) | reinterpret_cast<uintptr_t>(vpool);
+  if (hd == 128 && qkv_stride % 2 == 0 && (ends & 7) == 0) {
+    const long long units = (long long)batch * (nq + 2 * nkv);
+    const cudaError_t e = launch_pdl(qknorm_rope_kvstore_h128_kernel, dim3((unsigned)((units + 7) / 8)), dim3(256), 0, stream, qkv, qkv_stride, q_norm,
+                                     k_norm, eps, rope_cos, rope_sin, positions, block_table, max_pages, q_out, nq, batch, pool, early);
+    return e == cudaSuccess ? BONSAI_CUDA_OK : BONSAI_CUDA_LAUNCH_FAILED;
+  }
+  qknorm_rope_kvstore_kernel<<<grid, hd, (hd + 32) * sizeof(float), stream>>>(qkv, qkv_stride, q_norm, k_norm, eps, rope_cos, rope_sin,
+                                                                              positions, block_table, max_pages, q_out, nq, pool);
+  return launch_status();
+}
 
 }  // namespace bonsai
 
@@ -719,22 +745,8 @@ int bonsai_qknorm_rope_kvstore(const float* qkv, int qkv_stride, const float* q_
                                const float* rope_cos, const float* rope_sin, const int* positions, const int* block_table,
                                int max_pages, float* q_out, int batch, int nq, int nkv, int hd, int kvt, int page_size,
                                void* kpool, void* vpool, float* kscale, float* vscale, cudaStream_t stream) {
-  using namespace bonsai;
-  if (hd % 32 != 0 || hd < 64 || hd > 256 || kvt < 0 || kvt > 3 || batch <= 0) return BONSAI_CUDA_BAD_ARG;
-  KvPool pool{(uint8_t*)kpool, (uint8_t*)vpool, kscale, vscale, page_size, nkv, hd, kvt};
-  dim3 grid(nq + 2 * nkv, batch);
-  const uintptr_t ends = reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(q_norm) | reinterpret_cast<uintptr_t>(k_norm) |
-                         reinterpret_cast<uintptr_t>(rope_cos) | reinterpret_cast<uintptr_t>(rope_sin) | reinterpret_cast<uintptr_t>(q_out) |
-                         reinterpret_cast<uintptr_t>(kpool) | reinterpret_cast<uintptr_t>(vpool);
-  if (hd == 128 && qkv_stride % 2 == 0 && (ends & 7) == 0) {
-    const long long units = (long long)batch * (nq + 2 * nkv);
-    const cudaError_t e = launch_pdl(qknorm_rope_kvstore_h128_kernel, dim3((unsigned)((units + 7) / 8)), dim3(256), 0, stream, qkv, qkv_stride, q_norm,
-                                     k_norm, eps, rope_cos, rope_sin, positions, block_table, max_pages, q_out, nq, batch, pool);
-    return e == cudaSuccess ? BONSAI_CUDA_OK : BONSAI_CUDA_LAUNCH_FAILED;
-  }
-  qknorm_rope_kvstore_kernel<<<grid, hd, (hd + 32) * sizeof(float), stream>>>(qkv, qkv_stride, q_norm, k_norm, eps, rope_cos, rope_sin,
-                                                                              positions, block_table, max_pages, q_out, nq, pool);
-  return launch_status();
+  return bonsai::qknorm_rope_kvstore(qkv, qkv_stride, q_norm, k_norm, eps, rope_cos, rope_sin, positions, block_table, max_pages, q_out, batch, nq, nkv, hd,
+                                     kvt, page_size, kpool, vpool, kscale, vscale, 0, stream);
 }
 
 // Whether bonsai_attn_decode_route sends quantised rows of this shape to the tensor cores.
@@ -744,13 +756,14 @@ int bonsai_attn_decode_on_tensor_cores(const float* q, int nq, int nkv, int hd, 
 }
 
 // q: f32 [batch][nq][hd] -> out f32 [batch][nq][hd].  Context length of sequence b is
-// positions[b] + 1 + extra_len.  ws_acc needs batch*nq*nsplit*hd floats, ws_ml batch*nq*nsplit*2,
+// positions[b] + 1 + extra_len.  ws_acc needs batch*nq*nsplit*hd floats, ws_ml batch*nq*nsplit*2 (ws_rows rows of each: at least these, and
+// with 1776 * nq / nkv of them quantised rows on the tensor cores may have every CTA that the device holds),
 // counters batch*nkv ints that are zero between launches (the kernel resets them).  f32_rows: INT8 / INT4 rows are multiplied in f32 on the
 // CUDA cores whatever their shape.
 int bonsai_attn_decode_route(const float* q, const int* positions, const int* block_table, int max_pages, int batch, int nq, int nkv,
                              int hd, int kvt, int page_size, const void* kpool, const void* vpool, const float* kscale,
-                             const float* vscale, int nsplit, float* ws_acc, float* ws_ml, int* counters, float* out, int extra_len,
-                             int f32_rows, cudaStream_t stream) {
+                             const float* vscale, int nsplit, float* ws_acc, float* ws_ml, long long ws_rows, int* counters, float* out,
+                             int extra_len, int f32_rows, cudaStream_t stream) {
   using namespace bonsai;
   if (hd % 32 != 0 || hd < 64 || hd > 256 || nq % nkv != 0 || nsplit < 1 || batch <= 0 || counters == nullptr) return BONSAI_CUDA_BAD_ARG;
   int G = nq / nkv, dpl = hd / 32;
@@ -765,9 +778,11 @@ int bonsai_attn_decode_route(const float* q, const int* positions, const int* bl
                                        ws_ml, counters, out, extra_len, sc, stream);
     if (rc != BONSAI_CUDA_BAD_ARG) return rc;
   }
-  if (bonsai_attn_decode_on_tensor_cores(q, nq, nkv, hd, kvt, page_size, kpool, vpool, f32_rows))
-    return attn_decode_quant(q, positions, block_table, max_pages, batch, nq, nkv, kvt, page_size, kpool, vpool, kscale, vscale, nsplit, ws_acc,
-                             ws_ml, counters, out, extra_len, sc, stream);
+  if (bonsai_attn_decode_on_tensor_cores(q, nq, nkv, hd, kvt, page_size, kpool, vpool, f32_rows)) {
+    const int rc = attn_decode_quant(q, positions, block_table, max_pages, batch, nq, nkv, kvt, page_size, kpool, vpool, kscale, vscale, nsplit, ws_acc,
+                                     ws_ml, ws_rows, counters, out, extra_len, sc, stream);
+    if (rc != BONSAI_CUDA_BAD_ARG) return rc;      // outputs or a workspace at odd addresses
+  }
   if (hd == 128 && kvt != KV_F32 && (G == 1 || G == 2 || G == 4) && (page_size & (page_size - 1)) == 0) {
     switch (kvt) {
       case KV_F16: return launch_decode_h128<KV_F16>(G, grid, smem, stream, q, positions, block_table, max_pages, pool, nq, sc, ws_acc, ws_ml, counters, out, extra_len);
@@ -789,7 +804,7 @@ int bonsai_attn_decode(const float* q, const int* positions, const int* block_ta
                        const float* vscale, int nsplit, float* ws_acc, float* ws_ml, int* counters, float* out, int extra_len,
                        cudaStream_t stream) {
   return bonsai_attn_decode_route(q, positions, block_table, max_pages, batch, nq, nkv, hd, kvt, page_size, kpool, vpool, kscale, vscale, nsplit,
-                                  ws_acc, ws_ml, counters, out, extra_len, 0, stream);
+                                  ws_acc, ws_ml, (long long)batch * nq * nsplit, counters, out, extra_len, 0, stream);
 }
 
 }  // extern "C"

@@ -25,7 +25,7 @@ int bonsai_qknorm_rope_kvstore(const float*, int, const float*, const float*, fl
                                const int*, int, float*, int, int, int, int, int, int, void*, void*, float*, float*, cudaStream_t);
 int bonsai_attn_decode_on_tensor_cores(const float*, int, int, int, int, int, const void*, const void*, int);
 int bonsai_attn_decode_route(const float*, const int*, const int*, int, int, int, int, int, int, int, const void*, const void*,
-                             const float*, const float*, int, float*, float*, int*, float*, int, int, cudaStream_t);
+                             const float*, const float*, int, float*, float*, long long, int*, float*, int, int, cudaStream_t);
 int bonsai_bitgemv_h2(const void*, const void*, const float*, const float*, float, float*, const float*, int, int, int, cudaStream_t);
 int bonsai_bitgemv_warp(const void*, const void*, const float*, const float*, float, float*, const float*, int, int, int, cudaStream_t);
 int bonsai_bitgemv_hmma(const void*, const void*, const float*, const float*, float, float*, const float*, int, int, int, cudaStream_t);
@@ -61,6 +61,10 @@ size_t bonsai_s16_bytes(int, int);
 
 namespace bonsai {
 
+int attn_decode_quant_splits(int pairs);
+int qknorm_rope_kvstore(const float*, int, const float*, const float*, float, const float*, const float*, const int*, const int*, int, float*, int, int,
+                        int, int, int, int, void*, void*, float*, float*, int early, cudaStream_t);
+
 enum LayerPtr {
   LP_QKV_CODES = 0, LP_QKV_SCALES, LP_O_CODES, LP_O_SCALES, LP_GU_CODES, LP_GU_SCALES, LP_DOWN_CODES, LP_DOWN_SCALES,
   LP_ATTN_NORM, LP_FFN_NORM, LP_Q_NORM, LP_K_NORM, LP_KPOOL, LP_VPOOL, LP_KSCALE, LP_VSCALE,
@@ -72,7 +76,9 @@ enum GlobalPtr {
 };
 enum IntCfg {
   IC_HIDDEN = 0, IC_INTER_LOCAL, IC_LAYERS, IC_HEADS_LOCAL, IC_KV_HEADS_LOCAL, IC_HEAD_DIM, IC_VOCAB, IC_LM_ROWS_LOCAL,
-  IC_KVT, IC_PAGE_SIZE, IC_MAX_PAGES, IC_NSPLIT, IC_TP_SIZE, IC_TP_RANK, IC_FAST, IC_NSPLIT_BATCHED, IC_COUNT
+  IC_KVT, IC_PAGE_SIZE, IC_MAX_PAGES, IC_NSPLIT, IC_TP_SIZE, IC_TP_RANK, IC_FAST, IC_NSPLIT_BATCHED,
+  IC_WS_ROWS,   // rows of the split workspace (SP_WS_ACC, SP_WS_ML)
+  IC_COUNT
 };
 enum StepPtr {
   SP_TOKENS = 0, SP_POSITIONS, SP_BLOCK_TABLE, SP_H, SP_QKV, SP_Q, SP_ATTN, SP_ACT, SP_LOGITS, SP_WS_ACC, SP_WS_ML,
@@ -135,14 +141,20 @@ static int qkv_attention_run(Runner& r, const uint64_t* lp, const uint64_t* sp, 
     if (rc != BONSAI_CUDA_BAD_ARG) return rc;   // bad argument = not a shape of the fused kernel
   }
   const bool f32_rows = r.ic[IC_FAST] == 0;      // exact mode: quantised rows in f32
-  // INT8 / INT4 pages on the tensor cores: two CTAs on an SM; more splits than fill those only add partial sums
-  if (n > 1 && bonsai_attn_decode_on_tensor_cores(q, nq, nkv, hd, kvt, r.ic[IC_PAGE_SIZE], P<void>(pool.k), P<void>(pool.v), f32_rows))
-    nsplit = std::max(1, std::min(nsplit, 2 * 148 / (nkv * n)));
-  RC(bonsai_qknorm_rope_kvstore(qkv, qkv_n, P<float>(lp[LP_Q_NORM]), P<float>(lp[LP_K_NORM]), r.eps, P<float>(r.gp[GP_ROPE_COS]),
-                                P<float>(r.gp[GP_ROPE_SIN]), positions, bt, mp, q, n, nq, nkv, hd, kvt, r.ic[IC_PAGE_SIZE], P<void>(pool.k),
-                                P<void>(pool.v), P<float>(pool.ks), P<float>(pool.vs), st));
+  long long ws_rows = (long long)n * nq * nsplit;
+  // INT8 / INT4 pages on the tensor cores: as many CTAs as the device holds, over the whole workspace (the kernel ahead has left it)
+  const bool quant = bonsai_attn_decode_on_tensor_cores(q, nq, nkv, hd, kvt, r.ic[IC_PAGE_SIZE], P<void>(pool.k), P<void>(pool.v), f32_rows);
+  if (quant) {
+    nsplit = attn_decode_quant_splits(nkv * n);
+    ws_acc = P<float>(sp[SP_WS_ACC]);
+    ws_ml = P<float>(sp[SP_WS_ML]);
+    ws_rows = r.ic[IC_WS_ROWS];
+  }
+  RC(qknorm_rope_kvstore(qkv, qkv_n, P<float>(lp[LP_Q_NORM]), P<float>(lp[LP_K_NORM]), r.eps, P<float>(r.gp[GP_ROPE_COS]),
+                         P<float>(r.gp[GP_ROPE_SIN]), positions, bt, mp, q, n, nq, nkv, hd, kvt, r.ic[IC_PAGE_SIZE], P<void>(pool.k),
+                         P<void>(pool.v), P<float>(pool.ks), P<float>(pool.vs), quant, st));
   return bonsai_attn_decode_route(q, positions, bt, mp, n, nq, nkv, hd, kvt, r.ic[IC_PAGE_SIZE], P<void>(pool.k), P<void>(pool.v),
-                                  P<float>(pool.ks), P<float>(pool.vs), nsplit, ws_acc, ws_ml, counters, attn, 0, f32_rows, st);
+                                  P<float>(pool.ks), P<float>(pool.vs), nsplit, ws_acc, ws_ml, ws_rows, counters, attn, 0, f32_rows, st);
 }
 
 // The same for slots 0 .. batch-1: one launch (pair) per run of consecutive slots that share a page format.
@@ -359,15 +371,17 @@ static int prefill_chunk(Runner& r, const uint64_t* sp, const uint64_t* pp, int 
     RC(to_f16(P<float>(lp[LP_ATTN_NORM])));
     RC(gemm(P<void>(lp[LP_QKV_CODES]), P<void>(lp[LP_QKV_SCALES]), xn, xn_ld, qkv, nullptr, nullptr, qkv_n, hidden, 0, qkv_n));
     // every row of the chunk uses the same page list: a block-table stride of zero
-    RC(bonsai_qknorm_rope_kvstore(qkv, qkv_n, P<float>(lp[LP_Q_NORM]), P<float>(lp[LP_K_NORM]), r.eps, P<float>(r.gp[GP_ROPE_COS]),
-                                  P<float>(r.gp[GP_ROPE_SIN]), positions, bt, 0, q, T, nq, nkv, hd, kvt,
-                                  r.ic[IC_PAGE_SIZE], P<void>(pool.k), P<void>(pool.v), P<float>(pool.ks),
-                                  P<float>(pool.vs), st));
+    const bool f32_rows = settled || r.ic[IC_FAST] == 0;
+    const bool early = small && bonsai_attn_decode_on_tensor_cores(q, nq, nkv, hd, kvt, r.ic[IC_PAGE_SIZE], P<void>(pool.k), P<void>(pool.v), f32_rows);
+    RC(qknorm_rope_kvstore(qkv, qkv_n, P<float>(lp[LP_Q_NORM]), P<float>(lp[LP_K_NORM]), r.eps, P<float>(r.gp[GP_ROPE_COS]),
+                           P<float>(r.gp[GP_ROPE_SIN]), positions, bt, 0, q, T, nq, nkv, hd, kvt,
+                           r.ic[IC_PAGE_SIZE], P<void>(pool.k), P<void>(pool.v), P<float>(pool.ks),
+                           P<float>(pool.vs), early, st));
     if (small) {
       float* attn32 = P<float>(pp[PP_SM_ATTN]);
       RC(bonsai_attn_decode_route(q, positions, bt, 0, T, nq, nkv, hd, kvt, r.ic[IC_PAGE_SIZE], P<void>(pool.k),
                                   P<void>(pool.v), P<float>(pool.ks), P<float>(pool.vs), sm_splits, P<float>(pp[PP_SM_ACC]),
-                                  P<float>(pp[PP_SM_ML]), P<int>(pp[PP_SM_CTR]), attn32, 0, settled || r.ic[IC_FAST] == 0, st));
+                                  P<float>(pp[PP_SM_ML]), (long long)kSmallChunk * nq * kSmallSplits, P<int>(pp[PP_SM_CTR]), attn32, 0, f32_rows, st));
       RC(hm ? bonsai_norm_to_f16_hmma(attn32, qd, nullptr, r.eps, T, qd, attn, qd, st)
             : bonsai_norm_to_f16_paired(attn32, qd, nullptr, r.eps, T, qd, attn, qd, 0, st));
     } else {

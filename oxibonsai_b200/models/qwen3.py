@@ -312,8 +312,9 @@ class Qwen3Runner(SlotState):
         else:
             self.logits = torch.zeros((B, cfg.vocab), **f32)
             self.partial = torch.zeros((B, cfg.hidden), **f32)
-        self.ws_acc = torch.zeros((B, nq, self.nsplit, hd), **f32)
-        self.ws_ml = torch.zeros((B, nq, self.nsplit, 2), **f32)
+        self.ws_rows = max(B * nq * self.nsplit, K.attn_workspace_rows(nq, nkv))
+        self.ws_acc = torch.zeros((self.ws_rows, hd), **f32)
+        self.ws_ml = torch.zeros((self.ws_rows, 2), **f32)
         self.out_tokens = torch.zeros(B, **i32)
         self.attn_counters = torch.zeros(B * max(1, nkv), **i32)
         cos, sin = rope_table(hd, max_seq, cfg.rope_base)
@@ -328,8 +329,8 @@ class Qwen3Runner(SlotState):
         lib = K.lib()
         w, kv, cfg = self.w, self.kv, self.cfg
         nlp, nsp = lib.bonsai_runner_layer_ptr_count(), lib.bonsai_runner_step_ptr_count()
-        icfg = (C.c_int * 16)(cfg.hidden, w.inter_local, cfg.layers, w.heads_local, w.kv_heads_local, cfg.head_dim, cfg.vocab,
-                              w.lm_head.shape[0], kv.kvt, kv.page_size, self.max_pages, self.nsplit, w.tp_size, w.tp_rank, int(self.fast), self.nsplit)
+        icfg = (C.c_int * 17)(cfg.hidden, w.inter_local, cfg.layers, w.heads_local, w.kv_heads_local, cfg.head_dim, cfg.vocab,
+                              w.lm_head.shape[0], kv.kvt, kv.page_size, self.max_pages, self.nsplit, w.tp_size, w.tp_rank, int(self.fast), self.nsplit, self.ws_rows)
         gp = (C.c_uint64 * 5)(w.embd.data_ptr(), w.lm_head.data_ptr(), w.out_norm.data_ptr(), self.rope_cos.data_ptr(), self.rope_sin.data_ptr())
         lp = (C.c_uint64 * (nlp * cfg.layers))()
         for l, lw in enumerate(w.layers):

@@ -28,6 +28,7 @@ _SIG = {
     "bonsai_embed_f16": [_vp, _vp, _vp, _i, _i, _vp],
     "bonsai_qknorm_rope_kvstore": [_vp, _i, _vp, _vp, _f, _vp, _vp, _vp, _vp, _i, _vp, _i, _i, _i, _i, _i, _i, _vp, _vp, _vp, _vp, _vp],
     "bonsai_attn_decode": [_vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _vp, _vp, _vp, _vp, _i, _vp, _vp, _vp, _vp, _i, _vp],
+    "bonsai_attn_decode_route": [_vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _vp, _vp, _vp, _vp, _i, _vp, _vp, C.c_longlong, _vp, _vp, _i, _i, _vp],
     "bonsai_attn_decode_force_cuda_cores": [_i],
     "bonsai_attn_decode_qkv_f16": [_vp, _i, _vp, _vp, _f, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _vp, _vp, _i, _vp, _vp, _vp, _vp, _vp],
     "bonsai_sample": [_vp, _i, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _i, _vp, _i, _vp],
@@ -384,18 +385,24 @@ def qknorm_rope_kvstore(qkv, q_norm, k_norm, eps, rope_cos, rope_sin, positions,
                                            ptr(kscale), ptr(vscale), stream()), "qknorm_rope_kvstore")
 
 
+def attn_workspace_rows(nq: int, nkv: int) -> int:
+    """Rows of the split workspace with which decode attention over INT8 / INT4 pages may use every CTA that the device holds: two partial sums of
+    a kv head's queries from each of 888."""
+    return 1776 * (nq // max(1, nkv))
+
+
 def attn_decode(q, positions, block_table, nq, nkv, hd, kvt, page_size, kpool, vpool, kscale=None, vscale=None, nsplit=8,
                 extra_len=0, out=None) -> torch.Tensor:
     batch = q.shape[0]
-    ws_acc = torch.empty((batch, nq, nsplit, hd), dtype=torch.float32, device=q.device)
-    ws_ml = torch.empty((batch, nq, nsplit, 2), dtype=torch.float32, device=q.device)
+    rows = max(batch * nq * nsplit, attn_workspace_rows(nq, nkv) if kvt in (KV_Q8, KV_Q4) else 0)
+    ws_acc = torch.empty((rows, hd), dtype=torch.float32, device=q.device)
+    ws_ml = torch.empty((rows, 2), dtype=torch.float32, device=q.device)
     counters = torch.zeros(batch * nkv, dtype=torch.int32, device=q.device)
     if out is None:
         out = torch.empty((batch, nq, hd), dtype=torch.float32, device=q.device)
-    check(lib().bonsai_attn_decode(q.data_ptr(), positions.data_ptr(), block_table.data_ptr(), block_table.shape[1], batch, nq, nkv, hd,
-                                   kvt, page_size, kpool.data_ptr(), vpool.data_ptr(), ptr(kscale), ptr(vscale), nsplit,
-                                   ws_acc.data_ptr(), ws_ml.data_ptr(), counters.data_ptr(), out.data_ptr(), extra_len, stream()),
-          "attn_decode")
+    check(lib().bonsai_attn_decode_route(q.data_ptr(), positions.data_ptr(), block_table.data_ptr(), block_table.shape[1], batch, nq, nkv, hd,
+                                         kvt, page_size, kpool.data_ptr(), vpool.data_ptr(), ptr(kscale), ptr(vscale), nsplit, ws_acc.data_ptr(),
+                                         ws_ml.data_ptr(), rows, counters.data_ptr(), out.data_ptr(), extra_len, 0, stream()), "attn_decode")
     return out
 
 

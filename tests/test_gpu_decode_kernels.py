@@ -426,6 +426,58 @@ def test_quantised_decode_attention_with_queries_and_probabilities_in_two_f16_te
             assert worst <= 1.0, (b, h, worst, moved.item(), (p @ vh.abs()).min().item())
 
 
+@pytest.mark.parametrize("lens,nq,nkv", [([768], 8, 8), ([769], 8, 8), ([5000, 1, 0, 300], 9, 9), ([385] * 5 + [17], 16, 8), ([384] * 6, 16, 8),
+                                         ([60] * 149 + [9000], 1, 1), ([128] * 150, 2, 1), ([40, 0, 700] * 30, 8, 2)])
+@pytest.mark.parametrize("kvt", [2, 3])
+def test_quantised_decode_attention_cut_into_pieces(lens, nq, nkv, kvt):
+    """CTAs of twelve, six and two warps; pairs that have a CTA each (up to four tiles a warp) and one token more; a pair in many pieces among short
+    ones; sequences without keys in the line; less workspace than every CTA could use, and a captured launch that sees other lengths."""
+    import math
+    from oxibonsai_b200.ops import cuda_ops as K
+    dev, page = _dev(), 16
+    g = torch.Generator(device=dev).manual_seed(len(lens) + nq)
+    rand = lambda *shape: torch.randn(shape, device=dev, generator=g)  # noqa: E731
+    pages = [max(1, -(-n // page)) for n in lens]
+    table, at = torch.zeros((len(lens), max(pages)), dtype=torch.int32, device=dev), 0
+    order = torch.randperm(sum(pages), device=dev, generator=g).to(torch.int32)
+    for b, n in enumerate(pages):
+        table[b, :n] = order[at:at + n]
+        at += n
+    pools, scales, values = [], [], []
+    for _ in range(2):
+        x = rand(at, nkv, page, 128)
+        s = (x.abs().amax(-1) / (127 if kvt == 2 else 7)).contiguous()
+        c = (x / s[..., None]).round()
+        pools.append((c.to(torch.int8) if kvt == 2 else ((c + 8).to(torch.uint8)[..., 0::2] | ((c + 8).to(torch.uint8)[..., 1::2] << 4))).contiguous())
+        scales.append(s)
+        values.append(c.double() * s.double()[..., None])
+    q, pos = rand(len(lens), nq, 128), torch.tensor([n - 1 for n in lens], dtype=torch.int32, device=dev)
+
+    def check(got, lens):
+        for b, n in enumerate(lens):
+            if n == 0:
+                assert not got[b].any()
+                continue
+            k, v = (x[table[b, :max(1, -(-n // page))].long()].transpose(0, 1).reshape(nkv, -1, 128)[:, :n].repeat_interleave(nq // nkv, 0) for x in values)
+            p = (torch.einsum("hd,hnd->hn", q[b].double(), k) / math.sqrt(128)).softmax(-1)
+            # scores and weights of 22 bits, exponentials of 2^-22: some 2^-18 of the weighted values
+            assert ((got[b].double() - torch.einsum("hn,hnd->hd", p, v)).abs() <= 2.0 ** -18 * torch.einsum("hn,hnd->hd", p, v.abs())).all(), b
+
+    check(K.attn_decode(q, pos, table, nq, nkv, 128, kvt, page, *pools, *scales, nsplit=8), lens)
+    small = [torch.empty((len(lens) * nq * 2, n), device=dev) for n in (128, 2)]      # the documented workspace of two splits
+    counters, out = torch.zeros(len(lens) * nkv, dtype=torch.int32, device=dev), torch.empty_like(q)
+    rc = K.lib().bonsai_attn_decode(q.data_ptr(), pos.data_ptr(), table.data_ptr(), table.shape[1], len(lens), nq, nkv, 128, kvt, page, pools[0].data_ptr(),
+                                    pools[1].data_ptr(), scales[0].data_ptr(), scales[1].data_ptr(), 2, small[0].data_ptr(), small[1].data_ptr(),
+                                    counters.data_ptr(), out.data_ptr(), 0, K.stream())
+    assert rc == 0 and not counters.any()
+    check(out, lens)
+    graph = K.capture_graph(dev, lambda: K.attn_decode(q, pos, table, nq, nkv, 128, kvt, page, *pools, *scales, nsplit=8, out=out))
+    fewer = [n // 3 for n in lens]
+    pos.copy_(torch.tensor([n - 1 for n in fewer], dtype=torch.int32))
+    graph.replay()
+    check(out, fewer)
+
+
 @pytest.mark.parametrize("nq,nkv,B", [(4, 2, 1), (3, 3, 37)])
 @pytest.mark.parametrize("kvt", [0, 1, 2, 3])
 def test_row_kernels_of_head_size_128_leave_the_same_bits(nq, nkv, B, kvt):
