@@ -18,6 +18,7 @@ kernels of the native engine.  The sub-2-bit formats (Q1_0_g128, TQ2_0_g128) sho
 """
 from __future__ import annotations
 
+import ctypes as C
 from typing import Iterator, Sequence
 
 import numpy as np
@@ -84,7 +85,7 @@ class GenericQwen3Engine:
         self.max_seq_len, self.max_batch = max_seq_len, max(1, int(max_batch))
         self.prefill_min, self.prefill_chunk = prefill_min, prefill_chunk
         self.prefill_min_tokens = prefill_min          # the name the scheduler reads
-        self._wscratch = None
+        self._prompt = self._row = None
         self.sampling = sampling or SamplingPreset.GREEDY.params()
         f, dev, B = self.gguf, self.device, self.max_batch
         self.kvt = {"f32": K.KV_F32, "f16": K.KV_F16, "q8": K.KV_Q8, "q4": K.KV_Q4}[kv_dtype]
@@ -206,6 +207,33 @@ class GenericQwen3Engine:
             K.sample(self.logits[s], self.temps[s], self.topks[s], self.topps[s], self.rng[s], positions=pos, advance=True,
                      allow_mask=self.allow_mask[s] if masked else None, out=self.token[s])
 
+    def _forward_row(self, slot: int) -> None:
+        """``_forward`` of one slot without sampling, all launches from one native call."""
+        if self._row is None:
+            c = self.config
+            rows = max(c.heads * self.nsplit, K.attn_workspace_rows(c.heads, c.kv_heads))
+            f32 = dict(dtype=torch.float32, device=self.device)
+            self._row = dict(layers=self._layer_words(), acc=torch.empty((rows, c.head_dim), **f32), ml=torch.empty((rows, 2), **f32),
+                             counters=torch.zeros(c.kv_heads, dtype=torch.int32, device=self.device))
+        c, r = self.config, self._row
+        s = [self.embd, self.lm_head, self.out_norm, self.cos, self.sin, self.token[slot:], self.pos[slot:], self.bt[slot], self.h[slot], self.qkv[slot],
+             self.q[slot], self.attn[slot], self.gu[slot], self.act[slot], self.logits[slot], r["acc"], r["ml"], r["counters"], self.status]
+        words = [t.data_ptr() for t in s] + [r["acc"].shape[0], c.hidden, c.inter, c.layers, c.heads, c.kv_heads, c.head_dim, c.vocab, self.lm_head.shape[0], self.kvt,
+                                             self.page, self.nsplit]
+        K.blocks_forward_row((C.c_uint64 * len(words))(*words), r["layers"], c.eps)
+
+    def _layer_words(self):
+        """The layers as csrc/cuda/blocks_prompt.cu reads them."""
+        words = []
+        for l, w in enumerate(self.layers):
+            for parts, single in ((w["qkv"], ("q", "k", "v")), ([w["o"]], ("o",)), (w["gate_up"], ("gate", "up")), ([w["down"]], ("down",))):
+                fused = [*parts, *[None] * (len(single) - 1)] if len(parts) == 1 else [w[k] for k in single]
+                for m in fused:
+                    words += [0, 0, 0] if m is None else [m.type, m.n, m.data.data_ptr()]
+            words += [w[k].data_ptr() for k in ("attn_norm", "ffn_norm", "q_norm", "k_norm")]
+            words += [self.kpool[l].data_ptr(), self.vpool[l].data_ptr(), *(0 if s is None else s[l].data_ptr() for s in (self.kscale, self.vscale))]
+        return (C.c_uint64 * len(words))(*words)
+
     # kept for callers of the single-stream engine
     def _step_eager(self) -> None:
         self._forward(0, 1, True)
@@ -219,44 +247,75 @@ class GenericQwen3Engine:
         """Runs ``tokens`` (int32 on the device) of the sequence in ``slot`` through every layer as chunks of up to
         ``prefill_chunk`` tokens, filling the KV cache for positions pos0 .. pos0 + len - 1.  Nothing is sampled and no logits
         are left: the caller feeds the prompt's last token through ``_forward``."""
-        c, eps, dev = self.config, self.config.eps, self.device
-        qd, kvd = c.heads * c.head_dim, c.kv_heads * c.head_dim
-        if self._wscratch is None:
-            self._wscratch = torch.empty(max(c.hidden * c.inter, qd * c.hidden), dtype=torch.float16, device=dev)
-        f32 = dict(dtype=torch.float32, device=dev)
-
-        def mm(lin: _Linear, x16: torch.Tensor, out: torch.Tensor, residual: torch.Tensor | None = None) -> None:
-            w16 = K.quant_to_f16(lin.type, lin.data, lin.n, lin.k, out=self._wscratch[: lin.n * lin.k].view(lin.n, lin.k), paired=True)
-            K.dense_gemm_f16(w16, x16, out=out, status=self.status, residual=residual)
-
+        b = self._prompt_buffers(slot)
         done = 0
         while done < tokens.numel():
             T = min(self.prefill_chunk, tokens.numel() - done)
             p0 = pos0 + done
-            h = torch.index_select(self.embd, 0, tokens[done:done + T].long()).float()
-            positions = torch.arange(p0, p0 + T, dtype=torch.int32, device=dev)
-            bt = self.bt[slot:slot + 1].expand(T, -1).contiguous()
-            qkv = torch.empty((T, qd + 2 * kvd), **f32)
-            q = torch.empty((T, c.heads, c.head_dim), **f32)
-            gate, up, act = (torch.empty((T, c.inter), **f32) for _ in range(3))
-            for l, w in enumerate(self.layers):
-                xn = K.norm_to_f16_paired(h, w["attn_norm"], eps)
-                mm(w["q"], xn, qkv[:, :qd])
-                mm(w["k"], xn, qkv[:, qd:qd + kvd])
-                mm(w["v"], xn, qkv[:, qd + kvd:])
-                ks = self.kscale[l] if self.kscale is not None else None
-                vs = self.vscale[l] if self.vscale is not None else None
-                K.qknorm_rope_kvstore(qkv, w["q_norm"], w["k_norm"], eps, self.cos, self.sin, positions, bt, q, c.heads, c.kv_heads, c.head_dim,
-                                      self.kvt, self.page, self.kpool[l], self.vpool[l], ks, vs)
-                a16 = K.attn_prefill(q, p0, self.bt[slot], c.heads, c.kv_heads, c.head_dim, self.kvt, self.page, self.kpool[l], self.vpool[l], ks, vs,
-                                     status=self.status)
-                mm(w["o"], a16, h, residual=h)
-                xn = K.norm_to_f16_paired(h, w["ffn_norm"], eps)
-                mm(w["gate"], xn, gate)
-                mm(w["up"], xn, up)
-                K.swiglu(gate, up, out=act)
-                mm(w["down"], K.norm_to_f16_paired(act, None, eps), h, residual=h)
+            if T <= 64:
+                self._short_chunk(tokens[done:done + T], p0, slot, b["scratch"])
+                done += T
+                continue
+            b["tokens"][:T].copy_(tokens[done:done + T], non_blocking=True)
+            torch.arange(p0, p0 + T, dtype=torch.int32, device=self.device, out=b["positions"][:T])
+            K.blocks_prompt_chunk(b["prompt"], b["layers"], self.config.eps, T, p0)
             done += T
+
+    def _short_chunk(self, tokens: torch.Tensor, p0: int, slot: int, scratch: torch.Tensor) -> None:
+        """Up to 64 tokens (the last of a prompt).  Their products are cut along K by the shape of every single matrix, so each matrix keeps a product of
+        its own: over INT4 pages another order of sums would show (``kInt4Tokens`` of the native runner)."""
+        c, eps, dev, T = self.config, self.config.eps, self.device, tokens.numel()
+        qd, kvd = c.heads * c.head_dim, c.kv_heads * c.head_dim
+        f32 = dict(dtype=torch.float32, device=dev)
+
+        def mm(lin: _Linear, x16: torch.Tensor, out: torch.Tensor, residual: torch.Tensor | None = None) -> None:
+            w16 = K.quant_to_f16(lin.type, lin.data, lin.n, lin.k, out=scratch[: lin.n * lin.k].view(lin.n, lin.k), paired=True)
+            K.dense_gemm_f16(w16, x16, out=out, status=self.status, residual=residual)
+
+        h = torch.index_select(self.embd, 0, tokens.long()).float()
+        positions = torch.arange(p0, p0 + T, dtype=torch.int32, device=dev)
+        bt = self.bt[slot:slot + 1].expand(T, -1).contiguous()
+        qkv = torch.empty((T, qd + 2 * kvd), **f32)
+        q = torch.empty((T, c.heads, c.head_dim), **f32)
+        gate, up, act = (torch.empty((T, c.inter), **f32) for _ in range(3))
+        for l, w in enumerate(self.layers):
+            xn = K.norm_to_f16_paired(h, w["attn_norm"], eps)
+            mm(w["q"], xn, qkv[:, :qd])
+            mm(w["k"], xn, qkv[:, qd:qd + kvd])
+            mm(w["v"], xn, qkv[:, qd + kvd:])
+            ks = self.kscale[l] if self.kscale is not None else None
+            vs = self.vscale[l] if self.vscale is not None else None
+            K.qknorm_rope_kvstore(qkv, w["q_norm"], w["k_norm"], eps, self.cos, self.sin, positions, bt, q, c.heads, c.kv_heads, c.head_dim,
+                                  self.kvt, self.page, self.kpool[l], self.vpool[l], ks, vs)
+            a16 = K.attn_prefill(q, p0, self.bt[slot], c.heads, c.kv_heads, c.head_dim, self.kvt, self.page, self.kpool[l], self.vpool[l], ks, vs,
+                                 status=self.status)
+            mm(w["o"], a16, h, residual=h)
+            xn = K.norm_to_f16_paired(h, w["ffn_norm"], eps)
+            mm(w["gate"], xn, gate)
+            mm(w["up"], xn, up)
+            K.swiglu(gate, up, out=act)
+            mm(w["down"], K.norm_to_f16_paired(act, None, eps), h, residual=h)
+
+    def _prompt_buffers(self, slot: int) -> dict:
+        """Activations of one prompt chunk, the scratch matrix and the pointer tables of the native chunk (allocated by the first prompt)."""
+        c, dev = self.config, self.device
+        qd, kvd = c.heads * c.head_dim, c.kv_heads * c.head_dim
+        if self._prompt is None:
+            n = self.prefill_chunk
+            f32, f16, i32 = (dict(dtype=d, device=dev) for d in (torch.float32, torch.float16, torch.int32))
+            # the widest matrix; gate and up together where 104 MB hold them
+            scratch = max(c.hidden * c.inter, qd * c.hidden, min(2 * c.hidden * c.inter, 52 << 20))
+            b = dict(tokens=torch.zeros(n, **i32), positions=torch.zeros(n, **i32), h=torch.empty((n, c.hidden), **f32), qkv=torch.empty((n, qd + 2 * kvd), **f32),
+                     q=torch.empty((n, qd), **f32), xn=torch.empty((n, c.hidden), **f16), attn=torch.empty((n, qd), **f16), act=torch.empty((n, c.inter), **f16),
+                     scratch=torch.empty(scratch, **f16), ws=K.gemm_workspace(dev))
+            b["layers"] = self._layer_words()
+            self._prompt = b
+        b = self._prompt
+        words = [self.embd, self.cos, self.sin, b["tokens"], b["positions"], self.bt[slot], b["h"], b["qkv"], b["q"], b["xn"], b["attn"], b["act"], b["scratch"]]
+        words = [t.data_ptr() for t in words] + [b["scratch"].numel(), b["ws"].data_ptr(), b["ws"].numel() * b["ws"].element_size(), self.status.data_ptr(), c.hidden,
+                                                 c.inter, c.layers, c.heads, c.kv_heads, c.head_dim, c.vocab, self.kvt, self.page]
+        b["prompt"] = (C.c_uint64 * len(words))(*words)
+        return b
 
     def step(self, batch: int = 1, masked: bool = False) -> None:
         """One token for the first ``batch`` slots (tokens and positions are read from device buffers); replays a graph
@@ -322,7 +381,7 @@ class GenericQwen3Engine:
         for i in range(first, n):
             self.token[slot:slot + 1].copy_(toks[i:i + 1], non_blocking=True)
             self.pos[slot] = pos0 + i
-            self._forward(slot, slot + 1, False)
+            self._forward_row(slot)
 
     def finish_sequence(self, prompt: Sequence[int], slot: int = 0, mask=None) -> int:
         """Samples the first token of ``slot`` from the logits the prompt left; the slot is then ready for ``step_batch``."""

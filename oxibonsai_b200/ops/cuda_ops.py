@@ -217,6 +217,11 @@ _QG_SIG = {
     "bonsai_quant_gemv_rows": [_i, _vp, _i, _i],
     "bonsai_swiglu_rows": [_vp, _i, _vp, _i, _i, _i, _vp],
     "bonsai_quant_to_f16": [_i, _vp, _vp, _i, _i, _i, _vp],
+    "bonsai_blocks_prompt_chunk": [_vp, _vp, _f, _i, _i, _vp],
+    "bonsai_blocks_forward_row": [_vp, _vp, _f, _vp],
+    "bonsai_blocks_prompt_words": [],
+    "bonsai_blocks_row_words": [],
+    "bonsai_blocks_layer_words": [],
 }
 _qg_declared = False
 
@@ -309,6 +314,20 @@ def quant_to_f16(type_id: int, w: torch.Tensor, n: int, k: int, out: torch.Tenso
     assert out.dtype == torch.float16 and out.is_contiguous() and out.numel() >= n * k
     check(_qg().bonsai_quant_to_f16(type_id, w.data_ptr(), out.data_ptr(), n, k, int(paired), stream()), "quant_to_f16")
     return out
+
+
+def blocks_prompt_chunk(prompt, layers, eps: float, n_tokens: int, pos0: int) -> None:
+    """One prompt chunk of a model in GGUF blocks; ``prompt`` and ``layers``: the structures of csrc/cuda/blocks_prompt.cu as arrays of 64-bit words."""
+    l = _qg()
+    assert len(prompt) == l.bonsai_blocks_prompt_words() and len(layers) % l.bonsai_blocks_layer_words() == 0
+    check(l.bonsai_blocks_prompt_chunk(prompt, layers, eps, n_tokens, pos0, stream()), "blocks_prompt_chunk")
+
+
+def blocks_forward_row(row, layers, eps: float) -> None:
+    """One token of one sequence of a model in GGUF blocks, to its logits; ``row`` and ``layers`` as above."""
+    l = _qg()
+    assert len(row) == l.bonsai_blocks_row_words() and len(layers) % l.bonsai_blocks_layer_words() == 0
+    check(l.bonsai_blocks_forward_row(row, layers, eps, stream()), "blocks_forward_row")
 
 
 def swiglu(gate: torch.Tensor, up: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:

@@ -220,3 +220,43 @@ def test_streamed_rows_of_every_format(name, tid, tol, n, k):
         # every sum runs over at most K / 32 + 64 rounded steps of terms whose magnitudes add up to |x| |W|, with minima taken off separately
         terms = xn.abs() @ wd.abs().T * (3.0 if name in ("Q2_K", "Q4_K", "Q5_K") else 1.0) + res.abs()
         assert ((y - (xn @ wd.T + res.double())).abs() <= 2.0 ** -23 * (k / 32 + 64) * terms).all(), (name, batch)
+
+
+@pytest.mark.parametrize("name,tid,tol", TYPES)
+@pytest.mark.parametrize("n,k", [(1, 256), (3, 512), (77, 1280)])
+def test_rows_decoded_from_whole_words_are_those_of_single_values(name, tid, tol, n, k):
+    """Warps of 32 blocks that cross rows and end early, the last block of a matrix; a matrix at an odd address keeps the kernel that reads bytes."""
+    from oxibonsai_b200.core.blocks import quantize
+    from oxibonsai_b200.ops import cuda_ops as K
+    rng = np.random.default_rng(n)
+    raw = torch.from_numpy(quantize(tid, rng.normal(size=(n, k)).astype(np.float32) * 0.05).reshape(-1).view(np.uint8).copy()).cuda()
+    room = torch.empty(raw.numel() + 8, dtype=torch.uint8, device="cuda")
+    room[4:4 + raw.numel()] = raw
+    for paired in (True, False):
+        assert torch.equal(K.quant_to_f16(tid, raw, n, k, paired=paired), K.quant_to_f16(tid, room[4:4 + raw.numel()], n, k, paired=paired)), name
+
+
+@pytest.mark.parametrize("fmt", ["q8_0", "q4_k"])
+@pytest.mark.parametrize("kv", ["f16", "q4"])
+def test_native_prompt_chunk_leaves_the_bits_of_its_kernels_one_by_one(fmt, kv, tiny_gguf, tmp_path):
+    from oxibonsai_b200 import cli
+    from oxibonsai_b200.models.qwen3_generic import GenericQwen3Engine
+    path = str(tmp_path / f"tiny_{fmt}.gguf")
+    cli.requantize_gguf(tiny_gguf, path, fmt)
+    tokens = torch.from_numpy(np.random.default_rng(9).integers(0, 1000, 150).astype(np.int32)).cuda()
+    caches = []
+    for slabs in (None, 1, 0):
+        eng = GenericQwen3Engine(path, max_seq_len=256, kv_dtype=kv, prefill_chunk=100)
+        eng._bind(0)
+        buffers = eng._prompt_buffers(0)
+        if slabs == 1:                       # half of the gate and up rows at a time
+            c = eng.config
+            buffers["scratch"] = buffers["scratch"][:max(c.hidden * c.inter, c.heads * c.head_dim * c.hidden, (c.heads + 2 * c.kv_heads) * c.head_dim * c.hidden)]
+        if slabs is None:
+            for at in (0, 100):
+                eng._short_chunk(tokens[at:at + 100], at, 0, buffers["scratch"])
+        else:
+            eng.prefill(tokens, 0, 0)
+        caches.append([t.clone() for t in (eng.kpool, eng.vpool, eng.kscale, eng.vscale) if t is not None])
+    for other in caches[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(caches[0], other))
