@@ -26,6 +26,9 @@
 // Per (tile, group) block a thread issues 16 logic ops, 4 MMAs, 4 loads, 8 integer multiplies that build the
 // zero-padded B operands and a dozen f32 ops: ~0.8 instructions per weight.  The whole kernel executes twice that (24576 x 4096: 4.93 M warp
 // instructions, 1.57 per weight): every CTA quantises the activations, and waits, reductions and stores come on top.
+// Around the main loop a CTA spends, in cycles: set-up 1300 (before the wait for the kernel ahead), inputs and their norm 1200, quantising 1300 per 4096
+// inputs, reduction and store 600 to 1100.  Quantising was 2300 per 4096 while a thread took one chunk after the other, each with trips to L2 of its
+// own: 6144 x 4096 5.9 -> 5.2 us, 4096 x 4096 4.5 -> 4.1, 24576 x 4096 10.7 -> 10.2, 4096 x 12288 8.9 -> 7.7 in chains of themselves, a layer's four 28.2 -> 25.5.
 //
 // Epilogues: store, residual add, SwiGLU over interleaved gate/up rows, and the tensor-parallel one: every finished
 // row goes to all peers as one 8-byte {value, tag} store and the same thread polls its own slots for the peers'
@@ -68,6 +71,12 @@ __device__ __forceinline__ uint32_t s16_mul(uint32_t a, uint32_t b) {
   uint32_t d;
   asm("mul.lo.u32 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
   return d;
+}
+
+__device__ __forceinline__ float s16_warp_max(float v) {
+  float m;
+  asm("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(m) : "f"(v));
+  return m;
 }
 
 // 512 consumer threads only (the producer warp never joins)
@@ -188,8 +197,9 @@ __global__ void __launch_bounds__(kS16Threads, 1) bitgemv_s16_kernel(S16Args a, 
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int ntiles = (a.N + 15) >> 4;
-  const int tile_lo = (int)(((long long)blockIdx.x * ntiles) / gridDim.x);
-  const int tile_hi = (int)(((long long)(blockIdx.x + 1) * ntiles) / gridDim.x);
+  // blockIdx.x * ntiles / gridDim.x without a 64-bit division
+  const unsigned per = (unsigned)ntiles / gridDim.x, over = (unsigned)ntiles - per * gridDim.x;
+  const int tile_lo = (int)(per * blockIdx.x + over * blockIdx.x / gridDim.x), tile_hi = (int)(per * (blockIdx.x + 1) + over * (blockIdx.x + 1) / gridDim.x);
   const int nb_total = (tile_hi - tile_lo) * ng;           // blocks of this CTA's stream
   const int nstage_total = (nb_total + kS16StageBlocks - 1) / kS16StageBlocks;
   const uint8_t* wbase = a.w + (size_t)tile_lo * ng * kS16BlockBytes;
@@ -252,24 +262,33 @@ __global__ void __launch_bounds__(kS16Threads, 1) bitgemv_s16_kernel(S16Args a, 
 
   // ---- consumers ----
   constexpr int NT = kS16Warps * 32;
-  for (int i = tid; i < kS16MaxTiles * kS16Warps * 16; i += NT) part[i] = 0.0f;   // nothing here depends on an earlier kernel
+  // Nothing from here to the wait depends on an earlier kernel: the partial sums' zeros, the norm weights of the thread's first four chunks, the place
+  // of the warp's first block.
+  for (int i = tid; i < (tile_hi - tile_lo) * kS16Warps * 4; i += NT) reinterpret_cast<float4*>(part)[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  const int nch = K >> 2, g = lane >> 2, t = lane & 3;
+  const float4* x4 = reinterpret_cast<const float4*>(a.x);
+  const float4* w4 = reinterpret_cast<const float4*>(a.norm_w);
+  const float4 none = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  float4 nw[4], keep[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) nw[i] = w4 != nullptr && tid + i * NT < nch ? __ldg(w4 + tid + i * NT) : none;
+  int tl = (kS16Bpw * warp) / ng, grp = (kS16Bpw * warp) - tl * ng;       // (tile, group) of the warp's first block of the current stage
   asm volatile("griddepcontrol.wait;" ::: "memory");
   {
     // Activations: f32 -> (RMS-normalised) -> two int8 terms per 128-input group.  Thread tid + i * NT holds the four
-    // inputs of chunk c; a warp's 32 chunks are one group and lanes 8j..8j+7 hold the 32 inputs of MMA step j.
-    const int nch = K >> 2;
-    const float4* x4 = reinterpret_cast<const float4*>(a.x);
-    float4 keep[2];
+    // inputs of chunk c; a warp's 32 chunks are one group and lanes 8j..8j+7 hold the 32 inputs of MMA step j.  Inputs and norm weights are
+    // requested four chunks ahead.
     float ss = 0.0f;
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
+    for (int i = 0; i < 4; ++i) {
       const int c = tid + i * NT;
-      keep[i] = c < nch ? x4[c] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-      ss += keep[i].x * keep[i].x + keep[i].y * keep[i].y + keep[i].z * keep[i].z + keep[i].w * keep[i].w;
+      keep[i] = c < nch ? x4[c] : none;
     }
     float inv = 1.0f;
     if (a.norm_w != nullptr) {
-      for (int c = tid + 2 * NT; c < nch; c += NT) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) ss += keep[i].x * keep[i].x + keep[i].y * keep[i].y + keep[i].z * keep[i].z + keep[i].w * keep[i].w;
+      for (int c = tid + 4 * NT; c < nch; c += NT) {
         const float4 v = x4[c];
         ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
       }
@@ -280,61 +299,75 @@ __global__ void __launch_bounds__(kS16Threads, 1) bitgemv_s16_kernel(S16Args a, 
       tsum = warp_sum(tsum);
       inv = 1.0f / sqrtf(tsum / (float)K + a.eps);
     }
-    auto emit = [&](int c, float4 v) {      // whole warps enter (K % 128 == 0): c / 32 is the warp's group
-      if (a.norm_w != nullptr) {
-        const float4 ww = reinterpret_cast<const float4*>(a.norm_w)[c];
-        v.x *= ww.x * inv; v.y *= ww.y * inv; v.z *= ww.z * inv; v.w *= ww.w * inv;
+    // Two chunks c and c + NT side by side: a chunk is a chain of some 900 cycles (maximum over the group, division, rounding, sums), whatever runs
+    // beside it.  Whole warps enter (K % 128 == 0): c / 32 is the warp's group.
+    auto emit = [&](int c, const float4 (&in)[2], const float4 (&norm)[2]) {
+      float v[2][4], sx[2];
+      uint32_t w1[2] = {0u, 0u}, w2[2] = {0u, 0u};
+      int sums[2];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const float4 x = in[u], ww = norm[u];
+        v[u][0] = x.x; v[u][1] = x.y; v[u][2] = x.z; v[u][3] = x.w;
+        if (a.norm_w != nullptr) { v[u][0] *= ww.x * inv; v[u][1] *= ww.y * inv; v[u][2] *= ww.z * inv; v[u][3] *= ww.w * inv; }
+        const float amax = s16_warp_max(fmaxf(fmaxf(fabsf(v[u][0]), fabsf(v[u][1])), fmaxf(fabsf(v[u][2]), fabsf(v[u][3]))));
+        sx[u] = amax > 0.0f ? amax * (1.0f / 127.0f) : 1.0f;
       }
-      const float amax = warp_max(fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
-      const float sx = amax > 0.0f ? amax * (1.0f / 127.0f) : 1.0f;
-      const float rs = 1.0f / sx;
       // Round with the 1.5 * 2^23 trick: (f + magic) holds rint(f) in its low mantissa bits (two's complement, so the low
       // byte is the int8 value) and (f + magic) - magic is rint(f) as a float.  |f| <= 127 and |f - rint(f)| * 254 <= 127
       // by construction, so nothing needs clamping.
       constexpr float kMagic = 12582912.0f;
-      const float f[4] = {v.x * rs, v.y * rs, v.z * rs, v.w * rs};
-      uint32_t w1 = 0, w2 = 0;
-      float fs1 = 0.0f, fs2 = 0.0f;
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float m1 = f[e] + kMagic, r1 = m1 - kMagic;
-        const float m2 = (f[e] - r1) * kS16Term2 + kMagic, r2 = m2 - kMagic;
-        w1 |= (__float_as_uint(m1) & 255u) << (8 * e);
-        w2 |= (__float_as_uint(m2) & 255u) << (8 * e);
-        fs1 += r1;
-        fs2 += r2;
-      }
-      reinterpret_cast<uint32_t*>(xq)[c] = w1;
-      reinterpret_cast<uint32_t*>(xq + term_stride)[c] = w2;
-      // sums over the eight lanes of a step
+      for (int u = 0; u < 2; ++u) {
+        const float rs = 1.0f / sx[u];
 #pragma unroll
-      for (int o = 4; o > 0; o >>= 1) {      // sums of small integers: exact in f32
-        fs1 += __shfl_xor_sync(0xffffffffu, fs1, o);
-        fs2 += __shfl_xor_sync(0xffffffffu, fs2, o);
+        for (int e = 0; e < 4; ++e) {
+          const float f = v[u][e] * rs, m1 = f + kMagic, m2 = (f - (m1 - kMagic)) * kS16Term2 + kMagic;
+          w1[u] |= (__float_as_uint(m1) & 255u) << (8 * e);
+          w2[u] |= (__float_as_uint(m2) & 255u) << (8 * e);
+        }
+        // both terms' sums over the eight lanes of a step in one word: at most 32 * 127 each
+        sums[u] = __dp4a((int)w1[u], 0x01010101, 0) * 65536 + __dp4a((int)w2[u], 0x01010101, 0);
       }
-      if ((lane & 7) == 0) {
-        const int j = lane >> 3;
-        const int s1 = (int)fs1, s2 = (int)fs2;
-        S16Step r;
-        r.og0 = -s1 * (1 << (2 * j));
-        r.og1 = -s2 * (1 << (2 * j));
-        r.sx = sx * (1.0f / (float)(1 << (2 * j)));
-        r.pad = 0.0f;
-        steps[(size_t)(c >> 5) * 4 + j] = r;
+#pragma unroll
+      for (int o = 4; o > 0; o >>= 1)
+#pragma unroll
+        for (int u = 0; u < 2; ++u) sums[u] += __shfl_xor_sync(0xffffffffu, sums[u], o);
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int at = c + u * NT;
+        if (at >= nch) continue;
+        reinterpret_cast<uint32_t*>(xq)[at] = w1[u];
+        reinterpret_cast<uint32_t*>(xq + term_stride)[at] = w2[u];
+        if ((lane & 7) == 0) {
+          const int j = lane >> 3, s2 = (int)(short)(sums[u] & 0xffff), s1 = (sums[u] - s2) >> 16;
+          S16Step r;
+          r.og0 = -s1 * (1 << (2 * j));
+          r.og1 = -s2 * (1 << (2 * j));
+          r.sx = sx[u] * (1.0f / (float)(1 << (2 * j)));
+          r.pad = 0.0f;
+          steps[(size_t)(at >> 5) * 4 + j] = r;
+        }
       }
     };
+#pragma unroll 1
+    for (int c = tid; c - tid < nch; c += 2 * NT) {          // every warp of the block takes part to the end: its tail chunks are zeros
+      const float4 now[2] = {keep[0], keep[1]}, norm[2] = {nw[0], nw[1]};
+      keep[0] = keep[2]; keep[1] = keep[3];
+      nw[0] = nw[2]; nw[1] = nw[3];
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const int c = tid + i * NT;
-      if (c < nch) emit(c, keep[i]);
+      for (int i = 0; i < 2; ++i) {
+        const int ahead = c + (4 + i) * NT;
+        keep[2 + i] = ahead < nch ? x4[ahead] : none;
+        nw[2 + i] = w4 != nullptr && ahead < nch ? __ldg(w4 + ahead) : none;
+      }
+      emit(c, now, norm);
     }
-    for (int c = tid + 2 * NT; c < nch; c += NT) emit(c, x4[c]);
     s16_bar();
   }
 
   // ---- main loop: kS16Bpw consecutive blocks per warp per stage ----
   {
-    const int g = lane >> 2, t = lane & 3;
     // this lane supplies output column n = g = 2 * step + term of every B operand
     const int my_step = g >> 1;
     const uint32_t sel[4] = {my_step == 0 ? 1u : 0u, my_step == 1 ? 1u : 0u, my_step == 2 ? 1u : 0u, my_step == 3 ? 1u : 0u};
@@ -356,9 +389,7 @@ __global__ void __launch_bounds__(kS16Threads, 1) bitgemv_s16_kernel(S16Args a, 
       }
       tot_lo = tot_hi = 0.0f;
     };
-    // (tile, group) of the warp's first block of the current stage, advanced by one stage's blocks per iteration
-    int tl = (kS16Bpw * warp) / ng, grp = (kS16Bpw * warp) - tl * ng;
-    int slot = 0;
+    int slot = 0;                                                        // (tl, grp) advances by one stage's blocks per iteration
     uint32_t phase = 0;
     for (int s = 0; s < nstage_total; ++s) {
       if (!s16_wait(&full[slot], phase, lane, abort_flag)) break;
