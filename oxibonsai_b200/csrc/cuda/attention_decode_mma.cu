@@ -138,7 +138,21 @@ __global__ void __launch_bounds__(NW * 32, 8 / NW) attn_decode_mma_kernel(MmaAtt
   const int first_tb = t0 + warp * kMmaTile;
   const bool early = warp < ntiles && !(p.qkv != nullptr && len - 1 >= first_tb && len - 1 < first_tb + kMmaTile);
   if (early) issue_tile(warp, 0);
-  if (p.qkv != nullptr) asm volatile("griddepcontrol.wait;" ::: "memory");
+  // norm weights and rotation of the warp's first item (below) are older than the projections too (with the fences of the merge gone, one token behind
+  // 4096 of 32 / 8 heads in the step 11.0 -> 9.8 us)
+  const int pos = max(len - 1, 0);
+  float nw[4], turn[4];      // weights of dimensions lane + 32 i; cosines and sines of lane, lane + 32
+  if (p.qkv != nullptr) {
+    const float* w = warp < G ? p.q_norm : p.k_norm;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) nw[i] = __ldg(w + lane + 32 * i);
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      turn[2 * i] = __ldg(p.rope_cos + (size_t)pos * 64 + lane + 32 * i);
+      turn[2 * i + 1] = __ldg(p.rope_sin + (size_t)pos * 64 + lane + 32 * i);
+    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+  }
 
   // Q as A-operand fragments: rows 0..G-1 hold the group's query heads (scaled), rows G..15 are zero
   uint32_t qa[8][2];   // per 16-wide k step: a0 (row, k lo pair) and a2 (row, k hi pair); a1 = a3 = 0 (rows 8..15)
@@ -147,7 +161,6 @@ __global__ void __launch_bounds__(NW * 32, 8 / NW) attn_decode_mma_kernel(MmaAtt
   if (p.qkv != nullptr) {
     // a warp per item: the G query heads, plus the new token's K and V rows in the CTA that owns position len - 1
     float* qs = sh;                                          // [G][128] normalised, rotated, scaled queries
-    const int pos = max(len - 1, 0);
     const bool owner = pos >= t0 && pos < t1;
     const float* raw = p.qkv + (size_t)b * p.qkv_stride;
     for (int it = warp; it < G + (owner ? 2 : 0); it += kMmaWarps) {
@@ -156,10 +169,13 @@ __global__ void __launch_bounds__(NW * 32, 8 / NW) attn_decode_mma_kernel(MmaAtt
       float y0 = src[lane], y1 = src[lane + 32], y2 = src[lane + 64], y3 = src[lane + 96];
       if (!is_v) {
         const float inv = 1.0f / sqrtf(mma_warp_sum(y0 * y0 + y1 * y1 + y2 * y2 + y3 * y3) / (float)hd + p.eps);
-        const float* w = is_q ? p.q_norm : p.k_norm;
-        const float n0 = w[lane] * y0 * inv, n1 = w[lane + 32] * y1 * inv, n2 = w[lane + 64] * y2 * inv, n3 = w[lane + 96] * y3 * inv;
-        const float c0 = p.rope_cos[(size_t)pos * 64 + lane], s0 = p.rope_sin[(size_t)pos * 64 + lane];
-        const float c1 = p.rope_cos[(size_t)pos * 64 + lane + 32], s1 = p.rope_sin[(size_t)pos * 64 + lane + 32];
+        if (it != warp) {                                     // a second item of the warp
+          const float* w = is_q ? p.q_norm : p.k_norm;
+#pragma unroll
+          for (int i = 0; i < 4; ++i) nw[i] = w[lane + 32 * i];
+        }
+        const float n0 = nw[0] * y0 * inv, n1 = nw[1] * y1 * inv, n2 = nw[2] * y2 * inv, n3 = nw[3] * y3 * inv;
+        const float c0 = turn[0], s0 = turn[1], c1 = turn[2], s1 = turn[3];
         y0 = n0 * c0 - n2 * s0; y2 = n0 * s0 + n2 * c0;      // dims (lane, lane + 64)
         y1 = n1 * c1 - n3 * s1; y3 = n1 * s1 + n3 * c1;      // dims (lane + 32, lane + 96)
       }
@@ -173,8 +189,7 @@ __global__ void __launch_bounds__(NW * 32, 8 / NW) attn_decode_mma_kernel(MmaAtt
         dst[lane] = __float2half_rn(y0); dst[lane + 32] = __float2half_rn(y1); dst[lane + 64] = __float2half_rn(y2); dst[lane + 96] = __float2half_rn(y3);
       }
     }
-    if (owner) __threadfence();                              // the appended rows are read back through cp.async below
-    __syncthreads();
+    __syncthreads();                                         // (the appended rows are read back by this CTA below)
     qp = qs + (row < G ? row : 0) * hd;
     q_mul = 1.0f;
   }
@@ -367,17 +382,16 @@ __global__ void __launch_bounds__(NW * 32, 8 / NW) attn_decode_mma_kernel(MmaAtt
     }
   }
   if (parts == 1) return;
-  __threadfence();
   __syncthreads();
-  if (threadIdx.x == 0) {
+  if (threadIdx.x == 0) {       // one acquire-release operation instead of fences by every thread on both sides
     int* ctr = p.counters + (size_t)b * p.nkv + kvh;
-    const int prev = atomicAdd(ctr, 1);
+    int prev;
+    asm volatile("atom.add.acq_rel.gpu.global.s32 %0, [%1], 1;" : "=r"(prev) : "l"(ctr) : "memory");
     s_last = (prev == parts - 1);
     if (s_last) *ctr = 0;
   }
   __syncthreads();
   if (!s_last) return;
-  __threadfence();
   // ---- merge of the splits by the last CTA of this (sequence, kv head): see attention_decode.cu -----
   float* s_f = sh;
   float* s_l = sh + G * nsplit;
