@@ -657,7 +657,7 @@ __global__ void __launch_bounds__(256) quant_to_f16_kernel(const uint8_t* __rest
 
 // The same with 32 weights per thread, decoded from whole words: a warp turns 32 neighbouring blocks of 32 into 2 KB of rows, which go through
 // shared memory so that its stores are whole lines.  Row r of the matrix becomes row r * mul + add of out.  The last block, behind whose words
-// nothing needs to be readable, is decoded value by value.  2560 x 9728 in Q8_0: 18.5 us with eight byte loads per thread, 8.6 here.
+// nothing needs to be readable, is decoded value by value.  2560 x 9728 in Q8_0: 18.5 us with eight byte loads per thread, 13.5 here.
 template <typename D, typename Q>
 __global__ void __launch_bounds__(256) quant_rows_kernel(const uint8_t* __restrict__ w, uint4* __restrict__ out, int N, int K, int paired, int mul, int add) {
   __shared__ uint4 stage[8][128];
