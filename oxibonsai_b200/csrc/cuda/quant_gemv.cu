@@ -4,13 +4,17 @@
 // Replaces the reference's per-format single-GEMV wrappers cuda_gemv_q4_0 / q8_0, cuda_gemv_q{2..8}k
 // and cuda_gemv_fp8_* (crates/oxibonsai-kernels/src/gpu_backend/cuda_q_std_kernels.rs:200-,
 // cuda_k_quant_kernels.rs:640-, cuda_fp8_kernels.rs:300-) with kernels templated on the block decoder.
-// Products and sums are f32, with optional fused RMSNorm of the input and residual add.
-// quant_stream_kernel (below) serves matrices whose rows can be copied in 16-byte units; quant_gemv_kernel and its
+// Products and sums are f32 (exact integers inside a block in one kernel), with optional fused RMSNorm of the input and residual add.
+// quant_stream_imma_kernel serves Q4_0, Q8_0 and Q4_K of whole 256-input units, its sums of 32 products exact integers; quant_stream_kernel the other
+// matrices whose rows can be copied in 16-byte units; quant_gemv_kernel and its
 // batched form take the rest: one warp owns a row, for 32-element blocks every lane decodes a whole block per step
 // (32 blocks = 1024 inputs per warp step), for 256-element super-blocks the 32 lanes share a block, eight elements each.
 // Block layouts are the ones documented in csrc/core/blocks.hpp and csrc/core/kquants.hpp.
 #include <cuda_bf16.h>
 #include <cuda_fp8.h>
+
+#include <atomic>
+#include <type_traits>
 
 #include "common.cuh"
 #include "tcgen05.cuh"
@@ -486,6 +490,361 @@ static int qs_launch(const QsParams& p, int grid, size_t smem, cudaStream_t st) 
   return e == cudaSuccess ? BONSAI_CUDA_OK : BONSAI_CUDA_LAUNCH_FAILED;
 }
 
+// ---- one or two tokens on the integer tensor cores ----------------------------------------------------------------------------------
+// Q4_0, Q8_0 and Q4_K rows: a block of 32 codes times 32 inputs is one K extent of mma.sync.m16n8k32, for sixteen rows at once.  The inputs of a
+// block are four int8 terms of seven bits, x = s (q1 + q2 / 2^7 + q3 / 2^14 + q4 / 2^21) with s a power of two: 28 bits of the block's largest value,
+// every step of the split exact.  The terms are four columns.  Of one token two neighbouring blocks share an accumulator, the inputs of the first in
+// columns 0-3 and those of the second in 4-7 (zeros elsewhere); a second token has columns 4-7 instead.  Products and their sums are exact integers;
+// scales, minima (times the sum of the block's inputs) and the sums over blocks are f32.
+// A CTA owns tiles of sixteen rows.  A producer warp copies them, a segment of K at a time, row by row into a ring whose pitch keeps the rows' words
+// apart; a consumer warp takes 256 inputs of every segment and keeps its rows' sums to the end of the tile; the warps' sums meet in warp order.
+// Bound by the codes' way from shared memory to operands and the blocks' scales, some two instructions per weight where the kernel above takes six; the
+// large matrices come near the memory's rate.  One token, us above -> here: Q4_K 6144 x 4096 10.9 -> 7.0, 24576 x 4096 30.7 -> 17.9 (8.8 at the copy
+// rate), 4096 x 12288 19.9 -> 12.2; Q4_0 24576 x 4096 30.4 -> 16.7; Q8_0 24576 x 4096 29.4 -> 23.2 (16.6).  Two tokens: Q4_K 24576 x 4096 37.1 -> 21.4,
+// Q8_0 38.3 -> 27.2.  Relative error against 64 bits there: Q4_K 2.4e-7 -> 1.4e-7, Q4_0 9.5e-8 -> 8.6e-8, Q8_0 8.5e-8 -> 7.4e-8.
+struct QiParams {
+  const uint8_t* w;
+  const float *x, *norm_w, *residual;
+  float* out;
+  int* status;
+  float eps;
+  int N, K, nseg, warps, stages, pitch;      // segments of K; consumer warps = 256-input units of a segment
+  int x_ld, out_ld;
+};
+constexpr int kQiMaxWarps = 20, kQiMaxTiles = 12, kQiMaxStages = 4;
+
+template <bool SIGNED>
+__device__ __forceinline__ void qi_mma(int* d, const uint32_t* a, uint32_t b0, uint32_t b1, bool fresh) {
+  const int z = 0;
+  if (fresh) {
+    if (SIGNED)
+      asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+          : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "r"(z));
+    else
+      asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+          : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "r"(z));
+  } else {
+    if (SIGNED)
+      asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+          : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+    else
+      asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+          : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+  }
+}
+__device__ __forceinline__ uint32_t qi_word(const uint8_t* p) { return *reinterpret_cast<const uint32_t*>(p); }      // 4-byte aligned
+// word number i of bytes that lie two behind a 4-byte boundary
+__device__ __forceinline__ uint32_t qi_word2(const uint8_t* p, int i) {
+  const uint32_t* a = reinterpret_cast<const uint32_t*>(p - 2) + i;
+  return __funnelshift_r(a[0], a[1], 16);
+}
+
+// A unit of a row: 256 weights, kUnit bytes at `p` (16-byte aligned).  codes: the lane's share (t of four) of block j as the first operand's two words.
+// factor: what block j is multiplied with, or (of_sum) what the sum of its inputs is multiplied with.
+struct QiQ4_0 { static constexpr int kUnit = 144; static constexpr bool kSigned = true, kNibbles = true, kSums = false;
+  const uint8_t* p;
+  __device__ void load(const uint8_t* at) { p = at; }
+  __device__ void codes(int j, int t, uint32_t& lo, uint32_t& hi) const {
+    const uint8_t* b = p + 18 * j + 2;                        // two bytes off a boundary for even j
+    const uint32_t w = (j & 1) ? qi_word(b + 4 * t) : qi_word2(b, t);
+    lo = ((w << 4) & 0xF0F0F0F0u) ^ 0x80808080u; hi = (w & 0xF0F0F0F0u) ^ 0x80808080u; }      // 16 (q - 8)
+  __device__ float factor(int j, bool) const { return qs_f16(p + 18 * j) * 0.0625f; } };
+struct QiQ8_0 { static constexpr int kUnit = 272; static constexpr bool kSigned = true, kNibbles = false, kSums = false;
+  const uint8_t* p;
+  __device__ void load(const uint8_t* at) { p = at; }
+  __device__ void codes(int j, int t, uint32_t& lo, uint32_t& hi) const {
+    const uint8_t* b = p + 34 * j + 2;
+    if (j & 1) { lo = qi_word(b + 4 * t); hi = qi_word(b + 16 + 4 * t); }
+    else { lo = qi_word2(b, t); hi = qi_word2(b, t + 4); } }
+  __device__ float factor(int j, bool) const { return qs_f16(p + 34 * j); } };
+struct QiQ4K { static constexpr int kUnit = 144; static constexpr bool kSigned = false, kNibbles = true, kSums = true;
+  const uint8_t* p;
+  uint4 head;                // d and dmin, twelve bytes of scales
+  __device__ void load(const uint8_t* at) { p = at; head = *reinterpret_cast<const uint4*>(at); }
+  __device__ void codes(int j, int t, uint32_t& lo, uint32_t& hi) const {
+    const uint32_t w = qi_word(p + 16 + 16 * j + 4 * t);
+    lo = w & 0x0F0F0F0Fu; hi = (w >> 4) & 0x0F0F0F0Fu; }
+  __device__ float factor(int j, bool of_sum) const {
+    const __half2 dd = *reinterpret_cast<const __half2*>(&head.x);
+    const uint32_t low = of_sum ? head.z : head.y, high = of_sum ? head.w >> 16 : head.w;
+    const float q = qs_int(((low >> (4 * j)) & 15u) | (((high >> (2 * j)) & 3u) << 4));
+    return (of_sum ? -__high2float(dd) : __low2float(dd)) * q; } };
+
+template <typename D, int NB>
+__global__ void __launch_bounds__((kQiMaxWarps + 1) * 32, 1) quant_stream_imma_kernel(const __grid_constant__ QiParams p) {
+  extern __shared__ __align__(128) uint8_t qi_smem[];      // ring, [NB][4][K + 64] terms, [NB][K / 32] {unit, sum of inputs}, [tiles][warps][NB][16] sums
+  __shared__ uint64_t full[kQiMaxStages], empty[kQiMaxStages];
+  __shared__ float s_sq[NB][kQiMaxWarps];
+  __shared__ int s_failed;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nthr = p.warps * 32;
+  const int stage_bytes = 16 * p.pitch, plane = p.K + 64;
+  int8_t* xq = reinterpret_cast<int8_t*>(qi_smem + p.stages * stage_bytes);
+  float2* blocks = reinterpret_cast<float2*>(xq + NB * 4 * plane);
+  float* part = reinterpret_cast<float*>(blocks + NB * (p.K >> 5));
+  const unsigned ntiles = (unsigned)(p.N + 15) >> 4, per = ntiles / gridDim.x, over = ntiles - per * gridDim.x;
+  const int tile_lo = (int)(per * blockIdx.x + over * blockIdx.x / gridDim.x), tile_hi = (int)(per * (blockIdx.x + 1) + over * (blockIdx.x + 1) / gridDim.x);
+  const int units = p.K >> 8, steps = (tile_hi - tile_lo) * p.nseg;
+  const long long row_bytes = (long long)units * D::kUnit;
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (tid < kQiMaxStages) {
+    tc::mbar_init(&full[tid], 1);
+    tc::mbar_init(&empty[tid], p.warps);
+    tc::mbar_fence_init();
+  }
+  if (tid == 0) s_failed = 0;
+  __syncthreads();
+  bool failed = false;
+
+  if (warp == p.warps) {
+    // ---- producer: lanes 0-15 copy a row's piece each; weights depend on no earlier kernel --------------------------------------------------
+    int s = 0, seg = 0, tile = tile_lo, issued = 0;
+    uint32_t phase = 1;
+    for (; issued < steps; ++issued) {
+      if (!__all_sync(0xffffffffu, tc::mbar_wait_sleep<40>(&empty[s], phase))) { failed = true; break; }
+      const int u0 = seg * p.warps, nu = min(p.warps, units - u0);
+      const uint32_t bytes = (uint32_t)nu * D::kUnit;
+      if (lane == 0) tc::mbar_arrive_expect_tx(&full[s], 16 * bytes);
+      __syncwarp();
+      if (lane < 16)
+        tc::bulk_g2s(qi_smem + s * stage_bytes + lane * p.pitch, p.w + (long long)min(tile * 16 + lane, p.N - 1) * row_bytes + (long long)u0 * D::kUnit, bytes, &full[s]);
+      if (++s == p.stages) { s = 0; phase ^= 1; }
+      if (++seg == p.nseg) { seg = 0; ++tile; }
+    }
+    if (lane == 0) tc::mbar_drain(full, issued, p.stages);
+    __syncwarp();
+  } else if (warp < p.warps) {
+    const int g = lane >> 2, t = lane & 3;
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    // ---- inputs: a thread has four neighbours, eight lanes a block of 32 -----------------------------------------------------------------------------------
+#pragma unroll 1
+    for (int n = 0; n < NB; ++n) {
+      const float4 *x4 = reinterpret_cast<const float4*>(p.x + (size_t)n * p.x_ld), *w4 = reinterpret_cast<const float4*>(p.norm_w);
+      const int nch = p.K >> 2;
+      float sq = 0.0f;
+#pragma unroll 2
+      for (int c = tid; c < nch; c += nthr) {          // whole warps: K is a multiple of 256, so nch of 64
+        float4 v = x4[c];
+        sq += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
+        if (w4 != nullptr) {
+          const float4 ww = __ldg(w4 + c);
+          v.x *= ww.x; v.y *= ww.y; v.z *= ww.z; v.w *= ww.w;
+        }
+        float top = fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)));
+        const float all = (v.x + v.y) + (v.z + v.w);
+        const bool finite = __all_sync(0xffffffffu, all - all == 0.0f);
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+        // the largest input comes to [2^5, 2^6)
+        float unit = __uint_as_float(__float_as_uint(fminf(fmaxf(top, 7.9e-31f), 3.0e38f)) & 0x7F800000u) * 0.03125f;
+        const float back = __uint_as_float(0x7F000000u - __float_as_uint(unit));
+        // (f + 1.5 * 2^23) holds rint(f) in its low byte; what is left, at most a half, is up to 64 of the next term's units
+        constexpr float kMagic = 12582912.0f;
+        float f[4] = {v.x * back, v.y * back, v.z * back, v.w * back};
+        const int blk = c >> 3, i = c & 7;
+        if (!finite) {           // a block with infinities keeps their signs, in units of infinity; one with a NaN is NaN
+          bool inf = false, nan = false;
+          const float e4[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            inf |= isinf(e4[e]);
+            nan |= isnan(e4[e]);
+          }
+          const uint32_t mine = 0xFFu << (lane & 24), infs = __ballot_sync(0xffffffffu, inf) & mine, nans = __ballot_sync(0xffffffffu, nan) & mine;
+          if ((infs | nans) != 0) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) f[e] = isinf(e4[e]) ? copysignf(1.0f, e4[e]) : 0.0f;
+            unit = nans != 0 ? __int_as_float(0x7FFFFFFF) : __int_as_float(0x7F800000);
+          }
+        }
+        uint32_t word[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          uint32_t q[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float m = f[e] + kMagic;
+            q[e] = __float_as_uint(m);
+            f[e] = (f[e] - (m - kMagic)) * 128.0f;
+          }
+          // nibbles: lane t's codes are those of inputs 8t .. 8t + 7, the even ones, then the odd ones;  bytes: inputs 4t .. 4t + 3, then 16 + 4t ..
+          word[k] = D::kNibbles ? __byte_perm(__byte_perm(q[0], q[2], 0x0040), __byte_perm(q[1], q[3], 0x0040), 0x5410)
+                                : __byte_perm(__byte_perm(q[0], q[1], 0x0040), __byte_perm(q[2], q[3], 0x0040), 0x5410);
+          int8_t* dst = xq + (n * 4 + k) * plane + blk * 32;
+          if (D::kNibbles) {
+            *reinterpret_cast<uint16_t*>(dst + (i >> 1) * 8 + (i & 1) * 2) = (uint16_t)word[k];
+            *reinterpret_cast<uint16_t*>(dst + (i >> 1) * 8 + 4 + (i & 1) * 2) = (uint16_t)(word[k] >> 16);
+          } else {
+            *reinterpret_cast<uint32_t*>(dst + (i & 3) * 8 + (i >> 2) * 4) = word[k];
+          }
+        }
+        float sum = 0.0f;
+        if (D::kSums) {      // of the terms, exactly: two of them in a word, at most 2048 each
+          int s12 = __dp4a((int)word[0], 0x01010101, 0) * 65536 + __dp4a((int)word[1], 0x01010101, 0);
+          int s34 = __dp4a((int)word[2], 0x01010101, 0) * 65536 + __dp4a((int)word[3], 0x01010101, 0);
+#pragma unroll
+          for (int o = 4; o > 0; o >>= 1) {
+            s12 += __shfl_xor_sync(0xffffffffu, s12, o);
+            s34 += __shfl_xor_sync(0xffffffffu, s34, o);
+          }
+          const int s2 = (int)(short)(s12 & 0xffff), s4 = (int)(short)(s34 & 0xffff);
+          sum = unit * fmaf((float)((s34 - s4) / 65536 * 128 + s4), 1.0f / 2097152.0f, (float)((s12 - s2) / 65536 * 128 + s2) * (1.0f / 128.0f));
+        }
+        if (i == 0) blocks[n * (p.K >> 5) + blk] = make_float2(unit, sum);
+      }
+      sq = warp_sum(sq);
+      if (lane == 0) s_sq[n][warp] = sq;
+    }
+    asm volatile("bar.sync 1, %0;" ::"r"(nthr) : "memory");
+    // ---- rows -----------------------------------------------------------------------------------------------------------------------------------
+    const int term = g & 3, second = g >> 2;                 // the lane's column of the second operand
+    const uint32_t keep0 = second == 0 ? 0xffffffffu : 0u, keep1 = ~keep0;
+    const int8_t* xcol = xq + (NB == 2 ? 4 * second + term : term) * plane + (NB == 2 ? 0 : second * 32) + t * 8;
+    const bool of_sum = t & 1;                               // odd lanes hold the last two terms, and add what goes with the sum of the inputs
+    int s = 0, seg = 0, tl = 0;
+    uint32_t phase = 0;
+    float tot0 = 0.0f, tot1 = 0.0f, odd0 = 0.0f, odd1 = 0.0f;      // of two tokens the odd blocks apart
+    for (int n = 0; n < steps; ++n) {
+      if (!__all_sync(0xffffffffu, tc::mbar_wait(&full[s], phase))) { failed = true; break; }
+      const int unit = seg * p.warps + warp;
+      if (unit < units) {
+        const uint8_t* at = qi_smem + s * stage_bytes + g * p.pitch + warp * D::kUnit;
+        D r0, r1;
+        r0.load(at);
+        r1.load(at + 8 * p.pitch);
+        const int8_t* xu = xcol + unit * 256;
+        const float2* bu = blocks + (NB == 2 ? (t >> 1) * (p.K >> 5) : t >> 1) + unit * 8;
+#pragma unroll
+        for (int pr = 0; pr < 4; ++pr) {
+          uint32_t a[4], b[4];
+          r0.codes(2 * pr, t, a[0], a[2]);
+          r1.codes(2 * pr, t, a[1], a[3]);
+          r0.codes(2 * pr + 1, t, b[0], b[2]);
+          r1.codes(2 * pr + 1, t, b[1], b[3]);
+          // what an accumulator holds for block j of this lane: even lanes terms one and two, odd lanes three and four
+          auto add = [&](const int* acc, int j, float2 bl, float& s0, float& s1) {
+            float v0 = fmaf((float)acc[1], 1.0f / 128.0f, (float)acc[0]), v1 = fmaf((float)acc[3], 1.0f / 128.0f, (float)acc[2]);
+            v0 = fmaf(__shfl_xor_sync(0xffffffffu, v0, 1), 1.0f / 16384.0f, v0);
+            v1 = fmaf(__shfl_xor_sync(0xffffffffu, v1, 1), 1.0f / 16384.0f, v1);
+            if (D::kSums || !of_sum) {
+              const float m = of_sum ? bl.y : bl.x;
+              s0 = fmaf(r0.factor(j, of_sum) * m, of_sum ? 1.0f : v0, s0);
+              s1 = fmaf(r1.factor(j, of_sum) * m, of_sum ? 1.0f : v1, s1);
+            }
+          };
+          int acc[4];
+          if (NB == 1) {
+            const uint2 xb = *reinterpret_cast<const uint2*>(xu + 64 * pr);
+            qi_mma<D::kSigned>(acc, a, xb.x & keep0, xb.y & keep0, true);
+            qi_mma<D::kSigned>(acc, b, xb.x & keep1, xb.y & keep1, false);
+            add(acc, 2 * pr + (t >> 1), bu[2 * pr], tot0, tot1);
+          } else {
+            const uint2 xa = *reinterpret_cast<const uint2*>(xu + 64 * pr), xb = *reinterpret_cast<const uint2*>(xu + 64 * pr + 32);
+            int acc2[4];
+            qi_mma<D::kSigned>(acc, a, xa.x, xa.y, true);
+            qi_mma<D::kSigned>(acc2, b, xb.x, xb.y, true);
+            add(acc, 2 * pr, bu[2 * pr], tot0, tot1);
+            add(acc2, 2 * pr + 1, bu[2 * pr + 1], odd0, odd1);
+          }
+        }
+      }
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(&empty[s]);
+      if (++s == p.stages) { s = 0; phase ^= 1; }
+      if (++seg == p.nseg) {
+        if (NB == 2) {
+          tot0 += odd0;
+          tot1 += odd1;
+        }
+        tot0 += __shfl_xor_sync(0xffffffffu, tot0, 1);
+        tot1 += __shfl_xor_sync(0xffffffffu, tot1, 1);
+        if (NB == 1) {
+          tot0 += __shfl_xor_sync(0xffffffffu, tot0, 2);
+          tot1 += __shfl_xor_sync(0xffffffffu, tot1, 2);
+        }
+        if (t == 0 || (NB == 2 && t == 2)) {
+          float* dst = part + ((tl * p.warps + warp) * NB + (t >> 1)) * 16 + g;
+          dst[0] = tot0;
+          dst[8] = tot1;
+        }
+        tot0 = tot1 = odd0 = odd1 = 0.0f;
+        seg = 0;
+        ++tl;
+      }
+    }
+  }
+  if (failed) {                  // a copy that never arrived: its rows come out as NaN instead of numbers made of old data
+    s_failed = 1;
+    if (lane == 0 && p.status != nullptr) atomicExch(p.status, 5);
+  }
+  __syncthreads();
+  if (warp >= p.warps) return;
+  const int row0 = tile_lo * 16, rows = min(tile_hi * 16, p.N) - row0;
+#pragma unroll
+  for (int n = 0; n < NB; ++n) {
+    float inv = 1.0f;
+    if (p.norm_w != nullptr) {
+      float ss = 0.0f;
+      for (int k = 0; k < p.warps; ++k) ss += s_sq[n][k];
+      inv = 1.0f / sqrtf(ss / (float)p.K + p.eps);
+    }
+    for (int i = tid; i < rows; i += nthr) {
+      float a[4] = {};           // four short sums: one of them long would round more than the rest together
+      for (int k = 0; k < p.warps; k += 4) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (k + e < p.warps) a[e] += part[(((i >> 4) * p.warps + k + e) * NB + n) * 16 + (i & 15)];
+      }
+      const float v = (a[0] + a[1]) + (a[2] + a[3]);
+      const size_t o = (size_t)n * p.out_ld + row0 + i;
+      p.out[o] = s_failed ? __int_as_float(0x7FFFFFFF) : (p.residual ? p.residual[o] : 0.0f) + v * inv;
+    }
+  }
+}
+
+// Of the matrices that can be streamed: whole units of 256 inputs, a tile of rows at least.  Rows of more than 12288 leave a ring of few short segments
+// beside their inputs (2560 x 14336 in Q8_0: 15.2 us in the kernel above, 16.8 here; Q4_K, two tokens: 20.7 and 22.7).  A second token's inputs are
+// split in turn by every CTA, which small matrices do not earn back (2048 x 2048 in Q4_K: 5.3 us above, 6.0 here; 2560 x 2560: 8.0 and 6.8).
+template <typename D, int NB>
+static bool qi_launch(const QsParams& q, cudaStream_t st, int& rc) {
+  const int N = q.N, K = q.K;
+  if (K % 256 != 0 || K > 12288 || N < 16 || (NB == 2 && (long long)N * K < 6000000)) return false;
+  QiParams p{q.w, q.x, q.norm_w, q.residual, q.out, q.status, q.eps, N, K, 0, 0, 0, 0, q.x_ld, q.out_ld};
+  const int units = K / 256;
+  p.nseg = (units + kQiMaxWarps - 1) / kQiMaxWarps;
+  size_t smem = 0;
+  for (;; ++p.nseg) {
+    p.warps = (units + p.nseg - 1) / p.nseg;
+    p.pitch = p.warps * D::kUnit;
+    if ((p.pitch / 16) % 2 == 0) p.pitch += 16;
+    const size_t rest = NB * ((size_t)4 * (K + 64) + (size_t)(K / 32) * 8 + (size_t)kQiMaxTiles * p.warps * 16 * 4);
+    p.stages = (int)((220 * 1024 - (long long)rest) / (16 * p.pitch));
+    if (p.stages > kQiMaxStages) p.stages = kQiMaxStages;
+    smem = rest + (size_t)p.stages * 16 * p.pitch;
+    if (p.stages >= 2) break;
+    if (p.warps <= 2) return false;
+  }
+  const int tiles = (N + 15) / 16;
+  int grid = tiles < 148 ? tiles : 148;
+  if ((tiles + grid - 1) / grid > kQiMaxTiles) grid = (tiles + kQiMaxTiles - 1) / kQiMaxTiles;
+  static std::atomic<bool> configured[64];
+  int dev = 0;
+  rc = BONSAI_CUDA_LAUNCH_FAILED;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return true;
+  if (!configured[dev].load(std::memory_order_acquire)) {
+    if (cudaFuncSetAttribute(quant_stream_imma_kernel<D, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024) != cudaSuccess) return true;
+    configured[dev].store(true, std::memory_order_release);
+  }
+  if (launch_pdl(quant_stream_imma_kernel<D, NB>, dim3(grid), dim3((p.warps + 1) * 32), smem, st, p) == cudaSuccess) rc = BONSAI_CUDA_OK;
+  return true;
+}
+template <typename D, int NB>
+static bool qi_try(const QsParams& p, cudaStream_t st, int& rc) {
+  if constexpr (std::is_same_v<D, DecQ4_0>) return qi_launch<QiQ4_0, NB>(p, st, rc);
+  else if constexpr (std::is_same_v<D, DecQ8_0>) return qi_launch<QiQ8_0, NB>(p, st, rc);
+  else if constexpr (std::is_same_v<D, DecQ4K>) return qi_launch<QiQ4K, NB>(p, st, rc);
+  else return false;
+}
+
 template <typename D>
 __global__ void __launch_bounds__(256) quant_gemv_kernel(const uint8_t* __restrict__ w, const float* __restrict__ x,
                                                         const float* __restrict__ norm_w, float eps, float* __restrict__ out,
@@ -532,7 +891,10 @@ static int launch_quant_gemv(const void* w, const float* x, const float* norm_w,
   QsParams p = qs_params<D>(w, x, K, norm_w, eps, out, residual, N, N, K, status);
   int sgrid;
   size_t smem;
-  if (qs_plan<Q>(p, sgrid, smem, 1)) return qs_launch<Q, 1>(p, sgrid, smem, st);
+  if (qs_plan<Q>(p, sgrid, smem, 1)) {
+    int rc;
+    return qi_try<D, 1>(p, st, rc) ? rc : qs_launch<Q, 1>(p, sgrid, smem, st);
+  }
   int grid = (N + 7) / 8;
   if (grid > 148 * 8) grid = 148 * 8;
   quant_gemv_kernel<D><<<grid, 256, 0, st>>>((const uint8_t*)w, x, norm_w, eps, out, residual, N, K);
@@ -613,7 +975,9 @@ static int launch_quant_gemv_batched(const void* w, const float* x, int x_ld, co
         p.x = x + (size_t)b * x_ld;
         p.out = out + (size_t)b * out_ld;
         p.residual = residual ? residual + (size_t)b * out_ld : nullptr;
-        rc = b + 1 < B ? qs_launch<Q, 2>(p, sgrid, smem, st) : qs_launch<Q, 1>(p, sgrid, smem, st);
+        const bool two = b + 1 < B;
+        if (two ? qi_try<D, 2>(p, st, rc) : qi_try<D, 1>(p, st, rc)) continue;
+        rc = two ? qs_launch<Q, 2>(p, sgrid, smem, st) : qs_launch<Q, 1>(p, sgrid, smem, st);
       }
       return rc;
     }

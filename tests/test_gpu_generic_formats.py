@@ -222,6 +222,39 @@ def test_streamed_rows_of_every_format(name, tid, tol, n, k):
         assert ((y - (xn @ wd.T + res.double())).abs() <= 2.0 ** -23 * (k / 32 + 64) * terms).all(), (name, batch)
 
 
+@pytest.mark.parametrize("tid", [G.Q4_0, G.Q8_0, G.Q4_K])
+@pytest.mark.parametrize("n,k,batch", [(16, 256, 1), (77, 512, 1), (2000, 2560, 1), (28700, 256, 1), (300, 9728, 1), (24, 12288, 1), (24, 12544, 1),
+                                       (24000, 256, 2), (23437, 256, 2), (2347, 2560, 3), (490, 12288, 2)])
+def test_rows_of_exact_block_products(tid, n, k, batch):
+    """Tiles of sixteen rows that end inside the matrix, several tiles and segments per CTA, the widest rows and one beyond, matrices on both sides
+    of the least for two tokens; block inputs of very different size, zero blocks, inputs that are not finite."""
+    from oxibonsai_b200.core.blocks import dequantize, quantize
+    from oxibonsai_b200.ops import cuda_ops as K
+    dev = torch.device("cuda:0")
+    rng = np.random.default_rng(n + k + batch)
+    few = quantize(tid, rng.normal(size=(8, k)).astype(np.float32) * 0.05).reshape(8, -1)
+    pick = rng.integers(0, 8, n)
+    wd, qd = torch.from_numpy(dequantize(tid, few.reshape(-1)).reshape(8, k)[pick]).double(), torch.from_numpy(few[pick].copy()).to(dev)
+    x = rng.normal(size=(batch, k)).astype(np.float32) * np.exp2(rng.integers(-60, 3, (batch, k // 32)).repeat(32, 1)).astype(np.float32)
+    x[:, 32:64] = 0
+    x[:, 64:256:37] = 3e4
+    room = torch.zeros(batch, k + 8)
+    room[:, :k] = torch.from_numpy(x)
+    y = K.quant_gemv_batched(tid, qd, n, k, room.to(dev)[:, :k]).cpu().double()
+    xd = torch.from_numpy(x).double()
+    # inputs are held to 2^-28 of their block's largest, the sums run over at most 64 rounded steps
+    # of terms whose magnitudes add up to |x| |W| (three times that where minima are taken off separately)
+    held = xd.abs().view(batch, -1, 32).amax(2).repeat_interleave(32, 1) * 2.0 ** -28
+    terms = (xd.abs() * (64 * 2.0 ** -24) + held) @ wd.abs().T * (3.0 if tid == G.Q4_K else 1.0)
+    assert ((y - xd @ wd.T).abs() <= terms).all()
+    for bad in (float("nan"), float("inf")):
+        room[0, k - 1] = bad
+        y = K.quant_gemv_batched(tid, qd, n, k, room.to(dev)[:, :k])
+        assert not torch.isfinite(y[0]).any() and torch.isfinite(y[1:]).all()
+        if bad == float("inf") and tid != G.Q4_K:          # (minima come off separately: infinity minus infinity)
+            assert torch.equal(y[0].cpu().nan_to_num(7.0), (wd[:, k - 1].float() * bad).nan_to_num(7.0))
+
+
 @pytest.mark.parametrize("name,tid,tol", TYPES)
 @pytest.mark.parametrize("n,k", [(1, 256), (3, 512), (77, 1280)])
 def test_rows_decoded_from_whole_words_are_those_of_single_values(name, tid, tol, n, k):
