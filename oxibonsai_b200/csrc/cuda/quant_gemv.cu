@@ -84,7 +84,8 @@ struct DecF32 { static constexpr int kElems = 32, kBytes = 128;
 // What bounds it: instructions.  24576 x 4096 in Q4_0 takes 19.6 M warp instructions (some six per weight with addresses, shuffles and
 // the hand-over of stages), half of the issue slots; more rows side by side do not help.  24576 x 4096, one token: Q4_0 27.8 us, Q8_0
 // 25.9 (4.1 TB/s), Q4_K 27.9, Q6_K 40.8, F16 40.7 (4.9 TB/s).  Before (a warp per row, one byte load per weight) the matrices of a
-// quarter-depth 8B model in Q4_K took 113 us on average, now 20; a token of it 4370 us, now 850.
+// quarter-depth 8B model in Q4_K took 113 us on average, 20 here; a token of it 4370 us, 815 here (555 with the integer form further down, which
+// takes Q4_0, Q8_0 and Q4_K of whole 256-input units).
 constexpr int kQsMaxWarps = 16;
 constexpr int kQsMaxStages = 8;
 constexpr int kQsRing = 112 * 1024;

@@ -11,7 +11,8 @@ GEMV streams every matrix once for two activation rows (a matrix that cannot be 
 are the batch kernels of the native engine.  The engine has the slot interface the continuous-batching scheduler drives
 (``begin_sequence`` / ``prefill`` / ``finish_sequence`` / ``step_batch`` / ``move_slot`` / ``close_sequence``).  Prompts of at least ``prefill_min`` tokens run in chunks through the tensor cores: each weight
 matrix is decoded once per chunk into an f16 scratch matrix (csrc/cuda/quant_gemv.cu, bonsai_quant_to_f16) and multiplied
-by all the chunk's tokens with the dense tcgen05 GEMM, with the prompt-attention kernel of the native engine in between;
+by all the chunk's tokens with the dense tcgen05 GEMM, with the prompt-attention kernel of the native engine in between (a chunk of more than 64
+tokens is one native call, csrc/cuda/blocks_prompt.cu);
 shorter prompts go through the decode step token by token (all f32).  Attention, KV append, LM head and sampler are the
 kernels of the native engine.  The sub-2-bit formats (Q1_0_g128, TQ2_0_g128) should use
 ``oxibonsai_b200.runtime.InferenceEngine``, which is several times faster.
