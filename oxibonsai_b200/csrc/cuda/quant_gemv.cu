@@ -493,16 +493,19 @@ static int qs_launch(const QsParams& p, int grid, size_t smem, cudaStream_t st) 
 
 // ---- one or two tokens on the integer tensor cores ----------------------------------------------------------------------------------
 // Q4_0, Q8_0 and Q4_K rows: a block of 32 codes times 32 inputs is one K extent of mma.sync.m16n8k32, for sixteen rows at once.  The inputs of a
-// block are four int8 terms of seven bits, x = s (q1 + q2 / 2^7 + q3 / 2^14 + q4 / 2^21) with s a power of two: 28 bits of the block's largest value,
-// every step of the split exact.  The terms are four columns.  Of one token two neighbouring blocks share an accumulator, the inputs of the first in
-// columns 0-3 and those of the second in 4-7 (zeros elsewhere); a second token has columns 4-7 instead.  Products and their sums are exact integers;
-// scales, minima (times the sum of the block's inputs) and the sums over blocks are f32.
-// A CTA owns tiles of sixteen rows.  A producer warp copies them, a segment of K at a time, row by row into a ring whose pitch keeps the rows' words
-// apart; a consumer warp takes 256 inputs of every segment and keeps its rows' sums to the end of the tile; the warps' sums meet in warp order.
-// Bound by the codes' way from shared memory to operands and the blocks' scales, some two instructions per weight where the kernel above takes six; the
-// large matrices come near the memory's rate.  One token, us above -> here: Q4_K 6144 x 4096 10.9 -> 7.0, 24576 x 4096 30.7 -> 17.9 (8.8 at the copy
-// rate), 4096 x 12288 19.9 -> 12.2; Q4_0 24576 x 4096 30.4 -> 16.7; Q8_0 24576 x 4096 29.4 -> 23.2 (16.6).  Two tokens: Q4_K 24576 x 4096 37.1 -> 21.4,
-// Q8_0 38.3 -> 27.2.  Relative error against 64 bits there: Q4_K 2.4e-7 -> 1.4e-7, Q4_0 9.5e-8 -> 8.6e-8, Q8_0 8.5e-8 -> 7.4e-8.
+// block are eight int8 terms of seven bits, x = s (q1 + q2 / 2^7 + ... + q8 / 2^49) with s a power of two that brings the block's largest input to
+// [2^5, 2^6), every step of the split exact: an input of at least 2^-31 of the largest is held to its last bit (four terms, 28 bits of the largest,
+// lost what stood beside an outlier whose code is zero: 3e-5 of the result for outliers of 10^4).  A block with a smaller one, an infinity or a NaN
+// is multiplied in f32 instead.  The terms are the eight columns, so that a token has an accumulator per block.  Products and their sums are exact
+// integers; scales, minima (times the sum of the block's inputs) and the sums over blocks are f32.
+// A CTA owns tiles of sixteen rows and goes through them a segment of K at a time.  A producer warp copies a tile's piece row by row into a ring whose
+// pitch keeps the rows' words apart; a consumer warp has 256 inputs of the segment, which it alone splits, and adds to its sums of the tile; the warps'
+// sums meet in warp order at the end.  The warps and the order of additions follow from the matrix alone.
+// Bound by the codes' way from shared memory to operands and the blocks' scales, some two instructions per weight where the kernel above takes six.
+// One token, us above -> here: Q4_K 6144 x 4096 10.9 -> 7.5, 24576 x 4096 30.6 -> 18.8 (8.8 at the copy rate; 17.1 with four terms), 4096 x 12288 20.0 -> 14.3;
+// Q4_0 24576 x 4096 30.7 -> 17.4; Q8_0 24576 x 4096 30.5 -> 23.4 (16.6).  Two tokens: Q4_K 24576 x 4096 37.4 -> 27.1, Q8_0 38.7 -> 29.1.  Relative error
+// against 64 bits, with an input of twenty times the others in every third block: Q4_K 2.0e-7 -> 1.4e-7, Q4_0 1.1e-7 -> 8.0e-8, Q8_0 1.1e-7 -> 8.0e-8; with
+// inputs of 30 to 10^14 under zero codes in every block 0.4 to 4.1e-7 -> 0.3 to 2.3e-7.
 struct QiParams {
   const uint8_t* w;
   const float *x, *norm_w, *residual;
@@ -512,26 +515,24 @@ struct QiParams {
   int N, K, nseg, warps, stages, pitch;      // segments of K; consumer warps = 256-input units of a segment
   int x_ld, out_ld;
 };
-constexpr int kQiMaxWarps = 20, kQiMaxTiles = 12, kQiMaxStages = 4;
+constexpr int kQiMaxWarps = 20, kQiMaxTiles = 12, kQiMaxStages = 4, kQiTerms = 8;
+constexpr int kQiSmem = 226 * 1024;
+constexpr int kQiUnitBytes = kQiTerms * 256 + 8 * 8;      // of shared memory for a token's unit of inputs: terms and {scale, sum} of its blocks
 
+// d = kQiZero + a b as floats: the sums start at the bits of 1.5 * 2^23, so that an integer below 2^22 comes out in that float's last places
+constexpr float kQiZero = 12582912.0f;
 template <bool SIGNED>
-__device__ __forceinline__ void qi_mma(int* d, const uint32_t* a, uint32_t b0, uint32_t b1, bool fresh) {
-  const int z = 0;
-  if (fresh) {
-    if (SIGNED)
-      asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
-          : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "r"(z));
-    else
-      asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
-          : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "r"(z));
-  } else {
-    if (SIGNED)
-      asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-          : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-    else
-      asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-          : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-  }
+__device__ __forceinline__ void qi_mma(float* d, const uint32_t* a, uint2 b) {
+  int r[4];
+  const int z = __float_as_int(kQiZero);
+  if (SIGNED)
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b.x), "r"(b.y), "r"(z));
+  else
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b.x), "r"(b.y), "r"(z));
+#pragma unroll
+  for (int i = 0; i < 4; ++i) d[i] = __int_as_float(r[i]);
 }
 __device__ __forceinline__ uint32_t qi_word(const uint8_t* p) { return *reinterpret_cast<const uint32_t*>(p); }      // 4-byte aligned
 // word number i of bytes that lie two behind a 4-byte boundary
@@ -541,47 +542,44 @@ __device__ __forceinline__ uint32_t qi_word2(const uint8_t* p, int i) {
 }
 
 // A unit of a row: 256 weights, kUnit bytes at `p` (16-byte aligned).  codes: the lane's share (t of four) of block j as the first operand's two words.
-// factor: what block j is multiplied with, or (of_sum) what the sum of its inputs is multiplied with.
+// A Head has what the scales of a row's unit are made of; scale and (kSums) minimum of block j, the latter for the sum of its inputs.
 struct QiQ4_0 { static constexpr int kUnit = 144; static constexpr bool kSigned = true, kNibbles = true, kSums = false;
-  const uint8_t* p;
-  __device__ void load(const uint8_t* at) { p = at; }
-  __device__ void codes(int j, int t, uint32_t& lo, uint32_t& hi) const {
+  struct Head { const uint8_t* p; };
+  static __device__ Head head(const uint8_t* p) { return Head{p}; }
+  static __device__ void codes(const uint8_t* p, int j, int t, uint32_t& lo, uint32_t& hi) {
     const uint8_t* b = p + 18 * j + 2;                        // two bytes off a boundary for even j
     const uint32_t w = (j & 1) ? qi_word(b + 4 * t) : qi_word2(b, t);
     lo = ((w << 4) & 0xF0F0F0F0u) ^ 0x80808080u; hi = (w & 0xF0F0F0F0u) ^ 0x80808080u; }      // 16 (q - 8)
-  __device__ float factor(int j, bool) const { return qs_f16(p + 18 * j) * 0.0625f; } };
+  static __device__ float scale(const Head& h, int j) { return qs_f16(h.p + 18 * j) * 0.0625f; }
+  static __device__ float minimum(const Head&, int) { return 0.0f; } };
 struct QiQ8_0 { static constexpr int kUnit = 272; static constexpr bool kSigned = true, kNibbles = false, kSums = false;
-  const uint8_t* p;
-  __device__ void load(const uint8_t* at) { p = at; }
-  __device__ void codes(int j, int t, uint32_t& lo, uint32_t& hi) const {
+  struct Head { const uint8_t* p; };
+  static __device__ Head head(const uint8_t* p) { return Head{p}; }
+  static __device__ void codes(const uint8_t* p, int j, int t, uint32_t& lo, uint32_t& hi) {
     const uint8_t* b = p + 34 * j + 2;
     if (j & 1) { lo = qi_word(b + 4 * t); hi = qi_word(b + 16 + 4 * t); }
     else { lo = qi_word2(b, t); hi = qi_word2(b, t + 4); } }
-  __device__ float factor(int j, bool) const { return qs_f16(p + 34 * j); } };
+  static __device__ float scale(const Head& h, int j) { return qs_f16(h.p + 34 * j); }
+  static __device__ float minimum(const Head&, int) { return 0.0f; } };
 struct QiQ4K { static constexpr int kUnit = 144; static constexpr bool kSigned = false, kNibbles = true, kSums = true;
-  const uint8_t* p;
-  uint4 head;                // d and dmin, twelve bytes of scales
-  __device__ void load(const uint8_t* at) { p = at; head = *reinterpret_cast<const uint4*>(at); }
-  __device__ void codes(int j, int t, uint32_t& lo, uint32_t& hi) const {
+  struct Head { uint4 v; };  // d and dmin, twelve bytes of scales
+  static __device__ Head head(const uint8_t* p) { return Head{*reinterpret_cast<const uint4*>(p)}; }
+  static __device__ void codes(const uint8_t* p, int j, int t, uint32_t& lo, uint32_t& hi) {
     const uint32_t w = qi_word(p + 16 + 16 * j + 4 * t);
     lo = w & 0x0F0F0F0Fu; hi = (w >> 4) & 0x0F0F0F0Fu; }
-  __device__ float factor(int j, bool of_sum) const {
-    const __half2 dd = *reinterpret_cast<const __half2*>(&head.x);
-    const uint32_t low = of_sum ? head.z : head.y, high = of_sum ? head.w >> 16 : head.w;
-    const float q = qs_int(((low >> (4 * j)) & 15u) | (((high >> (2 * j)) & 3u) << 4));
-    return (of_sum ? -__high2float(dd) : __low2float(dd)) * q; } };
+  static __device__ float six(uint32_t low, uint32_t high, int j) { return qs_int(((low >> (4 * j)) & 15u) | (((high >> (2 * j)) & 3u) << 4)); }
+  static __device__ float scale(const Head& h, int j) { return __low2float(*reinterpret_cast<const __half2*>(&h.v.x)) * six(h.v.y, h.v.w, j); }
+  static __device__ float minimum(const Head& h, int j) { return -__high2float(*reinterpret_cast<const __half2*>(&h.v.x)) * six(h.v.z, h.v.w >> 16, j); } };
 
 template <typename D, int NB>
 __global__ void __launch_bounds__((kQiMaxWarps + 1) * 32, 1) quant_stream_imma_kernel(const __grid_constant__ QiParams p) {
-  extern __shared__ __align__(128) uint8_t qi_smem[];      // ring, [NB][4][K + 64] terms, [NB][K / 32] {unit, sum of inputs}, [tiles][warps][NB][16] sums
+  extern __shared__ __align__(128) uint8_t qi_smem[];      // ring, [warps][NB] units of inputs, [tiles][warps][NB][16] sums
   __shared__ uint64_t full[kQiMaxStages], empty[kQiMaxStages];
   __shared__ float s_sq[NB][kQiMaxWarps];
   __shared__ int s_failed;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nthr = p.warps * 32;
-  const int stage_bytes = 16 * p.pitch, plane = p.K + 64;
-  int8_t* xq = reinterpret_cast<int8_t*>(qi_smem + p.stages * stage_bytes);
-  float2* blocks = reinterpret_cast<float2*>(xq + NB * 4 * plane);
-  float* part = reinterpret_cast<float*>(blocks + NB * (p.K >> 5));
+  const int stage_bytes = 16 * p.pitch;
+  float* part = reinterpret_cast<float*>(qi_smem + p.stages * stage_bytes + p.warps * NB * kQiUnitBytes);
   const unsigned ntiles = (unsigned)(p.N + 15) >> 4, per = ntiles / gridDim.x, over = ntiles - per * gridDim.x;
   const int tile_lo = (int)(per * blockIdx.x + over * blockIdx.x / gridDim.x), tile_hi = (int)(per * (blockIdx.x + 1) + over * (blockIdx.x + 1) / gridDim.x);
   const int units = p.K >> 8, steps = (tile_hi - tile_lo) * p.nseg;
@@ -602,175 +600,185 @@ __global__ void __launch_bounds__((kQiMaxWarps + 1) * 32, 1) quant_stream_imma_k
     uint32_t phase = 1;
     for (; issued < steps; ++issued) {
       if (!__all_sync(0xffffffffu, tc::mbar_wait_sleep<40>(&empty[s], phase))) { failed = true; break; }
-      const int u0 = seg * p.warps, nu = min(p.warps, units - u0);
+      const int first = seg * p.warps, nu = min(p.warps, units - first);
       const uint32_t bytes = (uint32_t)nu * D::kUnit;
       if (lane == 0) tc::mbar_arrive_expect_tx(&full[s], 16 * bytes);
       __syncwarp();
       if (lane < 16)
-        tc::bulk_g2s(qi_smem + s * stage_bytes + lane * p.pitch, p.w + (long long)min(tile * 16 + lane, p.N - 1) * row_bytes + (long long)u0 * D::kUnit, bytes, &full[s]);
+        tc::bulk_g2s(qi_smem + s * stage_bytes + lane * p.pitch, p.w + (long long)min(tile * 16 + lane, p.N - 1) * row_bytes + (long long)first * D::kUnit, bytes, &full[s]);
       if (++s == p.stages) { s = 0; phase ^= 1; }
-      if (++seg == p.nseg) { seg = 0; ++tile; }
+      if (++tile == tile_hi) { tile = tile_lo; ++seg; }
     }
     if (lane == 0) tc::mbar_drain(full, issued, p.stages);
     __syncwarp();
   } else if (warp < p.warps) {
+    // A lane has terms 2t + 1 and 2t + 2 of rows g and g + 8; of a pair of blocks it comes to add up block t / 2 of row g + 8 (t & 1).
     const int g = lane >> 2, t = lane & 3;
+    const bool second = t >> 1, lower = t & 1;
+    const float u0 = __uint_as_float((127u - 14u * t) << 23), u1 = u0 * (1.0f / 128.0f), zero = -kQiZero * (u0 + u1);
+    // the warp's inputs: block j of term k at 32 (j ^ k) of its 256 bytes, so that the eight terms' words meet no bank twice
+    int8_t* const xq = reinterpret_cast<int8_t*>(qi_smem + p.stages * stage_bytes + warp * NB * kQiUnitBytes);
+    float2* const blocks = reinterpret_cast<float2*>(xq + NB * kQiTerms * 256);
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    // ---- inputs: a thread has four neighbours, eight lanes a block of 32 -----------------------------------------------------------------------------------
-#pragma unroll 1
-    for (int n = 0; n < NB; ++n) {
-      const float4 *x4 = reinterpret_cast<const float4*>(p.x + (size_t)n * p.x_ld), *w4 = reinterpret_cast<const float4*>(p.norm_w);
-      const int nch = p.K >> 2;
-      float sq = 0.0f;
-#pragma unroll 2
-      for (int c = tid; c < nch; c += nthr) {          // whole warps: K is a multiple of 256, so nch of 64
-        float4 v = x4[c];
-        sq += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
-        if (w4 != nullptr) {
-          const float4 ww = __ldg(w4 + c);
-          v.x *= ww.x; v.y *= ww.y; v.z *= ww.z; v.w *= ww.w;
-        }
-        float top = fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)));
-        const float all = (v.x + v.y) + (v.z + v.w);
-        const bool finite = __all_sync(0xffffffffu, all - all == 0.0f);
+    float sq[NB] = {};
+    uint32_t apart[NB] = {};       // bit j: block j of the unit is multiplied in f32
+    float4 x[2 * NB], nw[2];       // the unit's inputs and norm weights, first and second half, requested a segment ahead
+    auto request = [&](int unit) {
 #pragma unroll
-        for (int o = 4; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
-        // the largest input comes to [2^5, 2^6)
-        float unit = __uint_as_float(__float_as_uint(fminf(fmaxf(top, 7.9e-31f), 3.0e38f)) & 0x7F800000u) * 0.03125f;
-        const float back = __uint_as_float(0x7F000000u - __float_as_uint(unit));
-        // (f + 1.5 * 2^23) holds rint(f) in its low byte; what is left, at most a half, is up to 64 of the next term's units
-        constexpr float kMagic = 12582912.0f;
-        float f[4] = {v.x * back, v.y * back, v.z * back, v.w * back};
-        const int blk = c >> 3, i = c & 7;
-        if (!finite) {           // a block with infinities keeps their signs, in units of infinity; one with a NaN is NaN
-          bool inf = false, nan = false;
-          const float e4[4] = {v.x, v.y, v.z, v.w};
+      for (int h = 0; h < 2; ++h) {
+        const int c = unit * 64 + h * 32 + lane;
+        nw[h] = p.norm_w != nullptr ? __ldg(reinterpret_cast<const float4*>(p.norm_w) + c) : make_float4(1.0f, 1.0f, 1.0f, 1.0f);
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            inf |= isinf(e4[e]);
-            nan |= isnan(e4[e]);
-          }
-          const uint32_t mine = 0xFFu << (lane & 24), infs = __ballot_sync(0xffffffffu, inf) & mine, nans = __ballot_sync(0xffffffffu, nan) & mine;
-          if ((infs | nans) != 0) {
-#pragma unroll
-            for (int e = 0; e < 4; ++e) f[e] = isinf(e4[e]) ? copysignf(1.0f, e4[e]) : 0.0f;
-            unit = nans != 0 ? __int_as_float(0x7FFFFFFF) : __int_as_float(0x7F800000);
-          }
-        }
-        uint32_t word[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          uint32_t q[4];
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const float m = f[e] + kMagic;
-            q[e] = __float_as_uint(m);
-            f[e] = (f[e] - (m - kMagic)) * 128.0f;
-          }
-          // nibbles: lane t's codes are those of inputs 8t .. 8t + 7, the even ones, then the odd ones;  bytes: inputs 4t .. 4t + 3, then 16 + 4t ..
-          word[k] = D::kNibbles ? __byte_perm(__byte_perm(q[0], q[2], 0x0040), __byte_perm(q[1], q[3], 0x0040), 0x5410)
-                                : __byte_perm(__byte_perm(q[0], q[1], 0x0040), __byte_perm(q[2], q[3], 0x0040), 0x5410);
-          int8_t* dst = xq + (n * 4 + k) * plane + blk * 32;
-          if (D::kNibbles) {
-            *reinterpret_cast<uint16_t*>(dst + (i >> 1) * 8 + (i & 1) * 2) = (uint16_t)word[k];
-            *reinterpret_cast<uint16_t*>(dst + (i >> 1) * 8 + 4 + (i & 1) * 2) = (uint16_t)(word[k] >> 16);
-          } else {
-            *reinterpret_cast<uint32_t*>(dst + (i & 3) * 8 + (i >> 2) * 4) = word[k];
-          }
-        }
-        float sum = 0.0f;
-        if (D::kSums) {      // of the terms, exactly: two of them in a word, at most 2048 each
-          int s12 = __dp4a((int)word[0], 0x01010101, 0) * 65536 + __dp4a((int)word[1], 0x01010101, 0);
-          int s34 = __dp4a((int)word[2], 0x01010101, 0) * 65536 + __dp4a((int)word[3], 0x01010101, 0);
-#pragma unroll
-          for (int o = 4; o > 0; o >>= 1) {
-            s12 += __shfl_xor_sync(0xffffffffu, s12, o);
-            s34 += __shfl_xor_sync(0xffffffffu, s34, o);
-          }
-          const int s2 = (int)(short)(s12 & 0xffff), s4 = (int)(short)(s34 & 0xffff);
-          sum = unit * fmaf((float)((s34 - s4) / 65536 * 128 + s4), 1.0f / 2097152.0f, (float)((s12 - s2) / 65536 * 128 + s2) * (1.0f / 128.0f));
-        }
-        if (i == 0) blocks[n * (p.K >> 5) + blk] = make_float2(unit, sum);
+        for (int n = 0; n < NB; ++n) x[2 * n + h] = reinterpret_cast<const float4*>(p.x + (size_t)n * p.x_ld)[c];
       }
-      sq = warp_sum(sq);
-      if (lane == 0) s_sq[n][warp] = sq;
-    }
-    asm volatile("bar.sync 1, %0;" ::"r"(nthr) : "memory");
-    // ---- rows -----------------------------------------------------------------------------------------------------------------------------------
-    const int term = g & 3, second = g >> 2;                 // the lane's column of the second operand
-    const uint32_t keep0 = second == 0 ? 0xffffffffu : 0u, keep1 = ~keep0;
-    const int8_t* xcol = xq + (NB == 2 ? 4 * second + term : term) * plane + (NB == 2 ? 0 : second * 32) + t * 8;
-    const bool of_sum = t & 1;                               // odd lanes hold the last two terms, and add what goes with the sum of the inputs
-    int s = 0, seg = 0, tl = 0;
+    };
+    request(warp);
+    int s = 0;
     uint32_t phase = 0;
-    float tot0 = 0.0f, tot1 = 0.0f, odd0 = 0.0f, odd1 = 0.0f;      // of two tokens the odd blocks apart
-    for (int n = 0; n < steps; ++n) {
-      if (!__all_sync(0xffffffffu, tc::mbar_wait(&full[s], phase))) { failed = true; break; }
+    for (int seg = 0; seg < p.nseg && !failed; ++seg) {
       const int unit = seg * p.warps + warp;
       if (unit < units) {
-        const uint8_t* at = qi_smem + s * stage_bytes + g * p.pitch + warp * D::kUnit;
-        D r0, r1;
-        r0.load(at);
-        r1.load(at + 8 * p.pitch);
-        const int8_t* xu = xcol + unit * 256;
-        const float2* bu = blocks + (NB == 2 ? (t >> 1) * (p.K >> 5) : t >> 1) + unit * 8;
+        // ---- inputs: a lane has four neighbours, eight lanes a block of 32 ---------------------------------------------------------------------------
 #pragma unroll
-        for (int pr = 0; pr < 4; ++pr) {
-          uint32_t a[4], b[4];
-          r0.codes(2 * pr, t, a[0], a[2]);
-          r1.codes(2 * pr, t, a[1], a[3]);
-          r0.codes(2 * pr + 1, t, b[0], b[2]);
-          r1.codes(2 * pr + 1, t, b[1], b[3]);
-          // what an accumulator holds for block j of this lane: even lanes terms one and two, odd lanes three and four
-          auto add = [&](const int* acc, int j, float2 bl, float& s0, float& s1) {
-            float v0 = fmaf((float)acc[1], 1.0f / 128.0f, (float)acc[0]), v1 = fmaf((float)acc[3], 1.0f / 128.0f, (float)acc[2]);
-            v0 = fmaf(__shfl_xor_sync(0xffffffffu, v0, 1), 1.0f / 16384.0f, v0);
-            v1 = fmaf(__shfl_xor_sync(0xffffffffu, v1, 1), 1.0f / 16384.0f, v1);
-            if (D::kSums || !of_sum) {
-              const float m = of_sum ? bl.y : bl.x;
-              s0 = fmaf(r0.factor(j, of_sum) * m, of_sum ? 1.0f : v0, s0);
-              s1 = fmaf(r1.factor(j, of_sum) * m, of_sum ? 1.0f : v1, s1);
+        for (int n = 0; n < NB; ++n) {
+          apart[n] = 0;
+#pragma unroll 1
+          for (int half = 0; half < 2; ++half) {
+            const int i = lane & 7, j = half * 4 + (lane >> 3);
+            float4 v = half ? x[2 * n + 1] : x[2 * n];
+            const float4 ww = half ? nw[1] : nw[0];
+            sq[n] += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
+            v.x *= ww.x; v.y *= ww.y; v.z *= ww.z; v.w *= ww.w;
+            float top = fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))), sum = (v.x + v.y) + (v.z + v.w);
+            bool odd = !(sum - sum == 0.0f);           // an infinity or a NaN, or close to it
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) {
+              top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+              if (D::kSums) sum += __shfl_xor_sync(0xffffffffu, sum, o);
             }
-          };
-          int acc[4];
-          if (NB == 1) {
-            const uint2 xb = *reinterpret_cast<const uint2*>(xu + 64 * pr);
-            qi_mma<D::kSigned>(acc, a, xb.x & keep0, xb.y & keep0, true);
-            qi_mma<D::kSigned>(acc, b, xb.x & keep1, xb.y & keep1, false);
-            add(acc, 2 * pr + (t >> 1), bu[2 * pr], tot0, tot1);
-          } else {
-            const uint2 xa = *reinterpret_cast<const uint2*>(xu + 64 * pr), xb = *reinterpret_cast<const uint2*>(xu + 64 * pr + 32);
-            int acc2[4];
-            qi_mma<D::kSigned>(acc, a, xa.x, xa.y, true);
-            qi_mma<D::kSigned>(acc2, b, xb.x, xb.y, true);
-            add(acc, 2 * pr, bu[2 * pr], tot0, tot1);
-            add(acc2, 2 * pr + 1, bu[2 * pr + 1], odd0, odd1);
+            // the largest input comes to [2^5, 2^6)
+            float scale = __uint_as_float(__float_as_uint(fminf(fmaxf(top, 7.9e-31f), 3.0e38f)) & 0x7F800000u) * 0.03125f;
+            const float back = __uint_as_float(0x7F000000u - __float_as_uint(scale));
+            float f[4] = {v.x, v.y, v.z, v.w};
+            if (D::kNibbles) {     // of eight neighbours the even ones to the even lane, the odd ones to the odd lane, as their codes lie in the words
+              const float a = __shfl_xor_sync(0xffffffffu, i & 1 ? f[0] : f[1], 1), b = __shfl_xor_sync(0xffffffffu, i & 1 ? f[2] : f[3], 1);
+              const float own0 = i & 1 ? f[1] : f[0], own1 = i & 1 ? f[3] : f[2];
+              f[0] = i & 1 ? a : own0; f[1] = i & 1 ? b : own1;
+              f[2] = i & 1 ? own0 : a; f[3] = i & 1 ? own1 : b;
+            }
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const bool some = f[e] != 0.0f;
+              f[e] *= back;
+              odd |= some && fabsf(f[e]) < 0x1p-26f;   // its last places lie below those of the eighth term
+            }
+            const uint32_t lanes = __ballot_sync(0xffffffffu, odd);
+            if (lanes != 0) {
+#pragma unroll
+              for (int b = 0; b < 4; ++b) apart[n] |= ((lanes >> (8 * b)) & 255u) != 0 ? 1u << (half * 4 + b) : 0u;
+              if ((apart[n] >> j) & 1) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) f[e] = 0.0f;
+                scale = 0.0f;
+              }
+            }
+            // (f + 1.5 * 2^23) holds rint(f) in its low byte, and with 2^-7 of it the next term; what is left, at most a half, is up to 64 of the next
+            // term's units.  A lane's codes of a block are those of inputs 8t .. 8t + 7, even before odd (nibbles), or 4t .. 4t + 3 and 16 + 4t .. (bytes).
+            int8_t* dst = xq + n * kQiTerms * 256 + (D::kNibbles ? (i >> 1) * 8 + (i & 1) * 4 : (i & 3) * 8 + (i >> 2) * 4);
+#pragma unroll
+            for (int k = 0; k < kQiTerms; ++k) {
+              constexpr float kUnits[kQiTerms] = {1.0f, 0x1p-7f, 0x1p-14f, 0x1p-21f, 0x1p-28f, 0x1p-35f, 0x1p-42f, 0x1p-49f};
+              const float z = kQiZero * kUnits[k];
+              uint32_t q[4];
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                const float m = f[e] + z;
+                q[e] = __float_as_uint(m);
+                f[e] -= m - z;
+              }
+              *reinterpret_cast<uint32_t*>(dst + k * 256 + 32 * (j ^ k)) = __byte_perm(__byte_perm(q[0], q[1], 0x0040), __byte_perm(q[2], q[3], 0x0040), 0x5410);
+            }
+            if (i == 0) blocks[n * 8 + j] = make_float2(scale, sum);
           }
         }
+        if (unit + p.warps < units) request(unit + p.warps);
+        __syncwarp();
       }
-      __syncwarp();
-      if (lane == 0) tc::mbar_arrive(&empty[s]);
-      if (++s == p.stages) { s = 0; phase ^= 1; }
-      if (++seg == p.nseg) {
-        if (NB == 2) {
-          tot0 += odd0;
-          tot1 += odd1;
+      // ---- rows -----------------------------------------------------------------------------------------------------------------------------------
+      for (int tl = 0; tl < tile_hi - tile_lo; ++tl) {
+        if (!__all_sync(0xffffffffu, tc::mbar_wait(&full[s], phase))) { failed = true; break; }
+        if (unit < units) {
+          const uint8_t *r0 = qi_smem + s * stage_bytes + g * p.pitch + warp * D::kUnit, *r1 = r0 + 8 * p.pitch;
+          const auto head = D::head(lower ? r1 : r0);
+          float tot[NB] = {};
+#pragma unroll
+          for (int pr = 0; pr < 4; ++pr) {
+            uint32_t a[4], b[4];
+            D::codes(r0, 2 * pr, t, a[0], a[2]);
+            D::codes(r1, 2 * pr, t, a[1], a[3]);
+            D::codes(r0, 2 * pr + 1, t, b[0], b[2]);
+            D::codes(r1, 2 * pr + 1, t, b[1], b[3]);
+            const int j = 2 * pr + second;
+            const float scale = D::scale(head, j), minimum = D::minimum(head, j);
+#pragma unroll
+            for (int n = 0; n < NB; ++n) {
+              const int8_t* xu = xq + (n * kQiTerms + g) * 256 + t * 8;
+              const float2 bl = blocks[n * 8 + j];
+              float da[4], db[4];
+              qi_mma<D::kSigned>(da, a, *reinterpret_cast<const uint2*>(xu + 32 * ((2 * pr) ^ g)));
+              qi_mma<D::kSigned>(db, b, *reinterpret_cast<const uint2*>(xu + 32 * ((2 * pr + 1) ^ g)));
+              // two terms of a sum: the inner step is exact (integers below 2^19 in units of u0)
+              const float a0 = fmaf(da[1], u1, fmaf(da[0], u0, zero)), a1 = fmaf(da[3], u1, fmaf(da[2], u0, zero));
+              const float b0 = fmaf(db[1], u1, fmaf(db[0], u0, zero)), b1 = fmaf(db[3], u1, fmaf(db[2], u0, zero));
+              const float v0 = (second ? b0 : a0) + __shfl_xor_sync(0xffffffffu, second ? a0 : b0, 2);
+              const float v1 = (second ? b1 : a1) + __shfl_xor_sync(0xffffffffu, second ? a1 : b1, 2);
+              const float v = (lower ? v1 : v0) + __shfl_xor_sync(0xffffffffu, lower ? v0 : v1, 1);
+              tot[n] = fmaf(scale * bl.x, v, tot[n]);
+              if (D::kSums) tot[n] = fmaf(minimum, bl.y, tot[n]);
+            }
+          }
+#pragma unroll
+          for (int n = 0; n < NB; ++n) {
+#pragma unroll 1
+            for (uint32_t left = apart[n]; left != 0; left &= left - 1) {
+              const int j = __ffs(left) - 1;
+              uint32_t w[2][2];
+              D::codes(r0, j, t, w[0][0], w[0][1]);
+              D::codes(r1, j, t, w[1][0], w[1][1]);
+              float v[2] = {0.0f, 0.0f};
+#pragma unroll 1
+              for (int e = 0; e < 8; ++e) {
+                const int k = unit * 256 + j * 32 + (D::kNibbles ? 8 * t + 2 * (e & 3) + (e >> 2) : 16 * (e >> 2) + 4 * t + (e & 3));
+                const float in = p.x[(size_t)n * p.x_ld + k] * (p.norm_w != nullptr ? __ldg(p.norm_w + k) : 1.0f);
+#pragma unroll
+                for (int r = 0; r < 2; ++r) {
+                  const uint32_t q = (e < 4 ? w[r][0] : w[r][1]) >> (8 * (e & 3));
+                  v[r] = fmaf(D::kSigned ? (float)(int8_t)q : (float)(q & 255u), in, v[r]);
+                }
+              }
+#pragma unroll
+              for (int r = 0; r < 2; ++r) {
+                v[r] += __shfl_xor_sync(0xffffffffu, v[r], 1);
+                v[r] += __shfl_xor_sync(0xffffffffu, v[r], 2);
+              }
+              if (!second) tot[n] += D::scale(head, j) * (lower ? v[1] : v[0]);
+            }
+            const float v = tot[n] + __shfl_xor_sync(0xffffffffu, tot[n], 2);
+            if (!second) {
+              float* sum = part + ((tl * p.warps + warp) * NB + n) * 16 + g + 8 * lower;
+              *sum = seg == 0 ? v : *sum + v;
+            }
+          }
         }
-        tot0 += __shfl_xor_sync(0xffffffffu, tot0, 1);
-        tot1 += __shfl_xor_sync(0xffffffffu, tot1, 1);
-        if (NB == 1) {
-          tot0 += __shfl_xor_sync(0xffffffffu, tot0, 2);
-          tot1 += __shfl_xor_sync(0xffffffffu, tot1, 2);
-        }
-        if (t == 0 || (NB == 2 && t == 2)) {
-          float* dst = part + ((tl * p.warps + warp) * NB + (t >> 1)) * 16 + g;
-          dst[0] = tot0;
-          dst[8] = tot1;
-        }
-        tot0 = tot1 = odd0 = odd1 = 0.0f;
-        seg = 0;
-        ++tl;
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive(&empty[s]);
+        if (++s == p.stages) { s = 0; phase ^= 1; }
       }
+    }
+#pragma unroll
+    for (int n = 0; n < NB; ++n) {
+      sq[n] = warp_sum(sq[n]);
+      if (lane == 0) s_sq[n][warp] = sq[n];
     }
   }
   if (failed) {                  // a copy that never arrived: its rows come out as NaN instead of numbers made of old data
@@ -802,37 +810,38 @@ __global__ void __launch_bounds__((kQiMaxWarps + 1) * 32, 1) quant_stream_imma_k
   }
 }
 
-// Of the matrices that can be streamed: whole units of 256 inputs, a tile of rows at least.  Rows of more than 12288 leave a ring of few short segments
-// beside their inputs (2560 x 14336 in Q8_0: 15.2 us in the kernel above, 16.8 here; Q4_K, two tokens: 20.7 and 22.7).  A second token's inputs are
-// split in turn by every CTA, which small matrices do not earn back (2048 x 2048 in Q4_K: 5.3 us above, 6.0 here; 2560 x 2560: 8.0 and 6.8).
+// Of the matrices that can be streamed: whole units of 256 inputs, a tile of rows at least.  Rows of more than 12288 are split by
+// every CTA for few tiles of its own: two tokens lose what one gains (2560 x 14336 in Q4_K: 16.4 us above and 15.5 here, two tokens 20.9 and 24.9), and so do
+// those of small matrices (2048 x 2048 in Q4_K: two tokens 5.4 us above, 6.7 here; 2560 x 2560: 8.0 and 7.6).
+// Warps and segments leave room for two tokens, whether there is a second or not.
 template <typename D, int NB>
 static bool qi_launch(const QsParams& q, cudaStream_t st, int& rc) {
   const int N = q.N, K = q.K;
   if (K % 256 != 0 || K > 12288 || N < 16 || (NB == 2 && (long long)N * K < 6000000)) return false;
   QiParams p{q.w, q.x, q.norm_w, q.residual, q.out, q.status, q.eps, N, K, 0, 0, 0, 0, q.x_ld, q.out_ld};
-  const int units = K / 256;
-  p.nseg = (units + kQiMaxWarps - 1) / kQiMaxWarps;
-  size_t smem = 0;
-  for (;; ++p.nseg) {
+  const int units = K / 256, tiles = (N + 15) / 16;
+  int grid = tiles < 148 ? tiles : 148;
+  if ((tiles + grid - 1) / grid > kQiMaxTiles) grid = (tiles + kQiMaxTiles - 1) / kQiMaxTiles;
+  const int per = (tiles + grid - 1) / grid;
+  int token, stage;
+  p.nseg = (units + kQiMaxWarps - 1) / kQiMaxWarps - 1;
+  do {                           // (with one warp it is far less)
+    ++p.nseg;
     p.warps = (units + p.nseg - 1) / p.nseg;
     p.pitch = p.warps * D::kUnit;
     if ((p.pitch / 16) % 2 == 0) p.pitch += 16;
-    const size_t rest = NB * ((size_t)4 * (K + 64) + (size_t)(K / 32) * 8 + (size_t)kQiMaxTiles * p.warps * 16 * 4);
-    p.stages = (int)((220 * 1024 - (long long)rest) / (16 * p.pitch));
-    if (p.stages > kQiMaxStages) p.stages = kQiMaxStages;
-    smem = rest + (size_t)p.stages * 16 * p.pitch;
-    if (p.stages >= 2) break;
-    if (p.warps <= 2) return false;
-  }
-  const int tiles = (N + 15) / 16;
-  int grid = tiles < 148 ? tiles : 148;
-  if ((tiles + grid - 1) / grid > kQiMaxTiles) grid = (tiles + kQiMaxTiles - 1) / kQiMaxTiles;
+    token = p.warps * (kQiUnitBytes + per * 16 * 4);
+    stage = 16 * p.pitch;
+  } while (2 * (token + stage) > kQiSmem);
+  p.stages = (kQiSmem - NB * token) / stage;
+  if (p.stages > kQiMaxStages) p.stages = kQiMaxStages;
+  const size_t smem = (size_t)NB * token + (size_t)p.stages * stage;
   static std::atomic<bool> configured[64];
   int dev = 0;
   rc = BONSAI_CUDA_LAUNCH_FAILED;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return true;
   if (!configured[dev].load(std::memory_order_acquire)) {
-    if (cudaFuncSetAttribute(quant_stream_imma_kernel<D, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024) != cudaSuccess) return true;
+    if (cudaFuncSetAttribute(quant_stream_imma_kernel<D, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, kQiSmem) != cudaSuccess) return true;
     configured[dev].store(true, std::memory_order_release);
   }
   if (launch_pdl(quant_stream_imma_kernel<D, NB>, dim3(grid), dim3((p.warps + 1) * 32), smem, st, p) == cudaSuccess) rc = BONSAI_CUDA_OK;

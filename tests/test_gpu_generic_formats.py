@@ -255,6 +255,31 @@ def test_rows_of_exact_block_products(tid, n, k, batch):
             assert torch.equal(y[0].cpu().nan_to_num(7.0), (wd[:, k - 1].float() * bad).nan_to_num(7.0))
 
 
+@pytest.mark.parametrize("tid", [G.Q4_0, G.Q8_0, G.Q4_K])
+@pytest.mark.parametrize("n,k,batch", [(48, 512, 1), (2000, 4096, 2), (300, 9728, 1), (24576, 256, 2)])
+@pytest.mark.parametrize("size", [2.0 ** 16, 2.0 ** 31, 2.0 ** 33, 1e20])
+def test_block_rows_keep_inputs_beside_an_outlier(tid, n, k, batch, size):
+    """An outlier whose codes are zero leaves its neighbours every bit they have: sizes that the inputs' terms span, the largest they do, and
+    two beyond, whose blocks are multiplied in f32."""
+    from oxibonsai_b200.core.blocks import dequantize, quantize
+    from oxibonsai_b200.ops import cuda_ops as K
+    rng = np.random.default_rng(n + k)
+    src = rng.normal(size=(8, k)).astype(np.float32) * 0.05
+    if tid == G.Q4_K:
+        src = np.abs(src)                # no minima: code zero is weight zero
+    src[:, 5::96] = 0
+    few = quantize(tid, src).reshape(8, -1)
+    pick = rng.integers(0, 8, n)
+    wd, qd = torch.from_numpy(dequantize(tid, few.reshape(-1)).reshape(8, k)[pick]).double(), torch.from_numpy(few[pick].copy()).cuda()
+    assert not wd[:, 5::96].any()
+    x = rng.normal(size=(batch, k)).astype(np.float32)
+    x[:, 5::96] = size
+    y = K.quant_gemv_batched(tid, qd, n, k, torch.from_numpy(x).cuda()).cpu().double()
+    xd = torch.from_numpy(x).double()
+    # at most 64 rounded steps of terms whose magnitudes add up to |x| |W|
+    assert ((y - xd @ wd.T).abs() <= 64 * 2.0 ** -24 * (xd.abs() @ wd.abs().T)).all()
+
+
 @pytest.mark.parametrize("name,tid,tol", TYPES)
 @pytest.mark.parametrize("n,k", [(1, 256), (3, 512), (77, 1280)])
 def test_rows_decoded_from_whole_words_are_those_of_single_values(name, tid, tol, n, k):
