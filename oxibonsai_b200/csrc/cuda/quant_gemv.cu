@@ -500,7 +500,7 @@ static int qs_launch(const QsParams& p, int grid, size_t smem, cudaStream_t st) 
 // integers; scales, minima (times the sum of the block's inputs) and the sums over blocks are f32.
 // A CTA owns tiles of sixteen rows and goes through them a segment of K at a time.  A producer warp copies a tile's piece row by row into a ring whose
 // pitch keeps the rows' words apart; a consumer warp has 256 inputs of the segment, which it alone splits, and adds to its sums of the tile; the warps'
-// sums meet in warp order at the end.  The warps and the order of additions follow from the matrix alone.
+// sums meet in warp order at the end.  The warps and the order of additions follow from the matrix alone, whatever tokens there are.
 // Bound by the codes' way from shared memory to operands and the blocks' scales, some two instructions per weight where the kernel above takes six.
 // One token, us above -> here: Q4_K 6144 x 4096 10.9 -> 7.5, 24576 x 4096 30.6 -> 18.8 (8.8 at the copy rate; 17.1 with four terms), 4096 x 12288 20.0 -> 14.3;
 // Q4_0 24576 x 4096 30.7 -> 17.4; Q8_0 24576 x 4096 30.5 -> 23.4 (16.6).  Two tokens: Q4_K 24576 x 4096 37.4 -> 27.1, Q8_0 38.7 -> 29.1.  Relative error
@@ -810,14 +810,15 @@ __global__ void __launch_bounds__((kQiMaxWarps + 1) * 32, 1) quant_stream_imma_k
   }
 }
 
-// Of the matrices that can be streamed: whole units of 256 inputs, a tile of rows at least.  Rows of more than 12288 are split by
-// every CTA for few tiles of its own: two tokens lose what one gains (2560 x 14336 in Q4_K: 16.4 us above and 15.5 here, two tokens 20.9 and 24.9), and so do
-// those of small matrices (2048 x 2048 in Q4_K: two tokens 5.4 us above, 6.7 here; 2560 x 2560: 8.0 and 7.6).
-// Warps and segments leave room for two tokens, whether there is a second or not.
+// Of the matrices that can be streamed: whole units of 256 inputs, a tile of rows at least, and what makes the split of the inputs by every CTA worth
+// its time whether there is a second token or not.  Rows of more than 12288 gain with one token and lose with two (2560 x 14336 in Q4_K: 16.4 us above
+// and 15.5 here, two tokens 20.9 and 24.9), small matrices with two (2048 x 2048 in Q4_K: 4.0 and 4.0, two tokens 5.4 and 6.7; 2560 x 2560: 6.0 and 5.0,
+// 8.0 and 7.6).  The rule looks at the matrix alone, and warps and segments leave room for two tokens: a token's sums are the same with and without a
+// second one.
 template <typename D, int NB>
 static bool qi_launch(const QsParams& q, cudaStream_t st, int& rc) {
   const int N = q.N, K = q.K;
-  if (K % 256 != 0 || K > 12288 || N < 16 || (NB == 2 && (long long)N * K < 6000000)) return false;
+  if (K % 256 != 0 || K > 12288 || N < 16 || (long long)N * K < 6000000) return false;
   QiParams p{q.w, q.x, q.norm_w, q.residual, q.out, q.status, q.eps, N, K, 0, 0, 0, 0, q.x_ld, q.out_ld};
   const int units = K / 256, tiles = (N + 15) / 16;
   int grid = tiles < 148 ? tiles : 148;

@@ -280,6 +280,24 @@ def test_block_rows_keep_inputs_beside_an_outlier(tid, n, k, batch, size):
     assert ((y - xd @ wd.T).abs() <= 64 * 2.0 ** -24 * (xd.abs() @ wd.abs().T)).all()
 
 
+@pytest.mark.parametrize("tid", [G.Q4_0, G.Q8_0, G.Q4_K])
+@pytest.mark.parametrize("n,k", [(16, 256), (1000, 2560), (2048, 2048), (2343, 2560), (2344, 2560), (620, 9728), (490, 12288), (480, 12544)])
+def test_a_row_of_a_batch_is_the_row_alone(tid, n, k):
+    """Sequences come and go beside one another without moving results: the same bits alone, as one of a pair and as the last of an odd batch, on both
+    sides of the sizes at which the streamed kernels change."""
+    from oxibonsai_b200.core.blocks import quantize
+    from oxibonsai_b200.ops import cuda_ops as K
+    rng = np.random.default_rng(n)
+    few = quantize(tid, rng.normal(size=(8, k)).astype(np.float32) * 0.05).reshape(8, -1)
+    w = torch.from_numpy(few.view(np.uint8).reshape(8, -1)[rng.integers(0, 8, n)].copy()).cuda()
+    x, norm = (torch.from_numpy(rng.normal(size=s).astype(np.float32)).cuda() for s in ((3, k), (k,)))
+    x[1, ::64] *= 1e12
+    both = K.quant_gemv_batched(tid, w, n, k, x, norm, 1e-6)
+    for b in range(3):
+        assert torch.equal(both[b], K.quant_gemv_batched(tid, w, n, k, x[b:b + 1], norm, 1e-6)[0]), b
+        assert torch.equal(both[b], K.quant_gemv(tid, w, n, k, x[b], norm, 1e-6)), b
+
+
 @pytest.mark.parametrize("name,tid,tol", TYPES)
 @pytest.mark.parametrize("n,k", [(1, 256), (3, 512), (77, 1280)])
 def test_rows_decoded_from_whole_words_are_those_of_single_values(name, tid, tol, n, k):
