@@ -73,7 +73,7 @@ static int chunk(const BlockPrompt& p, const BlockLayer* layers, float eps, int 
   };
   auto product = [&](const BlockMatrix& m, const void* x, int K, float* out, const float* residual, int out_ld) -> int {
     const long long row_bytes = quant_row_bytes((int)m.type, K), most = p.scratch_elems / K;
-    if (row_bytes < 0 || most < 256) return BONSAI_CUDA_BAD_ARG;
+    if (row_bytes < 0 || (m.rows > most && most < 256)) return BONSAI_CUDA_BAD_ARG;
     const int step = (int)(m.rows <= most ? m.rows : most / 256 * 256);
     for (int r0 = 0; r0 < m.rows; r0 += step) {
       const int rows = (int)(m.rows - r0 < step ? m.rows - r0 : step);
@@ -101,7 +101,7 @@ static int chunk(const BlockPrompt& p, const BlockLayer* layers, float eps, int 
       BlockMatrix u = w.m[BM_UP];
       if (u.rows == 0) u = {g.type, inter, g.data + inter * quant_row_bytes((int)g.type, hidden)};
       const long long gb = quant_row_bytes((int)g.type, hidden), ub = quant_row_bytes((int)u.type, hidden), most = p.scratch_elems / hidden / 2;      // pairs of rows
-      if (gb < 0 || ub < 0 || most < 128) return BONSAI_CUDA_BAD_ARG;
+      if (gb < 0 || ub < 0 || (inter > most && most < 128)) return BONSAI_CUDA_BAD_ARG;
       const int slabs = (int)((inter + most - 1) / most), per = ((inter + slabs - 1) / slabs + 127) / 128 * 128, step = slabs == 1 ? inter : (per <= most ? per : (int)(most / 128 * 128));
       for (int r0 = 0; r0 < inter; r0 += step) {
         const int rows = inter - r0 < step ? inter - r0 : step;

@@ -336,3 +336,29 @@ def test_native_prompt_chunk_leaves_the_bits_of_its_kernels_one_by_one(fmt, kv, 
         caches.append([t.clone() for t in (eng.kpool, eng.vpool, eng.kscale, eng.vscale) if t is not None])
     for other in caches[1:]:
         assert all(torch.equal(a, b) for a, b in zip(caches[0], other))
+
+
+def _token_by_token(path, prompt, **kw):
+    """Logits and cache of an engine that feeds the prompt through the decode step."""
+    from oxibonsai_b200.models.qwen3_generic import GenericQwen3Engine
+    eng = GenericQwen3Engine(path, prefill_min=10**9, **kw)
+    eng.generate(prompt, 1, stop_at_eos=False)
+    return eng
+
+
+@pytest.mark.parametrize("hidden,inter,heads", [(128, 256, 4), (128, 128, 1), (256, 128, 8)])
+def test_prompts_of_narrow_models(hidden, inter, heads, tmp_path):
+    """Matrices of fewer rows than a slab of the scratch matrix, which they fit as a whole."""
+    from oxibonsai_b200 import cli
+    from oxibonsai_b200.core import Qwen3Config, write_synthetic_gguf
+    from oxibonsai_b200.models.qwen3_generic import GenericQwen3Engine
+    cfg = Qwen3Config(hidden=hidden, inter=inter, layers=2, heads=heads, kv_heads=1, head_dim=128, vocab=512, context=256, name="narrow")
+    write_synthetic_gguf(str(tmp_path / "a.gguf"), cfg, tied=False, seed=3)
+    path = str(tmp_path / "b.gguf")
+    cli.requantize_gguf(str(tmp_path / "a.gguf"), path, "q8_0")
+    prompt = [int(t) for t in np.random.default_rng(1).integers(0, 500, 100)]
+    slow = _token_by_token(path, prompt, max_seq_len=128, kv_dtype="f32")
+    fast = GenericQwen3Engine(path, max_seq_len=128, kv_dtype="f32")
+    assert fast.prefill_supported() and len(fast.generate(prompt, 1, stop_at_eos=False)) == 1
+    la, lb = slow.logits[0], fast.logits[0]
+    assert (la - lb).abs().max().item() <= 0.03 * la.abs().max().item()          # f16 operands in the prompt path only
