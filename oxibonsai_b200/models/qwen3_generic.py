@@ -86,7 +86,7 @@ class GenericQwen3Engine:
         self.max_seq_len, self.max_batch = max_seq_len, max(1, int(max_batch))
         self.prefill_min, self.prefill_chunk = prefill_min, prefill_chunk
         self.prefill_min_tokens = prefill_min          # the name the scheduler reads
-        self._prompt = self._row = None
+        self._prompt = self._row = self._table = self._wscratch = None
         self.sampling = sampling or SamplingPreset.GREEDY.params()
         f, dev, B = self.gguf, self.device, self.max_batch
         self.kvt = {"f32": K.KV_F32, "f16": K.KV_F16, "q8": K.KV_Q8, "q4": K.KV_Q4}[kv_dtype]
@@ -214,26 +214,32 @@ class GenericQwen3Engine:
             c = self.config
             rows = max(c.heads * self.nsplit, K.attn_workspace_rows(c.heads, c.kv_heads))
             f32 = dict(dtype=torch.float32, device=self.device)
-            self._row = dict(layers=self._layer_words(), acc=torch.empty((rows, c.head_dim), **f32), ml=torch.empty((rows, 2), **f32),
+            self._row = dict(acc=torch.empty((rows, c.head_dim), **f32), ml=torch.empty((rows, 2), **f32),
                              counters=torch.zeros(c.kv_heads, dtype=torch.int32, device=self.device))
         c, r = self.config, self._row
         s = [self.embd, self.lm_head, self.out_norm, self.cos, self.sin, self.token[slot:], self.pos[slot:], self.bt[slot], self.h[slot], self.qkv[slot],
              self.q[slot], self.attn[slot], self.gu[slot], self.act[slot], self.logits[slot], r["acc"], r["ml"], r["counters"], self.status]
         words = [t.data_ptr() for t in s] + [r["acc"].shape[0], c.hidden, c.inter, c.layers, c.heads, c.kv_heads, c.head_dim, c.vocab, self.lm_head.shape[0], self.kvt,
                                              self.page, self.nsplit]
-        K.blocks_forward_row((C.c_uint64 * len(words))(*words), r["layers"], c.eps)
+        K.blocks_forward_row((C.c_uint64 * len(words))(*words), self._layer_words(), c.eps)
 
     def _layer_words(self):
-        """The layers as csrc/cuda/blocks_prompt.cu reads them."""
-        words = []
+        """The layers as csrc/cuda/blocks_prompt.cu reads them: laid out once, with the tensors that the words point to."""
+        if self._table is not None:
+            return self._table[0]
+        words, keep = [], [self.kpool, self.vpool, self.kscale, self.vscale]
         for l, w in enumerate(self.layers):
             for parts, single in ((w["qkv"], ("q", "k", "v")), ([w["o"]], ("o",)), (w["gate_up"], ("gate", "up")), ([w["down"]], ("down",))):
                 fused = [*parts, *[None] * (len(single) - 1)] if len(parts) == 1 else [w[k] for k in single]
                 for m in fused:
                     words += [0, 0, 0] if m is None else [m.type, m.n, m.data.data_ptr()]
-            words += [w[k].data_ptr() for k in ("attn_norm", "ffn_norm", "q_norm", "k_norm")]
+                    keep.append(None if m is None else m.data)
+            norms = [w[k] for k in ("attn_norm", "ffn_norm", "q_norm", "k_norm")]
+            words += [t.data_ptr() for t in norms]
+            keep += norms
             words += [self.kpool[l].data_ptr(), self.vpool[l].data_ptr(), *(0 if s is None else s[l].data_ptr() for s in (self.kscale, self.vscale))]
-        return (C.c_uint64 * len(words))(*words)
+        self._table = (C.c_uint64 * len(words))(*words), keep
+        return self._table[0]
 
     # kept for callers of the single-stream engine
     def _step_eager(self) -> None:
@@ -248,19 +254,28 @@ class GenericQwen3Engine:
         """Runs ``tokens`` (int32 on the device) of the sequence in ``slot`` through every layer as chunks of up to
         ``prefill_chunk`` tokens, filling the KV cache for positions pos0 .. pos0 + len - 1.  Nothing is sampled and no logits
         are left: the caller feeds the prompt's last token through ``_forward``."""
-        b = self._prompt_buffers(slot)
         done = 0
         while done < tokens.numel():
             T = min(self.prefill_chunk, tokens.numel() - done)
             p0 = pos0 + done
             if T <= 64:
-                self._short_chunk(tokens[done:done + T], p0, slot, b["scratch"])
+                self._short_chunk(tokens[done:done + T], p0, slot, self._scratch())
                 done += T
                 continue
+            b = self._prompt_buffers(slot, T)
             b["tokens"][:T].copy_(tokens[done:done + T], non_blocking=True)
             torch.arange(p0, p0 + T, dtype=torch.int32, device=self.device, out=b["positions"][:T])
-            K.blocks_prompt_chunk(b["prompt"], b["layers"], self.config.eps, T, p0)
+            K.blocks_prompt_chunk(b["prompt"], self._layer_words(), self.config.eps, T, p0)
             done += T
+
+    def _scratch(self) -> torch.Tensor:
+        """The scratch matrix of short chunks: the widest matrix of a layer, or that of the native chunks once there is one."""
+        if self._prompt is not None:
+            return self._prompt["scratch"]
+        if self._wscratch is None:
+            c = self.config
+            self._wscratch = torch.empty(max(c.hidden * c.inter, c.heads * c.head_dim * c.hidden), dtype=torch.float16, device=self.device)
+        return self._wscratch
 
     def _short_chunk(self, tokens: torch.Tensor, p0: int, slot: int, scratch: torch.Tensor) -> None:
         """Up to 64 tokens (the last of a prompt).  Their products are cut along K by the shape of every single matrix, so each matrix keeps a product of
@@ -297,20 +312,20 @@ class GenericQwen3Engine:
             K.swiglu(gate, up, out=act)
             mm(w["down"], K.norm_to_f16_paired(act, None, eps), h, residual=h)
 
-    def _prompt_buffers(self, slot: int) -> dict:
-        """Activations of one prompt chunk, the scratch matrix and the pointer tables of the native chunk (allocated by the first prompt)."""
-        c, dev = self.config, self.device
+    def _prompt_buffers(self, slot: int, T: int = 0) -> dict:
+        """Activations of a native chunk of ``T`` tokens (0: the longest there is), its scratch matrix, and the structure that points to them and to the
+        slot's pages.  Sized by the chunks that run: a longer one than before has its activations allocated anew."""
+        c, dev, T = self.config, self.device, T or self.prefill_chunk
         qd, kvd = c.heads * c.head_dim, c.kv_heads * c.head_dim
-        if self._prompt is None:
-            n = self.prefill_chunk
+        if self._prompt is None or self._prompt["tokens"].numel() < T:
             f32, f16, i32 = (dict(dtype=d, device=dev) for d in (torch.float32, torch.float16, torch.int32))
-            # the widest matrix; gate and up together where 104 MB hold them
-            scratch = max(c.hidden * c.inter, qd * c.hidden, min(2 * c.hidden * c.inter, 52 << 20))
-            b = dict(tokens=torch.zeros(n, **i32), positions=torch.zeros(n, **i32), h=torch.empty((n, c.hidden), **f32), qkv=torch.empty((n, qd + 2 * kvd), **f32),
-                     q=torch.empty((n, qd), **f32), xn=torch.empty((n, c.hidden), **f16), attn=torch.empty((n, qd), **f16), act=torch.empty((n, c.inter), **f16),
-                     scratch=torch.empty(scratch, **f16), ws=K.gemm_workspace(dev))
-            b["layers"] = self._layer_words()
-            self._prompt = b
+            scratch = None if self._prompt is None else self._prompt["scratch"]
+            self._prompt = self._wscratch = None           # given back first
+            if scratch is None:                            # the widest matrix; gate and up together where 104 MB hold them
+                scratch = torch.empty(max(c.hidden * c.inter, qd * c.hidden, min(2 * c.hidden * c.inter, 52 << 20)), **f16)
+            self._prompt = dict(tokens=torch.zeros(T, **i32), positions=torch.zeros(T, **i32), h=torch.empty((T, c.hidden), **f32),
+                                qkv=torch.empty((T, qd + 2 * kvd), **f32), q=torch.empty((T, qd), **f32), xn=torch.empty((T, c.hidden), **f16),
+                                attn=torch.empty((T, qd), **f16), act=torch.empty((T, c.inter), **f16), scratch=scratch, ws=K.gemm_workspace(dev))
         b = self._prompt
         words = [self.embd, self.cos, self.sin, b["tokens"], b["positions"], self.bt[slot], b["h"], b["qkv"], b["q"], b["xn"], b["attn"], b["act"], b["scratch"]]
         words = [t.data_ptr() for t in words] + [b["scratch"].numel(), b["ws"].data_ptr(), b["ws"].numel() * b["ws"].element_size(), self.status.data_ptr(), c.hidden,

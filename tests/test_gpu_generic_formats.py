@@ -362,3 +362,38 @@ def test_prompts_of_narrow_models(hidden, inter, heads, tmp_path):
     assert fast.prefill_supported() and len(fast.generate(prompt, 1, stop_at_eos=False)) == 1
     la, lb = slow.logits[0], fast.logits[0]
     assert (la - lb).abs().max().item() <= 0.03 * la.abs().max().item()          # f16 operands in the prompt path only
+
+
+def test_prompts_pay_for_the_chunks_that_run(tiny_gguf, tmp_path):
+    """Short prompts allocate no more than one matrix and what they free again; longer ones activations of their length, also when the chunks are
+    made longer behind the first."""
+    from oxibonsai_b200 import cli
+    from oxibonsai_b200.models.qwen3_generic import GenericQwen3Engine
+    from oxibonsai_b200.ops import cuda_ops as K
+    path = str(tmp_path / "tiny_q8_0.gguf")
+    cli.requantize_gguf(tiny_gguf, path, "q8_0")
+    prompt = [int(t) for t in np.random.default_rng(9).integers(0, 1000, 400)]
+    eng = GenericQwen3Engine(path, max_seq_len=448)
+    c = eng.config
+    K.gemm_workspace(eng.device)
+
+    def grown(n):
+        before = torch.cuda.memory_allocated()
+        eng.begin_sequence(prompt[:n], n + 1, 0)
+        eng.prefill_slot(prompt[:n], 0)
+        eng.finish_sequence(prompt[:n], 0)
+        logits = eng.logits[0].clone()
+        eng.close_sequence(0)
+        return torch.cuda.memory_allocated() - before, logits
+
+    grown(2)                                  # the last token's step has buffers of its own
+    matrix = 2 * max(c.hidden * c.inter, c.heads * c.head_dim * c.hidden)
+    token = 16 * c.hidden + 8 * (c.heads + c.kv_heads) * c.head_dim + 4 * c.heads * c.head_dim + 2 * c.inter + 1024
+    first, short = grown(41)
+    assert first <= matrix + (64 << 10)
+    assert grown(101)[0] <= matrix + 100 * token + (64 << 10)
+    eng.prefill_chunk = 100
+    want = grown(400)[1]
+    eng.prefill_chunk = 399
+    _, got = grown(400)
+    assert torch.nn.functional.cosine_similarity(want, got, dim=0).item() > 0.999 and torch.equal(grown(41)[1], short)
