@@ -701,7 +701,7 @@ int launch_decode_d(int dpl, int G, dim3 grid, size_t smem, cudaStream_t st, con
 }
 
 int attn_decode_quant(const float*, const int*, const int*, int, int, int, int, int, int, const void*, const void*, const float*, const float*, int, float*,
-                      float*, long long, int*, float*, int, float, cudaStream_t);
+                      float*, long long, int*, float*, int, int, float, cudaStream_t);
 bool attn_decode_quant_takes(const float*, int, int, int, const void*, const void*);
 int attn_decode_mma_f16(const float* q, const int* positions, const int* block_table, int max_pages, int batch, int nq, int nkv,
                         int page_size, const void* kpool, const void* vpool, int nsplit, float* ws_acc, float* ws_ml, int* counters,
@@ -759,11 +759,12 @@ int bonsai_attn_decode_on_tensor_cores(const float* q, int nq, int nkv, int hd, 
 // positions[b] + 1 + extra_len.  ws_acc needs batch*nq*nsplit*hd floats, ws_ml batch*nq*nsplit*2 (ws_rows rows of each: at least these, and
 // with 1776 * nq / nkv of them quantised rows on the tensor cores may have every CTA that the device holds),
 // counters batch*nkv ints that are zero between launches (the kernel resets them).  f32_rows: INT8 / INT4 rows are multiplied in f32 on the
-// CUDA cores whatever their shape.
+// CUDA cores whatever their shape.  older: the kernel directly ahead in the stream wrote neither positions nor block_table, so that they may be read
+// before it has ended.
 int bonsai_attn_decode_route(const float* q, const int* positions, const int* block_table, int max_pages, int batch, int nq, int nkv,
                              int hd, int kvt, int page_size, const void* kpool, const void* vpool, const float* kscale,
                              const float* vscale, int nsplit, float* ws_acc, float* ws_ml, long long ws_rows, int* counters, float* out,
-                             int extra_len, int f32_rows, cudaStream_t stream) {
+                             int extra_len, int f32_rows, int older, cudaStream_t stream) {
   using namespace bonsai;
   if (hd % 32 != 0 || hd < 64 || hd > 256 || nq % nkv != 0 || nsplit < 1 || batch <= 0 || counters == nullptr) return BONSAI_CUDA_BAD_ARG;
   int G = nq / nkv, dpl = hd / 32;
@@ -780,7 +781,7 @@ int bonsai_attn_decode_route(const float* q, const int* positions, const int* bl
   }
   if (bonsai_attn_decode_on_tensor_cores(q, nq, nkv, hd, kvt, page_size, kpool, vpool, f32_rows)) {
     const int rc = attn_decode_quant(q, positions, block_table, max_pages, batch, nq, nkv, kvt, page_size, kpool, vpool, kscale, vscale, nsplit, ws_acc,
-                                     ws_ml, ws_rows, counters, out, extra_len, sc, stream);
+                                     ws_ml, ws_rows, counters, out, extra_len, older, sc, stream);
     if (rc != BONSAI_CUDA_BAD_ARG) return rc;      // outputs or a workspace at odd addresses
   }
   if (hd == 128 && kvt != KV_F32 && (G == 1 || G == 2 || G == 4) && (page_size & (page_size - 1)) == 0) {
@@ -804,7 +805,7 @@ int bonsai_attn_decode(const float* q, const int* positions, const int* block_ta
                        const float* vscale, int nsplit, float* ws_acc, float* ws_ml, int* counters, float* out, int extra_len,
                        cudaStream_t stream) {
   return bonsai_attn_decode_route(q, positions, block_table, max_pages, batch, nq, nkv, hd, kvt, page_size, kpool, vpool, kscale, vscale, nsplit,
-                                  ws_acc, ws_ml, (long long)batch * nq * nsplit, counters, out, extra_len, 0, stream);
+                                  ws_acc, ws_ml, (long long)batch * nq * nsplit, counters, out, extra_len, 0, 0, stream);
 }
 
 }  // extern "C"

@@ -45,7 +45,7 @@ struct QaParams {
   float* ws_ml;              // [CTA][2][G][2]
   int* counters;             // [batch][nkv], zero between launches
   float* out;                // [batch][nq][128]
-  int batch, max_pages, nq, nkv, page_size, extra_len, ctas;
+  int batch, max_pages, nq, nkv, page_size, extra_len, ctas, older;
   float sm_scale;
 };
 
@@ -119,8 +119,9 @@ __global__ void __launch_bounds__(NW * 32, kQaSmWarps / NW) attn_decode_quant_ke
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5, row = lane >> 2, c = lane & 3;
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if (cta >= p.ctas) return;
-  // Positions are not written by the kernel ahead (it appends rows and queries): the line is laid out before it has ended.  A sequence without
-  // keys has one empty tile, which writes its zeros.
+  // Where positions and page lists are older than the kernel ahead (a model's step: it appends rows and queries), the line is laid out before that
+  // has ended.  A sequence without keys has one empty tile, which writes its zeros.
+  if (!p.older) asm volatile("griddepcontrol.wait;" ::: "memory");
   if (warp == 0) {
     int sum = 0, most = 0;
     for (int b0 = 0; b0 < p.batch; b0 += 32) {
@@ -581,10 +582,11 @@ int attn_decode_quant_splits(int pairs) {
 }
 
 // kvt 2 (INT8) or 3 (INT4); BAD_ARG for what the caller's other kernels take.  ws_rows: rows of 128 floats in ws_acc (of 2 in ws_ml); a CTA may leave
-// two partial sums of G rows, so fewer CTAs run where there is room for fewer.
+// two partial sums of G rows, so fewer CTAs run where there is room for fewer.  older: positions and block_table were not written by the kernel
+// directly ahead in the stream.
 int attn_decode_quant(const float* q, const int* positions, const int* block_table, int max_pages, int batch, int nq, int nkv, int kvt, int page_size,
                       const void* kpool, const void* vpool, const float* kscale, const float* vscale, int nsplit, float* ws_acc, float* ws_ml, long long ws_rows,
-                      int* counters, float* out, int extra_len, float sm_scale, cudaStream_t st) {
+                      int* counters, float* out, int extra_len, int older, float sm_scale, cudaStream_t st) {
   if (!attn_decode_quant_takes(q, nq, nkv, page_size, kpool, vpool)) return BONSAI_CUDA_BAD_ARG;
   if (((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(ws_acc)) & 15) != 0 || (reinterpret_cast<uintptr_t>(ws_ml) & 7) != 0) return BONSAI_CUDA_BAD_ARG;
   const int G = nq / nkv;
@@ -597,7 +599,7 @@ int attn_decode_quant(const float* q, const int* positions, const int* block_tab
     if (ctas > ws_rows / (2 * G)) ctas = ws_rows / (2 * G);
     QaParams p{q + (size_t)b0 * nq * 128, positions + b0, block_table + (size_t)b0 * max_pages, (const uint8_t*)kpool, (const uint8_t*)vpool, kscale, vscale,
                ws_acc, ws_ml, counters + (size_t)b0 * nkv, out + (size_t)b0 * nq * 128, n, max_pages, nq, nkv, page_size, extra_len,
-               ctas < 1 ? 1 : (int)ctas, sm_scale * 1.4426950408889634f};
+               ctas < 1 ? 1 : (int)ctas, older, sm_scale * 1.4426950408889634f};
     const dim3 grid(nkv, nsplit, n);
     int rc;
 #define BONSAI_QA_W(k, g) (warps == 2 ? qa_launch<k, g, 2>(p, grid, st) : (warps == 6 ? qa_launch<k, g, 6>(p, grid, st) : qa_launch<k, g, 12>(p, grid, st)))

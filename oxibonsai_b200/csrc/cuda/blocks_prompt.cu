@@ -16,7 +16,7 @@ int bonsai_attn_prefill_ws(const float*, int, int, const int*, int, int, int, in
                            void*, size_t, int*, cudaStream_t);
 int bonsai_quant_gemv_batched_status(int, const void*, const float*, int, const float*, float, float*, const float*, int, int, int, int, int*, cudaStream_t);
 int bonsai_attn_decode_route(const float*, const int*, const int*, int, int, int, int, int, int, int, const void*, const void*, const float*, const float*, int,
-                             float*, float*, long long, int*, float*, int, int, cudaStream_t);
+                             float*, float*, long long, int*, float*, int, int, int, cudaStream_t);
 int bonsai_swiglu_rows(const float*, int, float*, int, int, int, cudaStream_t);
 int bonsai_f16gemv(const void*, const float*, const float*, float, float*, int, int, cudaStream_t);
 int bonsai_bitgemm_prefill_ws(const void*, const void*, const void*, int, float*, const float*, void*, int*, int, int, int, int, int, int, const void*, void*,
@@ -128,7 +128,7 @@ static int forward_row(const BlockRow& p, const BlockLayer* layers, float eps, c
     RC(bonsai_qknorm_rope_kvstore(p.qkv, qkv_n, w.q_norm, w.k_norm, eps, p.rope_cos, p.rope_sin, p.position, p.block_table, 0, p.q, 1, nq, nkv, hd, kvt, page,
                                   w.kpool, w.vpool, w.kscale, w.vscale, st));
     RC(bonsai_attn_decode_route(p.q, p.position, p.block_table, 0, 1, nq, nkv, hd, kvt, page, w.kpool, w.vpool, w.kscale, w.vscale, (int)p.nsplit, p.ws_acc,
-                                p.ws_ml, p.ws_rows, p.counters, p.attn, 0, 0, st));
+                                p.ws_ml, p.ws_rows, p.counters, p.attn, 0, 0, 1, st));
     RC(product(w.m[BM_O], p.attn, qd, nullptr, p.h, p.h, hidden));
     for (int i = BM_GATE, c0 = 0; i <= BM_UP; c0 += (int)w.m[i++].rows) RC(product(w.m[i], p.h, hidden, w.ffn_norm, p.gu + c0, nullptr, 2 * inter));
     RC(bonsai_swiglu_rows(p.gu, 2 * inter, p.act, inter, inter, 1, st));

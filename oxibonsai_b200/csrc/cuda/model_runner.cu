@@ -25,7 +25,7 @@ int bonsai_qknorm_rope_kvstore(const float*, int, const float*, const float*, fl
                                const int*, int, float*, int, int, int, int, int, int, void*, void*, float*, float*, cudaStream_t);
 int bonsai_attn_decode_on_tensor_cores(const float*, int, int, int, int, int, const void*, const void*, int);
 int bonsai_attn_decode_route(const float*, const int*, const int*, int, int, int, int, int, int, int, const void*, const void*,
-                             const float*, const float*, int, float*, float*, long long, int*, float*, int, int, cudaStream_t);
+                             const float*, const float*, int, float*, float*, long long, int*, float*, int, int, int, cudaStream_t);
 int bonsai_bitgemv_h2(const void*, const void*, const float*, const float*, float, float*, const float*, int, int, int, cudaStream_t);
 int bonsai_bitgemv_warp(const void*, const void*, const float*, const float*, float, float*, const float*, int, int, int, cudaStream_t);
 int bonsai_bitgemv_hmma(const void*, const void*, const float*, const float*, float, float*, const float*, int, int, int, cudaStream_t);
@@ -154,7 +154,7 @@ static int qkv_attention_run(Runner& r, const uint64_t* lp, const uint64_t* sp, 
                          P<float>(r.gp[GP_ROPE_SIN]), positions, bt, mp, q, n, nq, nkv, hd, kvt, r.ic[IC_PAGE_SIZE], P<void>(pool.k),
                          P<void>(pool.v), P<float>(pool.ks), P<float>(pool.vs), quant, st));
   return bonsai_attn_decode_route(q, positions, bt, mp, n, nq, nkv, hd, kvt, r.ic[IC_PAGE_SIZE], P<void>(pool.k), P<void>(pool.v),
-                                  P<float>(pool.ks), P<float>(pool.vs), nsplit, ws_acc, ws_ml, ws_rows, counters, attn, 0, f32_rows, st);
+                                  P<float>(pool.ks), P<float>(pool.vs), nsplit, ws_acc, ws_ml, ws_rows, counters, attn, 0, f32_rows, 1, st);
 }
 
 // The same for slots 0 .. batch-1: one launch (pair) per run of consecutive slots that share a page format.
@@ -381,7 +381,7 @@ static int prefill_chunk(Runner& r, const uint64_t* sp, const uint64_t* pp, int 
       float* attn32 = P<float>(pp[PP_SM_ATTN]);
       RC(bonsai_attn_decode_route(q, positions, bt, 0, T, nq, nkv, hd, kvt, r.ic[IC_PAGE_SIZE], P<void>(pool.k),
                                   P<void>(pool.v), P<float>(pool.ks), P<float>(pool.vs), sm_splits, P<float>(pp[PP_SM_ACC]),
-                                  P<float>(pp[PP_SM_ML]), (long long)kSmallChunk * nq * kSmallSplits, P<int>(pp[PP_SM_CTR]), attn32, 0, f32_rows, st));
+                                  P<float>(pp[PP_SM_ML]), (long long)kSmallChunk * nq * kSmallSplits, P<int>(pp[PP_SM_CTR]), attn32, 0, f32_rows, 1, st));
       RC(hm ? bonsai_norm_to_f16_hmma(attn32, qd, nullptr, r.eps, T, qd, attn, qd, st)
             : bonsai_norm_to_f16_paired(attn32, qd, nullptr, r.eps, T, qd, attn, qd, 0, st));
     } else {

@@ -28,7 +28,7 @@ _SIG = {
     "bonsai_embed_f16": [_vp, _vp, _vp, _i, _i, _vp],
     "bonsai_qknorm_rope_kvstore": [_vp, _i, _vp, _vp, _f, _vp, _vp, _vp, _vp, _i, _vp, _i, _i, _i, _i, _i, _i, _vp, _vp, _vp, _vp, _vp],
     "bonsai_attn_decode": [_vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _vp, _vp, _vp, _vp, _i, _vp, _vp, _vp, _vp, _i, _vp],
-    "bonsai_attn_decode_route": [_vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _vp, _vp, _vp, _vp, _i, _vp, _vp, C.c_longlong, _vp, _vp, _i, _i, _vp],
+    "bonsai_attn_decode_route": [_vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _vp, _vp, _vp, _vp, _i, _vp, _vp, C.c_longlong, _vp, _vp, _i, _i, _i, _vp],
     "bonsai_attn_decode_force_cuda_cores": [_i],
     "bonsai_attn_decode_qkv_f16": [_vp, _i, _vp, _vp, _f, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _vp, _vp, _i, _vp, _vp, _vp, _vp, _vp],
     "bonsai_sample": [_vp, _i, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _i, _vp, _i, _vp],
@@ -421,7 +421,7 @@ def attn_decode(q, positions, block_table, nq, nkv, hd, kvt, page_size, kpool, v
         out = torch.empty((batch, nq, hd), dtype=torch.float32, device=q.device)
     check(lib().bonsai_attn_decode_route(q.data_ptr(), positions.data_ptr(), block_table.data_ptr(), block_table.shape[1], batch, nq, nkv, hd,
                                          kvt, page_size, kpool.data_ptr(), vpool.data_ptr(), ptr(kscale), ptr(vscale), nsplit, ws_acc.data_ptr(),
-                                         ws_ml.data_ptr(), rows, counters.data_ptr(), out.data_ptr(), extra_len, 0, stream()), "attn_decode")
+                                         ws_ml.data_ptr(), rows, counters.data_ptr(), out.data_ptr(), extra_len, 0, 0, stream()), "attn_decode")
     return out
 
 

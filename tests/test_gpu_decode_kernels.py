@@ -478,6 +478,31 @@ def test_quantised_decode_attention_cut_into_pieces(lens, nq, nkv, kvt):
     check(out, fewer)
 
 
+@pytest.mark.parametrize("kvt", [2, 3])
+def test_quantised_decode_attention_behind_the_kernel_that_writes_positions(kvt):
+    """The entry point waits for the kernel ahead before it reads positions and page lists, whoever wrote them."""
+    from oxibonsai_b200.ops import cuda_ops as K
+    dev, page, nkv, B = _dev(), 16, 2, 40
+    g = torch.Generator(device=dev).manual_seed(kvt)
+    shape = (B * 20, nkv, page)
+    pools = [torch.randint(0, 255, (*shape, 128 if kvt == 2 else 64), dtype=torch.uint8, device=dev, generator=g) for _ in range(2)]
+    scales = [torch.rand(shape, device=dev, generator=g) for _ in range(2)]
+    q, out = torch.randn((B, nkv, 128), device=dev, generator=g), torch.empty((B, nkv, 128), device=dev)
+    tables = [torch.randperm(B * 20, device=dev, generator=g).to(torch.int32).view(B, 20) for _ in range(2)]
+    lens = [torch.randint(1, 320, (B,), dtype=torch.int32, device=dev, generator=g) for _ in range(2)]
+    want = [K.attn_decode(q, p, t, nkv, nkv, 128, kvt, page, *pools, *scales) for p, t in zip(lens, tables)]
+    ws = [torch.empty((B * nkv * 8, n), device=dev) for n in (128, 2)]
+    counters, pos, table = torch.zeros(B * nkv, dtype=torch.int32, device=dev), lens[0].clone(), tables[0].clone()
+    zero = torch.zeros((), dtype=torch.int32, device=dev)
+    for i in range(20):
+        torch.add(tables[i % 2], zero, out=table)
+        torch.add(lens[i % 2], zero, out=pos)
+        assert K.lib().bonsai_attn_decode(q.data_ptr(), pos.data_ptr(), table.data_ptr(), 20, B, nkv, nkv, 128, kvt, page, pools[0].data_ptr(), pools[1].data_ptr(),
+                                          scales[0].data_ptr(), scales[1].data_ptr(), 8, ws[0].data_ptr(), ws[1].data_ptr(), counters.data_ptr(), out.data_ptr(),
+                                          0, K.stream()) == 0
+        assert torch.allclose(out, want[i % 2], rtol=1e-4, atol=1e-5), i
+
+
 @pytest.mark.parametrize("nq,nkv,B", [(4, 2, 1), (3, 3, 37)])
 @pytest.mark.parametrize("kvt", [0, 1, 2, 3])
 def test_row_kernels_of_head_size_128_leave_the_same_bits(nq, nkv, B, kvt):
