@@ -24,6 +24,7 @@
 // 1500, INT4 31 / 22, one of 20001 22.4 / 20.7, one of 300 9.2 / 6.2.
 #include <cuda_fp16.h>
 
+#include <algorithm>
 #include <atomic>
 
 #include "common.cuh"
@@ -41,11 +42,11 @@ struct QaParams {
   const uint8_t* v;
   const float* k_scale;
   const float* v_scale;
-  float* ws_acc;             // [CTA][2][G][128]: partial sums of a CTA's first and last pair
-  float* ws_ml;              // [CTA][2][G][2]
+  float* ws_acc;             // [CTA][2][G][128]: partial sums of a CTA's first and last pair; close: [CTA + pair][G][128]
+  float* ws_ml;              // [..][G][2]
   int* counters;             // [batch][nkv], zero between launches
   float* out;                // [batch][nq][128]
-  int batch, max_pages, nq, nkv, page_size, extra_len, ctas, older;
+  int batch, max_pages, nq, nkv, page_size, extra_len, ctas, older, alone, close;
   float sm_scale;
 };
 
@@ -148,7 +149,7 @@ __global__ void __launch_bounds__(NW * 32, kQaSmWarps / NW) attn_decode_quant_ke
   // pair has more than four tiles for each warp of a CTA and every pair has its CTA, each gets a whole one: merging parts takes as long as four tiles
   // (one sequence of 300 tokens 11.3 us cut, 6.6 whole).
   constexpr int kParts = 65 * NW;
-  const bool whole = s_first <= 4 * NW && p.batch * p.nkv <= p.ctas;
+  const bool whole = p.alone || (s_first <= 4 * NW && p.batch * p.nkv <= p.ctas);
   const int per = whole ? 1 << 30 : (max((total + p.ctas - 1) / p.ctas, max(kAhead + 1, (s_first + kParts - 3) / (kParts - 2))) + NW - 1) / NW * NW;
   const int begin = whole ? 0 : cta * per;
   int end = min(total, begin + per);
@@ -283,7 +284,9 @@ __global__ void __launch_bounds__(NW * 32, kQaSmWarps / NW) attn_decode_quant_ke
   for (;;) {
     const int cta0 = run.at / per, parts = (run.at + run.n - 1) / per - cta0 + 1;
     // a CTA's first pair has its first partial sum, any other pair that it does not finish is its last
-    auto slot = [&](int i) { return (2 * i + (run.at - kAhead > i * per ? 1 : 0)) * G; };
+    auto second = [&](int i) { return run.at - kAhead > i * per ? 1 : 0; };
+    // (close: along the line a part has a later CTA or a later pair than the one before it)
+    auto slot = [&](int i) { return (p.close ? i + run.b * p.nkv + run.h : 2 * i + second(i)) * G; };
     float2 o[16];            // dimensions 32 c + i and 32 c + 16 + i of head `row`
 #pragma unroll
     for (int i = 0; i < 16; ++i) o[i] = make_float2(0.0f, 0.0f);
@@ -519,7 +522,7 @@ __global__ void __launch_bounds__(NW * 32, kQaSmWarps / NW) attn_decode_quant_ke
       }
     }
     if (!merging) {
-      if (parts > 1 && t == 0) s_open[slot(cta) == 2 * cta * G ? 0 : 1] = run;
+      if (parts > 1 && t == 0) s_open[second(cta)] = run;
       if (next_run(run)) {
         load_queries(run);
         __syncthreads();         // the sums have been read
@@ -581,9 +584,12 @@ int attn_decode_quant_splits(int pairs) {
   return n < 1 ? 1 : n;
 }
 
-// kvt 2 (INT8) or 3 (INT4); BAD_ARG for what the caller's other kernels take.  ws_rows: rows of 128 floats in ws_acc (of 2 in ws_ml); a CTA may leave
-// two partial sums of G rows, so fewer CTAs run where there is room for fewer.  older: positions and block_table were not written by the kernel
-// directly ahead in the stream.
+// kvt 2 (INT8) or 3 (INT4); BAD_ARG for what the caller's other kernels take.  ws_rows: rows of 128 floats in ws_acc (of 2 in ws_ml).  A CTA may leave
+// two partial sums of G rows, but n CTAs and m pairs no more than n + m - 1 together: with less room than two for every CTA they stand close, and where
+// that leaves fewer CTAs than pairs (one split) each pair has its own, whatever the lengths are.  Half the CTAs, with two places each, took
+// 61 / 26 / 18 / 15 us for one sequence of 4000 tokens over INT8 rows and 1 / 4 / 8 / 16 splits where it now takes 33 / 21 / 16 / 15, and 29 / 15 us for
+// four of 1000 and 1 / 4 splits where it takes 12 / 14.
+// older: positions and block_table were not written by the kernel directly ahead in the stream.
 int attn_decode_quant(const float* q, const int* positions, const int* block_table, int max_pages, int batch, int nq, int nkv, int kvt, int page_size,
                       const void* kpool, const void* vpool, const float* kscale, const float* vscale, int nsplit, float* ws_acc, float* ws_ml, long long ws_rows,
                       int* counters, float* out, int extra_len, int older, float sm_scale, cudaStream_t st) {
@@ -593,13 +599,14 @@ int attn_decode_quant(const float* q, const int* positions, const int* block_tab
   constexpr int kMost = 1024;              // sequences of a launch: their lengths stand in shared memory
   for (int b0 = 0; b0 < batch; b0 += kMost) {
     const int n = batch - b0 < kMost ? batch - b0 : kMost;
-    long long ctas = (long long)nkv * nsplit * n;
+    const long long pairs = (long long)nkv * n, room = ws_rows / G;
     const int warps = qa_warps(nkv * n);
-    if (ctas > qa_ctas(warps)) ctas = qa_ctas(warps);
-    if (ctas > ws_rows / (2 * G)) ctas = ws_rows / (2 * G);
+    const long long most = std::min(pairs * nsplit, (long long)qa_ctas(warps));
+    const bool tight = 2 * most > room, alone = tight && std::max(room / 2, room - pairs + 1) < pairs && pairs <= most, close = tight && room - pairs + 1 > room / 2;
+    const long long ctas = !tight ? most : (alone ? pairs : std::min(most, close ? room - pairs + 1 : room / 2));
     QaParams p{q + (size_t)b0 * nq * 128, positions + b0, block_table + (size_t)b0 * max_pages, (const uint8_t*)kpool, (const uint8_t*)vpool, kscale, vscale,
                ws_acc, ws_ml, counters + (size_t)b0 * nkv, out + (size_t)b0 * nq * 128, n, max_pages, nq, nkv, page_size, extra_len,
-               ctas < 1 ? 1 : (int)ctas, older, sm_scale * 1.4426950408889634f};
+               ctas < 1 ? 1 : (int)ctas, older, alone, close, sm_scale * 1.4426950408889634f};
     const dim3 grid(nkv, nsplit, n);
     int rc;
 #define BONSAI_QA_W(k, g) (warps == 2 ? qa_launch<k, g, 2>(p, grid, st) : (warps == 6 ? qa_launch<k, g, 6>(p, grid, st) : qa_launch<k, g, 12>(p, grid, st)))

@@ -600,3 +600,44 @@ def test_decode_attention_over_no_tokens_is_zero(kvt, nsplit):
     out = torch.full((2, nq, 128), float("nan"), device=dev)
     K.attn_decode(q, pos, table, nq, nkv, 128, kvt, 64, *pools, *scales, nsplit=nsplit, out=out)
     assert not out[0].any() and torch.isfinite(out[1]).all() and out[1].any()
+
+
+@pytest.mark.parametrize("lens,nq,nkv,nsplit,least", [([8000], 32, 8, 1, -1), ([8000], 32, 8, 2, 14), ([8000], 32, 8, 4, 28), ([8000], 32, 8, 16, 112), ([300, 2000, 1, 5000], 32, 8, 1, -1),
+                                                      ([300, 2000, 0, 5000], 8, 4, 3, 34), ([40, 900] * 60, 8, 2, 1, -1), ([3000, 80, 700] * 150, 2, 2, 1, 1)])
+@pytest.mark.parametrize("kvt", [2, 3])
+def test_quantised_decode_attention_uses_the_documented_workspace(lens, nq, nkv, nsplit, least, kvt):
+    """batch * nq * nsplit rows give room for nearly a CTA per split, or for a pair each: partial sums side by side, at least so many (-1: none), and
+    nothing behind the workspace."""
+    import math
+    from oxibonsai_b200.ops import cuda_ops as K
+    dev, page, B, G = _dev(), 16, len(lens), nq // nkv
+    g = torch.Generator(device=dev).manual_seed(B + nsplit)
+    most = max(1, -(-max(lens) // page))
+    table = torch.stack([torch.randperm(most, device=dev, generator=g) for _ in range(B)]).to(torch.int32)      # the sequences share their pages
+    pools, scales, values = [], [], []
+    for _ in range(2):
+        x = torch.randn((most, nkv, page, 128), device=dev, generator=g)
+        sc = (x.abs().amax(-1) / (127 if kvt == 2 else 7)).contiguous()
+        c = (x / sc[..., None]).round()
+        pools.append((c.to(torch.int8) if kvt == 2 else ((c + 8).to(torch.uint8)[..., 0::2] | ((c + 8).to(torch.uint8)[..., 1::2] << 4))).contiguous())
+        scales.append(sc)
+        values.append(c.double() * sc.double()[..., None])
+    q, pos = torch.randn((B, nq, 128), device=dev, generator=g), torch.tensor([n - 1 for n in lens], dtype=torch.int32, device=dev)
+    rows = B * nq * nsplit
+    acc, ml = torch.full((rows + 4096, 128), 7.0, device=dev), torch.full((rows + 4096, 2), -1.0, device=dev)
+    counters, out = torch.zeros(B * nkv, dtype=torch.int32, device=dev), torch.empty_like(q)
+    for _ in range(2):
+        assert K.lib().bonsai_attn_decode(q.data_ptr(), pos.data_ptr(), table.data_ptr(), most, B, nq, nkv, 128, kvt, page, pools[0].data_ptr(), pools[1].data_ptr(),
+                                          scales[0].data_ptr(), scales[1].data_ptr(), nsplit, acc.data_ptr(), ml.data_ptr(), counters.data_ptr(), out.data_ptr(),
+                                          0, K.stream()) == 0
+        assert not counters.any() and (acc[rows:] == 7.0).all() and (ml[rows:] == -1.0).all()
+    left = int((ml[:rows:G, 1] > 0).sum())
+    assert left >= least and (least >= 0 or left == 0)
+    for b, n in list(enumerate(lens))[::max(1, B // 8)]:
+        if n == 0:
+            assert not out[b].any()
+            continue
+        k, v = (x[table[b].long()].transpose(0, 1).reshape(nkv, -1, 128)[:, :n].repeat_interleave(G, 0) for x in values)
+        p = (torch.einsum("hd,hnd->hn", q[b].double(), k) / math.sqrt(128)).softmax(-1)
+        # scores and weights of 22 bits, exponentials of 2^-22: some 2^-18 of the weighted values
+        assert ((out[b].double() - torch.einsum("hn,hnd->hd", p, v)).abs() <= 2.0 ** -18 * torch.einsum("hn,hnd->hd", p, v.abs())).all(), b
