@@ -397,3 +397,67 @@ def test_prompts_pay_for_the_chunks_that_run(tiny_gguf, tmp_path):
     eng.prefill_chunk = 399
     _, got = grown(400)
     assert torch.nn.functional.cosine_similarity(want, got, dim=0).item() > 0.999 and torch.equal(grown(41)[1], short)
+
+
+def _requantise_by_name(src, dst, choose):
+    """``src`` with every matrix in the block type that ``choose`` gives its name."""
+    from oxibonsai_b200.core import GgufFile, GgufWriter, dequantize, quantize
+    f, w = GgufFile.open(src), GgufWriter()
+    for k, v in f.metadata.items():
+        w.add(k, v)
+    for t in f.tensors:
+        raw = f.tensor_bytes(t.name)
+        if len(t.dims) == 2 and not t.name.endswith("norm.weight"):
+            tid = choose(t.name)
+            w.add_tensor(t.name, t.dims, tid, quantize(tid, dequantize(t.type, raw) if t.type != G.F32 else np.frombuffer(raw, dtype=np.float32)))
+        else:
+            w.add_tensor(t.name, t.dims, t.type, np.frombuffer(raw, dtype=np.uint8))
+    w.write(dst)
+    return dst
+
+
+MIXED = {"blk.0.attn_v": G.Q6_K, "blk.0.ffn_up": G.Q4_K, "blk.1.attn_q": G.Q4_0, "blk.1.attn_k": G.Q5_K, "blk.1.ffn_gate": G.F8_E4M3, "blk.1.ffn_down": G.BF16}
+
+
+@pytest.mark.parametrize("kv", ["f32", "f16", "q8"])
+@pytest.mark.parametrize("mixed", [False, True])
+def test_native_prompt_chunks_match_token_by_token(kv, mixed, tiny_gguf, tmp_path):
+    """Two native chunks and the last token's native step, over every page format whose codes do not hang on the last digits; matrices of one type side by
+    side, and layers in which Q / K / V or gate / up are of different types."""
+    from oxibonsai_b200.models.qwen3_generic import GenericQwen3Engine
+    path = _requantise_by_name(tiny_gguf, str(tmp_path / "a.gguf"), lambda name: MIXED.get(name.removesuffix(".weight"), G.Q8_0) if mixed else G.Q8_0)
+    prompt = [int(t) for t in np.random.default_rng(9).integers(0, 1000, 190)]
+    slow = _token_by_token(path, prompt, max_seq_len=256, kv_dtype=kv)
+    fast = GenericQwen3Engine(path, max_seq_len=256, kv_dtype=kv, prefill_chunk=100)
+    assert [len(w["qkv"]) for w in fast.layers] == ([2, 3] if mixed else [1, 1]) and [len(w["gate_up"]) for w in fast.layers] == ([2, 2] if mixed else [1, 1])
+    fast.generate(prompt, 1, stop_at_eos=False)
+    la, lb = slow.logits[0], fast.logits[0]
+    assert torch.nn.functional.cosine_similarity(la, lb, dim=0).item() > 0.999          # f16 operands in the prompt path only
+    assert (la - lb).abs().max().item() <= 0.03 * la.abs().max().item()
+
+
+def test_expired_waits_of_native_prompt_chunks_are_reported(tiny_gguf, tmp_path, monkeypatch):
+    """The status word that a native chunk is given is the one that the engine reads with the prompt's first token."""
+    from oxibonsai_b200.models.qwen3_generic import GenericQwen3Engine
+    from oxibonsai_b200.ops import cuda_ops as K
+    eng = GenericQwen3Engine(_requantise_by_name(tiny_gguf, str(tmp_path / "a.gguf"), lambda name: G.Q8_0), max_seq_len=256, max_batch=2)
+    prompt = [int(t) for t in np.random.default_rng(9).integers(0, 1000, 120)]
+
+    def first_token(slot):
+        eng.begin_sequence(prompt, 130, slot)
+        eng.prefill_slot(prompt, slot)
+        return eng.finish_sequence(prompt, slot)
+
+    good = [first_token(0), first_token(1)]
+    chunk = K.blocks_prompt_chunk
+
+    def stalled(prompt, layers, *args):
+        chunk(prompt, layers, *args)
+        assert eng.status.data_ptr() in list(prompt)
+        eng.status.fill_(1)              # what a product of the chunk does whose pipeline stalls
+
+    monkeypatch.setattr(K, "blocks_prompt_chunk", stalled)
+    with pytest.raises(K.CudaKernelError, match="stalled"):
+        first_token(1)
+    monkeypatch.setattr(K, "blocks_prompt_chunk", chunk)
+    assert [first_token(0), first_token(1)] == good
