@@ -31,7 +31,7 @@ long long quant_row_bytes(int type, int K);      // -1: not a block type
 
 // one matrix of a layer: block type, rows, bytes
 struct BlockMatrix { long long type, rows; const uint8_t* data; };
-enum { BM_Q, BM_K, BM_V, BM_O, BM_GATE, BM_UP, BM_DOWN, BM_COUNT };      // K and V (UP) with rows 0: their rows stand behind those of Q (GATE)
+enum { BM_Q, BM_K, BM_V, BM_O, BM_GATE, BM_UP, BM_DOWN, BM_COUNT };      // rows 0: in the matrix before, behind its own
 struct BlockLayer {
   BlockMatrix m[BM_COUNT];
   const float *attn_norm, *ffn_norm, *q_norm, *k_norm;

@@ -230,8 +230,10 @@ class GenericQwen3Engine:
         words, keep = [], [self.kpool, self.vpool, self.kscale, self.vscale]
         for l, w in enumerate(self.layers):
             for parts, single in ((w["qkv"], ("q", "k", "v")), ([w["o"]], ("o",)), (w["gate_up"], ("gate", "up")), ([w["down"]], ("down",))):
-                fused = [*parts, *[None] * (len(single) - 1)] if len(parts) == 1 else [w[k] for k in single]
-                for m in fused:
+                rest, left = iter(parts), 0             # a matrix of the decode step stands in the place of the first of those that it holds
+                for k in single:
+                    m = next(rest) if left == 0 else None
+                    left = (left or m.n) - w[k].n
                     words += [0, 0, 0] if m is None else [m.type, m.n, m.data.data_ptr()]
                     keep.append(None if m is None else m.data)
             norms = [w[k] for k in ("attn_norm", "ffn_norm", "q_norm", "k_norm")]

@@ -436,6 +436,27 @@ def test_native_prompt_chunks_match_token_by_token(kv, mixed, tiny_gguf, tmp_pat
     assert (la - lb).abs().max().item() <= 0.03 * la.abs().max().item()
 
 
+@pytest.mark.parametrize("kv", ["f16", "q8", "q4"])
+def test_the_last_token_of_a_prompt_runs_the_matrices_of_a_decode_step(kv, tmp_path):
+    """Query and key rows in one matrix beside values of another type (how K-quant checkpoints are made), of sizes at which the pair and the single
+    matrices have different kernels: the same bits as the decode step, in logits and cache."""
+    from oxibonsai_b200.core import Qwen3Config, write_synthetic_gguf
+    from oxibonsai_b200.models.qwen3_generic import GenericQwen3Engine
+    cfg = Qwen3Config(hidden=2048, inter=256, layers=2, heads=16, kv_heads=8, head_dim=128, vocab=512, context=128, name="mixed")
+    write_synthetic_gguf(str(tmp_path / "a.gguf"), cfg, tied=False, seed=3)
+    path = _requantise_by_name(str(tmp_path / "a.gguf"), str(tmp_path / "b.gguf"), lambda name: G.Q8_0 if "attn_v" in name else G.Q4_0)
+    caches = []
+    for native in (True, False):
+        eng = GenericQwen3Engine(path, max_seq_len=64, kv_dtype=kv)
+        eng._bind(0)
+        assert [m.n for m in eng.layers[0]["qkv"]] == [3072, 1024]
+        for i, t in enumerate((5, 300, 17)):
+            eng.token[0], eng.pos[0] = t, i
+            eng._forward_row(0) if native else eng._forward(0, 1, False)
+        caches.append([t.clone() for t in (eng.logits, eng.kpool, eng.vpool, eng.kscale, eng.vscale) if t is not None])
+    assert all(torch.equal(a, b) for a, b in zip(*caches))
+
+
 def test_expired_waits_of_native_prompt_chunks_are_reported(tiny_gguf, tmp_path, monkeypatch):
     """The status word that a native chunk is given is the one that the engine reads with the prompt's first token."""
     from oxibonsai_b200.models.qwen3_generic import GenericQwen3Engine
