@@ -322,7 +322,10 @@ class GenericQwen3Engine:
         if self._prompt is None or self._prompt["tokens"].numel() < T:
             f32, f16, i32 = (dict(dtype=d, device=dev) for d in (torch.float32, torch.float16, torch.int32))
             scratch = None if self._prompt is None else self._prompt["scratch"]
-            self._prompt = self._wscratch = None           # given back first
+            for t in (self._wscratch, *(self._prompt or {}).values()):
+                if isinstance(t, torch.Tensor):
+                    t.record_stream(torch.cuda.current_stream(dev))      # which may still use what another one allocated
+            self._prompt = self._wscratch = t = None       # given back first
             if scratch is None:                            # the widest matrix; gate and up together where 104 MB hold them
                 scratch = torch.empty(max(c.hidden * c.inter, qd * c.hidden, min(2 * c.hidden * c.inter, 52 << 20)), **f16)
             self._prompt = dict(tokens=torch.zeros(T, **i32), positions=torch.zeros(T, **i32), h=torch.empty((T, c.hidden), **f32),

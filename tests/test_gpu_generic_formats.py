@@ -482,3 +482,32 @@ def test_expired_waits_of_native_prompt_chunks_are_reported(tiny_gguf, tmp_path,
         first_token(1)
     monkeypatch.setattr(K, "blocks_prompt_chunk", chunk)
     assert [first_token(0), first_token(1)] == good
+
+
+@pytest.mark.parametrize("first", [40, 70])
+def test_prompt_buffers_outlive_the_stream_that_uses_them(first, tiny_gguf, tmp_path):
+    """Buffers that one stream allocated and another still uses when a longer prompt replaces them are not handed out meanwhile."""
+    from oxibonsai_b200.models.qwen3_generic import GenericQwen3Engine
+    eng = GenericQwen3Engine(_requantise_by_name(tiny_gguf, str(tmp_path / "a.gguf"), lambda name: G.Q8_0), max_seq_len=256)
+    eng._bind(0)
+    tokens = torch.arange(1, 201, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    a, b = torch.cuda.Stream(), torch.cuda.Stream()
+    with torch.cuda.stream(a):
+        eng.prefill(tokens[:first])
+        torch.cuda.synchronize()
+    old = [eng._wscratch] if first <= 64 else [eng._prompt[k] for k in ("tokens", "h", "q", "act")]
+    used = [(t.data_ptr(), t.data_ptr() + t.numel() * t.element_size()) for t in old]
+    sizes = [t.numel() * t.element_size() for t in old]
+    del old
+    with torch.cuda.stream(b):
+        torch.cuda._sleep(1 << 30)                 # half a second
+        eng.prefill(tokens[:first])
+        eng.prefill(tokens)
+        waiting = torch.cuda.Event()
+        waiting.record()
+    with torch.cuda.stream(a):
+        taken = [torch.empty(n, dtype=torch.uint8, device="cuda") for n in sizes for _ in range(16)]
+    assert not waiting.query()
+    assert not any(t.data_ptr() < hi and lo < t.data_ptr() + t.numel() for t in taken for lo, hi in used)
+    torch.cuda.synchronize()
