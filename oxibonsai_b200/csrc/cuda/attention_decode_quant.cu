@@ -34,6 +34,8 @@ namespace bonsai {
 constexpr int kQaStages = 3, kQaSmWarps = 12;
 constexpr int qa_ctas(int warps) { return 148 * kQaSmWarps / warps; }      // that the device holds, by warps of a CTA
 
+// mode: see attn_decode_quant (words of their own made the parameters larger, and the compiler spilled: 20001 tokens 472 -> 482 us a step)
+enum { kQaOlder = 1, kQaAlone = 2, kQaClose = 4 };
 struct QaParams {
   const float* q;            // [batch][nq][128]
   const int* positions;
@@ -46,7 +48,7 @@ struct QaParams {
   float* ws_ml;              // [..][G][2]
   int* counters;             // [batch][nkv], zero between launches
   float* out;                // [batch][nq][128]
-  int batch, max_pages, nq, nkv, page_size, extra_len, ctas, older, alone, close;
+  int batch, max_pages, nq, nkv, page_size, extra_len, ctas, mode;
   float sm_scale;
 };
 
@@ -105,7 +107,8 @@ __device__ __forceinline__ void qa_copy4(uint32_t dst, const void* src, bool rea
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(real ? 4 : 0) : "memory");
 }
 
-template <int KVT, int G, int NW>
+// TIGHT: a workspace with less room than two partial sums a CTA (the two cases cost the others up to 3 % in spilled registers)
+template <int KVT, int G, int NW, bool TIGHT>
 __global__ void __launch_bounds__(NW * 32, kQaSmWarps / NW) attn_decode_quant_kernel(QaParams p) {
   constexpr int hd = 128, RB = KVT == 2 ? 128 : 64, KW = KVT == 2 ? 2 : 1;
   constexpr int kTile = 32 * RB + 128, kChunks = RB / 16;       // a tile: 16 rows of keys, 16 of values, 32 scales
@@ -122,7 +125,7 @@ __global__ void __launch_bounds__(NW * 32, kQaSmWarps / NW) attn_decode_quant_ke
   if (cta >= p.ctas) return;
   // Where positions and page lists are older than the kernel ahead (a model's step: it appends rows and queries), the line is laid out before that
   // has ended.  A sequence without keys has one empty tile, which writes its zeros.
-  if (!p.older) asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (!(p.mode & kQaOlder)) asm volatile("griddepcontrol.wait;" ::: "memory");
   if (warp == 0) {
     int sum = 0, most = 0;
     for (int b0 = 0; b0 < p.batch; b0 += 32) {
@@ -149,7 +152,7 @@ __global__ void __launch_bounds__(NW * 32, kQaSmWarps / NW) attn_decode_quant_ke
   // pair has more than four tiles for each warp of a CTA and every pair has its CTA, each gets a whole one: merging parts takes as long as four tiles
   // (one sequence of 300 tokens 11.3 us cut, 6.6 whole).
   constexpr int kParts = 65 * NW;
-  const bool whole = p.alone || (s_first <= 4 * NW && p.batch * p.nkv <= p.ctas);
+  const bool whole = (TIGHT && (p.mode & kQaAlone)) || (s_first <= 4 * NW && p.batch * p.nkv <= p.ctas);
   const int per = whole ? 1 << 30 : (max((total + p.ctas - 1) / p.ctas, max(kAhead + 1, (s_first + kParts - 3) / (kParts - 2))) + NW - 1) / NW * NW;
   const int begin = whole ? 0 : cta * per;
   int end = min(total, begin + per);
@@ -284,9 +287,8 @@ __global__ void __launch_bounds__(NW * 32, kQaSmWarps / NW) attn_decode_quant_ke
   for (;;) {
     const int cta0 = run.at / per, parts = (run.at + run.n - 1) / per - cta0 + 1;
     // a CTA's first pair has its first partial sum, any other pair that it does not finish is its last
-    auto second = [&](int i) { return run.at - kAhead > i * per ? 1 : 0; };
     // (close: along the line a part has a later CTA or a later pair than the one before it)
-    auto slot = [&](int i) { return (p.close ? i + run.b * p.nkv + run.h : 2 * i + second(i)) * G; };
+    auto slot = [&](int i) { return (TIGHT && (p.mode & kQaClose) ? i + run.b * p.nkv + run.h : 2 * i + (run.at - kAhead > i * per ? 1 : 0)) * G; };
     float2 o[16];            // dimensions 32 c + i and 32 c + 16 + i of head `row`
 #pragma unroll
     for (int i = 0; i < 16; ++i) o[i] = make_float2(0.0f, 0.0f);
@@ -522,7 +524,7 @@ __global__ void __launch_bounds__(NW * 32, kQaSmWarps / NW) attn_decode_quant_ke
       }
     }
     if (!merging) {
-      if (parts > 1 && t == 0) s_open[second(cta)] = run;
+      if (parts > 1 && t == 0) s_open[run.at - kAhead > cta * per ? 1 : 0] = run;
       if (next_run(run)) {
         load_queries(run);
         __syncthreads();         // the sums have been read
@@ -553,17 +555,17 @@ __global__ void __launch_bounds__(NW * 32, kQaSmWarps / NW) attn_decode_quant_ke
   }
 }
 
-template <int KVT, int G, int NW>
+template <int KVT, int G, int NW, bool TIGHT = false>
 static int qa_launch(const QaParams& p, dim3 grid, cudaStream_t st) {
   static std::atomic<bool> configured[64];
   const size_t smem = (size_t)NW * kQaStages * (32 * (KVT == 2 ? 128 : 64) + 128) + (size_t)NW * G * 130 * sizeof(float) + (size_t)p.batch * 2 * sizeof(int);
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return BONSAI_CUDA_LAUNCH_FAILED;
   if (!configured[dev].load(std::memory_order_acquire)) {
-    if (cudaFuncSetAttribute(attn_decode_quant_kernel<KVT, G, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, NW == 12 ? 226 * 1024 : 113 * 1024) != cudaSuccess) return BONSAI_CUDA_LAUNCH_FAILED;
+    if (cudaFuncSetAttribute(attn_decode_quant_kernel<KVT, G, NW, TIGHT>, cudaFuncAttributeMaxDynamicSharedMemorySize, NW == 12 ? 226 * 1024 : 113 * 1024) != cudaSuccess) return BONSAI_CUDA_LAUNCH_FAILED;
     configured[dev].store(true, std::memory_order_release);
   }
-  return launch_pdl(attn_decode_quant_kernel<KVT, G, NW>, grid, dim3(NW * 32), smem, st, p) == cudaSuccess ? BONSAI_CUDA_OK : BONSAI_CUDA_LAUNCH_FAILED;
+  return launch_pdl(attn_decode_quant_kernel<KVT, G, NW, TIGHT>, grid, dim3(NW * 32), smem, st, p) == cudaSuccess ? BONSAI_CUDA_OK : BONSAI_CUDA_LAUNCH_FAILED;
 }
 
 // Head size 128, INT8 or INT4 rows: the group sizes, pages and alignments of this kernel.
@@ -585,10 +587,10 @@ int attn_decode_quant_splits(int pairs) {
 }
 
 // kvt 2 (INT8) or 3 (INT4); BAD_ARG for what the caller's other kernels take.  ws_rows: rows of 128 floats in ws_acc (of 2 in ws_ml).  A CTA may leave
-// two partial sums of G rows, but n CTAs and m pairs no more than n + m - 1 together: with less room than two for every CTA they stand close, and where
-// that leaves fewer CTAs than pairs (one split) each pair has its own, whatever the lengths are.  Half the CTAs, with two places each, took
-// 61 / 26 / 18 / 15 us for one sequence of 4000 tokens over INT8 rows and 1 / 4 / 8 / 16 splits where it now takes 33 / 21 / 16 / 15, and 29 / 15 us for
-// four of 1000 and 1 / 4 splits where it takes 12 / 14.
+// two partial sums of G rows, but n CTAs and m pairs no more than n + m - 1 together: where two places each would leave a third of the CTAs idle they are
+// CTAs of twelve warps whose sums stand close, and where these are fewer than the pairs (one split) each pair has its own, whatever the lengths are.
+// Fewer CTAs, with two places each, took 61 / 26 / 18 / 15 us for one sequence of 4000 tokens over INT8 rows and 1 / 4 / 8 / 16 splits where it now takes
+// 33 / 21 / 16 / 15, 29 / 15 us for four of 1000 and 1 / 4 splits where it takes 12 / 14, 34 for sixteen of 1000 and one split where it takes 14.
 // older: positions and block_table were not written by the kernel directly ahead in the stream.
 int attn_decode_quant(const float* q, const int* positions, const int* block_table, int max_pages, int batch, int nq, int nkv, int kvt, int page_size,
                       const void* kpool, const void* vpool, const float* kscale, const float* vscale, int nsplit, float* ws_acc, float* ws_ml, long long ws_rows,
@@ -600,16 +602,24 @@ int attn_decode_quant(const float* q, const int* positions, const int* block_tab
   for (int b0 = 0; b0 < batch; b0 += kMost) {
     const int n = batch - b0 < kMost ? batch - b0 : kMost;
     const long long pairs = (long long)nkv * n, room = ws_rows / G;
-    const int warps = qa_warps(nkv * n);
-    const long long most = std::min(pairs * nsplit, (long long)qa_ctas(warps));
-    const bool tight = 2 * most > room, alone = tight && std::max(room / 2, room - pairs + 1) < pairs && pairs <= most, close = tight && room - pairs + 1 > room / 2;
-    const long long ctas = !tight ? most : (alone ? pairs : std::min(most, close ? room - pairs + 1 : room / 2));
+    int warps = qa_warps(nkv * n);
+    long long most = std::min(pairs * nsplit, (long long)qa_ctas(warps)), ctas = std::min(most, room / 2);
+    bool alone = false, close = false;
+    if (3 * ctas < 2 * most) {
+      warps = 12;
+      most = std::min(pairs * nsplit, (long long)qa_ctas(warps));
+      ctas = std::min(most, std::max(room / 2, room - pairs + 1));
+      alone = ctas < pairs && pairs <= most;
+      close = !alone && ctas > room / 2;
+      if (alone) ctas = pairs;
+    }
     QaParams p{q + (size_t)b0 * nq * 128, positions + b0, block_table + (size_t)b0 * max_pages, (const uint8_t*)kpool, (const uint8_t*)vpool, kscale, vscale,
                ws_acc, ws_ml, counters + (size_t)b0 * nkv, out + (size_t)b0 * nq * 128, n, max_pages, nq, nkv, page_size, extra_len,
-               ctas < 1 ? 1 : (int)ctas, older, alone, close, sm_scale * 1.4426950408889634f};
+               ctas < 1 ? 1 : (int)ctas, (older ? kQaOlder : 0) | (alone ? kQaAlone : 0) | (close ? kQaClose : 0), sm_scale * 1.4426950408889634f};
     const dim3 grid(nkv, nsplit, n);
     int rc;
-#define BONSAI_QA_W(k, g) (warps == 2 ? qa_launch<k, g, 2>(p, grid, st) : (warps == 6 ? qa_launch<k, g, 6>(p, grid, st) : qa_launch<k, g, 12>(p, grid, st)))
+#define BONSAI_QA_12(k, g) (alone || close ? qa_launch<k, g, 12, true>(p, grid, st) : qa_launch<k, g, 12>(p, grid, st))
+#define BONSAI_QA_W(k, g) (warps == 2 ? qa_launch<k, g, 2>(p, grid, st) : (warps == 6 ? qa_launch<k, g, 6>(p, grid, st) : BONSAI_QA_12(k, g)))
 #define BONSAI_QA(g) (kvt == 2 ? BONSAI_QA_W(2, g) : BONSAI_QA_W(3, g))
     switch (G) {
       case 1: rc = BONSAI_QA(1); break;
@@ -619,6 +629,7 @@ int attn_decode_quant(const float* q, const int* positions, const int* block_tab
     }
 #undef BONSAI_QA
 #undef BONSAI_QA_W
+#undef BONSAI_QA_12
     if (rc != BONSAI_CUDA_OK) return rc;
   }
   return BONSAI_CUDA_OK;

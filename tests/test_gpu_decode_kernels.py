@@ -603,7 +603,7 @@ def test_decode_attention_over_no_tokens_is_zero(kvt, nsplit):
 
 
 @pytest.mark.parametrize("lens,nq,nkv,nsplit,least", [([8000], 32, 8, 1, -1), ([8000], 32, 8, 2, 14), ([8000], 32, 8, 4, 28), ([8000], 32, 8, 16, 112), ([300, 2000, 1, 5000], 32, 8, 1, -1),
-                                                      ([300, 2000, 0, 5000], 8, 4, 3, 34), ([40, 900] * 60, 8, 2, 1, -1), ([3000, 80, 700] * 150, 2, 2, 1, 1)])
+                                                      ([300, 2000, 0, 5000], 8, 4, 3, 34), ([900, 200] * 8, 8, 8, 1, -1), ([900, 200] * 8, 8, 8, 2, 140), ([40, 900] * 60, 8, 2, 1, 100), ([3000, 80, 700] * 150, 2, 2, 1, 100)])
 @pytest.mark.parametrize("kvt", [2, 3])
 def test_quantised_decode_attention_uses_the_documented_workspace(lens, nq, nkv, nsplit, least, kvt):
     """batch * nq * nsplit rows give room for nearly a CTA per split, or for a pair each: partial sums side by side, at least so many (-1: none), and
