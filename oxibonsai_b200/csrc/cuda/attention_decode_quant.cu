@@ -16,7 +16,8 @@
 // Work: the tiles of all (sequence, kv head) pairs stand in one line, which is cut into equal pieces, one per CTA, whatever the
 // lengths are.  A pair that lies in one piece is finished there; of any other each CTA leaves a partial sum (a CTA has two at most, of
 // its first and of its last pair), and the last one to do so merges them.  The lengths are read on the device, so that a
-// captured launch serves every step.  Rows come through a ring of three tiles per warp in shared memory (cp.async), two ahead and across the
+// captured launch serves every step.  The cuts follow from the lengths of all sequences of the launch: the last bits of a sequence's result depend on
+// its neighbours' lengths, as they do on their number (the CUDA-core kernel's splits: on the number alone).  Rows come through a ring of three tiles per warp in shared memory (cp.async), two ahead and across the
 // pairs, which leaves registers for three warps per scheduler.
 // What bounds it: not the rows (a warp waits 20 cycles for its next tile) but its instructions, some 400 per tile of 16 tokens in 2100 cycles with
 // three warps in turn; turning to another pair 3000 to 4000 cycles, and merging parts 5 to 7 us at the end, a chain of launch-cold code and L2 trips.
@@ -148,9 +149,10 @@ __global__ void __launch_bounds__(NW * 32, kQaSmWarps / NW) attn_decode_quant_ke
   }
   __syncthreads();
   const int total = (ends[p.batch - 1] + kAhead * p.batch) * p.nkv;
-  // Places of the line that a CTA takes: at least a pair's start and a tile, and so many that no pair has more parts than the merge holds.  Where no
-  // pair has more than four tiles for each warp of a CTA and every pair has its CTA, each gets a whole one: merging parts takes as long as four tiles
-  // (one sequence of 300 tokens 11.3 us cut, 6.6 whole).
+  // Places of the line that a CTA takes: at least a pair's start and a tile, and so many that no pair has more than 65 parts for each warp of the CTA
+  // that adds them up, one after the other (one kv head, 149 sequences of 60 tokens and one of 9000, in CTAs of two warps: 33.4 us over INT8 rows
+  // in 94 parts, 40.8 in 141).  Where no pair has more than four tiles for each warp of a CTA and every pair has its CTA, each gets a whole one:
+  // merging parts takes as long as four tiles (one sequence of 300 tokens 11.3 us cut, 6.6 whole).
   constexpr int kParts = 65 * NW;
   const bool whole = (TIGHT && (p.mode & kQaAlone)) || (s_first <= 4 * NW && p.batch * p.nkv <= p.ctas);
   const int per = whole ? 1 << 30 : (max((total + p.ctas - 1) / p.ctas, max(kAhead + 1, (s_first + kParts - 3) / (kParts - 2))) + NW - 1) / NW * NW;
@@ -576,7 +578,10 @@ bool attn_decode_quant_takes(const float* q, int nq, int nkv, int page_size, con
 }
 
 // The more warps in a CTA, the more sums meet in shared memory and the fewer parts of a long context are left to merge; the fewer, the less they wait
-// for one another at the end of a run.  A CTA has an SM up to four sequences of eight heads, a sixth of one from a pair per SM on.
+// for one another at the end of a run.  A CTA has an SM up to four sequences of eight heads, a sixth of one from a pair per SM on.  us over INT8 rows with
+// twelve / six / two warps, 32 / 8 heads: one sequence of 300 tokens 6.5 / 8.4 / 8.9, four of up to 530 8.3 / 10.9 / 12.0 (whole pairs), four of 4000
+// 19.5 / 18.1 / 26.4, five of 100 to 1377 13.1 / 12.2 / 15.6, one of 20001 22.0 / 22.1 / 44.0; 18 of 100 to 1496 17.9 / 16.6 / 19.2, 24 22.2 / 19.8 / 21.6, 32
+// 26.8 / 25.1 / 25.3, 64 44.5 / 37.9 / 37.6: between 19 and 32 sequences six warps would be up to a tenth faster, from there on it is even.
 static int qa_warps(int pairs) { return pairs >= 148 ? 2 : (pairs > 36 ? 6 : 12); }
 // Splits (grid rows per pair) that give every SM its CTAs: whole ones, a further one where these would leave more than a quarter of the places empty.
 int attn_decode_quant_splits(int pairs) {

@@ -303,8 +303,8 @@ __global__ void __launch_bounds__(kGbThreads, 1) bitgemm_batch_kernel(const __gr
   if (S > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
   if (warp < kGbMmaWarp) {
     // A tile's end is a chain (drain, exchange, sum, store): few, wide accesses and short loops.  Warps 12-15 take it beside the expansion of the next
-    // tile; the last tile has the expanders' warps too, every group a quarter of the tokens.  us of 64 / 24 / 5 tokens with four warps, a store per
-    // value and loops unrolled over tokens (the start's form): 6144 x 4096 16.2 / 12.3 / 10.0, 24576 x 4096 40.2 / 26.6 / 19.5.
+    // tile; the last tile has the expanders' warps too, every group a quarter of the tokens.  us of 64 / 24 / 5 tokens with four warps for every tile, a
+    // 4-byte store per value and loops unrolled over tokens: 6144 x 4096 16.2 / 12.3 / 10.0, 24576 x 4096 40.2 / 26.6 / 19.5.
     asm volatile("griddepcontrol.wait;" ::: "memory");
     constexpr int CB = 16;
     const int a = t & 127, part = warp >= kGbEpiWarp ? 0 : 1 + (warp >> 2);
@@ -488,7 +488,8 @@ int bonsai_bitgemm_batch(const void* codes, const void* scales, const void* x_f1
     // exchange, six blocks' time), and for the cluster's size what waiting for one more CTA costs: 1.5 blocks' time, 2.8 with the 33 to 64 tokens' sums to
     // exchange, where more than four CTAs never paid.  us by split 1 / 2 / 3 / 4 / 6 behind the norm at 8 tokens: 6144 x 4096 13.0 / 9.7 / 13.1 / 9.4 / 10.2;
     // 24576 x 4096 22.0 / 18.6 / 20.3 / 20.6 / 26.4; 4096 x 12288 28.6 / 17.9 / 16.2 / 12.7 / 16.0; 2560 x 4096 13.0 / 9.2 / 8.0 / 6.9 / 7.0; 2560 x 9728 23.7 / 15.1 / 12.5 /
-    // 10.9 / 10.1; at 64 tokens 2560 x 4096 14.3 / 10.3 / 9.4 / 8.5 / 10.3, 2560 x 9728 25.6 / 16.4 / 14.9 / 11.8 / 14.2.
+    // 10.9 / 10.1; at 64 tokens 2560 x 4096 14.3 / 10.3 / 9.4 / 8.5 / 10.3, 2560 x 9728 25.6 / 16.4 / 14.9 / 11.8 / 14.2.  A tensor-core sum is cut off where
+    // f32 would round it, so that more CTAs have less error (4096 x 12288, normal inputs: 5.9 / 2.8 / 1.8 / 1.4 / 0.9e-6 of the result by split 1 / 2 / 3 / 4 / 6).
     long long best = -1;
     for (int s = 1; s <= (T > 32 && most > 4 ? 4 : most); ++s) {
       if (held[s] < 1) continue;

@@ -13,7 +13,7 @@ are the batch kernels of the native engine.  The engine has the slot interface t
 matrix is decoded once per chunk into an f16 scratch matrix (csrc/cuda/quant_gemv.cu, bonsai_quant_to_f16) and multiplied
 by all the chunk's tokens with the dense tcgen05 GEMM, with the prompt-attention kernel of the native engine in between (a chunk of more than 64
 tokens is one native call, csrc/cuda/blocks_prompt.cu);
-shorter prompts go through the decode step token by token (all f32).  Attention, KV append, LM head and sampler are the
+shorter prompts go through the decode step token by token (inputs and sums in f32, or in integers that hold every bit of them).  Attention, KV append, LM head and sampler are the
 kernels of the native engine.  The sub-2-bit formats (Q1_0_g128, TQ2_0_g128) should use
 ``oxibonsai_b200.runtime.InferenceEngine``, which is several times faster.
 """
